@@ -60,7 +60,8 @@ constexpr int kMaxSlots = 2 * kMaxProbes + kMaxPorts;
 constexpr int kPostThreads = 1024;   // k_post: one block
 constexpr int kMaxGridY = 65535;     // launches over node planes are split into chunks of this many
 constexpr int kPostStage = 4096;     // probe edge products staged in shared memory
-constexpr unsigned kFlagDisp = 1, kFlagSrc = 2, kFlagMode = 4;   // table entry flags: Debye, lumped source, mode source
+// table entry flags: Debye, lumped source, mode source, surface-impedance edge
+constexpr unsigned kFlagDisp = 1, kFlagSrc = 2, kFlagMode = 4, kFlagSibc = 8;
 
 // ---------------------------------------------------------------- arguments
 
@@ -194,6 +195,23 @@ struct PostArgs {
     long long *dstep;
     float *srcv;             // source values of the step the E update runs next
     int advance;             // 1: count this step
+};
+
+// A run of whole steps. Probe and port edges are sampled by blocks of the
+// update launches themselves, where nothing writes the family they read: E of
+// a step in the H launch of the next one, H in the E launch. The samples (one
+// row per step) become rows of the sample ring after the run (k_rows).
+struct RunArgs {
+    const uint4 *samples;    // entries of E, then of H: component (0..5), index, place in the row
+    int nsample[2];
+    int nent;                // samples of a row
+    float *raw;
+    const float2 *src;       // per step of the run: lumped and modal source values
+    float2 *srcv;            // the current step's, which the E update reads
+    int *at;                 // [0] step of the run in progress, [1] the next one
+    int on;                  // whether the launch belongs to a run
+    int first;               // blocks of the launch before the update's own: sampling, surface impedance
+    unsigned skip;           // table flags whose points the E update leaves to those blocks
 };
 
 // --------------------------------------------------------------- helpers
@@ -678,6 +696,157 @@ __device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r)
     h_points<C>(a, i, j, k4, H + q, w, e2, e2n, e1, e1n, h);
 }
 
+__device__ __forceinline__ float4 all4(float v) { return make_float4(v, v, v, v); }
+
+__device__ __forceinline__ float4 sub4(const float4 &a, const float4 &b) {
+    return make_float4(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z), __fsub_rn(a.w, b.w));
+}
+__device__ __forceinline__ float4 add4(const float4 &a, const float4 &b) {
+    return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+}
+__device__ __forceinline__ float4 mul4(const float4 &a, const float4 &b) {
+    return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
+}
+__device__ __forceinline__ float4 fma4(const float4 &a, const float4 &b, const float4 &c) {
+    return make_float4(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y), __fmaf_rn(a.z, b.z, c.z),
+                       __fmaf_rn(a.w, b.w, c.w));
+}
+
+// the points of `in` from v, the others as they are
+__device__ __forceinline__ void pick4(float4 &to, const float4 &v, unsigned in) {
+    if (in & 1u) to.x = v.x;
+    if (in & 2u) to.y = v.y;
+    if (in & 4u) to.z = v.z;
+    if (in & 8u) to.w = v.w;
+}
+
+// One difference term of an update, d * c, and where auxiliaries lie (in: the
+// points that have one, psi their values) the CPML recursion psi_next and the
+// auxiliary's share: + dth * psi' for H, + psi' for E.
+template <bool E>
+__device__ __forceinline__ float4 term(const float4 &d, const float4 &c, float dth, float4 &psi, const float4 &b,
+                                       const float4 &cd, unsigned in) {
+    float4 t = mul4(d, c);
+    if (!in) return t;
+    const float4 n = fma4(b, psi, fma4(cd, d, psi));
+    const float4 u = E ? add4(t, n) : fma4(all4(dth), n, t);
+    if (in == 15u) {
+        psi = n;
+        return u;
+    }
+    pick4(psi, n, in);
+    pick4(t, u, in);
+    return t;
+}
+
+// E component C of four points from the curl: t per point (ca-1, cb, cs,
+// flags), J the pole currents (Debye, jo4 >= 0), sv the source values. own:
+// the points the component has; skip: table flags whose points are left alone.
+// Stores E and the currents. Each rounding is
+// that of e_finish and debye_next.
+template <int C, int P>
+__device__ __forceinline__ void e_four(const StepArgs &a, int j, int k4, int q, const float4 &ev, const float4 &curl,
+                                       const uint2 mv, unsigned own, int jo4, float4 (&J)[P > 0 ? P : 1],
+                                       const float2 sv, unsigned skip) {
+    constexpr int NB = (P + 3) / 4;
+    const int m0 = (int)(mv.x & 0xffffu), m1 = (int)(mv.x >> 16), m2 = (int)(mv.y & 0xffffu), m3 = (int)(mv.y >> 16);
+    const float4 t0 = __ldg(a.tab4[C] + m0);
+    float4 t1 = t0, t2 = t0, t3 = t0;
+    const bool same = m0 == m1 && mv.x == mv.y;
+    if (!same) {
+        t1 = __ldg(a.tab4[C] + m1);
+        t2 = __ldg(a.tab4[C] + m2);
+        t3 = __ldg(a.tab4[C] + m3);
+    }
+    const unsigned f0 = __float_as_uint(t0.w), f1 = __float_as_uint(t1.w), f2 = __float_as_uint(t2.w),
+                   f3 = __float_as_uint(t3.w);
+    const unsigned any = f0 | f1 | f2 | f3;
+    const float4 ca = make_float4(t0.x, t1.x, t2.x, t3.x), cb = make_float4(t0.y, t1.y, t2.y, t3.y);
+    float4 js = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (P > 0) {
+#pragma unroll
+        for (int p = 0; p < P; p++) js = fma4(all4(a.hk[p]), J[p], js);
+    }
+    float4 v;
+    if (!any) {
+        v = fma4(cb, curl, fma4(ca, ev, ev));
+    } else {
+        const float4 base = fma4(ca, ev, ev);
+        float4 c = curl;
+        if (f0 & kFlagDisp) c.x = __fsub_rn(c.x, js.x);
+        if (f1 & kFlagDisp) c.y = __fsub_rn(c.y, js.y);
+        if (f2 & kFlagDisp) c.z = __fsub_rn(c.z, js.z);
+        if (f3 & kFlagDisp) c.w = __fsub_rn(c.w, js.w);
+        v = fma4(cb, c, base);
+        if (any & (kFlagSrc | kFlagMode | skip)) {
+            const float cs[4] = {t0.z, t1.z, t2.z, t3.z};
+            const unsigned fl[4] = {f0, f1, f2, f3};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                float x = lane4(v, e);
+                if (fl[e] & kFlagSrc) x = __fmaf_rn(cs[e], sv.x, x);
+                if (C > 0 && (fl[e] & kFlagMode)) {
+                    const float w = __ldg(a.wsrc[C - 1] + j * (a.g.n[2] + 1) + k4 + e);
+                    if (w != 0.f) x = __fmaf_rn(w, sv.y, x);
+                }
+                set4(v, e, x);
+                if (fl[e] & skip) own &= ~(1u << e);
+            }
+        }
+    }
+    float *E = a.E[C] + q;
+    const float4 de = sub4(v, ev);
+    if (own == 15u) {
+        st4(E, v);
+    } else if (any & skip) {   // another block writes the points left out
+        if (own & 1u) E[0] = v.x;
+        if (own & 2u) E[1] = v.y;
+        if (own & 4u) E[2] = v.z;
+        if (own & 8u) E[3] = v.w;
+    } else {
+        float4 r = ev;
+        if (own & 1u) r.x = v.x;
+        if (own & 2u) r.y = v.y;
+        if (own & 4u) r.z = v.z;
+        if (own & 8u) r.w = v.w;
+        st4(E, r);
+    }
+    if (P == 0 || jo4 < 0) return;
+    const unsigned disp = own & ((f0 & kFlagDisp ? 1u : 0u) | (f1 & kFlagDisp ? 2u : 0u) | (f2 & kFlagDisp ? 4u : 0u) |
+                                 (f3 & kFlagDisp ? 8u : 0u));
+    if (!disp) return;
+    float *Jc = a.J[C];
+    const int jvol = jbox_volume<C>(a);
+    const int mi[4] = {m0, m1, m2, m3};
+    if (same && disp == 15u) {
+#pragma unroll
+        for (int h = 0; h < NB; h++) {
+            const float4 b = __ldg(a.beta4[C] + m0 * NB + h);
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (4 * h + e < P) {
+                    float4 &x = J[4 * h + e];
+                    x = fma4(all4(lane4(b, e)), de, fma4(all4(-a.omk[4 * h + e]), x, x));
+                }
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            if (!(disp >> e & 1u)) continue;
+#pragma unroll
+            for (int h = 0; h < NB; h++) {
+                const float4 b = __ldg(a.beta4[C] + mi[e] * NB + h);
+#pragma unroll
+                for (int x = 0; x < 4; x++)
+                    if (4 * h + x < P)
+                        set4(J[4 * h + x], e, debye_next(a, 4 * h + x, lane4(b, x), lane4(de, e), lane4(J[4 * h + x], e)));
+            }
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < P; p++) st4(Jc + jaddr(P, jvol, p, jo4), J[p]);
+}
+
 // e_where: as h_where for E; CPML planes of nodes, and the Debye box
 template <int C, int P>
 __device__ __forceinline__ Where e_where(const StepArgs &a, int i, int j, int k4) {
@@ -699,107 +868,53 @@ __device__ __forceinline__ Where e_where(const StepArgs &a, int i, int j, int k4
 // E component C at points k4 .. k4+3 of row (i, j) from the H values there
 // (h2 = H_{C+2}, h1 = H_{C+1}) and one step back along the derivative axes
 // (h2m along C+1, h1m along C+2), the old E ev and the material indices mv,
-// w from e_where; the new E goes to eq. Points with no CPML on a derivative
-// axis and outside the Debye box take a short path (sources included); the
-// others update CPML auxiliaries and Debye currents, the currents of all
-// four points read in one pass (sum_p hk_p J_p) and re-read from L1 for
-// their update.
+// w from e_where; the new E goes to E[C] + q. Points with no CPML on a derivative
+// axis take no auxiliaries, those outside the Debye box no currents.
 template <int C, int P>
-__device__ __forceinline__ void e_points(const StepArgs &a, int i, int j, int k4, float *eq, const Where &w,
+__device__ __forceinline__ void e_points(const StepArgs &a, int i, int j, int k4, int q, const Where &w,
                                          const float4 &h2, const float4 &h2m, const float4 &h1, const float4 &h1m,
-                                         float4 ev, const uint2 mv, const float2 sv) {
+                                         const float4 &ev, const uint2 mv, const float2 sv, unsigned skip) {
     constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
     const int nz = a.g.n[2];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float ci = a.ec[0][i], cj = a.ec[1][j];
+    const float ci = __ldg(a.ec[0] + i), cj = __ldg(a.ec[1] + j);
     const float4 ck = ldg4(a.ec[2] + k4);
-    const int pi = w.pi, pj = w.pj;
-    const int4 pk = w.pk;
-    const int pa[3] = {pi, pj, max(max(pk.x, pk.y), max(pk.z, pk.w))};
-    const int jo4 = w.jo4;
-    const bool box = jo4 >= 0;
-    const int mi[4] = {(int)(mv.x & 0xffffu), (int)(mv.x >> 16), (int)(mv.y & 0xffffu), (int)(mv.y >> 16)};
-    float4 t[4];
-    unsigned flags = 0;
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        t[e] = __ldg(a.tab4[C] + mi[e]);   // index 0 (PEC, padding) for points E does not own
-        flags |= __float_as_uint(t[e].w);
+    const float4 c1 = A1 == 0 ? all4(ci) : (A1 == 1 ? all4(cj) : ck), c2 = A2 == 0 ? all4(ci) : (A2 == 1 ? all4(cj) : ck);
+    unsigned own = k4 + 4 > nz ? (1u << max(nz - k4, 0)) - 1u : 15u;
+    if (C != 2 && k4 == 0) own &= ~1u;
+    const unsigned inz = (w.pk.x >= 0 ? 1u : 0u) | (w.pk.y >= 0 ? 2u : 0u) | (w.pk.z >= 0 ? 4u : 0u) | (w.pk.w >= 0 ? 8u : 0u);
+    const int pa[3] = {w.pi, w.pj, inz ? 0 : -1};
+    const unsigned in1 = (A1 == 2 ? inz : (pa[A1] >= 0 ? 15u : 0u)) & own, in2 = (A2 == 2 ? inz : (pa[A2] >= 0 ? 15u : 0u)) & own;
+    // auxiliaries and currents: all loads before the arithmetic
+    float4 s1 = z4, s2 = z4, b1 = z4, b2 = z4, d1 = z4, d2 = z4;
+    int x1 = 0, x2 = 0;
+    if (in1) {
+        x1 = psi_at<A1, true>(a, pa[A1], i, j, k4);
+        s1 = ld4(a.psiE[C][0] + x1);
+        b1 = A1 == 2 ? ldg4(a.pml[2].bm1_e + k4) : all4(__ldg(a.pml[A1].bm1_e + (A1 == 0 ? i : j)));
+        d1 = A1 == 2 ? ldg4(a.pml[2].cid_e + k4) : all4(__ldg(a.pml[A1].cid_e + (A1 == 0 ? i : j)));
     }
-    // sources (lumped and modal) need no general path: their flags are
-    // handled by e_finish; dispersive edges lie inside the Debye box
-    if (!w.gen) {
-        float s = 0.f;
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int k = k4 + e;
-            if (!(C == 2 ? k < nz : (k >= 1 && k < nz))) continue;
-            const float c[3] = {ci, cj, lane4(ck, e)};
-            set4(ev, e, e_value<C>(a, t[e], i, j, k, sv, lane4(ev, e), __fsub_rn(lane4(h2, e), lane4(h2m, e)),
-                                   __fsub_rn(lane4(h1, e), lane4(h1m, e)), c[A1], c[A2], false, false, s, s, 0.f));
-        }
-        st4(eq, ev);
-        return;
+    if (in2) {
+        x2 = psi_at<A2, true>(a, pa[A2], i, j, k4);
+        s2 = ld4(a.psiE[C][1] + x2);
+        b2 = A2 == 2 ? ldg4(a.pml[2].bm1_e + k4) : all4(__ldg(a.pml[A2].bm1_e + (A2 == 0 ? i : j)));
+        d2 = A2 == 2 ? ldg4(a.pml[2].cid_e + k4) : all4(__ldg(a.pml[A2].cid_e + (A2 == 0 ? i : j)));
     }
-    const bool any1 = pa[A1] >= 0, any2 = pa[A2] >= 0;
-    const int x1 = any1 ? psi_at<A1, true>(a, pa[A1], i, j, k4) : 0;
-    const int x2 = any2 ? psi_at<A2, true>(a, pa[A2], i, j, k4) : 0;
-    float4 s1 = any1 ? ld4(a.psiE[C][0] + x1) : z4;
-    float4 s2 = any2 ? ld4(a.psiE[C][1] + x2) : z4;
-    float jsum[4] = {0.f, 0.f, 0.f, 0.f};
+    float4 J[P > 0 ? P : 1];
     const int jvol = P > 0 ? jbox_volume<C>(a) : 0;
-    // sum_p hk_p J_p of the four points (currents of points that are not
-    // dispersive are never written and stay zero; their sum is unused)
-    if (P > 0 && box) {
 #pragma unroll
-        for (int p = 0; p < (P > 0 ? P : 1); p++) {
-            const float4 jp = ld4(a.J[C] + jaddr(P, jvol, p, jo4));
-#pragma unroll
-            for (int e = 0; e < 4; e++) jsum[e] = debye_term(a, p, lane4(jp, e), jsum[e]);
-        }
-    }
-    float4 eo = ev;
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const int k = k4 + e;
-        if (!(C == 2 ? k < nz : (k >= 1 && k < nz))) continue;
-        const bool in1 = A1 == 2 ? lane4i(pk, e) >= 0 : any1;
-        const bool in2 = A2 == 2 ? lane4i(pk, e) >= 0 : any2;
-        float q1 = lane4(s1, e), q2 = lane4(s2, e);
-        const float c[3] = {ci, cj, lane4(ck, e)};
-        set4(ev, e, e_value<C>(a, t[e], i, j, k, sv, lane4(ev, e), __fsub_rn(lane4(h2, e), lane4(h2m, e)),
-                               __fsub_rn(lane4(h1, e), lane4(h1m, e)), c[A1], c[A2], in1, in2, q1, q2, jsum[e]));
-        set4(s1, e, q1);
-        set4(s2, e, q2);
-    }
-    st4(eq, ev);
-    if (any1) st4(a.psiE[C][0] + x1, s1);
-    if (any2) st4(a.psiE[C][1] + x2, s2);
-    if (P > 0 && box && (flags & kFlagDisp)) {
-        bool disp[4];
-        float de[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int k = k4 + e;
-            disp[e] = (C == 2 ? k < nz : (k >= 1 && k < nz)) && (__float_as_uint(t[e].w) & kFlagDisp);
-            de[e] = __fsub_rn(lane4(ev, e), lane4(eo, e));
-        }
-#pragma unroll
-        for (int p = 0; p < (P > 0 ? P : 1); p++) {
-            float *jp = a.J[C] + jaddr(P, jvol, p, jo4);
-            float4 jv = ld4(jp);
-#pragma unroll
-            for (int e = 0; e < 4; e++)
-                if (disp[e]) set4(jv, e, debye_next(a, p, beta_at<C>(a, mi[e], p), de[e], lane4(jv, e)));
-            st4(jp, jv);
-        }
-    }
+    for (int p = 0; p < P; p++) J[p] = w.jo4 >= 0 ? ld4(a.J[C] + jaddr(P, jvol, p, w.jo4)) : z4;
+    const float4 t1 = term<true>(sub4(h2, h2m), c1, 0.f, s1, b1, d1, in1);
+    const float4 t2 = term<true>(sub4(h1, h1m), c2, 0.f, s2, b2, d2, in2);
+    if (in1) st4(a.psiE[C][0] + x1, s1);
+    if (in2) st4(a.psiE[C][1] + x2, s2);
+    e_four<C, P>(a, j, k4, q, ev, sub4(t1, t2), mv, own, w.jo4, J, sv, skip);
 }
 
 // E component C on points k4 .. k4+3 of row (i, j) (segment [ks, ke));
 // FAST as for h_vec: no CPML auxiliary and no Debye current in the block.
 template <int C, int P, bool FAST>
-__device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r, const float2 sv) {
+__device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r, const float2 sv, unsigned skip) {
     const int j = r.j, k4 = r.k4;
     const int m = j * a.g.sj + k4;
     constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
@@ -829,7 +944,7 @@ __device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r,
     if (A1 == 2) h2m = prev_k(h2, H2 + q, row && k4 > 0, edge);
     if (A2 == 2) h1m = prev_k(h1, H1 + q, row && k4 > 0, edge);
     if (!row) return;
-    e_points<C, P>(a, i, j, k4, E + q, w, h2, h2m, h1, h1m, ev, mv, sv);
+    e_points<C, P>(a, i, j, k4, q, w, h2, h2m, h1, h1m, ev, mv, sv, skip);
 }
 
 // whether the group at k4 of a lean kernel's row lies in a z tail (StepArgs::zt)
@@ -895,7 +1010,7 @@ __device__ __forceinline__ void h_lean(const StepArgs &a, int i, const RowPos &p
 // short path of e_points (material table, sources; no auxiliaries, no Debye
 // currents), every rounding the same; groups of a z tail take e_points itself
 template <int C>
-__device__ __forceinline__ void e_lean(const StepArgs &a, int i, const RowPos &p, const float2 sv) {
+__device__ __forceinline__ void e_lean(const StepArgs &a, int i, const RowPos &p, const float2 sv, unsigned skip) {
     constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
     constexpr bool kz = A1 == 2 || A2 == 2;
     const int ny = a.g.n[1], nz = a.g.n[2];
@@ -922,24 +1037,16 @@ __device__ __forceinline__ void e_lean(const StepArgs &a, int i, const RowPos &p
     if (A2 == 2) h1m = prev_k(h1, H1 + q, row && k4 > 0, first);
     if (!row) return;
     if (kz && in_ztail(a.zt[1], k4)) {
-        e_points<C, 0>(a, i, j, k4, E + q, ztail_where(a.pml[2].plane_e, k4), h2, h2m, h1, h1m, ev, mv, sv);
+        e_points<C, 0>(a, i, j, k4, q, ztail_where(a.pml[2].plane_e, k4), h2, h2m, h1, h1m, ev, mv, sv, skip);
         return;
     }
     const float ci = __ldg(a.ec[0] + i), cj = __ldg(a.ec[1] + j);
     const float4 ck = ldg4(a.ec[2] + k4);
-    const int mi[4] = {(int)(mv.x & 0xffffu), (int)(mv.x >> 16), (int)(mv.y & 0xffffu), (int)(mv.y >> 16)};
-    float s = 0.f;
-    float4 r = ev;
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const int k = k4 + e;
-        const float4 t = __ldg(a.tab4[C] + mi[e]);
-        const float c[3] = {ci, cj, lane4(ck, e)};
-        const float v = e_value<C>(a, t, i, j, k, sv, lane4(ev, e), __fsub_rn(lane4(h2, e), lane4(h2m, e)),
-                                   __fsub_rn(lane4(h1, e), lane4(h1m, e)), c[A1], c[A2], false, false, s, s, 0.f);
-        if (C == 2 ? k < nz : (k >= 1 && k < nz)) set4(r, e, v);
-    }
-    st4(E + q, r);
+    const float4 c1 = A1 == 0 ? all4(ci) : (A1 == 1 ? all4(cj) : ck), c2 = A2 == 0 ? all4(ci) : (A2 == 1 ? all4(cj) : ck);
+    unsigned own = k4 + 4 > nz ? (1u << max(nz - k4, 0)) - 1u : 15u;
+    if (kz && k4 == 0) own &= ~1u;
+    float4 J[1];
+    e_four<C, 0>(a, j, k4, q, ev, sub4(mul4(sub4(h2, h2m), c1), mul4(sub4(h1, h1m), c2)), mv, own, -1, J, sv, skip);
 }
 
 // E component C at points k4 .. k4+3 of row (i, j) of a Debye piece: no
@@ -949,9 +1056,9 @@ __device__ __forceinline__ void e_lean(const StepArgs &a, int i, const RowPos &p
 // registers for both sum_p hk_p J_p and their own update, then written once;
 // beta_p/dt comes packed per table entry. Every rounding is that of e_points.
 template <int C, int P>
-__device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &p, const float2 sv) {
+__device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &p, const float2 sv, unsigned skip) {
     constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
-    constexpr int NB = (P + 3) / 4;
+    constexpr bool kz = A1 == 2 || A2 == 2;
     const int ny = a.g.n[1], nz = a.g.n[2];
     const int j = p.j, k4 = p.k4;
     const bool row = p.act && (C == 0 || i >= 1) && (C == 1 ? j < ny : (j >= 1 && j < ny));
@@ -984,49 +1091,75 @@ __device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &
     if (!row) return;
     // a z tail above the box (tails exist only where no box reaches a z slab)
     if ((A1 == 2 || A2 == 2) && in_ztail(a.zt[1], k4)) {
-        e_points<C, 0>(a, i, j, k4, E + q, ztail_where(a.pml[2].plane_e, k4), h2, h2m, h1, h1m, ev, mv, sv);
+        e_points<C, 0>(a, i, j, k4, q, ztail_where(a.pml[2].plane_e, k4), h2, h2m, h1, h1m, ev, mv, sv, skip);
         return;
     }
     const float ci = __ldg(a.ec[0] + i), cj = __ldg(a.ec[1] + j);
     const float4 ck = ldg4(a.ec[2] + k4);
-    const int mi[4] = {(int)(mv.x & 0xffffu), (int)(mv.x >> 16), (int)(mv.y & 0xffffu), (int)(mv.y >> 16)};
-    float s = 0.f;
-    float4 r = ev;
-    float de[4];
-    bool disp[4];
-    bool any = false;
+    const float4 c1 = A1 == 0 ? all4(ci) : (A1 == 1 ? all4(cj) : ck), c2 = A2 == 0 ? all4(ci) : (A2 == 1 ? all4(cj) : ck);
+    unsigned own = k4 + 4 > nz ? (1u << max(nz - k4, 0)) - 1u : 15u;
+    if (kz && k4 == 0) own &= ~1u;
+    e_four<C, P>(a, j, k4, q, ev, sub4(mul4(sub4(h2, h2m), c1), mul4(sub4(h1, h1m), c2)), mv, own, jo4, J, sv, skip);
+}
+
+// E = sum_k c_k (J - y_k) with y_k += (1 - e_k)(J - y_k), J from the faces' H.
+// (reference sibc.c:256-269)
+__device__ __forceinline__ void sibc_edge(const SibcArgs &a, int e) {
+    // every load first: face tables (16-byte vectors), the convolution
+    // states, then the H values of the faces
+    const float4 w4 = __ldg(a.hw + e);
+    const uint4 i4 = __ldg(a.hidx + e);
+    const uchar4 c4 = __ldg(a.hcomp + e);
+    const unsigned char ec = __ldg(a.ecomp + e);
+    const unsigned ei = __ldg(a.eidx + e);
+    float y[kSibcTerms];
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const int k = k4 + e;
-        const float4 t = __ldg(a.tab4[C] + mi[e]);
-        float jsum = 0.f;
+    for (int k = 0; k < kSibcTerms; k++)
+        if (k < a.K) y[k] = a.y[(long long)k * a.ns + e];
+    const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+    const unsigned hi[4] = {i4.x, i4.y, i4.z, i4.w};
+    const int hc[4] = {c4.x, c4.y, c4.z, c4.w};
+    float h[4];
 #pragma unroll
-        for (int pp = 0; pp < P; pp++) jsum = debye_term(a, pp, lane4(J[pp], e), jsum);
-        const float c[3] = {ci, cj, lane4(ck, e)};
-        const float v = e_value<C>(a, t, i, j, k, sv, lane4(ev, e), __fsub_rn(lane4(h2, e), lane4(h2m, e)),
-                                   __fsub_rn(lane4(h1, e), lane4(h1m, e)), c[A1], c[A2], false, false, s, s, jsum);
-        const bool own = C == 2 ? k < nz : (k >= 1 && k < nz);
-        if (own) set4(r, e, v);
-        disp[e] = own && jo4 >= 0 && (__float_as_uint(t.w) & kFlagDisp);
-        de[e] = __fsub_rn(v, lane4(ev, e));
-        any = any || disp[e];
-    }
-    st4(E + q, r);
-    if (!any) return;
+    for (int f = 0; f < 4; f++) h[f] = w[f] != 0.f ? __ldg(a.H[hc[f]] + hi[f]) : 0.f;
+    // explicit roundings: the same bits in every kernel that inlines this
+    float J = 0.f;
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-        if (!disp[e]) continue;
-        float b[4 * (NB > 0 ? NB : 1)];
+    for (int f = 0; f < 4; f++)
+        if (w[f] != 0.f) J = __fmaf_rn(w[f], h[f], J);
+    float E = 0.f;
 #pragma unroll
-        for (int h = 0; h < NB; h++) {
-            const float4 v = __ldg(a.beta4[C] + mi[e] * NB + h);
-            b[4 * h] = v.x; b[4 * h + 1] = v.y; b[4 * h + 2] = v.z; b[4 * h + 3] = v.w;
+    for (int k = 0; k < kSibcTerms; k++) {
+        if (k < a.K) {
+            y[k] = __fmaf_rn(a.ome[k], __fsub_rn(J, y[k]), y[k]);
+            E = __fmaf_rn(a.c[k], __fsub_rn(J, y[k]), E);
         }
-#pragma unroll
-        for (int pp = 0; pp < P; pp++) set4(J[pp], e, debye_next(a, pp, b[pp], de[e], lane4(J[pp], e)));
     }
 #pragma unroll
-    for (int pp = 0; pp < P; pp++) st4(Jc + jaddr(P, jvol, pp, jo4), J[pp]);
+    for (int k = 0; k < kSibcTerms; k++)
+        if (k < a.K) a.y[(long long)k * a.ns + e] = y[k];
+    a.E[ec][ei] = E;
+}
+
+// samples of family u (0 E, 1 H) into the row of step t, by one block
+__device__ __forceinline__ void sample_family(const StepArgs &a, const RunArgs &r, int u, int t) {
+    const uint4 *s = r.samples + (u ? r.nsample[0] : 0);
+    for (int e = threadIdx.x; e < r.nsample[u]; e += blockDim.x) {
+        const uint4 v = __ldg(s + e);
+        r.raw[(size_t)t * r.nent + v.z] = __ldg((u ? a.H[v.x - 3] : a.E[v.x]) + v.y);
+    }
+}
+
+// H launch of a run: E of the step before, and the new step's source values
+__device__ __forceinline__ void begin_step(const StepArgs &a, const RunArgs &r) {
+    const int t = r.at[1];
+    if (t > 0) sample_family(a, r, 0, t - 1);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *r.srcv = r.src[t];
+        r.at[0] = t;
+        r.at[1] = t + 1;
+    }
 }
 
 // H over node planes [i0, i0 + gridDim.y) (cem_mt_H and the unfused step)
@@ -1052,7 +1185,11 @@ __device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &
 
 // H on the fast rectangles of node planes [i0, i0 + gridDim.y); block x:
 // block x / 3 of the space, component x % 3
-__global__ void __launch_bounds__(kBlock, CB2_HF_MINBLOCKS) k_update_h_fast(const StepArgs a, int i0) {
+__global__ void __launch_bounds__(kBlock, CB2_HF_MINBLOCKS) k_update_h_fast(const StepArgs a, int i0, const RunArgs r) {
+    if (r.first && blockIdx.x == gridDim.x - 1) {   // one column more: the run's own work
+        if (blockIdx.y == 0) begin_step(a, r);
+        return;
+    }
     const int comp = blockIdx.x % 3;
     const RowPos p = space_pos(a.sp[0][kFast], blockIdx.x / 3);
     const int i = i0 + blockIdx.y;
@@ -1062,14 +1199,18 @@ __global__ void __launch_bounds__(kBlock, CB2_HF_MINBLOCKS) k_update_h_fast(cons
 }
 
 // E on the fast rectangles of node planes [i0, i0 + gridDim.y)
-__global__ void __launch_bounds__(kBlock, CB2_EF_MINBLOCKS) k_update_e_fast(const StepArgs a, int i0) {
+__global__ void __launch_bounds__(kBlock, CB2_EF_MINBLOCKS) k_update_e_fast(const StepArgs a, int i0, const RunArgs r) {
+    if (r.first && blockIdx.x == gridDim.x - 1) {
+        if (blockIdx.y == 0) sample_family(a, r, 1, r.at[0]);
+        return;
+    }
     const int comp = blockIdx.x % 3;
     const RowPos p = space_pos(a.sp[1][kFast], blockIdx.x / 3);
     const int i = i0 + blockIdx.y;
     const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
-    if (comp == 0) e_lean<0>(a, i, p, sv);
-    else if (comp == 1) e_lean<1>(a, i, p, sv);
-    else e_lean<2>(a, i, p, sv);
+    if (comp == 0) e_lean<0>(a, i, p, sv, r.skip);
+    else if (comp == 1) e_lean<1>(a, i, p, sv, r.skip);
+    else e_lean<2>(a, i, p, sv, r.skip);
 }
 
 #ifndef CB2_ED_MINBLOCKS
@@ -1078,14 +1219,14 @@ __global__ void __launch_bounds__(kBlock, CB2_EF_MINBLOCKS) k_update_e_fast(cons
 
 // E on the Debye rectangles of node planes [i0, i0 + gridDim.y) (P poles)
 template <int P>
-__global__ void __launch_bounds__(kBlock, CB2_ED_MINBLOCKS) k_update_e_debye(const StepArgs a, int i0) {
+__global__ void __launch_bounds__(kBlock, CB2_ED_MINBLOCKS) k_update_e_debye(const StepArgs a, int i0, const RunArgs r) {
     const int comp = blockIdx.x % 3;
     const RowPos p = space_pos(a.sp[1][kDebye], blockIdx.x / 3);
     const int i = i0 + blockIdx.y;
     const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
-    if (comp == 0) e_debye<0, P>(a, i, p, sv);
-    else if (comp == 1) e_debye<1, P>(a, i, p, sv);
-    else e_debye<2, P>(a, i, p, sv);
+    if (comp == 0) e_debye<0, P>(a, i, p, sv, r.skip);
+    else if (comp == 1) e_debye<1, P>(a, i, p, sv, r.skip);
+    else e_debye<2, P>(a, i, p, sv, r.skip);
 }
 
 // Position in the general space of update U: the general rectangles on an
@@ -1097,25 +1238,35 @@ __device__ __forceinline__ RowPos general_pos(const StepArgs &a, int i, int b) {
 
 // Work entry of the general blocks: x node plane, y block of the plane's
 // general space (component y % 3, block y / 3).
-__global__ void __launch_bounds__(kBlock, CB2_H_MINBLOCKS) k_update_h(const StepArgs a, const int2 *work) {
-    const int2 w = work[blockIdx.x];
+__global__ void __launch_bounds__(kBlock, CB2_H_MINBLOCKS) k_update_h(const StepArgs a, const int2 *work, const RunArgs r) {
+    if ((int)blockIdx.x < r.first) {
+        begin_step(a, r);
+        return;
+    }
+    const int2 w = work[blockIdx.x - r.first];
     const int comp = w.y % 3;
-    const RowPos r = general_pos<0>(a, w.x, w.y / 3);
-    if (comp == 0) h_vec<0, false>(a, w.x, r);
-    else if (comp == 1) h_vec<1, false>(a, w.x, r);
-    else h_vec<2, false>(a, w.x, r);
+    const RowPos p = general_pos<0>(a, w.x, w.y / 3);
+    if (comp == 0) h_vec<0, false>(a, w.x, p);
+    else if (comp == 1) h_vec<1, false>(a, w.x, p);
+    else h_vec<2, false>(a, w.x, p);
 }
 
 // E over the general blocks (P Debye poles)
 template <int P>
-__global__ void __launch_bounds__(kBlock, CB2_E_MINBLOCKS) k_update_e(const StepArgs a, const int2 *work) {
-    const int2 w = work[blockIdx.x];
+__global__ void __launch_bounds__(kBlock, CB2_E_MINBLOCKS) k_update_e(const StepArgs a, const int2 *work, const RunArgs r, const SibcArgs s) {
+    if ((int)blockIdx.x < r.first) {   // H samples, then the surface-impedance edges (their E is left alone below)
+        const int e = ((int)blockIdx.x - 1) * kBlock + threadIdx.x;
+        if (blockIdx.x == 0) sample_family(a, r, 1, r.at[0]);
+        else if (e < s.ns) sibc_edge(s, e);
+        return;
+    }
+    const int2 w = work[blockIdx.x - r.first];
     const int comp = w.y % 3;
-    const RowPos r = general_pos<1>(a, w.x, w.y / 3);
+    const RowPos p = general_pos<1>(a, w.x, w.y / 3);
     const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
-    if (comp == 0) e_vec<0, P, false>(a, w.x, r, sv);
-    else if (comp == 1) e_vec<1, P, false>(a, w.x, r, sv);
-    else e_vec<2, P, false>(a, w.x, r, sv);
+    if (comp == 0) e_vec<0, P, false>(a, w.x, p, sv, r.skip);
+    else if (comp == 1) e_vec<1, P, false>(a, w.x, p, sv, r.skip);
+    else e_vec<2, P, false>(a, w.x, p, sv, r.skip);
 }
 
 constexpr unsigned kWaitLimit = 1u << 24;
@@ -1323,8 +1474,8 @@ __global__ void __launch_bounds__(kFT, 3) k_step_fused(const StepArgs a, const F
 }
 
 // launchers of the pole-count instantiations
-using EKernel = void (*)(StepArgs, const int2 *);
-using HKernel = void (*)(StepArgs, int);
+using EKernel = void (*)(StepArgs, const int2 *, RunArgs, SibcArgs);
+using HKernel = void (*)(StepArgs, int, RunArgs);
 using FKernel = void (*)(StepArgs, FusedArgs, TmaMaps);
 #define CB2_POLES(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
 #define CB2_EK(p) k_update_e<p>,
@@ -1339,45 +1490,6 @@ const HKernel kEDKernels[] = {CB2_POLES(CB2_DK)};
 #undef CB2_POLES
 
 // ------------------------------------------------------------------- SIBC
-
-// E = sum_k c_k (J - y_k) with y_k += (1 - e_k)(J - y_k), J from the faces' H.
-// (reference sibc.c:256-269)
-__device__ __forceinline__ void sibc_edge(const SibcArgs &a, int e) {
-    // every load first: face tables (16-byte vectors), the convolution
-    // states, then the H values of the faces
-    const float4 w4 = __ldg(a.hw + e);
-    const uint4 i4 = __ldg(a.hidx + e);
-    const uchar4 c4 = __ldg(a.hcomp + e);
-    const unsigned char ec = __ldg(a.ecomp + e);
-    const unsigned ei = __ldg(a.eidx + e);
-    float y[kSibcTerms];
-#pragma unroll
-    for (int k = 0; k < kSibcTerms; k++)
-        if (k < a.K) y[k] = a.y[(long long)k * a.ns + e];
-    const float w[4] = {w4.x, w4.y, w4.z, w4.w};
-    const unsigned hi[4] = {i4.x, i4.y, i4.z, i4.w};
-    const int hc[4] = {c4.x, c4.y, c4.z, c4.w};
-    float h[4];
-#pragma unroll
-    for (int f = 0; f < 4; f++) h[f] = w[f] != 0.f ? __ldg(a.H[hc[f]] + hi[f]) : 0.f;
-    // explicit roundings: the same bits in every kernel that inlines this
-    float J = 0.f;
-#pragma unroll
-    for (int f = 0; f < 4; f++)
-        if (w[f] != 0.f) J = __fmaf_rn(w[f], h[f], J);
-    float E = 0.f;
-#pragma unroll
-    for (int k = 0; k < kSibcTerms; k++) {
-        if (k < a.K) {
-            y[k] = __fmaf_rn(a.ome[k], __fsub_rn(J, y[k]), y[k]);
-            E = __fmaf_rn(a.c[k], __fsub_rn(J, y[k]), E);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < kSibcTerms; k++)
-        if (k < a.K) a.y[(long long)k * a.ns + e] = y[k];
-    a.E[ec][ei] = E;
-}
 
 __global__ void __launch_bounds__(kBlock) k_sibc(const SibcArgs a) {
     const int e = blockIdx.x * kBlock + threadIdx.x;
@@ -1456,6 +1568,74 @@ __device__ __forceinline__ void post_block(const PostArgs &a) {
 }
 
 __global__ void __launch_bounds__(kPostThreads) k_post(const PostArgs a) { post_block(a); }
+
+// the same as a launch of its own, where no update launch carries it
+__global__ void __launch_bounds__(kBlock) k_begin_step(const StepArgs a, const RunArgs r) { begin_step(a, r); }
+__global__ void __launch_bounds__(kBlock) k_sample_h(const StepArgs a, const RunArgs r) { sample_family(a, r, 1, r.at[0]); }
+
+// before a run: its step count to zero, the source values of its steps
+__global__ void k_run_begin(const RunArgs r, const PostArgs p, float *src, int steps, long long step0) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
+    if (t == 0) r.at[1] = 0;
+    for (int q = t; q < steps; q += n) source_values(p, step0 + q, src + 2 * q);
+}
+
+// after a run: the ring rows of its steps from the samples, block q step
+// step0 + q, the sums in post_block's order (E of the last step, which no
+// launch has sampled, from the field). Block 0 also carries the port voltages,
+// the step count and the source values on.
+constexpr int kRowThreads = 256;
+__global__ void __launch_bounds__(kRowThreads) k_rows(const RunArgs r, const PostArgs a, int steps, long long step0) {
+    __shared__ double now[kMaxSlots], old[kMaxPorts];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto sum = [&](int q, int s) {
+        const float *raw = r.raw + (size_t)q * r.nent;
+        double v = 0;
+        for (int e = a.off[s] + lane; e < a.off[s + 1]; e += 32) {
+            const float x = q == steps - 1 && a.ecomp[e] < 3 ? a.F[a.ecomp[e]][a.eidx[e]] : raw[e];
+            v = __dadd_rn(v, __dmul_rn((double)x, a.ew[e]));
+        }
+        return warp_sum(v);
+    };
+    const int q = blockIdx.x;
+    for (int s = warp; s < a.nin + a.nport; s += kRowThreads / 32) {
+        const int p = s - a.nin;   // the ports once more, a step earlier
+        if (p >= 0 && q == 0) {
+            if (lane == 0) old[p] = a.vold[p];
+            continue;
+        }
+        const double v = p < 0 ? sum(q, s) : sum(q - 1, a.nip + p);
+        if (lane == 0) (p < 0 ? now[s] : old[p]) = v;
+    }
+    __syncthreads();
+    const long long step = step0 + q;
+    double *row = a.ring + (long long)(step % kRing) * a.nslot;
+    const double tH = __dmul_rn(__dadd_rn((double)step, 0.5), a.dt);
+    const double vs = a.src_port >= 0 ? gauss(tH, a.src_amp, a.src_t0, a.src_tau) : 0.0;
+    for (int s = threadIdx.x; s < a.nip; s += kRowThreads) row[s] = now[s];
+    for (int p = threadIdx.x; p < a.nport; p += kRowThreads) {
+        const double V = __dmul_rn(0.5, __dadd_rn(now[a.nip + p], old[p]));
+        const double I = __ddiv_rn(__dsub_rn(p == a.src_port ? vs : 0.0, V), a.R[p]);
+        row[a.nip + 2 * p] = V;
+        row[a.nip + 2 * p + 1] = I;
+    }
+    if (threadIdx.x == 0) {
+        double src = a.src_port >= 0 ? vs : 0.0;
+        if (a.msrc_on) src = __dadd_rn(src, dgauss(tH, a.m_t0, a.m_tau));
+        row[a.nip + 2 * a.nport] = src;
+    }
+    for (int s = threadIdx.x; s < a.nvp; s += kRowThreads) row[a.nip + 2 * a.nport + 1 + s] = now[a.nip + a.nport + s];
+    if (q != 0) return;
+    __syncthreads();   // block 0 alone reads and writes vold
+    for (int p = warp; p < a.nport; p += kRowThreads / 32) {
+        const double v = sum(steps - 1, a.nip + p);
+        if (lane == 0) a.vold[p] = v;
+    }
+    if (threadIdx.x == 0) {
+        *a.dstep = step0 + steps;
+        source_values(a, step0 + steps, a.srcv);
+    }
+}
 
 // source values for the step count held on the device (after it was set from the host)
 __global__ void k_source_values(const PostArgs a) { source_values(a, *a.dstep, a.srcv); }
@@ -1583,13 +1763,13 @@ __global__ void __launch_bounds__(kBlock, FAST ? CB2_EF_MINBLOCKS : CB2_E_MINBLO
         const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
         const int comp = w.y % 3;
         if (FAST) {
-            if (comp == 0) e_lean<0>(a, w.z, r, sv);
-            else if (comp == 1) e_lean<1>(a, w.z, r, sv);
-            else e_lean<2>(a, w.z, r, sv);
+            if (comp == 0) e_lean<0>(a, w.z, r, sv, 0u);
+            else if (comp == 1) e_lean<1>(a, w.z, r, sv, 0u);
+            else e_lean<2>(a, w.z, r, sv, 0u);
         } else {
-            if (comp == 0) e_vec<0, P, false>(a, w.z, r, sv);
-            else if (comp == 1) e_vec<1, P, false>(a, w.z, r, sv);
-            else e_vec<2, P, false>(a, w.z, r, sv);
+            if (comp == 0) e_vec<0, P, false>(a, w.z, r, sv, 0u);
+            else if (comp == 1) e_vec<1, P, false>(a, w.z, r, sv, 0u);
+            else e_vec<2, P, false>(a, w.z, r, sv, 0u);
         }
     }
 }
@@ -1790,6 +1970,14 @@ struct Device {
     // with z tails, E rows are not cut at the Debye boxes: a row that meets a box is one
     // piece of the Debye space, air and tail included (CEM_B200_ROWS=0/1)
     bool whole_rows = false;
+    // runs of whole steps (RunArgs)
+    int run_steps = 0;                // most steps of a run (sample rows)
+    bool sibc_flagged = false;        // the tables mark the surface-impedance edges
+    RunArgs run{};
+    DevBuf<uint4> samples;
+    DevBuf<float> raw;
+    DevBuf<float2> run_src;
+    DevBuf<int> run_at;
     bool tune = false, tuned = false, tuned_from_cache = false;
     double tuned_ms = 0;
     cudaEvent_t tev[2] = {nullptr, nullptr};   // tuner timing
@@ -2105,6 +2293,36 @@ bool build_tables(cem_sim *s, Device &D) {
         unsigned short *m = out[c]->mat.data();
         for (size_t q = (size_t)x.i0 * D.g.si; q < (size_t)x.i1 * D.g.si; q++) m[q] = (unsigned short)rm[m[q]];
     });
+    // surface-impedance edges as entries of their own, so that the E update can leave them to the edges' own
+    // update in the same launch (not where the tables have no room: that update then follows in its own launch)
+    size_t nsib[3] = {0, 0, 0};
+    std::vector<std::vector<int>> marked(3);
+    D.sibc_flagged = s->nsb > 0;
+    for (int c = 0; c < 3; c++) {
+        if (out[c]->overflow) continue;
+        const size_t n0 = out[c]->tb.flags.size();
+        std::vector<char> seen(n0, 0);
+        for (int e = 0; e < s->nsb; e++)
+            if (s->sb_comp[e] == c) {
+                char &x = seen[out[c]->mat[dev_index(s, D, s->sb_idx[e])]];
+                nsib[c] += !x;
+                x = 1;
+            }
+        if (n0 + nsib[c] > 65536) D.sibc_flagged = false;
+        marked[c].assign(n0, -1);
+    }
+    for (int e = 0; D.sibc_flagged && e < s->nsb; e++) {
+        Built &b = *out[s->sb_comp[e]];
+        if (b.overflow) continue;
+        unsigned short &id = b.mat[dev_index(s, D, s->sb_idx[e])];
+        if (id >= marked[s->sb_comp[e]].size()) continue;   // listed twice
+        int &to = marked[s->sb_comp[e]][id];
+        if (to < 0) {
+            const std::vector<float> row(b.tb.rows.begin() + (size_t)id * nfields, b.tb.rows.begin() + (size_t)(id + 1) * nfields);
+            to = b.tb.add(row.data(), (unsigned char)(b.tb.flags[id] | kFlagSibc), b.tb.cb64[id]);
+        }
+        id = (unsigned short)to;
+    }
     for (int c = 0; c < 3; c++) {
         Built &b = *out[c];
         if (b.overflow) {
@@ -2276,10 +2494,27 @@ bool build_probes(cem_sim *s, Device &D) {
     if (!dev_upload(s, D.off, off) || !dev_upload(s, D.ecomp, comp) || !dev_upload(s, D.eidx, idx) ||
         !dev_upload(s, D.ew, w) || !dev_upload(s, D.R, R) || !dev_upload(s, D.omega, omega))
         return false;
+    // samples of a run: E entries, then H entries, each to its place in the row
+    std::vector<uint4> samp;
+    for (int u = 0; u < 2; u++) {
+        for (size_t e = 0; e < idx.size(); e++)
+            if ((comp[e] >= 3) == (u == 1)) samp.push_back(make_uint4(comp[e], idx[e], (unsigned)e, 0u));
+        D.run.nsample[u] = (int)samp.size() - (u ? D.run.nsample[0] : 0);
+    }
+    D.run.nent = (int)idx.size();
+    D.run_steps = (int)std::max(1ll, std::min((long long)kRing, (4ll << 20) / std::max(D.run.nent, 1)));
+    if (!dev_upload(s, D.samples, samp) || !dev_alloc(s, D.raw, (size_t)D.run_steps * D.run.nent) ||
+        !dev_alloc(s, D.run_src, kRing) || !dev_alloc(s, D.run_at, 2))
+        return false;
     if (!dev_alloc(s, D.vold, std::max(D.nport, 1)) || !dev_alloc(s, D.ring, (size_t)kRing * D.nslot) ||
         !dev_alloc(s, D.acc, (size_t)D.nslot * 2 * s->nf) || !dev_alloc(s, D.dstep, 1) ||
         !dev_alloc(s, D.srcv, 2))
         return false;
+    D.run.samples = D.samples.p;
+    D.run.raw = D.raw.p;
+    D.run.src = D.run_src.p;
+    D.run.srcv = reinterpret_cast<float2 *>(D.srcv.p);
+    D.run.at = D.run_at.p;
     return true;
 }
 
@@ -3034,24 +3269,34 @@ bool launch_fused_step(cem_sim *s) {
     return true;
 }
 
-bool launch_step(cem_sim *s, int phase_mask, int i0, int i1) {
+// The phases of phase_mask (1 H, 2 port voltages, 4 E, 8 surface impedance,
+// probes and step count) on node planes [i0, i1). run: a step of a run of whole
+// steps (march of run_steps); its samples and surface-impedance edges ride on the
+// update launches, and only the step count of the host advances.
+bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
     Device &D = *s->dev;
     if (phase_mask == (1 | 4 | 8) && i0 <= 0 && i1 > s->n[0] && D.use_fused) return launch_fused_step(s);
     const int nx = s->n[0];
     const dim3 blk(kBlock);
+    SibcArgs sb = D.sb[D.cur];
+    if (!run || !D.sibc_flagged) sb.ns = 0;
+    RunArgs none = D.run, carry = D.run;   // a launch with nothing of the run's, and the phase's one with it
+    none.first = carry.first = 0;
+    none.skip = carry.skip = sb.ns ? kFlagSibc : 0u;
     // general work-list entries of update u for node planes [a, b)
     auto span = [&](int u, int a, int b, const int2 *&p) {
         const std::vector<int> &st = D.wl_start[u];
         p = D.wl[u].p + st[a];
         return (unsigned)(st[b] - st[a]);
     };
-    // fast (or Debye) rectangles of update u on node planes [a, b)
-    auto fast = [&](int u, int a, int b, auto kernel, int cls = kFast) {
+    // fast (or Debye) rectangles of update u on node planes [a, b), with one block column more for r.first
+    auto fast = [&](int u, int a, int b, auto kernel, const RunArgs &r, int cls = kFast) {
         const int nb = space_blocks(D.sp[u][cls]);
         const int c0 = std::max(a, D.p0[u]), c1 = std::min(b, D.p1[u]);
         if (nb == 0) return;
-        for (int c = c0; c < c1; c += kMaxGridY)
-            kernel<<<dim3(3 * nb, std::min(kMaxGridY, c1 - c)), blk, 0, D.stream>>>(D.sa[D.cur], c);
+        RunArgs q = r;
+        for (int c = c0; c < c1; c += kMaxGridY, q.first = 0)
+            kernel<<<dim3(3 * nb + q.first, std::min(kMaxGridY, c1 - c)), blk, 0, D.stream>>>(D.sa[D.cur], c, q);
     };
     // the general blocks go to the side stream (after the work so far on the
     // main one), the fast pieces to the main stream, which then waits for both
@@ -3066,13 +3311,17 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1) {
             t_begin(0);
             const int2 *w;
             const unsigned n = span(0, a, b, w);
+            carry.first = run ? 1 : 0;
+            auto general = [&](cudaStream_t st) { k_update_h<<<n + carry.first, blk, 0, st>>>(D.sa[D.cur], w, carry); };
             if (n && D.side_on) {
                 fork();
-                k_update_h<<<n, blk, 0, D.side>>>(D.sa[D.cur], w);
+                general(D.side);
                 cudaEventRecord(D.join, D.side);
             }
-            fast(0, a, b, k_update_h_fast);
-            if (n && !D.side_on) k_update_h<<<n, blk, 0, D.stream>>>(D.sa[D.cur], w);
+            const bool here = !n && space_blocks(D.sp[0][kFast]);   // no general blocks: the fast launch carries the run's
+            fast(0, a, b, k_update_h_fast, here ? carry : none);
+            if (n && !D.side_on) general(D.stream);
+            if (run && !n && !here) k_begin_step<<<1, blk, 0, D.stream>>>(D.sa[D.cur], carry);
             if (n && D.side_on) join();
             t_end();
         }
@@ -3088,21 +3337,33 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1) {
             t_begin(1);
             const int2 *w;
             const unsigned n = span(1, a, b, w);
-            if (n && D.side_on) {
+            const bool own = n || sb.ns;   // the general launch carries the run's
+            carry.first = !run ? 0 : own ? 1 + (sb.ns + kBlock - 1) / kBlock : 1;
+            auto general = [&](cudaStream_t st) {
+                kEKernels[s->npole]<<<n + carry.first, blk, 0, st>>>(D.sa[D.cur], w, carry, sb);
+            };
+            if (own && D.side_on) {
                 fork();
-                kEKernels[s->npole]<<<n, blk, 0, D.side>>>(D.sa[D.cur], w);
+                general(D.side);
                 cudaEventRecord(D.join, D.side);
             }
-            fast(1, a, b, k_update_e_fast);
-            fast(1, a, b, kEDKernels[s->npole], kDebye);
-            if (n && !D.side_on) kEKernels[s->npole]<<<n, blk, 0, D.stream>>>(D.sa[D.cur], w);
-            if (n && D.side_on) join();
+            const bool here = !own && space_blocks(D.sp[1][kFast]);
+            fast(1, a, b, k_update_e_fast, here ? carry : none);
+            fast(1, a, b, kEDKernels[s->npole], none, kDebye);
+            if (own && !D.side_on) general(D.stream);
+            if (run && !own && !here) k_sample_h<<<1, blk, 0, D.stream>>>(D.sa[D.cur], carry);
+            if (own && D.side_on) join();
             t_end();
         }
     }
     if (phase_mask & 8) {   // surface impedance, probes, step count
-        if (D.ring_count == kRing && !flush_dft(s)) return false;
-        launch_sibc_post(s, D);
+        if (run) {
+            if (s->nsb && !D.sibc_flagged)
+                k_sibc<<<(unsigned)((s->nsb + kBlock - 1) / kBlock), kBlock, 0, D.stream>>>(D.sb[D.cur]);
+        } else {
+            if (D.ring_count == kRing && !flush_dft(s)) return false;
+            launch_sibc_post(s, D);
+        }
         D.ring_count++;
         s->step++;
     }
@@ -3162,25 +3423,25 @@ void engine_host_modified(cem_sim *s, unsigned groups) {
 
 namespace {
 
-constexpr int kGraphSteps = 32;   // divides kRing: graph runs fill the sample ring exactly
-
-// n whole steps. With graphs on (separate H and E kernels, not while kernels
-// are timed one by one), a run of kGraphSteps steps that needs no DFT flush
-// replays one graph captured from the same launches; the others go one by one.
-// The graph holds the kernels' arguments, which stay fixed for the life of
-// the device state.
-bool run_steps(cem_sim *s, long n) {
+// n whole steps, n at most Device::run_steps and the room in the sample ring:
+// source values, the steps (with graphs on, groups of graph_steps replay one
+// captured graph; the graph holds the kernels' arguments, which stay fixed for
+// the life of the device state), then the sample rows.
+bool run_chunk(cem_sim *s, long n) {
     Device &D = *s->dev;
-    const bool graphs = D.use_graphs && !D.use_fused && !g_timer;
+    const PostArgs &pa = D.pa[D.cur];
+    const long step0 = s->step;
+    k_run_begin<<<(unsigned)((n + 127) / 128), 128, 0, D.stream>>>(D.run, pa, reinterpret_cast<float *>(D.run_src.p), (int)n,
+                                                                  step0);
     for (long it = 0; it < n;) {
         const int gs = D.graph_steps;
-        if (graphs && n - it >= gs && D.ring_count + gs <= kRing) {
+        if (D.use_graphs && n - it >= gs) {
             if (!D.graph) {
                 const int rc = D.ring_count;
                 const long st = s->step;
                 CB2_CHECK(s, cudaStreamBeginCapture(D.stream, cudaStreamCaptureModeThreadLocal));
                 bool ok = true;
-                for (int q = 0; q < gs && ok; q++) ok = launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1);
+                for (int q = 0; q < gs && ok; q++) ok = launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1, true);
                 cudaGraph_t g = nullptr;
                 const cudaError_t ec = cudaStreamEndCapture(D.stream, &g);
                 D.ring_count = rc;
@@ -3200,9 +3461,25 @@ bool run_steps(cem_sim *s, long n) {
             s->step += gs;
             it += gs;
         } else {
-            if (!launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1)) return false;
+            if (!launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1, true)) return false;
             it++;
         }
+    }
+    k_rows<<<(unsigned)n, kRowThreads, 0, D.stream>>>(D.run, pa, (int)n, step0);
+    CB2_CHECK(s, cudaGetLastError());
+    return true;
+}
+
+// n whole steps: in runs with the separate kernels, one by one with the fused
+// kernel and while kernels are timed one by one
+bool run_steps(cem_sim *s, long n) {
+    Device &D = *s->dev;
+    const bool runs = !D.use_fused && !g_timer;
+    while (n > 0) {
+        if (D.ring_count == kRing && !flush_dft(s)) return false;
+        const long k = runs ? std::min<long>(n, std::min(D.run_steps, kRing - D.ring_count)) : 1;
+        if (runs ? !run_chunk(s, k) : !launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1)) return false;
+        n -= k;
     }
     CB2_CHECK(s, cudaGetLastError());
     return true;
