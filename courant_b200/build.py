@@ -27,7 +27,7 @@ CUDA_LIB = Path(NVCC).resolve().parent.parent / "lib64"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CXXFLAGS = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-ffp-contract=off", "-Wall", "-Wextra",
             "-Wno-unused-parameter", f'-DCEM_VERSION="{VERSION}"', f"-I{INCLUDE}"]
-NVFLAGS = ["-O3", "-std=c++17", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC,-fvisibility=hidden,-ffp-contract=off",
+NVFLAGS = ["-O3", "--split-compile=0", "-std=c++17", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC,-fvisibility=hidden,-ffp-contract=off",
            "-Xptxas", "-v", f'-DCEM_VERSION="{VERSION}"', f"-I{INCLUDE}"]
 
 
