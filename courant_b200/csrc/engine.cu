@@ -1,16 +1,19 @@
 // Device time stepping for libcourant_b200 (NVIDIA B200, sm_100a).
 //
 // Replaces the reference time loop (skyhoffert/CourantEM solver/src/sim.c:569-960,
-// dispersive.c:89-112, sibc.c:256-269, modeport.c:124-135) with four kernels
-// per step, all in stream order:
+// dispersive.c:89-112, sibc.c:256-269, modeport.c:124-135) with two phases per
+// step, each a few kernels side by side:
 //
-//   k_update_h   H bulk curl fused with the CPML psi_H recursions
-//   k_update_e   E bulk curl fused with the CPML psi_E recursions, PEC/sheet
+//   k_update_h*  H bulk curl fused with the CPML psi_H recursions
+//   k_update_e*  E bulk curl fused with the CPML psi_E recursions, PEC/sheet
 //                masking, the lumped and mode sources and the Debye ADE
-//                currents (correction and update in one pass per edge)
-//   k_sibc       surface-impedance edges (recursive convolution), if any
-//   k_post       probe/port line integrals by warp reductions into a sample
-//                ring; k_dft folds the ring into FP64 DFT accumulators
+//                currents (correction and update in one pass per edge); the
+//                surface-impedance edges (recursive convolution)
+//
+// Both sample the probe and port edges of the family they only read; after a
+// run of steps k_rows turns the samples into line integrals in a sample ring,
+// and k_dft folds the ring into FP64 DFT accumulators. (k_sibc and k_post do
+// the same step by step, for the cem_mt_* phases.)
 //
 // Layout in HBM: fields and auxiliary states are FP32, structure of arrays,
 // in the reference index space q = i*si + j*sj + k (k fastest), so a warp
@@ -200,7 +203,11 @@ struct PostArgs {
 // A run of whole steps. Probe and port edges are sampled by blocks of the
 // update launches themselves, where nothing writes the family they read: E of
 // a step in the H launch of the next one, H in the E launch. The samples (one
-// row per step) become rows of the sample ring after the run (k_rows).
+// row per step) become rows of the sample ring after the run (k_rows). A probe
+// kernel after each E update (one block, 4 us between two dependent launches)
+// was a quarter to a third of a small grid's step: 61 x 47 x 35 cavity 9.3 us
+// per step with it, 5.5 so; 121 x 62 x 40 line 16.8 and 12.8; 232 x 159 x 30
+// board 45.2 and 41.1.
 struct RunArgs {
     const uint4 *samples;    // entries of E, then of H: component (0..5), index, place in the row
     int nsample[2];
@@ -522,14 +529,14 @@ __device__ __forceinline__ void st4(float *p, const float4 &v) { *reinterpret_ca
 // Every lane of the warp must call it.
 __device__ __forceinline__ float4 next_k(const float4 &v, const float *p, bool need, bool edge) {
     float w = __shfl_down_sync(0xffffffffu, v.x, 1);
-    if (edge && need) w = __ldg(p + 4);
+    if (edge && need) w = p[4];
     return make_float4(v.y, v.z, v.w, w);
 }
 
 // values at q-1 .. q+2 (a lane that starts a run loads p[-1] when `need`)
 __device__ __forceinline__ float4 prev_k(const float4 &v, const float *p, bool need, bool edge) {
     float w = __shfl_up_sync(0xffffffffu, v.w, 1);
-    if (edge && need) w = __ldg(p - 1);
+    if (edge && need) w = p[-1];
     return make_float4(w, v.x, v.y, v.z);
 }
 
@@ -675,17 +682,17 @@ __device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r)
     const Where w = valid && !FAST ? h_where<C>(a, i, j, k4) : Where{-1, -1, make_int4(-1, -1, -1, -1), -1, false};
     const bool row = valid;
     const int q = i * (int)a.g.si + m;
-    const float *__restrict__ E2 = a.E[A2];
-    const float *__restrict__ E1 = a.E[A1];
-    float *__restrict__ H = a.H[C];
+    const float *E2 = a.E[A2];
+    const float *E1 = a.E[A1];
+    float *H = a.H[C];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 e2 = z4, e1 = z4, h = z4, e2n = z4, e1n = z4;
     if (row) {
-        e2 = ldg4(E2 + q);
-        e1 = ldg4(E1 + q);
+        e2 = ld4(E2 + q);
+        e1 = ld4(E1 + q);
         h = ld4(H + q);
-        if (A1 != 2) e2n = ldg4(E2 + q + stride_of<A1>(a));
-        if (A2 != 2) e1n = ldg4(E1 + q + stride_of<A2>(a));
+        if (A1 != 2) e2n = ld4(E2 + q + stride_of<A1>(a));
+        if (A2 != 2) e1n = ld4(E1 + q + stride_of<A2>(a));
     }
     // the next lane holds the next four points only if it is in the same run and loaded them
     const bool nb = __shfl_down_sync(0xffffffffu, row, 1);
@@ -924,19 +931,19 @@ __device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r,
     const Where w = valid && !FAST ? e_where<C, P>(a, i, j, k4) : Where{-1, -1, make_int4(-1, -1, -1, -1), -1, false};
     const bool row = valid;
     const int q = i * (int)a.g.si + m;
-    const float *__restrict__ H2 = a.H[A2];
-    const float *__restrict__ H1 = a.H[A1];
-    float *__restrict__ E = a.E[C];
+    const float *H2 = a.H[A2];
+    const float *H1 = a.H[A1];
+    float *E = a.E[C];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 h2 = z4, h1 = z4, ev = z4, h2m = z4, h1m = z4;
     uint2 mv = make_uint2(0, 0);
     if (row) {
-        h2 = ldg4(H2 + q);
-        h1 = ldg4(H1 + q);
+        h2 = ld4(H2 + q);
+        h1 = ld4(H1 + q);
         ev = ld4(E + q);
         mv = __ldg(reinterpret_cast<const uint2 *>(a.mat[C] + q));
-        if (A1 != 2) h2m = ldg4(H2 + q - stride_of<A1>(a));
-        if (A2 != 2) h1m = ldg4(H1 + q - stride_of<A2>(a));
+        if (A1 != 2) h2m = ld4(H2 + q - stride_of<A1>(a));
+        if (A2 != 2) h1m = ld4(H1 + q - stride_of<A2>(a));
     }
     // the previous lane holds the previous four points only if it is in the same run and loaded them
     const bool pb = __shfl_up_sync(0xffffffffu, row, 1);
@@ -972,17 +979,17 @@ __device__ __forceinline__ void h_lean(const StepArgs &a, int i, const RowPos &p
     const int j = p.j, k4 = p.k4;
     const bool row = p.act && (!(A1 == 0 || A2 == 0) || i < nx) && (!(A1 == 1 || A2 == 1) || j < ny);
     const int q = i * (int)a.g.si + j * a.g.sj + k4;
-    const float *__restrict__ E2 = a.E[A2];
-    const float *__restrict__ E1 = a.E[A1];
-    float *__restrict__ H = a.H[C];
+    const float *E2 = a.E[A2];
+    const float *E1 = a.E[A1];
+    float *H = a.H[C];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 e2 = z4, e1 = z4, h = z4, e2n = z4, e1n = z4;
     if (row) {
-        e2 = ldg4(E2 + q);
-        e1 = ldg4(E1 + q);
+        e2 = ld4(E2 + q);
+        e1 = ld4(E1 + q);
         h = ld4(H + q);
-        if (A1 != 2) e2n = ldg4(E2 + q + stride_of<A1>(a));
-        if (A2 != 2) e1n = ldg4(E1 + q + stride_of<A2>(a));
+        if (A1 != 2) e2n = ld4(E2 + q + stride_of<A1>(a));
+        if (A2 != 2) e1n = ld4(E1 + q + stride_of<A2>(a));
     }
     if (A1 == 2) e2n = next_k(e2, E2 + q, row && k4 + 4 <= nz, !p.cont);
     if (A2 == 2) e1n = next_k(e1, E1 + q, row && k4 + 4 <= nz, !p.cont);
@@ -1017,19 +1024,19 @@ __device__ __forceinline__ void e_lean(const StepArgs &a, int i, const RowPos &p
     const int j = p.j, k4 = p.k4;
     const bool row = p.act && (C == 0 || i >= 1) && (C == 1 ? j < ny : (j >= 1 && j < ny));
     const int q = i * (int)a.g.si + j * a.g.sj + k4;
-    const float *__restrict__ H2 = a.H[A2];
-    const float *__restrict__ H1 = a.H[A1];
-    float *__restrict__ E = a.E[C];
+    const float *H2 = a.H[A2];
+    const float *H1 = a.H[A1];
+    float *E = a.E[C];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 h2 = z4, h1 = z4, ev = z4, h2m = z4, h1m = z4;
     uint2 mv = make_uint2(0, 0);
     if (row) {
-        h2 = ldg4(H2 + q);
-        h1 = ldg4(H1 + q);
+        h2 = ld4(H2 + q);
+        h1 = ld4(H1 + q);
         ev = ld4(E + q);
         mv = __ldg(reinterpret_cast<const uint2 *>(a.mat[C] + q));
-        if (A1 != 2) h2m = ldg4(H2 + q - stride_of<A1>(a));
-        if (A2 != 2) h1m = ldg4(H1 + q - stride_of<A2>(a));
+        if (A1 != 2) h2m = ld4(H2 + q - stride_of<A1>(a));
+        if (A2 != 2) h1m = ld4(H1 + q - stride_of<A2>(a));
     }
     // the previous lane holds the previous four points unless this lane starts a warp or a row
     const bool first = (threadIdx.x & 31) == 0 || k4 == p.ks;
@@ -1063,10 +1070,10 @@ __device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &
     const int j = p.j, k4 = p.k4;
     const bool row = p.act && (C == 0 || i >= 1) && (C == 1 ? j < ny : (j >= 1 && j < ny));
     const int q = i * (int)a.g.si + j * a.g.sj + k4;
-    const float *__restrict__ H2 = a.H[A2];
-    const float *__restrict__ H1 = a.H[A1];
-    float *__restrict__ E = a.E[C];
-    float *__restrict__ Jc = a.J[C];
+    const float *H2 = a.H[A2];
+    const float *H1 = a.H[A1];
+    float *E = a.E[C];
+    float *Jc = a.J[C];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 h2 = z4, h1 = z4, ev = z4, h2m = z4, h1m = z4;
     uint2 mv = make_uint2(0, 0);
@@ -1076,12 +1083,12 @@ __device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &
     const int jvol = jbox_volume<C>(a);
     float4 J[P > 0 ? P : 1];
     if (row) {
-        h2 = ldg4(H2 + q);
-        h1 = ldg4(H1 + q);
+        h2 = ld4(H2 + q);
+        h1 = ld4(H1 + q);
         ev = ld4(E + q);
         mv = __ldg(reinterpret_cast<const uint2 *>(a.mat[C] + q));
-        if (A1 != 2) h2m = ldg4(H2 + q - stride_of<A1>(a));
-        if (A2 != 2) h1m = ldg4(H1 + q - stride_of<A2>(a));
+        if (A1 != 2) h2m = ld4(H2 + q - stride_of<A1>(a));
+        if (A2 != 2) h1m = ld4(H1 + q - stride_of<A2>(a));
     }
 #pragma unroll
     for (int pp = 0; pp < P; pp++) J[pp] = jo4 >= 0 ? ld4(Jc + jaddr(P, jvol, pp, jo4)) : z4;
@@ -1121,7 +1128,7 @@ __device__ __forceinline__ void sibc_edge(const SibcArgs &a, int e) {
     const int hc[4] = {c4.x, c4.y, c4.z, c4.w};
     float h[4];
 #pragma unroll
-    for (int f = 0; f < 4; f++) h[f] = w[f] != 0.f ? __ldg(a.H[hc[f]] + hi[f]) : 0.f;
+    for (int f = 0; f < 4; f++) h[f] = w[f] != 0.f ? a.H[hc[f]][hi[f]] : 0.f;
     // explicit roundings: the same bits in every kernel that inlines this
     float J = 0.f;
 #pragma unroll
@@ -1146,7 +1153,7 @@ __device__ __forceinline__ void sample_family(const StepArgs &a, const RunArgs &
     const uint4 *s = r.samples + (u ? r.nsample[0] : 0);
     for (int e = threadIdx.x; e < r.nsample[u]; e += blockDim.x) {
         const uint4 v = __ldg(s + e);
-        r.raw[(size_t)t * r.nent + v.z] = __ldg((u ? a.H[v.x - 3] : a.E[v.x]) + v.y);
+        r.raw[(size_t)t * r.nent + v.z] = (u ? a.H[v.x - 3] : a.E[v.x])[v.y];
     }
 }
 
@@ -1183,50 +1190,49 @@ __device__ __forceinline__ void begin_step(const StepArgs &a, const RunArgs &r) 
 #define CB2_EF_MINBLOCKS 8
 #endif
 
+// Chained launches (RunArgs::on): a launch that follows another on one stream
+// alone may start while that one ends; it works out its place meanwhile and
+// waits for the end before it touches what that one writes. (Fields are read by
+// plain loads for that: they change within the launch's life. The wait makes the
+// other's writes visible; the read-only path promises nothing there.) Parity
+// scene 6.8 to 5.9 us per step, lossy scene 8.2 to 6.9, cavity 5.8 to 5.4.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // H on the fast rectangles of node planes [i0, i0 + gridDim.y); block x:
 // block x / 3 of the space, component x % 3
 __global__ void __launch_bounds__(kBlock, CB2_HF_MINBLOCKS) k_update_h_fast(const StepArgs a, int i0, const RunArgs r) {
+    chain_next();
     if (r.first && blockIdx.x == gridDim.x - 1) {   // one column more: the run's own work
+        chain_wait();
         if (blockIdx.y == 0) begin_step(a, r);
         return;
     }
     const int comp = blockIdx.x % 3;
     const RowPos p = space_pos(a.sp[0][kFast], blockIdx.x / 3);
+    chain_wait();
     const int i = i0 + blockIdx.y;
     if (comp == 0) h_lean<0>(a, i, p);
     else if (comp == 1) h_lean<1>(a, i, p);
     else h_lean<2>(a, i, p);
 }
 
-// E on the fast rectangles of node planes [i0, i0 + gridDim.y)
+// E on the fast rectangles of node planes [i0, i0 + gridDim.y), from the last to the first
 __global__ void __launch_bounds__(kBlock, CB2_EF_MINBLOCKS) k_update_e_fast(const StepArgs a, int i0, const RunArgs r) {
+    chain_next();
     if (r.first && blockIdx.x == gridDim.x - 1) {
+        chain_wait();
         if (blockIdx.y == 0) sample_family(a, r, 1, r.at[0]);
         return;
     }
     const int comp = blockIdx.x % 3;
     const RowPos p = space_pos(a.sp[1][kFast], blockIdx.x / 3);
-    const int i = i0 + blockIdx.y;
+    chain_wait();
+    const int i = i0 + (int)(gridDim.y - 1 - blockIdx.y);   // E begins where H ended, on what L2 still holds
     const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
     if (comp == 0) e_lean<0>(a, i, p, sv, r.skip);
     else if (comp == 1) e_lean<1>(a, i, p, sv, r.skip);
     else e_lean<2>(a, i, p, sv, r.skip);
-}
-
-#ifndef CB2_ED_MINBLOCKS
-#define CB2_ED_MINBLOCKS 6
-#endif
-
-// E on the Debye rectangles of node planes [i0, i0 + gridDim.y) (P poles)
-template <int P>
-__global__ void __launch_bounds__(kBlock, CB2_ED_MINBLOCKS) k_update_e_debye(const StepArgs a, int i0, const RunArgs r) {
-    const int comp = blockIdx.x % 3;
-    const RowPos p = space_pos(a.sp[1][kDebye], blockIdx.x / 3);
-    const int i = i0 + blockIdx.y;
-    const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
-    if (comp == 0) e_debye<0, P>(a, i, p, sv, r.skip);
-    else if (comp == 1) e_debye<1, P>(a, i, p, sv, r.skip);
-    else e_debye<2, P>(a, i, p, sv, r.skip);
 }
 
 // Position in the general space of update U: the general rectangles on an
@@ -1239,34 +1245,137 @@ __device__ __forceinline__ RowPos general_pos(const StepArgs &a, int i, int b) {
 // Work entry of the general blocks: x node plane, y block of the plane's
 // general space (component y % 3, block y / 3).
 __global__ void __launch_bounds__(kBlock, CB2_H_MINBLOCKS) k_update_h(const StepArgs a, const int2 *work, const RunArgs r) {
+    chain_next();
     if ((int)blockIdx.x < r.first) {
+        chain_wait();
         begin_step(a, r);
         return;
     }
     const int2 w = work[blockIdx.x - r.first];
     const int comp = w.y % 3;
     const RowPos p = general_pos<0>(a, w.x, w.y / 3);
+    chain_wait();
     if (comp == 0) h_vec<0, false>(a, w.x, p);
     else if (comp == 1) h_vec<1, false>(a, w.x, p);
     else h_vec<2, false>(a, w.x, p);
 }
 
-// E over the general blocks (P Debye poles)
-template <int P>
-__global__ void __launch_bounds__(kBlock, CB2_E_MINBLOCKS) k_update_e(const StepArgs a, const int2 *work, const RunArgs r, const SibcArgs s) {
+// E over the general blocks (no Debye poles)
+__global__ void __launch_bounds__(kBlock, CB2_E_MINBLOCKS)
+    k_update_e(const StepArgs a, const int2 *work, const RunArgs r, const SibcArgs s) {
+    chain_next();
     if ((int)blockIdx.x < r.first) {   // H samples, then the surface-impedance edges (their E is left alone below)
         const int e = ((int)blockIdx.x - 1) * kBlock + threadIdx.x;
+        chain_wait();
         if (blockIdx.x == 0) sample_family(a, r, 1, r.at[0]);
         else if (e < s.ns) sibc_edge(s, e);
         return;
     }
-    const int2 w = work[blockIdx.x - r.first];
+    const int2 w = work[gridDim.x - 1 - blockIdx.x];
     const int comp = w.y % 3;
     const RowPos p = general_pos<1>(a, w.x, w.y / 3);
+    chain_wait();
     const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
-    if (comp == 0) e_vec<0, P, false>(a, w.x, p, sv, r.skip);
-    else if (comp == 1) e_vec<1, P, false>(a, w.x, p, sv, r.skip);
-    else e_vec<2, P, false>(a, w.x, p, sv, r.skip);
+    if (comp == 0) e_vec<0, 0, false>(a, w.x, p, sv, r.skip);
+    else if (comp == 1) e_vec<1, 0, false>(a, w.x, p, sv, r.skip);
+    else e_vec<2, 0, false>(a, w.x, p, sv, r.skip);
+}
+
+// All blocks of an update in one launch: the run's own work first, then the
+// general blocks (the slowest) of a work-list, then the interior planes, on
+// each the Debye and the fast rectangles. There is no second stream to fork and
+// join, consecutive launches chain, and the pieces of a row that a Debye and a
+// fast rectangle share are fetched from HBM once. The price is one register
+// count for all blocks: where bandwidth counts more than launches and there is
+// nothing to share, H and (without poles) E of a large grid keep a kernel per
+// class on two streams. us per step, kernel per class / one launch for E / for
+// both: line 121 x 62 x 40 12.6 / 12.6 / 10.4, 250 k-cell board 15.7 / 15.5 /
+// 13.1, 1.1 M-cell board 41.2 / 40.2 / 38.3, lossy line (6 poles, 3.6 M cells)
+// 102 / 99.4 / 101, 10.9 M-cell board 364 / 334 / 352, 5.7 M-cell line (no
+// poles) 123 / 125 / 128. (General blocks spread evenly over the launch
+// instead: 1.1 M-cell board 43.7, 10.9 M-cell 373.)
+struct Whole {
+    const int2 *work;    // general entries (node plane, block)
+    int n;
+    int p0, planes;      // interior node planes
+    int nd, nf;          // blocks of a plane's Debye and fast rectangles, components included
+    int flip;            // from the last plane to the first: E begins where H ended, on what L2 still holds
+};
+
+template <bool E>
+__device__ __forceinline__ int whole_place(const StepArgs &a, const Whole &l, int b, int &i, int &comp, RowPos &p) {
+    if (b < l.n) {
+        const int2 w = l.work[l.flip ? l.n - 1 - b : b];
+        i = w.x;
+        comp = w.y % 3;
+        p = general_pos<E ? 1 : 0>(a, w.x, w.y / 3);
+        return 2;
+    }
+    const int per = l.nd + l.nf, f = b - l.n, plane = f / per, x = f - plane * per;
+    i = l.p0 + (l.flip ? l.planes - 1 - plane : plane);
+    const bool deb = x < l.nd;
+    const int y = deb ? x : x - l.nd;
+    comp = y % 3;
+    p = space_pos(a.sp[E ? 1 : 0][deb ? kDebye : kFast], y / 3);
+    return deb ? 1 : 0;
+}
+
+// resident blocks per SM: 48 registers for H; for E 72, or 64 on large grids of up
+// to four poles (they spill a little on the CPML paths there, but a bandwidth-bound
+// launch gains more from the eighth block: 334 against 341 us per step on the
+// 10.9 M-cell board; 13.1 against 15.1 the other way on the 250 k-cell one)
+constexpr int kWholeH = 10, kWholeE = 7, kWholeELarge = 8;
+__global__ void __launch_bounds__(kBlock, kWholeH) k_whole_h(const StepArgs a, const Whole l, const RunArgs r) {
+    chain_next();
+    if ((int)blockIdx.x < r.first) {
+        chain_wait();
+        begin_step(a, r);
+        return;
+    }
+    int i, comp;
+    RowPos p;
+    const int kind = whole_place<false>(a, l, (int)blockIdx.x - r.first, i, comp, p);
+    chain_wait();
+    if (kind == 2) {
+        if (comp == 0) h_vec<0, false>(a, i, p);
+        else if (comp == 1) h_vec<1, false>(a, i, p);
+        else h_vec<2, false>(a, i, p);
+    } else {
+        if (comp == 0) h_lean<0>(a, i, p);
+        else if (comp == 1) h_lean<1>(a, i, p);
+        else h_lean<2>(a, i, p);
+    }
+}
+
+template <int P, int B>
+__global__ void __launch_bounds__(kBlock, P > 8 ? 4 : B)
+    k_whole_e(const StepArgs a, const Whole l, const RunArgs r, const SibcArgs s) {
+    chain_next();
+    if ((int)blockIdx.x < r.first) {   // H samples, then the surface-impedance edges (their E is left alone below)
+        const int e = ((int)blockIdx.x - 1) * kBlock + threadIdx.x;
+        chain_wait();
+        if (blockIdx.x == 0) sample_family(a, r, 1, r.at[0]);
+        else if (e < s.ns) sibc_edge(s, e);
+        return;
+    }
+    int i, comp;
+    RowPos p;
+    const int kind = whole_place<true>(a, l, (int)blockIdx.x - r.first, i, comp, p);
+    chain_wait();
+    const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
+    if (kind == 2) {
+        if (comp == 0) e_vec<0, P, false>(a, i, p, sv, r.skip);
+        else if (comp == 1) e_vec<1, P, false>(a, i, p, sv, r.skip);
+        else e_vec<2, P, false>(a, i, p, sv, r.skip);
+    } else if (P > 0 && kind == 1) {
+        if (comp == 0) e_debye<0, P>(a, i, p, sv, r.skip);
+        else if (comp == 1) e_debye<1, P>(a, i, p, sv, r.skip);
+        else e_debye<2, P>(a, i, p, sv, r.skip);
+    } else {
+        if (comp == 0) e_lean<0>(a, i, p, sv, r.skip);
+        else if (comp == 1) e_lean<1>(a, i, p, sv, r.skip);
+        else e_lean<2>(a, i, p, sv, r.skip);
+    }
 }
 
 constexpr unsigned kWaitLimit = 1u << 24;
@@ -1474,19 +1583,18 @@ __global__ void __launch_bounds__(kFT, 3) k_step_fused(const StepArgs a, const F
 }
 
 // launchers of the pole-count instantiations
-using EKernel = void (*)(StepArgs, const int2 *, RunArgs, SibcArgs);
 using HKernel = void (*)(StepArgs, int, RunArgs);
 using FKernel = void (*)(StepArgs, FusedArgs, TmaMaps);
+using WKernel = void (*)(StepArgs, Whole, RunArgs, SibcArgs);
 #define CB2_POLES(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
-#define CB2_EK(p) k_update_e<p>,
 #define CB2_FK(p) k_step_fused<p>,
-#define CB2_DK(p) k_update_e_debye<p>,
-const EKernel kEKernels[] = {CB2_POLES(CB2_EK)};
+#define CB2_WK(p) k_whole_e<p, kWholeE>,
 const FKernel kFKernels[] = {CB2_POLES(CB2_FK)};
-const HKernel kEDKernels[] = {CB2_POLES(CB2_DK)};
-#undef CB2_EK
+const WKernel kEWKernels[] = {CB2_POLES(CB2_WK)};
+const WKernel kEWLarge[] = {k_whole_e<0, kWholeELarge>, k_whole_e<1, kWholeELarge>, k_whole_e<2, kWholeELarge>,
+                            k_whole_e<3, kWholeELarge>, k_whole_e<4, kWholeELarge>};
 #undef CB2_FK
-#undef CB2_DK
+#undef CB2_WK
 #undef CB2_POLES
 
 // ------------------------------------------------------------------- SIBC
@@ -1973,6 +2081,8 @@ struct Device {
     // runs of whole steps (RunArgs)
     int run_steps = 0;                // most steps of a run (sample rows)
     bool sibc_flagged = false;        // the tables mark the surface-impedance edges
+    bool whole_h = true, whole_e = true;   // an update's blocks in one launch (Whole), or a kernel per class
+    bool chained = false;   // the last launch on the main stream is one of a run, nothing else since
     RunArgs run{};
     DevBuf<uint4> samples;
     DevBuf<float> raw;
@@ -2893,6 +3003,9 @@ bool create_device_impl(cem_sim *s) {
     if (const char *e = std::getenv("CEM_B200_FUSED")) D.use_fused = e[0] == '1';
     if (const char *e = std::getenv("CEM_B200_GRAPHS")) D.use_graphs = e[0] != '0';
     D.ztail = (long long)s->n[0] * s->n[1] * s->n[2] >= 2000000;
+    // one launch an update below 2 M cells; above, for E with poles (Whole has both sides measured)
+    D.whole_h = (long long)s->n[0] * s->n[1] * s->n[2] < 2000000;
+    D.whole_e = D.whole_h || s->npole > 0;
     if (const char *e = std::getenv("CEM_B200_ZTAIL")) {
         D.ztail = e[0] != '0';
         D.ztail_split = e[0] != '1';
@@ -3271,7 +3384,7 @@ bool launch_fused_step(cem_sim *s) {
 
 // The phases of phase_mask (1 H, 2 port voltages, 4 E, 8 surface impedance,
 // probes and step count) on node planes [i0, i1). run: a step of a run of whole
-// steps (march of run_steps); its samples and surface-impedance edges ride on the
+// steps (run_chunk); its samples and surface-impedance edges ride on the
 // update launches, and only the step count of the host advances.
 bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
     Device &D = *s->dev;
@@ -3289,6 +3402,30 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
         p = D.wl[u].p + st[a];
         return (unsigned)(st[b] - st[a]);
     };
+    // the general blocks go to the side stream (after the work so far on the
+    // main one), the fast pieces to the main stream, which then waits for both
+    auto fork = [&]() {
+        cudaEventRecord(D.fork, D.stream);
+        cudaStreamWaitEvent(D.side, D.fork, 0);
+    };
+    auto join = [&]() {
+        cudaStreamWaitEvent(D.stream, D.join, 0);
+        D.chained = false;
+    };
+    // a kernel on the main stream; of a run, chained to the one before it where only that one precedes it
+    auto launch = [&](auto kernel, dim3 grid, auto... args) {
+        cudaLaunchConfig_t c{};
+        c.gridDim = grid;
+        c.blockDim = blk;
+        c.stream = D.stream;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        c.attrs = &at;
+        c.numAttrs = run && D.chained ? 1 : 0;
+        cudaLaunchKernelEx(&c, kernel, args...);
+        D.chained = run;
+    };
     // fast (or Debye) rectangles of update u on node planes [a, b), with one block column more for r.first
     auto fast = [&](int u, int a, int b, auto kernel, const RunArgs &r, int cls = kFast) {
         const int nb = space_blocks(D.sp[u][cls]);
@@ -3296,33 +3433,45 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
         if (nb == 0) return;
         RunArgs q = r;
         for (int c = c0; c < c1; c += kMaxGridY, q.first = 0)
-            kernel<<<dim3(3 * nb + q.first, std::min(kMaxGridY, c1 - c)), blk, 0, D.stream>>>(D.sa[D.cur], c, q);
+            launch(kernel, dim3(3 * nb + q.first, std::min(kMaxGridY, c1 - c)), D.sa[D.cur], c, q);
     };
-    // the general blocks go to the side stream (after the work so far on the
-    // main one), the fast pieces to the main stream, which then waits for both
-    auto fork = [&]() {
-        cudaEventRecord(D.fork, D.stream);
-        cudaStreamWaitEvent(D.side, D.fork, 0);
+    auto whole = [&](int u, int a, int b, const int2 *w, unsigned n) {
+        Whole l{};
+        l.work = w;
+        l.n = (int)n;
+        l.p0 = std::max(a, D.p0[u]);
+        l.planes = std::max(0, std::min(b, D.p1[u]) - l.p0);
+        l.nd = 3 * space_blocks(D.sp[u][kDebye]);
+        l.nf = 3 * space_blocks(D.sp[u][kFast]);
+        l.flip = u;
+        return l;
     };
-    auto join = [&]() { cudaStreamWaitEvent(D.stream, D.join, 0); };
     if (phase_mask & 1) {   // H over node planes [i0, i1) within [0, nx]
         const int a = std::max(0, i0), b = std::min(nx + 1, i1);
         if (b > a) {
             t_begin(0);
             const int2 *w;
             const unsigned n = span(0, a, b, w);
+            const bool side = n && D.side_on && space_blocks(D.sp[0][kFast]);   // beside the fast launch
             carry.first = run ? 1 : 0;
-            auto general = [&](cudaStream_t st) { k_update_h<<<n + carry.first, blk, 0, st>>>(D.sa[D.cur], w, carry); };
-            if (n && D.side_on) {
-                fork();
-                general(D.side);
-                cudaEventRecord(D.join, D.side);
+            if (D.whole_h) {
+                const Whole l = whole(0, a, b, w, n);
+                launch(k_whole_h, dim3(carry.first + n + (unsigned)l.planes * (l.nd + l.nf)), D.sa[D.cur], l, carry);
+            } else {
+                if (side) {
+                    fork();
+                    k_update_h<<<n + carry.first, blk, 0, D.side>>>(D.sa[D.cur], w, carry);
+                    cudaEventRecord(D.join, D.side);
+                }
+                const bool here = !n && space_blocks(D.sp[0][kFast]);   // no general blocks: the fast launch carries the run's
+                fast(0, a, b, k_update_h_fast, here ? carry : none);
+                if (n && !side) launch(k_update_h, dim3(n + carry.first), D.sa[D.cur], w, carry);
+                if (run && !n && !here) {
+                    k_begin_step<<<1, blk, 0, D.stream>>>(D.sa[D.cur], carry);
+                    D.chained = false;
+                }
+                if (side) join();
             }
-            const bool here = !n && space_blocks(D.sp[0][kFast]);   // no general blocks: the fast launch carries the run's
-            fast(0, a, b, k_update_h_fast, here ? carry : none);
-            if (n && !D.side_on) general(D.stream);
-            if (run && !n && !here) k_begin_step<<<1, blk, 0, D.stream>>>(D.sa[D.cur], carry);
-            if (n && D.side_on) join();
             t_end();
         }
     }
@@ -3338,28 +3487,37 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
             const int2 *w;
             const unsigned n = span(1, a, b, w);
             const bool own = n || sb.ns;   // the general launch carries the run's
+            const bool side = own && D.side_on && space_blocks(D.sp[1][kFast]);
             carry.first = !run ? 0 : own ? 1 + (sb.ns + kBlock - 1) / kBlock : 1;
-            auto general = [&](cudaStream_t st) {
-                kEKernels[s->npole]<<<n + carry.first, blk, 0, st>>>(D.sa[D.cur], w, carry, sb);
-            };
-            if (own && D.side_on) {
-                fork();
-                general(D.side);
-                cudaEventRecord(D.join, D.side);
+            if (D.whole_e) {
+                const Whole l = whole(1, a, b, w, n);
+                const bool large = !D.whole_h && s->npole <= 4;
+                launch(large ? kEWLarge[s->npole] : kEWKernels[s->npole],
+                       dim3(carry.first + n + (unsigned)l.planes * (l.nd + l.nf)), D.sa[D.cur], l, carry, sb);
+            } else {   // no poles: no Debye rectangles
+                if (side) {
+                    fork();
+                    k_update_e<<<n + carry.first, blk, 0, D.side>>>(D.sa[D.cur], w, carry, sb);
+                    cudaEventRecord(D.join, D.side);
+                }
+                const bool here = !own && space_blocks(D.sp[1][kFast]);
+                fast(1, a, b, k_update_e_fast, here ? carry : none);
+                if (own && !side) launch(k_update_e, dim3(n + carry.first), D.sa[D.cur], w, carry, sb);
+                if (run && !own && !here) {
+                    k_sample_h<<<1, blk, 0, D.stream>>>(D.sa[D.cur], carry);
+                    D.chained = false;
+                }
+                if (side) join();
             }
-            const bool here = !own && space_blocks(D.sp[1][kFast]);
-            fast(1, a, b, k_update_e_fast, here ? carry : none);
-            fast(1, a, b, kEDKernels[s->npole], none, kDebye);
-            if (own && !D.side_on) general(D.stream);
-            if (run && !own && !here) k_sample_h<<<1, blk, 0, D.stream>>>(D.sa[D.cur], carry);
-            if (own && D.side_on) join();
             t_end();
         }
     }
     if (phase_mask & 8) {   // surface impedance, probes, step count
         if (run) {
-            if (s->nsb && !D.sibc_flagged)
+            if (s->nsb && !D.sibc_flagged) {
+                D.chained = false;
                 k_sibc<<<(unsigned)((s->nsb + kBlock - 1) / kBlock), kBlock, 0, D.stream>>>(D.sb[D.cur]);
+            }
         } else {
             if (D.ring_count == kRing && !flush_dft(s)) return false;
             launch_sibc_post(s, D);
@@ -3431,6 +3589,7 @@ bool run_chunk(cem_sim *s, long n) {
     Device &D = *s->dev;
     const PostArgs &pa = D.pa[D.cur];
     const long step0 = s->step;
+    D.chained = false;
     k_run_begin<<<(unsigned)((n + 127) / 128), 128, 0, D.stream>>>(D.run, pa, reinterpret_cast<float *>(D.run_src.p), (int)n,
                                                                   step0);
     for (long it = 0; it < n;) {
@@ -3440,6 +3599,7 @@ bool run_chunk(cem_sim *s, long n) {
                 const int rc = D.ring_count;
                 const long st = s->step;
                 CB2_CHECK(s, cudaStreamBeginCapture(D.stream, cudaStreamCaptureModeThreadLocal));
+                D.chained = false;
                 bool ok = true;
                 for (int q = 0; q < gs && ok; q++) ok = launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1, true);
                 cudaGraph_t g = nullptr;
@@ -3457,6 +3617,7 @@ bool run_chunk(cem_sim *s, long n) {
                 CB2_CHECK(s, ei);
             }
             CB2_CHECK(s, cudaGraphLaunch(D.graph, D.stream));
+            D.chained = false;
             D.ring_count += gs;
             s->step += gs;
             it += gs;
@@ -4067,18 +4228,19 @@ int cemx_sizes(const cem_sim *s, long long *out, int n) {
                  (long long)(D.ring.n + D.acc.n) * 8;
         v[11] = bytes;
     }
-    // kernels per step: H and E, each over its fast and general blocks (or one
-    // fused kernel), SIBC when present, the probe pass
+    // kernels per step: H and E, each over its fast and general blocks (or one fused kernel)
     int upd = 4;
-    if (s->dev && s->dev->use_fused) upd = 1;
-    else if (s->dev)
+    if (s->dev) {
+        const Device &D = *s->dev;
         for (int u = 0; u < 2; u++) {
-            const Device &D = *s->dev;
+            if (u ? D.whole_e : D.whole_h) { upd--; continue; }
             upd -= space_blocks(D.sp[u][kFast]) == 0 || D.p1[u] <= D.p0[u];
             upd -= D.wl_start[u].empty() || D.wl_start[u].back() == 0;
-            upd += u == 1 && space_blocks(D.sp[u][kDebye]) > 0 && D.p1[u] > D.p0[u];
         }
-    v[12] = upd + 1 + (s->nsb ? 1 : 0);
+    }
+    // with the fused kernel also the surface impedance and the probes
+    if (s->dev && s->dev->use_fused) v[12] = 2 + (s->nsb ? 1 : 0);
+    else v[12] = upd + (s->nsb && s->dev && !s->dev->sibc_flagged ? 1 : 0);
     // point-components each update class covers per step (4 points per thread,
     // 3 components): H fast, H general, E fast, E general, E Debye; and the
     // Debye boxes' points (pole currents move for all of them)
