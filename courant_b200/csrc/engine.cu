@@ -148,7 +148,6 @@ struct StepArgs {
     // [H, E]: k ranges [zt[u][0], zt[u][1]) and [zt[u][2], zt[u][3]) (four-point groups) where the
     // lean kernels' rows reach into a z CPML slab and take its auxiliaries (empty: they never do)
     int zt[2][4];
-    // thread spaces last: batched kernels stage the arguments before them
     Space sp[2][4];          // [H, E][kFast, kGeneral, kAll, kDebye]
     int p0[2], p1[2];        // interior node planes of H and E
 };
@@ -668,10 +667,8 @@ __device__ __forceinline__ void h_points(const StepArgs &a, int i, int j, int k4
     if (any2) st4(a.psiH[C][1] + x2, s2);
 }
 
-// H component C on points k4 .. k4+3 of row (i, j) (segment [ks, ke)).
-// FAST: the block lies where no point has a CPML auxiliary (short path only,
-// fewer registers); the arithmetic is the same.
-template <int C, bool FAST>
+// H component C on points k4 .. k4+3 of row (i, j) (segment [ks, ke))
+template <int C>
 __device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r) {
     const int j = r.j, k4 = r.k4;
     const int m = j * a.g.sj + k4;
@@ -679,7 +676,7 @@ __device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r)
     const int nx = a.g.n[0], ny = a.g.n[1], nz = a.g.n[2];
     // derivative axes x and y need i < nx, j < ny (the row's own axis goes to n)
     const bool valid = r.act && (!(A1 == 0 || A2 == 0) || i < nx) && (!(A1 == 1 || A2 == 1) || j < ny);
-    const Where w = valid && !FAST ? h_where<C>(a, i, j, k4) : Where{-1, -1, make_int4(-1, -1, -1, -1), -1, false};
+    const Where w = valid ? h_where<C>(a, i, j, k4) : Where{-1, -1, make_int4(-1, -1, -1, -1), -1, false};
     const bool row = valid;
     const int q = i * (int)a.g.si + m;
     const float *E2 = a.E[A2];
@@ -918,9 +915,8 @@ __device__ __forceinline__ void e_points(const StepArgs &a, int i, int j, int k4
     e_four<C, P>(a, j, k4, q, ev, sub4(t1, t2), mv, own, w.jo4, J, sv, skip);
 }
 
-// E component C on points k4 .. k4+3 of row (i, j) (segment [ks, ke));
-// FAST as for h_vec: no CPML auxiliary and no Debye current in the block.
-template <int C, int P, bool FAST>
+// E component C on points k4 .. k4+3 of row (i, j) (segment [ks, ke))
+template <int C, int P>
 __device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r, const float2 sv, unsigned skip) {
     const int j = r.j, k4 = r.k4;
     const int m = j * a.g.sj + k4;
@@ -928,7 +924,7 @@ __device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r,
     const int nx = a.g.n[0], ny = a.g.n[1];
     // own axis: index < n; transverse axes: 1 <= index < n
     const bool valid = r.act && i < nx && (C == 0 || i >= 1) && (C == 1 ? j < ny : (j >= 1 && j < ny));
-    const Where w = valid && !FAST ? e_where<C, P>(a, i, j, k4) : Where{-1, -1, make_int4(-1, -1, -1, -1), -1, false};
+    const Where w = valid ? e_where<C, P>(a, i, j, k4) : Where{-1, -1, make_int4(-1, -1, -1, -1), -1, false};
     const bool row = valid;
     const int q = i * (int)a.g.si + m;
     const float *H2 = a.H[A2];
@@ -1255,9 +1251,9 @@ __global__ void __launch_bounds__(kBlock, CB2_H_MINBLOCKS) k_update_h(const Step
     const int comp = w.y % 3;
     const RowPos p = general_pos<0>(a, w.x, w.y / 3);
     chain_wait();
-    if (comp == 0) h_vec<0, false>(a, w.x, p);
-    else if (comp == 1) h_vec<1, false>(a, w.x, p);
-    else h_vec<2, false>(a, w.x, p);
+    if (comp == 0) h_vec<0>(a, w.x, p);
+    else if (comp == 1) h_vec<1>(a, w.x, p);
+    else h_vec<2>(a, w.x, p);
 }
 
 // E over the general blocks (no Debye poles)
@@ -1276,9 +1272,9 @@ __global__ void __launch_bounds__(kBlock, CB2_E_MINBLOCKS)
     const RowPos p = general_pos<1>(a, w.x, w.y / 3);
     chain_wait();
     const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
-    if (comp == 0) e_vec<0, 0, false>(a, w.x, p, sv, r.skip);
-    else if (comp == 1) e_vec<1, 0, false>(a, w.x, p, sv, r.skip);
-    else e_vec<2, 0, false>(a, w.x, p, sv, r.skip);
+    if (comp == 0) e_vec<0, 0>(a, w.x, p, sv, r.skip);
+    else if (comp == 1) e_vec<1, 0>(a, w.x, p, sv, r.skip);
+    else e_vec<2, 0>(a, w.x, p, sv, r.skip);
 }
 
 // All blocks of an update in one launch: the run's own work first, then the
@@ -1337,9 +1333,9 @@ __global__ void __launch_bounds__(kBlock, kWholeH) k_whole_h(const StepArgs a, c
     const int kind = whole_place<false>(a, l, (int)blockIdx.x - r.first, i, comp, p);
     chain_wait();
     if (kind == 2) {
-        if (comp == 0) h_vec<0, false>(a, i, p);
-        else if (comp == 1) h_vec<1, false>(a, i, p);
-        else h_vec<2, false>(a, i, p);
+        if (comp == 0) h_vec<0>(a, i, p);
+        else if (comp == 1) h_vec<1>(a, i, p);
+        else h_vec<2>(a, i, p);
     } else {
         if (comp == 0) h_lean<0>(a, i, p);
         else if (comp == 1) h_lean<1>(a, i, p);
@@ -1364,9 +1360,9 @@ __global__ void __launch_bounds__(kBlock, P > 8 ? 4 : B)
     chain_wait();
     const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
     if (kind == 2) {
-        if (comp == 0) e_vec<0, P, false>(a, i, p, sv, r.skip);
-        else if (comp == 1) e_vec<1, P, false>(a, i, p, sv, r.skip);
-        else e_vec<2, P, false>(a, i, p, sv, r.skip);
+        if (comp == 0) e_vec<0, P>(a, i, p, sv, r.skip);
+        else if (comp == 1) e_vec<1, P>(a, i, p, sv, r.skip);
+        else e_vec<2, P>(a, i, p, sv, r.skip);
     } else if (P > 0 && kind == 1) {
         if (comp == 0) e_debye<0, P>(a, i, p, sv, r.skip);
         else if (comp == 1) e_debye<1, P>(a, i, p, sv, r.skip);
@@ -1773,133 +1769,6 @@ __global__ void k_dft(const double *ring, int nslot, int first_e_slot, long long
     a[0] = re;
     a[1] = im;
 }
-
-// ------------------------------------------------------- batched kernels
-//
-// Several simulations on one device advance together: each launch walks a
-// work-list of blocks across all of them. A block stages its simulation's
-// arguments in shared memory and then runs exactly the per-simulation code
-// (h_vec, e_vec, sibc_edge, post_block), so every simulation computes the
-// same bits alone and in a batch.
-
-// this simulation's arguments (their first `bytes`), copied to shared memory
-// by the whole block
-template <class T>
-__device__ __forceinline__ const T &stage_args(const T *src, unsigned *buf, int bytes = sizeof(T)) {
-    static_assert(sizeof(T) % 4 == 0, "arguments copied as 4-byte words");
-    const unsigned *s = reinterpret_cast<const unsigned *>(src);
-    for (int q = threadIdx.x; q < bytes / 4; q += blockDim.x) buf[q] = s[q];
-    __syncthreads();
-    return *reinterpret_cast<const T *>(buf);
-}
-
-// the update kernels stage the arguments before the thread spaces; a thread
-// reads its position from the spaces in global memory
-constexpr int kStaged = (int)offsetof(StepArgs, sp);
-static_assert(kStaged % 4 == 0, "staged arguments end on a 4-byte boundary");
-
-// work entry: x simulation, y block of the plane (component = y % 3), z node plane
-// A batched update block walks kPerBlock consecutive work entries (x
-// member, y block of the plane incl. component, z node plane) and stages a
-// member's arguments only when the member changes: the arguments before the
-// thread spaces, the interior planes and the spaces it walks (the fast one,
-// or the general one and the one of all rectangles), each at its own offset,
-// so the buffer reads as the member's StepArgs.
-constexpr int kPerBlock = 4;
-
-template <int U, bool FAST>
-__device__ __forceinline__ void stage_member(const StepArgs *args, int x, unsigned *buf) {
-    __syncthreads();   // every thread is done with the previous member
-    const unsigned *s = reinterpret_cast<const unsigned *>(args + x);
-    for (int q = threadIdx.x; q < kStaged / 4; q += blockDim.x) buf[q] = s[q];
-    constexpr int sw = (int)(sizeof(Space) / 4);
-    const int c0 = FAST ? kFast : kGeneral;
-    for (int c = c0; c < (FAST ? kFast + 1 : kSpaces); c++) {
-        const int off = (int)((offsetof(StepArgs, sp) + (U * kSpaces + c) * sizeof(Space)) / 4);
-        for (int q = threadIdx.x; q < sw; q += blockDim.x) buf[off + q] = s[off + q];
-    }
-    constexpr int po = (int)(offsetof(StepArgs, p0) / 4);
-    if (threadIdx.x < 4) buf[po + threadIdx.x] = s[po + threadIdx.x];   // p0[2], p1[2]
-    __syncthreads();
-}
-
-// FAST: the members' fast rectangles (the lean kernels' code), else their general blocks
-template <bool FAST>
-__global__ void __launch_bounds__(kBlock, FAST ? CB2_HF_MINBLOCKS : CB2_H_MINBLOCKS)
-    k_batch_h(const StepArgs *args, const int4 *work, int n) {
-    static_assert(offsetof(StepArgs, p0) % 4 == 0 && offsetof(StepArgs, p1) == offsetof(StepArgs, p0) + 8, "p0, p1");
-    __shared__ unsigned buf[sizeof(StepArgs) / 4];
-    const StepArgs &a = *reinterpret_cast<const StepArgs *>(buf);
-    int staged = -1;
-    const int e1 = min(n, (int)(blockIdx.x + 1) * kPerBlock);
-    for (int e = blockIdx.x * kPerBlock; e < e1; e++) {
-        const int4 w = work[e];
-        if (w.x != staged) {
-            stage_member<0, FAST>(args, w.x, buf);
-            staged = w.x;
-        }
-        const RowPos r = FAST ? space_pos(a.sp[0][kFast], w.y / 3) : general_pos<0>(a, w.z, w.y / 3);
-        const int comp = w.y % 3;
-        if (FAST) {
-            if (comp == 0) h_lean<0>(a, w.z, r);
-            else if (comp == 1) h_lean<1>(a, w.z, r);
-            else h_lean<2>(a, w.z, r);
-        } else {
-            if (comp == 0) h_vec<0, false>(a, w.z, r);
-            else if (comp == 1) h_vec<1, false>(a, w.z, r);
-            else h_vec<2, false>(a, w.z, r);
-        }
-    }
-}
-
-template <int P, bool FAST>
-__global__ void __launch_bounds__(kBlock, FAST ? CB2_EF_MINBLOCKS : CB2_E_MINBLOCKS)
-    k_batch_e(const StepArgs *args, const int4 *work, int n) {
-    __shared__ unsigned buf[sizeof(StepArgs) / 4];
-    const StepArgs &a = *reinterpret_cast<const StepArgs *>(buf);
-    int staged = -1;
-    const int e1 = min(n, (int)(blockIdx.x + 1) * kPerBlock);
-    for (int e = blockIdx.x * kPerBlock; e < e1; e++) {
-        const int4 w = work[e];
-        if (w.x != staged) {
-            stage_member<1, FAST>(args, w.x, buf);
-            staged = w.x;
-        }
-        // general entries: w.w = 1 for blocks of the Debye space (general code, the same bits)
-        const RowPos r = FAST ? space_pos(a.sp[1][kFast], w.y / 3)
-                              : (w.w ? space_pos(a.sp[1][kDebye], w.y / 3) : general_pos<1>(a, w.z, w.y / 3));
-        const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
-        const int comp = w.y % 3;
-        if (FAST) {
-            if (comp == 0) e_lean<0>(a, w.z, r, sv, 0u);
-            else if (comp == 1) e_lean<1>(a, w.z, r, sv, 0u);
-            else e_lean<2>(a, w.z, r, sv, 0u);
-        } else {
-            if (comp == 0) e_vec<0, P, false>(a, w.z, r, sv, 0u);
-            else if (comp == 1) e_vec<1, P, false>(a, w.z, r, sv, 0u);
-            else e_vec<2, P, false>(a, w.z, r, sv, 0u);
-        }
-    }
-}
-
-using BEKernel = void (*)(const StepArgs *, const int4 *, int);
-#define CB2_BE(p) k_batch_e<p, false>,
-const BEKernel kBEKernels[] = {CB2_BE(0) CB2_BE(1) CB2_BE(2) CB2_BE(3) CB2_BE(4) CB2_BE(5) CB2_BE(6) CB2_BE(7) CB2_BE(8)
-                                   CB2_BE(9) CB2_BE(10) CB2_BE(11) CB2_BE(12) CB2_BE(13) CB2_BE(14) CB2_BE(15)
-                                       CB2_BE(16)};
-#undef CB2_BE
-
-// work entry: x simulation, y first edge of the block
-__global__ void __launch_bounds__(kBlock) k_batch_sibc(const SibcArgs *args, const int2 *work) {
-    __shared__ unsigned buf[sizeof(SibcArgs) / 4];
-    const int2 w = work[blockIdx.x];
-    const SibcArgs &a = stage_args(args + w.x, buf);
-    const int e = w.y + threadIdx.x;
-    if (e < a.ns) sibc_edge(a, e);
-}
-
-// one block per simulation
-__global__ void __launch_bounds__(kPostThreads) k_batch_post(const PostArgs *args) { post_block(args[blockIdx.x]); }
 
 // ----------------------------------------------------------------- energy
 
@@ -3633,13 +3502,14 @@ bool run_chunk(cem_sim *s, long n) {
 
 // n whole steps: in runs with the separate kernels, one by one with the fused
 // kernel and while kernels are timed one by one
-bool run_steps(cem_sim *s, long n) {
+bool run_steps(cem_sim *s, long n, long *launches = nullptr) {
     Device &D = *s->dev;
     const bool runs = !D.use_fused && !g_timer;
     while (n > 0) {
         if (D.ring_count == kRing && !flush_dft(s)) return false;
         const long k = runs ? std::min<long>(n, std::min(D.run_steps, kRing - D.ring_count)) : 1;
         if (runs ? !run_chunk(s, k) : !launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1)) return false;
+        if (launches) *launches += runs ? k / D.graph_steps + k % D.graph_steps + 2 : 1;   // a graph counts once, as does a step
         n -= k;
     }
     CB2_CHECK(s, cudaGetLastError());
@@ -3938,254 +3808,41 @@ bool profiled_steps(cem_sim *s, long n, double *kernel_ms, long *launches) {
 
 // ------------------------------------------------------------------ batches
 
-// Simulations advanced together on one device (cemx_batch_*). Each member
-// keeps its own device state; the batch holds device copies of the members'
-// kernel arguments and the work-lists of the batched kernels, rebuilt when
-// the set of members still short of their step budget changes, and a CUDA
-// graph of `chunk` batched steps, captured once per work-list.
+// Simulations advanced together on one device (cemx_batch_*). Each member keeps
+// its own device state and steps on its own stream with its own replayed
+// graphs; the GPU runs the members' launches side by side, so small members
+// fill what one of them leaves idle, a change of members costs nothing, and a
+// member at the end of its budget holds none of the others up. (Work-lists of
+// all members' blocks in common launches, in lockstep: 189 us per step for
+// eight boards of 5e4-8e5 cells, 2.6 M in all.)
 struct cemx_batch {
     struct Member {
         cem_sim *s;
         long left;   // steps still to run
     };
     int device = 0;
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr;           // forks to the members' streams and joins them
     std::vector<Member> members;
-    std::vector<int> active;                 // members in the work-lists
-    DevBuf<StepArgs> args;
-    DevBuf<SibcArgs> sargs;
-    DevBuf<PostArgs> pargs;
-    DevBuf<int4> work_h[2];                  // H blocks: fast, general
-    DevBuf<int4> work_ef;                    // E fast blocks of all members
-    std::map<int, DevBuf<int4>> work_e;      // E general blocks, by pole count
-    DevBuf<int2> work_s;
-    size_t nh[2] = {0, 0}, nef = 0, ns = 0;
-    std::map<int, size_t> ne;
-    bool dirty = true;
-    int order = 0;                           // work-list order: 0 member-major, 1 plane-interleaved
-    int chunk = 256;                         // steps between the host's checks of budgets and rings
-    bool tune = false, tuned = false;
-    cudaGraphExec_t graph = nullptr;
-    int graph_steps = 0;
+    bool tune = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaEvent_t tev0 = nullptr, tev1 = nullptr;   // timing of the tuning chunks
-    cudaStream_t side = nullptr;             // general blocks beside the fast ones; SIBC beside the probes
-    bool sibc_beside = false;                // no member's probes read a SIBC edge
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaEvent_t join = nullptr;
     double last_ms = 0;
     long last_steps = 0, last_launches = 0;
 };
 
 namespace {
 
-bool batch_fail(const char *what, cudaError_t e) {
+int batch_fail(const char *what, cudaError_t e) {
     char msg[256];
     std::snprintf(msg, sizeof msg, "batch: CUDA %s: %s", what, cudaGetErrorString(e));
     set_error(msg);
-    return false;
+    return -1;
 }
 #define CB2_BCHECK(call)                                   \
     do {                                                   \
         cudaError_t e_ = (call);                           \
         if (e_ != cudaSuccess) return batch_fail(#call, e_); \
     } while (0)
-
-template <class T>
-bool batch_upload(DevBuf<T> &b, const std::vector<T> &v) {
-    if (b.p) { cudaFree(b.p); b.p = nullptr; b.n = 0; }
-    if (v.empty()) return true;
-    CB2_BCHECK(cudaMalloc(&b.p, v.size() * sizeof(T)));
-    b.n = v.size();
-    CB2_BCHECK(cudaMemcpy(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return true;
-}
-
-void batch_drop_graph(cemx_batch *b) {
-    if (b->graph) cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-    b->graph_steps = 0;
-}
-
-// work-lists of the members still short of their budget
-bool batch_rebuild(cemx_batch *b) {
-    batch_drop_graph(b);
-    b->active.clear();
-    for (int m = 0; m < (int)b->members.size(); m++)
-        if (b->members[m].left > 0) b->active.push_back(m);
-    std::vector<StepArgs> sa;
-    std::vector<SibcArgs> sb;
-    std::vector<PostArgs> pa;
-    std::vector<int4> wh[2], wef;
-    std::map<int, std::vector<int4>> we;
-    std::vector<int2> ws;
-    int maxp = 0;
-    for (int x = 0; x < (int)b->active.size(); x++) {
-        cem_sim *s = b->members[b->active[x]].s;
-        Device &D = *s->dev;
-        sa.push_back(D.sa[D.cur]);
-        sb.push_back(D.sb[D.cur]);
-        pa.push_back(D.pa[D.cur]);
-        pa.back().advance = 1;
-        maxp = std::max(maxp, s->n[0] + 1);
-        for (int e0 = 0; e0 < s->nsb; e0 += kBlock) ws.push_back(make_int2(x, e0));
-    }
-    // H over planes 0..nx, E over 0..nx-1; member-major, or plane by plane
-    // across members; fast and general blocks as the member's own lists
-    auto add_plane = [&](int x, int i) {
-        cem_sim *s = b->members[b->active[x]].s;
-        const Device &D = *s->dev;
-        // interior planes: the fast and the general space; elsewhere every rectangle
-        auto blocks = [&](int u, int c) { return 3 * space_blocks(D.sp[u][c]); };
-        const bool ih = i >= D.p0[0] && i < D.p1[0], ie = i >= D.p0[1] && i < D.p1[1];
-        if (i <= s->n[0]) {
-            for (int bx = 0; ih && bx < blocks(0, kFast); bx++) wh[0].push_back(make_int4(x, bx, i, 0));
-            for (int bx = 0; bx < blocks(0, ih ? kGeneral : kAll); bx++) wh[1].push_back(make_int4(x, bx, i, 0));
-        }
-        if (i < s->n[0]) {
-            for (int bx = 0; ie && bx < blocks(1, kFast); bx++) wef.push_back(make_int4(x, bx, i, 0));
-            for (int bx = 0; bx < blocks(1, ie ? kGeneral : kAll); bx++)
-                we[s->npole].push_back(make_int4(x, bx, i, 0));
-            for (int bx = 0; ie && bx < blocks(1, kDebye); bx++) we[s->npole].push_back(make_int4(x, bx, i, 1));
-        }
-    };
-    if (b->order == 0) {
-        for (int x = 0; x < (int)b->active.size(); x++)
-            for (int i = 0; i <= b->members[b->active[x]].s->n[0]; i++) add_plane(x, i);
-    } else {
-        for (int i = 0; i < maxp; i++)
-            for (int x = 0; x < (int)b->active.size(); x++) add_plane(x, i);
-    }
-    if (!batch_upload(b->args, sa) || !batch_upload(b->sargs, sb) || !batch_upload(b->pargs, pa) ||
-        !batch_upload(b->work_h[0], wh[0]) || !batch_upload(b->work_h[1], wh[1]) || !batch_upload(b->work_ef, wef) ||
-        !batch_upload(b->work_s, ws))
-        return false;
-    b->work_e.clear();
-    b->ne.clear();
-    for (auto &kv : we) {
-        if (!batch_upload(b->work_e[kv.first], kv.second)) return false;
-        b->ne[kv.first] = kv.second.size();
-    }
-    b->sibc_beside = true;
-    for (int m : b->active) b->sibc_beside = b->sibc_beside && b->members[m].s->dev->post_beside_sibc;
-    b->nh[0] = wh[0].size();
-    b->nh[1] = wh[1].size();
-    b->nef = wef.size();
-    b->ns = ws.size();
-    b->dirty = false;
-    return true;
-}
-
-// blocks of a batched update launch over n work entries
-unsigned blocks_for(size_t n) { return (unsigned)((n + kPerBlock - 1) / kPerBlock); }
-
-// one batched time step: H (fast, general blocks), E (fast blocks; general
-// blocks one launch per pole count), SIBC, probes
-int batch_step(cemx_batch *b) {
-    int launches = 0;
-    // general blocks on the side stream beside the fast ones, joined before the next phase
-    auto fork = [&]() {
-        cudaEventRecord(b->fork, b->stream);
-        cudaStreamWaitEvent(b->side, b->fork, 0);
-    };
-    auto join = [&]() {
-        cudaEventRecord(b->join, b->side);
-        cudaStreamWaitEvent(b->stream, b->join, 0);
-    };
-    if (b->nh[1]) {
-        fork();
-        k_batch_h<false><<<blocks_for(b->nh[1]), kBlock, 0, b->side>>>(b->args.p, b->work_h[1].p, (int)b->nh[1]);
-        launches++;
-    }
-    if (b->nh[0]) {
-        k_batch_h<true><<<blocks_for(b->nh[0]), kBlock, 0, b->stream>>>(b->args.p, b->work_h[0].p, (int)b->nh[0]);
-        launches++;
-    }
-    if (b->nh[1]) join();
-    bool side = false;
-    for (auto &kv : b->ne)
-        if (kv.second) {
-            if (!side) fork();
-            side = true;
-            kBEKernels[kv.first]<<<blocks_for(kv.second), kBlock, 0, b->side>>>(b->args.p, b->work_e[kv.first].p,
-                                                                               (int)kv.second);
-            launches++;
-        }
-    if (b->nef) {
-        k_batch_e<0, true><<<blocks_for(b->nef), kBlock, 0, b->stream>>>(b->args.p, b->work_ef.p, (int)b->nef);
-        launches++;
-    }
-    if (side) join();
-    const bool beside = b->ns && b->sibc_beside;
-    if (beside) fork();
-    if (b->ns) {
-        k_batch_sibc<<<(unsigned)b->ns, kBlock, 0, beside ? b->side : b->stream>>>(b->sargs.p, b->work_s.p);
-        launches++;
-    }
-    k_batch_post<<<(unsigned)b->active.size(), kPostThreads, 0, b->stream>>>(b->pargs.p);
-    if (beside) join();
-    return launches + 1;
-}
-
-// n batched steps, through the cached graph when n is the chunk length
-// n batched steps: whole runs of kBatchGraph steps replay the graph captured
-// for the current composition (captured once per composition, so a change of
-// members costs one short capture), the rest go step by step
-constexpr int kBatchGraph = 16;
-
-bool batch_launch(cemx_batch *b, int n) {
-    if (n >= kBatchGraph) {
-        if (!b->graph || b->graph_steps != kBatchGraph) {
-            batch_drop_graph(b);
-            cudaGraph_t g = nullptr;
-            CB2_BCHECK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-            for (int q = 0; q < kBatchGraph; q++) batch_step(b);
-            CB2_BCHECK(cudaStreamEndCapture(b->stream, &g));
-            const cudaError_t e = cudaGraphInstantiate(&b->graph, g, 0);
-            cudaGraphDestroy(g);
-            if (e != cudaSuccess) { b->graph = nullptr; return batch_fail("cudaGraphInstantiate", e); }
-            b->graph_steps = kBatchGraph;
-        }
-        for (int q = 0; q + kBatchGraph <= n; q += kBatchGraph) {
-            CB2_BCHECK(cudaGraphLaunch(b->graph, b->stream));
-            b->last_launches += 1;
-        }
-    }
-    for (int q = n / kBatchGraph * kBatchGraph; q < n; q++) b->last_launches += batch_step(b);
-    CB2_BCHECK(cudaGetLastError());
-    return true;
-}
-
-// Per-composition choice of chunk length and work-list order, found by timing
-// real batched steps once and kept for the process.
-std::mutex g_tune_mu;
-std::map<std::string, std::pair<int, int>> g_tuned;
-
-// cache-file key of a batch composition: FNV-1a hash of its signature and the member count
-std::string batch_key(const std::string &sig) {
-    unsigned long long h = 1469598103934665603ull;
-    int members = 0;
-    for (char c : sig) {
-        h = (h ^ (unsigned char)c) * 1099511628211ull;
-        members += c == ';';
-    }
-    char k[64];
-    std::snprintf(k, sizeof k, "batch/%016llx/%d", h, members);
-    return k;
-}
-
-std::string batch_signature(const cemx_batch *b) {
-    std::vector<std::string> v;
-    for (int m : b->active) {
-        const cem_sim *s = b->members[m].s;
-        char k[96];
-        std::snprintf(k, sizeof k, "%dx%dx%d/p%d/s%d", s->n[0], s->n[1], s->n[2], s->npole, s->nsb);
-        v.push_back(k);
-    }
-    std::sort(v.begin(), v.end());
-    std::string sig;
-    for (auto &x : v) sig += x + ";";
-    return sig;
-}
 
 }  // namespace
 
@@ -4340,9 +3997,6 @@ cemx_batch *cemx_batch_create(int device) {
     b->device = device;
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
-        cudaEventCreate(&b->tev0) != cudaSuccess || cudaEventCreate(&b->tev1) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming) != cudaSuccess) {
         set_error("batch: cannot create its stream");
         cemx_batch_destroy(b);
@@ -4355,15 +4009,9 @@ void cemx_batch_destroy(cemx_batch *b) {
     if (!b) return;
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
-    batch_drop_graph(b);
-    b->work_e.clear();
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
-    if (b->tev0) cudaEventDestroy(b->tev0);
-    if (b->tev1) cudaEventDestroy(b->tev1);
-    if (b->fork) cudaEventDestroy(b->fork);
     if (b->join) cudaEventDestroy(b->join);
-    if (b->side) cudaStreamDestroy(b->side);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
 }
@@ -4381,7 +4029,6 @@ int cemx_batch_add(cemx_batch *b, cem_sim *s, long steps) {
     if (!ok) return -1;
     if (s->dev->device != b->device) { set_error("batch: simulation lives on another device"); return -1; }
     b->members.push_back({s, steps});
-    b->dirty = true;
     return (int)b->members.size() - 1;
 }
 
@@ -4392,7 +4039,6 @@ int cemx_batch_remove(cemx_batch *b, cem_sim *s) {
             cudaSetDevice(b->device);
             cudaStreamSynchronize(b->stream);
             b->members.erase(b->members.begin() + m);
-            b->dirty = true;
             return 0;
         }
     set_error("batch: not a member");
@@ -4409,8 +4055,7 @@ long cemx_batch_left(const cemx_batch *b, const cem_sim *s) {
 int cemx_batch_tune(cemx_batch *b, int on) {
     if (!b) return -1;
     const int prev = b->tune ? 1 : 0;
-    b->tune = on != 0;
-    b->tuned = false;
+    b->tune = on != 0;   // nothing left to choose: kept for callers that set it
     return prev;
 }
 
@@ -4426,97 +4071,24 @@ int cemx_batch_run(cemx_batch *b, long max_steps) {
     b->last_ms = 0;
     b->last_steps = 0;
     b->last_launches = 0;
-    if (cudaEventRecord(b->ev0, b->stream) != cudaSuccess) { set_error("batch: event"); return -1; }
-    long done = 0;
-    while (done < max_steps) {
-        if (b->dirty && !batch_rebuild(b)) return -1;
-        if (b->active.empty()) break;
-        if (b->tune && !b->tuned) {
-            // chunk length and work-list order: cached per composition, else timed on real steps
-            const std::string sig = batch_signature(b);
-            std::pair<int, int> best{b->chunk, b->order};
-            bool cached = false;
-            {   // this process's choices, then the launch-shape cache file
-                std::lock_guard<std::mutex> lock(g_tune_mu);
-                auto it = g_tuned.find(sig);
-                if (it != g_tuned.end()) { best = it->second; cached = true; }
-            }
-            if (!cached) {
-                std::lock_guard<std::mutex> lock(g_shape_mu);
-                load_shapes();
-                auto it = g_shapes.find(batch_key(sig));
-                if (it != g_shapes.end()) { best = {(int)it->second[0], (int)it->second[1]}; cached = true; }
-            }
-            if (!cached) {
-                long minleft = max_steps - done;
-                for (int m : b->active) minleft = std::min(minleft, b->members[m].left);
-                float best_ms = 1e30f;
-                for (int order = 0; order < 2; order++)
-                    for (int ch : {64}) {
-                        if (2 * ch > minleft) continue;   // one warm-up and one timed chunk
-                        if (b->order != order) { b->order = order; if (!batch_rebuild(b)) return -1; }
-                        b->chunk = ch;
-                        float ms = 0;
-                        for (int rep = 0; rep < 2; rep++) {
-                            for (int m : b->active) {
-                                Device &D = *b->members[m].s->dev;
-                                if (D.ring_count + ch > kRing) {
-                                    const cudaError_t e = cudaStreamSynchronize(b->stream);
-                                    if (e != cudaSuccess) { batch_fail("cudaStreamSynchronize", e); return -1; }
-                                    if (!flush_dft(b->members[m].s) || cudaStreamSynchronize(D.stream) != cudaSuccess)
-                                        return -1;
-                                }
-                            }
-                            cudaError_t e = cudaEventRecord(b->tev0, b->stream);
-                            if (e != cudaSuccess) { batch_fail("cudaEventRecord", e); return -1; }
-                            if (!batch_launch(b, ch)) return -1;
-                            if ((e = cudaEventRecord(b->tev1, b->stream)) != cudaSuccess ||
-                                (e = cudaEventSynchronize(b->tev1)) != cudaSuccess ||
-                                (e = cudaEventElapsedTime(&ms, b->tev0, b->tev1)) != cudaSuccess)
-                            { batch_fail("tuning timer", e); return -1; }
-                            for (int m : b->active) {
-                                b->members[m].s->step += ch;
-                                b->members[m].s->dev->ring_count += ch;
-                                b->members[m].left -= ch;
-                            }
-                            done += ch;
-                            minleft -= ch;
-                            b->last_steps += ch;
-                        }
-                        if (ms / ch < best_ms) { best_ms = ms / ch; best = {ch, order}; }
-                    }
-                {
-                    std::lock_guard<std::mutex> lock(g_tune_mu);
-                    g_tuned[sig] = best;
-                }
-                std::lock_guard<std::mutex> lock(g_shape_mu);
-                store_shape(batch_key(sig), {(double)best.first, (double)best.second, 0.0, best_ms});
-            }
-            b->tuned = true;
-            if (b->order != best.second) { b->order = best.second; b->dirty = true; }
-            for (int m : b->active)
-                if (b->members[m].left <= 0) b->dirty = true;
-            continue;
+    // members take turns of kTurn steps at most, so that the host feeds all their streams
+    constexpr long kTurn = 256;
+    CB2_BCHECK(cudaEventRecord(b->ev0, b->stream));
+    for (cem_sim *s : touched) CB2_BCHECK(cudaStreamWaitEvent(s->dev->stream, b->ev0, 0));
+    for (long done = 0, more = 1; done < max_steps && more; done += kTurn) {
+        more = 0;
+        for (auto &m : b->members) {
+            if (m.left <= 0) continue;
+            const long n = std::min({m.left, kTurn, max_steps - done});
+            if (!run_steps(m.s, n, &b->last_launches)) return -1;
+            m.left -= n;
+            more += m.left > 0;
+            b->last_steps = std::max(b->last_steps, done + n);
         }
-        long n = std::min<long>(b->chunk, max_steps - done);
-        for (int m : b->active) n = std::min(n, b->members[m].left);
-        for (int m : b->active) {
-            Device &D = *b->members[m].s->dev;
-            if (D.ring_count + n > kRing) {   // room in the sample ring for n rows
-                cudaStreamSynchronize(b->stream);
-                if (!flush_dft(b->members[m].s) || cudaStreamSynchronize(D.stream) != cudaSuccess) return -1;
-            }
-        }
-        if (!batch_launch(b, (int)n)) return -1;
-        for (int m : b->active) {
-            cemx_batch::Member &mb = b->members[m];
-            mb.s->step += n;
-            mb.s->dev->ring_count += n;
-            mb.left -= n;
-            if (mb.left == 0) b->dirty = true;
-        }
-        done += n;
-        b->last_steps += n;
+    }
+    for (cem_sim *s : touched) {
+        CB2_BCHECK(cudaEventRecord(b->join, s->dev->stream));
+        CB2_BCHECK(cudaStreamWaitEvent(b->stream, b->join, 0));
     }
     float ms = 0;
     if (cudaEventRecord(b->ev1, b->stream) != cudaSuccess || cudaEventSynchronize(b->ev1) != cudaSuccess ||
@@ -4534,8 +4106,8 @@ int cemx_batch_run(cemx_batch *b, long max_steps) {
 
 int cemx_batch_stats(const cemx_batch *b, double *out, int n) {
     if (!b) return -1;
-    const double v[6] = {b->last_ms, (double)b->last_steps, (double)b->last_launches, (double)kBatchGraph,
-                         (double)b->order, (double)b->members.size()};
+    const double v[6] = {b->last_ms, (double)b->last_steps, (double)b->last_launches, 32.0, 0.0,
+                         (double)b->members.size()};
     for (int q = 0; q < n && q < 6; q++) out[q] = v[q];
     return 0;
 }
