@@ -113,7 +113,6 @@ struct Space {
     int n;
     int ks[kMaxRects], ke[kMaxRects], js[kMaxRects];
     int t0[kMaxRects + 1];                  // t0[n]: threads of the space
-    unsigned long long magic[kMaxRects];    // row in its rectangle of thread t - t0: ((t - t0) * magic) >> 40
 };
 // E only: kDebye, the interior rectangles that meet a Debye box but no CPML
 // slab (the lean Debye kernel's space; general otherwise).
@@ -148,7 +147,7 @@ struct StepArgs {
     // [H, E]: k ranges [zt[u][0], zt[u][1]) and [zt[u][2], zt[u][3]) (four-point groups) where the
     // lean kernels' rows reach into a z CPML slab and take its auxiliaries (empty: they never do)
     int zt[2][4];
-    Space sp[2][4];          // [H, E][kFast, kGeneral, kAll, kDebye]
+    const uint2 *item[2][4];   // [H, E][kFast, kGeneral, kAll, kDebye]: the spaces' threads (RowPos)
     int p0[2], p1[2];        // interior node planes of H and E
 };
 
@@ -540,29 +539,28 @@ __device__ __forceinline__ float4 prev_k(const float4 &v, const float *p, bool n
 }
 
 // Position of this thread (block b of a space): row j and first point k4 of
-// its four, the k range [ks, ke) of its rectangle, whether it has work
-// (`act`; a thread past the end takes the last thread's position) and whether
-// the next lane holds the next four points of the same row (`cont`).
+// its four, whether it has work (`act`; a thread past the end takes the last
+// thread's position), whether the next lane holds the next four points of the
+// same row (`cont`), whether the previous lane does not hold the previous four
+// (`first`) and whether the four lie in a z tail (StepArgs::zt). One word pair
+// per thread of the space from a table, the same for every plane: finding the
+// rectangle and dividing by its width took 60-80 of a thread's 300 instructions
+// and a chain of indexed constant loads.
 struct RowPos {
-    int j, k4, ks, ke;
-    bool act, cont;
+    int j, k4;
+    bool act, cont, first, tail;
 };
+constexpr unsigned kItemAct = 1u << 28, kItemCont = 1u << 29, kItemFirst = 1u << 30, kItemTail = 1u << 31;
 
-__device__ __forceinline__ RowPos space_pos(const Space &sp, int b) {
-    const int t = b * kBlock + threadIdx.x, nt = sp.t0[sp.n];
+__device__ __forceinline__ RowPos space_pos(const uint2 *item, int b) {
+    const uint2 w = __ldg(item + (size_t)b * kBlock + threadIdx.x);
     RowPos r;
-    r.act = t < nt;
-    const int tc = r.act ? t : nt - 1;
-    int q = 0;
-    while (q + 1 < sp.n && tc >= sp.t0[q + 1]) q++;
-    const int tl = tc - sp.t0[q];
-    r.ks = sp.ks[q];
-    r.ke = sp.ke[q];
-    const int nk4 = (r.ke - r.ks) >> 2;
-    const int row = (int)(((unsigned long long)tl * sp.magic[q]) >> 40);
-    r.j = sp.js[q] + row;
-    r.k4 = r.ks + 4 * (tl - row * nk4);
-    r.cont = (threadIdx.x & 31) != 31 && r.k4 + 4 < r.ke && t + 1 < nt;
+    r.j = (int)w.x;
+    r.k4 = (int)(w.y << 2 & 0x3fffffffu);
+    r.act = w.y & kItemAct;
+    r.cont = w.y & kItemCont;
+    r.first = w.y & kItemFirst;
+    r.tail = w.y & kItemTail;
     return r;
 }
 
@@ -693,7 +691,7 @@ __device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r)
     }
     // the next lane holds the next four points only if it is in the same run and loaded them
     const bool nb = __shfl_down_sync(0xffffffffu, row, 1);
-    const bool edge = (threadIdx.x & 31) == 31 || k4 + 4 >= r.ke || !nb;
+    const bool edge = !r.cont || !nb;
     if (A1 == 2) e2n = next_k(e2, E2 + q, row && k4 + 4 <= nz, edge);
     if (A2 == 2) e1n = next_k(e1, E1 + q, row && k4 + 4 <= nz, edge);
     if (!row) return;
@@ -943,16 +941,11 @@ __device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r,
     }
     // the previous lane holds the previous four points only if it is in the same run and loaded them
     const bool pb = __shfl_up_sync(0xffffffffu, row, 1);
-    const bool edge = (threadIdx.x & 31) == 0 || k4 == r.ks || !pb;
+    const bool edge = r.first || !pb;
     if (A1 == 2) h2m = prev_k(h2, H2 + q, row && k4 > 0, edge);
     if (A2 == 2) h1m = prev_k(h1, H1 + q, row && k4 > 0, edge);
     if (!row) return;
     e_points<C, P>(a, i, j, k4, q, w, h2, h2m, h1, h1m, ev, mv, sv, skip);
-}
-
-// whether the group at k4 of a lean kernel's row lies in a z tail (StepArgs::zt)
-__device__ __forceinline__ bool in_ztail(const int (&zt)[4], int k4) {
-    return (k4 >= zt[0] && k4 < zt[1]) || (k4 >= zt[2] && k4 < zt[3]);
 }
 
 // Where of a z-tail group: lean rows lie on interior planes outside the y
@@ -990,7 +983,7 @@ __device__ __forceinline__ void h_lean(const StepArgs &a, int i, const RowPos &p
     if (A1 == 2) e2n = next_k(e2, E2 + q, row && k4 + 4 <= nz, !p.cont);
     if (A2 == 2) e1n = next_k(e1, E1 + q, row && k4 + 4 <= nz, !p.cont);
     if (!row) return;
-    if (kz && in_ztail(a.zt[0], k4)) {
+    if (kz && p.tail) {
         h_points<C>(a, i, j, k4, H + q, ztail_where(a.pml[2].plane_h, k4), e2, e2n, e1, e1n, h);
         return;
     }
@@ -1035,11 +1028,10 @@ __device__ __forceinline__ void e_lean(const StepArgs &a, int i, const RowPos &p
         if (A2 != 2) h1m = ld4(H1 + q - stride_of<A2>(a));
     }
     // the previous lane holds the previous four points unless this lane starts a warp or a row
-    const bool first = (threadIdx.x & 31) == 0 || k4 == p.ks;
-    if (A1 == 2) h2m = prev_k(h2, H2 + q, row && k4 > 0, first);
-    if (A2 == 2) h1m = prev_k(h1, H1 + q, row && k4 > 0, first);
+    if (A1 == 2) h2m = prev_k(h2, H2 + q, row && k4 > 0, p.first);
+    if (A2 == 2) h1m = prev_k(h1, H1 + q, row && k4 > 0, p.first);
     if (!row) return;
-    if (kz && in_ztail(a.zt[1], k4)) {
+    if (kz && p.tail) {
         e_points<C, 0>(a, i, j, k4, q, ztail_where(a.pml[2].plane_e, k4), h2, h2m, h1, h1m, ev, mv, sv, skip);
         return;
     }
@@ -1088,12 +1080,11 @@ __device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &
     }
 #pragma unroll
     for (int pp = 0; pp < P; pp++) J[pp] = jo4 >= 0 ? ld4(Jc + jaddr(P, jvol, pp, jo4)) : z4;
-    const bool first = (threadIdx.x & 31) == 0 || k4 == p.ks;
-    if (A1 == 2) h2m = prev_k(h2, H2 + q, row && k4 > 0, first);
-    if (A2 == 2) h1m = prev_k(h1, H1 + q, row && k4 > 0, first);
+    if (A1 == 2) h2m = prev_k(h2, H2 + q, row && k4 > 0, p.first);
+    if (A2 == 2) h1m = prev_k(h1, H1 + q, row && k4 > 0, p.first);
     if (!row) return;
     // a z tail above the box (tails exist only where no box reaches a z slab)
-    if ((A1 == 2 || A2 == 2) && in_ztail(a.zt[1], k4)) {
+    if (kz && p.tail) {
         e_points<C, 0>(a, i, j, k4, q, ztail_where(a.pml[2].plane_e, k4), h2, h2m, h1, h1m, ev, mv, sv, skip);
         return;
     }
@@ -1205,7 +1196,7 @@ __global__ void __launch_bounds__(kBlock, CB2_HF_MINBLOCKS) k_update_h_fast(cons
         return;
     }
     const int comp = blockIdx.x % 3;
-    const RowPos p = space_pos(a.sp[0][kFast], blockIdx.x / 3);
+    const RowPos p = space_pos(a.item[0][kFast], blockIdx.x / 3);
     chain_wait();
     const int i = i0 + blockIdx.y;
     if (comp == 0) h_lean<0>(a, i, p);
@@ -1222,7 +1213,7 @@ __global__ void __launch_bounds__(kBlock, CB2_EF_MINBLOCKS) k_update_e_fast(cons
         return;
     }
     const int comp = blockIdx.x % 3;
-    const RowPos p = space_pos(a.sp[1][kFast], blockIdx.x / 3);
+    const RowPos p = space_pos(a.item[1][kFast], blockIdx.x / 3);
     chain_wait();
     const int i = i0 + (int)(gridDim.y - 1 - blockIdx.y);   // E begins where H ended, on what L2 still holds
     const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
@@ -1235,7 +1226,7 @@ __global__ void __launch_bounds__(kBlock, CB2_EF_MINBLOCKS) k_update_e_fast(cons
 // interior node plane i, all rectangles on the others
 template <int U>
 __device__ __forceinline__ RowPos general_pos(const StepArgs &a, int i, int b) {
-    return i >= a.p0[U] && i < a.p1[U] ? space_pos(a.sp[U][kGeneral], b) : space_pos(a.sp[U][kAll], b);
+    return space_pos(a.item[U][i >= a.p0[U] && i < a.p1[U] ? kGeneral : kAll], b);
 }
 
 // Work entry of the general blocks: x node plane, y block of the plane's
@@ -1312,7 +1303,7 @@ __device__ __forceinline__ int whole_place(const StepArgs &a, const Whole &l, in
     const bool deb = x < l.nd;
     const int y = deb ? x : x - l.nd;
     comp = y % 3;
-    p = space_pos(a.sp[E ? 1 : 0][deb ? kDebye : kFast], y / 3);
+    p = space_pos(a.item[E ? 1 : 0][deb ? kDebye : kFast], y / 3);
     return deb ? 1 : 0;
 }
 
@@ -1883,6 +1874,7 @@ struct Device {
     // (entries: node plane, block of the plane's general space incl.
     // component) in plane order; wl_start[u][i] is the first entry of plane i.
     Space sp[2][kSpaces]{};
+    DevBuf<uint2> item[2][kSpaces];
     int p0[2] = {0, 0}, p1[2] = {0, 0};
     int zt[2][4] = {};       // z CPML groups the lean kernels' rows reach (StepArgs::zt)
     DevBuf<int2> wl[2];
@@ -2055,6 +2047,14 @@ template <class T>
 bool dev_upload(cem_sim *s, DevBuf<T> &b, const std::vector<T> &v) {
     if (!dev_alloc(s, b, v.size())) return false;
     return h2d(s, b.p, v.data(), v.size() * sizeof(T));
+}
+
+// the same into a buffer that may hold an older table (of launches that have ended)
+template <class T>
+bool dev_renew(cem_sim *s, DevBuf<T> &b, const std::vector<T> &v) {
+    if (b.p) CB2_CHECK(s, cudaFree(b.p));
+    b.p = nullptr;
+    return dev_upload(s, b, v);
 }
 
 // length of a per-axis array of n cells / n+1 nodes, padded past round_up(n+1, 4)
@@ -2664,15 +2664,10 @@ bool build_spaces(cem_sim *s, Device &D, int u) {
         long long t = 0;
         for (const Rect &r : cls[c]) {
             const long long nk4 = (r.ke - r.ks) / 4, nr = r.je - r.js;
-            if (nr * nk4 * nk4 >= (1ll << 40)) {
-                set_error("grid too large for the update layout");
-                return false;
-            }
             sp.ks[sp.n] = r.ks;
             sp.ke[sp.n] = r.ke;
             sp.js[sp.n] = r.js;
             sp.t0[sp.n] = (int)t;
-            sp.magic[sp.n] = ((1ull << 40) + (unsigned long long)nk4 - 1) / (unsigned long long)nk4;
             sp.n++;
             t += nr * nk4;
         }
@@ -2681,6 +2676,21 @@ bool build_spaces(cem_sim *s, Device &D, int u) {
             return false;
         }
         sp.t0[sp.n] = (int)t;
+        std::vector<uint2> item;
+        item.reserve((size_t)(t + kBlock));
+        for (int q = 0; q < sp.n; q++)
+            for (int r = 0, nr = cls[c][q].je - cls[c][q].js; r < nr; r++)
+                for (int k = sp.ks[q]; k < sp.ke[q]; k += 4) {
+                    const size_t at = item.size();
+                    unsigned w = (unsigned)(k >> 2) | kItemAct;
+                    if (at % 32 != 31 && k + 4 < sp.ke[q]) w |= kItemCont;
+                    if (at % 32 == 0 || k == sp.ks[q]) w |= kItemFirst;
+                    if ((k >= D.zt[u][0] && k < D.zt[u][1]) || (k >= D.zt[u][2] && k < D.zt[u][3])) w |= kItemTail;
+                    item.push_back(make_uint2((unsigned)(sp.js[q] + r), w));
+                }
+        while (!item.empty() && item.size() % kBlock)
+            item.push_back(make_uint2(item.back().x, (item.back().y & ~(kItemAct | kItemCont)) | kItemFirst));
+        if (!dev_renew(s, D.item[u][c], item)) return false;
     }
     D.p0[u] = p0;
     D.p1[u] = p1;
@@ -2695,7 +2705,7 @@ bool build_spaces(cem_sim *s, Device &D, int u) {
         for (int b = 0; b < 3 * nb; b++) wl.push_back(make_int2(i, b));
     }
     st[planes] = (int)wl.size();
-    return wl.empty() || dev_upload(s, D.wl[u], wl);
+    return dev_renew(s, D.wl[u], wl);
 }
 
 bool build_sources(cem_sim *s, Device &D) {
@@ -2718,7 +2728,7 @@ void fill_args_for(cem_sim *s, Device &D, int cur) {
     a = StepArgs{};
     a.g = D.g;
     for (int u = 0; u < 2; u++) {
-        for (int c = 0; c < kSpaces; c++) a.sp[u][c] = D.sp[u][c];
+        for (int c = 0; c < kSpaces; c++) a.item[u][c] = D.item[u][c].p;
         a.p0[u] = D.p0[u];
         a.p1[u] = D.p1[u];
         for (int q = 0; q < 4; q++) a.zt[u][q] = D.zt[u][q];
