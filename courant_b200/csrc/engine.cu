@@ -1732,8 +1732,11 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(const RunArgs r, const Pos
     }
 }
 
-// source values for the step count held on the device (after it was set from the host)
-__global__ void k_source_values(const PostArgs a) { source_values(a, *a.dstep, a.srcv); }
+// the step count of the host, and its source values
+__global__ void k_set_step(const PostArgs a, long long step) {
+    *a.dstep = step;
+    source_values(a, step, a.srcv);
+}
 
 // acc[slot][f] += (sample * dt) e^{-j w t} for each pending row in step order,
 // t the slot's sampling time: (n + 1/2) dt for H-time slots, (n + 1) dt for
@@ -1952,10 +1955,12 @@ struct Device {
     bool tune = false, tuned = false, tuned_from_cache = false;
     double tuned_ms = 0;
     cudaEvent_t tev[2] = {nullptr, nullptr};   // tuner timing
-    cudaGraphExec_t graph = nullptr;
+    cudaGraphExec_t graph = nullptr, tail = nullptr;   // graph_steps steps; the rest of the last run
+    int tail_steps = 0;
 
     ~Device() {
         if (graph) cudaGraphExecDestroy(graph);
+        if (tail) cudaGraphExecDestroy(tail);
         for (cudaEvent_t e : tev)
             if (e) cudaEventDestroy(e);
         if (fork) cudaEventDestroy(fork);
@@ -3121,8 +3126,7 @@ bool upload_group(cem_sim *s, unsigned g, bool from_host) {
 bool download_group(cem_sim *s, unsigned g) {
     Device &D = *s->dev;
     if ((g & kGroupDft) && !flush_dft(s)) return false;
-    CB2_CHECK(s, cudaStreamSynchronize(D.stream));
-    for (int c = 0; c < 3; c++) {
+    for (int c = 0; c < 3; c++) {   // (each copy follows the work of the stream and is waited for)
         if ((g & (kGroupE0 << c)) && !download_field(s, s->E[c], D.E[D.cur][c].p)) return false;
         if ((g & (kGroupH0 << c)) && !download_field(s, s->H[c], D.H[D.cur][c].p)) return false;
     }
@@ -3168,25 +3172,29 @@ bool download_group(cem_sim *s, unsigned g) {
     return true;
 }
 
-// Make the device state current before a device operation.
-bool begin_device_op(cem_sim *s) {
+// Make the device state current before a device operation. What callers may
+// have written through a pointer they hold goes up again (the spectra are handed
+// out as const: they stay); steps: the operation advances the simulation, so
+// the step count, source values and port voltages are set and the host copies
+// cease to be current. Nothing waits for the device unless something goes up.
+// (Five waits and two small copies an operation were half of a ten-step call
+// on a small grid.)
+bool begin_device_op(cem_sim *s, bool steps = true) {
     if (!create_device(s)) return false;
     Device &D = *s->dev;
     if (D.failed) { set_error(D.error_msg.c_str()); return false; }
     CB2_CHECK(s, cudaSetDevice(D.device));
-    CB2_CHECK(s, cudaStreamSynchronize(D.stream));
-    const unsigned need = (~s->dev_valid | s->exposed) & kGroupAll;
+    const unsigned need = (~s->dev_valid | (s->exposed & ~kGroupDft)) & kGroupAll;
+    if (need) CB2_CHECK(s, cudaStreamSynchronize(D.stream));
     for (unsigned g = 1; g & kGroupAll; g <<= 1) {
         if (!(need & g)) continue;
         if (!upload_group(s, g, (s->host_valid & g) != 0)) return false;
     }
     s->dev_valid = kGroupAll;
+    if (!steps) return true;
     if (D.ring_count == 0) D.ring_first = s->step;
-    long long st = s->step;
-    CB2_CHECK(s, cudaMemcpyAsync(D.dstep.p, &st, sizeof st, cudaMemcpyHostToDevice, D.stream));
-    k_source_values<<<1, 1, 0, D.stream>>>(D.pa[D.cur]);
+    k_set_step<<<1, 1, 0, D.stream>>>(D.pa[D.cur], s->step);
     CB2_CHECK(s, cudaGetLastError());
-    CB2_CHECK(s, cudaStreamSynchronize(D.stream));
     if (!D.vold_valid && D.nport) {
         PostArgs pa = D.pa[D.cur];
         pa.advance = 0;
@@ -3212,9 +3220,10 @@ bool end_device_op(cem_sim *s) {
             return false;
         }
     }
-    if (s->exposed) {
-        if (!download_group(s, s->exposed)) return false;
-        s->host_valid |= s->exposed;
+    const unsigned stale = s->exposed & ~s->host_valid;
+    if (stale) {
+        if (!download_group(s, stale)) return false;
+        s->host_valid |= stale;
     }
     return true;
 }
@@ -3460,6 +3469,31 @@ void engine_host_modified(cem_sim *s, unsigned groups) {
 
 namespace {
 
+// n steps of a run as a graph; the host's counts stay
+bool capture_steps(cem_sim *s, int n, cudaGraphExec_t &exec) {
+    Device &D = *s->dev;
+    const int rc = D.ring_count;
+    const long st = s->step;
+    CB2_CHECK(s, cudaStreamBeginCapture(D.stream, cudaStreamCaptureModeThreadLocal));
+    D.chained = false;
+    bool ok = true;
+    for (int q = 0; q < n && ok; q++) ok = launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1, true);
+    cudaGraph_t g = nullptr;
+    const cudaError_t ec = cudaStreamEndCapture(D.stream, &g);
+    D.ring_count = rc;
+    s->step = st;
+    if (!ok) {
+        if (g) cudaGraphDestroy(g);
+        return false;
+    }
+    CB2_CHECK(s, ec);
+    const cudaError_t ei = cudaGraphInstantiate(&exec, g, 0);
+    cudaGraphDestroy(g);
+    if (ei != cudaSuccess) exec = nullptr;
+    CB2_CHECK(s, ei);
+    return true;
+}
+
 // n whole steps, n at most Device::run_steps and the room in the sample ring:
 // source values, the steps (with graphs on, groups of graph_steps replay one
 // captured graph; the graph holds the kernels' arguments, which stay fixed for
@@ -3471,40 +3505,32 @@ bool run_chunk(cem_sim *s, long n) {
     D.chained = false;
     k_run_begin<<<(unsigned)((n + 127) / 128), 128, 0, D.stream>>>(D.run, pa, reinterpret_cast<float *>(D.run_src.p), (int)n,
                                                                   step0);
-    for (long it = 0; it < n;) {
-        const int gs = D.graph_steps;
-        if (D.use_graphs && n - it >= gs) {
-            if (!D.graph) {
-                const int rc = D.ring_count;
-                const long st = s->step;
-                CB2_CHECK(s, cudaStreamBeginCapture(D.stream, cudaStreamCaptureModeThreadLocal));
-                D.chained = false;
-                bool ok = true;
-                for (int q = 0; q < gs && ok; q++) ok = launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1, true);
-                cudaGraph_t g = nullptr;
-                const cudaError_t ec = cudaStreamEndCapture(D.stream, &g);
-                D.ring_count = rc;
-                s->step = st;
-                if (!ok) {
-                    if (g) cudaGraphDestroy(g);
-                    return false;
-                }
-                CB2_CHECK(s, ec);
-                const cudaError_t ei = cudaGraphInstantiate(&D.graph, g, 0);
-                cudaGraphDestroy(g);
-                if (ei != cudaSuccess) D.graph = nullptr;
-                CB2_CHECK(s, ei);
-            }
-            CB2_CHECK(s, cudaGraphLaunch(D.graph, D.stream));
-            D.chained = false;
-            D.ring_count += gs;
-            s->step += gs;
-            it += gs;
-        } else {
-            if (!launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1, true)) return false;
-            it++;
+    auto replay = [&](cudaGraphExec_t &graph, int k) {
+        if (!graph && !capture_steps(s, k, graph)) return false;
+        CB2_CHECK(s, cudaGraphLaunch(graph, D.stream));
+        D.chained = false;
+        D.ring_count += k;
+        s->step += k;
+        return true;
+    };
+    long rest = n;
+    for (const int gs = D.graph_steps; D.use_graphs && rest >= gs; rest -= gs)
+        if (!replay(D.graph, gs)) return false;
+    // what is left over: one graph too when the run before left as much (a ten-step
+    // call spends 55 us of the host's time on its launches, 8 on the graph's)
+    if (rest && rest != D.tail_steps) {
+        if (D.tail) {
+            CB2_CHECK(s, cudaStreamSynchronize(D.stream));
+            cudaGraphExecDestroy(D.tail);
         }
+        D.tail = nullptr;
+        D.tail_steps = (int)rest;
+    } else if (rest > 2 && D.use_graphs) {
+        if (!replay(D.tail, (int)rest)) return false;
+        rest = 0;
     }
+    for (; rest > 0; rest--)
+        if (!launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1, true)) return false;
     k_rows<<<(unsigned)n, kRowThreads, 0, D.stream>>>(D.run, pa, (int)n, step0);
     CB2_CHECK(s, cudaGetLastError());
     return true;
@@ -3591,7 +3617,9 @@ bool apply_shape(cem_sim *s, Device &D, int thin, bool side, int graph, bool zta
     }
     if (respace || graph != D.graph_steps) {
         if (D.graph) cudaGraphExecDestroy(D.graph);
-        D.graph = nullptr;
+        if (D.tail) cudaGraphExecDestroy(D.tail);
+        D.graph = D.tail = nullptr;
+        D.tail_steps = 0;
         D.graph_steps = graph;
     }
     D.side_on = side;
@@ -3679,7 +3707,7 @@ int engine_phase(cem_sim *s, int phase, int i0, int i1) {
 
 namespace {
 bool energy_on_device(cem_sim *s, double *out) {
-    if (!begin_device_op(s)) return false;
+    if (!begin_device_op(s, false)) return false;
     Device &D = *s->dev;
     const int gx = (D.g.plane + kEnergyBlock - 1) / kEnergyBlock;
     for (int c0 = 0; c0 <= s->n[0]; c0 += kMaxGridY)

@@ -63,3 +63,15 @@ def test_run_past_the_sample_ring(lib):
         b.step(n)
     assert np.array_equal(a.checkpoint(), b.checkpoint())
     assert np.array_equal(a.portV(0), b.portV(0)) and np.array_equal(a.iprobe(0), b.iprobe(0))
+
+
+def test_repeated_short_runs(lib):
+    """A run's rest replays a graph once the run before left as much; other rests in between, single steps among them."""
+    a, b = SCENES["lossy"](lib), SCENES["lossy"](lib)
+    chunks = (10, 10, 10, 42, 10, 3, 3, 10, 10, 1, 1, 31, 31)
+    for n in chunks:
+        a.step(n)
+    for _ in range(sum(chunks)):
+        b.step(1)
+    assert np.array_equal(a.checkpoint(), b.checkpoint())
+    assert np.array_equal(a.portI(1), b.portI(1))
