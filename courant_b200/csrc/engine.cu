@@ -433,22 +433,9 @@ __device__ __forceinline__ int jbox_volume(const StepArgs &a) {
     return a.jbox[C][3] * a.jbox[C][4] * a.jbox[C][5];
 }
 
-// Element of pole p's current at offset o of a Debye box of `vol` points
-// with P poles. CB2_JLAYOUT 0: one box-sized plane per pole; 1: the P poles
-// of each four-point group side by side (one thread's currents are P
-// consecutive float4).
-#ifndef CB2_JLAYOUT
-#define CB2_JLAYOUT 0
-#endif
-__host__ __device__ __forceinline__ size_t jaddr(int P, size_t vol, int p, size_t o) {
-#if CB2_JLAYOUT
-    (void)vol;
-    return ((o >> 2) * (size_t)P + (size_t)p) * 4 + (o & 3);
-#else
-    (void)P;
-    return (size_t)p * vol + o;
-#endif
-}
+// Element of pole p's current at offset o of a Debye box of `vol` points:
+// one box-sized plane per pole.
+__host__ __device__ __forceinline__ size_t jaddr(size_t vol, int p, size_t o) { return (size_t)p * vol + o; }
 
 // E value with auxiliaries and Debye currents read and written in place
 // (fused step; p1, p2: CPML planes as for h_comp; mi: table index)
@@ -468,7 +455,7 @@ __device__ __forceinline__ float e_comp(const StepArgs &a, int i, int j, int k, 
     if (disp) {
         jo = jbox_at<C>(a, i, j, k);
 #pragma unroll
-        for (int p = 0; p < P; p++) jsum = debye_term(a, p, a.J[C][jaddr(P, jvol, p, jo)], jsum);
+        for (int p = 0; p < P; p++) jsum = debye_term(a, p, a.J[C][jaddr(jvol, p, jo)], jsum);
     }
     const float r = e_value<C>(a, t, i, j, k, sv, e, d1, d2, c1, c2, p1 >= 0, p2 >= 0, s1, s2, jsum);
     if (p1 >= 0) a.psiE[C][0][x1] = s1;
@@ -477,7 +464,7 @@ __device__ __forceinline__ float e_comp(const StepArgs &a, int i, int j, int k, 
         const float de = __fsub_rn(r, e);
 #pragma unroll
         for (int p = 0; p < P; p++) {
-            float *jp = a.J[C] + jaddr(P, jvol, p, jo);
+            float *jp = a.J[C] + jaddr(jvol, p, jo);
             *jp = debye_next(a, p, beta_at<C>(a, mi, p), de, *jp);
         }
     }
@@ -846,7 +833,7 @@ __device__ __forceinline__ void e_four(const StepArgs &a, int j, int k4, int q, 
         }
     }
 #pragma unroll
-    for (int p = 0; p < P; p++) st4(Jc + jaddr(P, jvol, p, jo4), J[p]);
+    for (int p = 0; p < P; p++) st4(Jc + jaddr(jvol, p, jo4), J[p]);
 }
 
 // e_where: as h_where for E; CPML planes of nodes, and the Debye box
@@ -905,7 +892,7 @@ __device__ __forceinline__ void e_points(const StepArgs &a, int i, int j, int k4
     float4 J[P > 0 ? P : 1];
     const int jvol = P > 0 ? jbox_volume<C>(a) : 0;
 #pragma unroll
-    for (int p = 0; p < P; p++) J[p] = w.jo4 >= 0 ? ld4(a.J[C] + jaddr(P, jvol, p, w.jo4)) : z4;
+    for (int p = 0; p < P; p++) J[p] = w.jo4 >= 0 ? ld4(a.J[C] + jaddr(jvol, p, w.jo4)) : z4;
     const float4 t1 = term<true>(sub4(h2, h2m), c1, 0.f, s1, b1, d1, in1);
     const float4 t2 = term<true>(sub4(h1, h1m), c2, 0.f, s2, b2, d2, in2);
     if (in1) st4(a.psiE[C][0] + x1, s1);
@@ -1079,7 +1066,7 @@ __device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &
         if (A2 != 2) h1m = ld4(H1 + q - stride_of<A2>(a));
     }
 #pragma unroll
-    for (int pp = 0; pp < P; pp++) J[pp] = jo4 >= 0 ? ld4(Jc + jaddr(P, jvol, pp, jo4)) : z4;
+    for (int pp = 0; pp < P; pp++) J[pp] = jo4 >= 0 ? ld4(Jc + jaddr(jvol, pp, jo4)) : z4;
     if (A1 == 2) h2m = prev_k(h2, H2 + q, row && k4 > 0, p.first);
     if (A2 == 2) h1m = prev_k(h1, H1 + q, row && k4 > 0, p.first);
     if (!row) return;
@@ -1828,6 +1815,60 @@ __global__ void k_sum(const double *partial, long long n, double *out) {
     if (threadIdx.x == 0) *out = red[0];
 }
 
+// ------------------------------------------------------------- state moves
+
+// The arrays of the state as one stream of words, in the reference's order: word
+// (a*B + b)*C + c of piece p is word a*sa + b*sb + c*sc of its device array
+// (map: map[c] for c).
+// 6 fields, 16 CPML auxiliaries (a z slab is a piece), a Debye pole of a component, SIBC, DFT
+constexpr int kMovePieces = 24 + 3 * kMaxPoles;
+struct MovePiece {
+    unsigned *dev;
+    const unsigned *map;
+    unsigned long long start;   // its first word of the stream
+    unsigned B, C;
+    unsigned long long sa, sb, sc;
+};
+struct MoveArgs {
+    MovePiece p[kMovePieces];
+    int n;
+    unsigned long long lo;   // this launch: stream words [lo, lo + count) <-> stage[0 ..]
+    unsigned count;
+    unsigned *stage;
+};
+
+// Out: device arrays -> stage; otherwise back. Bound by the copy that follows or
+// precedes it over the host link: one copy in place of one and a wait per array
+// (up to 72 of them, 12 us each whatever the size), of the state without its
+// padding. Saving a 6e3-cell scene with CPML and Debye edges: 248 us (668 before),
+// restoring it and stepping: 104 us of host time (359); saving a 1e5-cell cavity:
+// 838 us (1607).
+template <bool Out>
+__global__ void k_move(const MoveArgs m) {
+    for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < m.count; w += gridDim.x * blockDim.x) {
+        const unsigned long long at = m.lo + w;
+        int q = 0;
+        while (q + 1 < m.n && at >= m.p[q + 1].start) q++;
+        const MovePiece &p = m.p[q];
+        const unsigned r = (unsigned)(at - p.start), ab = r / p.C, c = r - ab * p.C, i = ab / p.B, b = ab - i * p.B;
+        unsigned *d = p.dev + i * p.sa + b * p.sb + (p.map ? p.map[c] : c) * p.sc;
+        if (Out) m.stage[w] = *d;
+        else *d = m.stage[w];
+    }
+}
+
+// Arrays to zero in one launch (what goes up starts from zeroed padding).
+struct ClearArgs {
+    unsigned *p[kMovePieces];
+    unsigned long long n[kMovePieces];
+};
+
+__global__ void k_clear(const ClearArgs c) {
+    unsigned *p = c.p[blockIdx.y];
+    const unsigned long long n = c.n[blockIdx.y];
+    for (unsigned long long w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x) p[w] = 0;
+}
+
 // ------------------------------------------------------------ device state
 
 template <class T>
@@ -1872,6 +1913,8 @@ struct Device {
     int ntab[3] = {0, 0, 0};
     DevBuf<float> J[3];
     int jbox[3][6] = {};
+    DevBuf<unsigned> jmap[3];   // offset in the box of each dispersive edge (made for the first move)
+    size_t jfirst[4] = {};      // first dispersive edge of each component
     // Update kernels [H, E]: thread spaces [kFast, kGeneral, kAll], the
     // interior node planes [p0, p1), and the work-list of the general blocks
     // (entries: node plane, block of the plane's general space incl.
@@ -1952,6 +1995,10 @@ struct Device {
     DevBuf<float> raw;
     DevBuf<float2> run_src;
     DevBuf<int> run_at;
+    // words that state moves pass through, on the device and on the host (kStageWords at most)
+    DevBuf<unsigned> stage;
+    std::vector<unsigned> stage_host;
+    cudaEvent_t stage_ev = nullptr;
     bool tune = false, tuned = false, tuned_from_cache = false;
     double tuned_ms = 0;
     cudaEvent_t tev[2] = {nullptr, nullptr};   // tuner timing
@@ -1963,6 +2010,7 @@ struct Device {
         if (tail) cudaGraphExecDestroy(tail);
         for (cudaEvent_t e : tev)
             if (e) cudaEventDestroy(e);
+        if (stage_ev) { cudaEventSynchronize(stage_ev); cudaEventDestroy(stage_ev); }
         if (fork) cudaEventDestroy(fork);
         if (join) cudaEventDestroy(join);
         if (side) cudaStreamDestroy(side);
@@ -2955,35 +3003,6 @@ bool create_device_impl(cem_sim *s) {
 
 // ----------------------------------------------------- host <-> device moves
 
-// a field in the reference layout -> the padded device layout, and back
-bool upload_field(cem_sim *s, float *dst, const std::vector<double> &src) {
-    const Device &D = *s->dev;
-    std::vector<float> tmp(D.Np, 0.f);
-    const int nx = s->n[0], ny = s->n[1], nz = s->n[2];
-    for (int i = 0; i <= nx; i++)
-        for (int j = 0; j <= ny; j++) {
-            const double *r = &src[(size_t)i * s->si + (size_t)j * s->sj];
-            float *o = &tmp[(size_t)i * D.g.si + (size_t)j * D.g.sj];
-            for (int k = 0; k <= nz; k++) o[k] = (float)r[k];
-        }
-    return h2d(s, dst, tmp.data(), tmp.size() * 4);
-}
-
-bool download_field(cem_sim *s, std::vector<double> &dst, const float *src) {
-    const Device &D = *s->dev;
-    std::vector<float> tmp(D.Np);
-    if (!d2h(s, tmp.data(), src, tmp.size() * 4)) return false;
-    dst.resize(s->N);
-    const int nx = s->n[0], ny = s->n[1], nz = s->n[2];
-    for (int i = 0; i <= nx; i++)
-        for (int j = 0; j <= ny; j++) {
-            const float *r = &tmp[(size_t)i * D.g.si + (size_t)j * D.g.sj];
-            double *o = &dst[(size_t)i * s->si + (size_t)j * s->sj];
-            for (int k = 0; k <= nz; k++) o[k] = r[k];
-        }
-    return true;
-}
-
 // pack the host DFT accumulators in slot order: I probes, port V/I, source, V probes
 std::vector<double *> dft_slots(cem_sim *s) {
     std::vector<double *> v;
@@ -3008,167 +3027,220 @@ bool flush_dft(cem_sim *s) {
     return true;
 }
 
-// Reference compact index -> device index of every auxiliary of array
-// (c, w) (derivative axis (c + w + 1) % 3), E (nodes) or H (cells).
-template <class F>
-void psi_map(const cem_sim *s, const Device &D, bool is_e, int c, int w, F visit) {
-    const int ax = (c + w + 1) % 3, nx = s->n[0], ny = s->n[1], nz = s->n[2];
-    const size_t per = pml_per(s, ax);
-    const int planes = D.pml_planes[ax];
-    for (int pl = 0; pl < planes; pl++) {
-        if (ax == 0) {
-            for (int j = 0; j <= ny; j++)
-                for (int k = 0; k <= nz; k++)
-                    visit(pl * per + (size_t)j * (nz + 1) + k, (size_t)pl * D.g.si + (size_t)j * D.g.sj + k);
-        } else if (ax == 1) {
-            for (int i = 0; i <= nx; i++)
-                for (int k = 0; k <= nz; k++)
-                    visit(pl * per + (size_t)i * (nz + 1) + k, ((size_t)i * planes + pl) * D.g.sj + k);
-        } else {
-            int r[2][2];
-            pml_ranges(s, 2, is_e, r);
-            const int nlo = r[0][1] >= r[0][0] ? r[0][1] - r[0][0] + 1 : 0;
-            const int kz = pl < nlo ? r[0][0] + pl : r[1][0] + (pl - nlo);
-            const size_t zw = is_e ? D.zw_e : D.zw_h, zo = D.zoff_host[is_e][kz];
-            for (int i = 0; i <= nx; i++)
-                for (int j = 0; j <= ny; j++)
-                    visit(pl * per + (size_t)i * (ny + 1) + j, ((size_t)i * (ny + 1) + j) * zw + zo);
+// The dispersive edges follow one another by component.
+bool make_jmap(cem_sim *s) {
+    Device &D = *s->dev;
+    if (D.jfirst[3]) return true;
+    size_t first[4] = {};
+    for (int c = 0; c < 3; c++) {
+        const int *bx = D.jbox[c];
+        std::vector<unsigned> map;
+        size_t e = first[c];
+        for (; e < (size_t)s->ndisp && s->d_comp[e] == c; e++) {
+            const size_t q = s->d_idx[e];
+            const int i = (int)(q / s->si), j = (int)((q % s->si) / s->sj), k = (int)(q % s->sj);
+            map.push_back((unsigned)(((size_t)(i - bx[0]) * bx[4] + (j - bx[1])) * bx[5] + (k - bx[2])));
         }
+        first[c + 1] = e;
+        if (!dev_renew(s, D.jmap[c], map)) return false;
     }
-}
-
-bool psi_upload(cem_sim *s, bool is_e, int c, int w, const std::vector<double> &v, float *dst) {
-    const Device &D = *s->dev;
-    const size_t n = is_e ? D.psi_dev_e[c][w] : D.psi_dev_h[c][w];
-    if (!n) return true;
-    std::vector<float> o(n + 4, 0.f);
-    if (!v.empty()) psi_map(s, D, is_e, c, w, [&](size_t r, size_t d) { o[d] = (float)v[r]; });
-    return h2d(s, dst, o.data(), o.size() * sizeof(float));
-}
-
-bool psi_download(cem_sim *s, bool is_e, int c, int w, std::vector<double> &v, const float *src) {
-    const Device &D = *s->dev;
-    const size_t n = is_e ? D.psi_dev_e[c][w] : D.psi_dev_h[c][w];
-    v.assign(is_e ? D.psi_len_e[c][w] : D.psi_len_h[c][w], 0.0);
-    if (!n) return true;
-    std::vector<float> o(n);
-    if (!d2h(s, o.data(), src, n * sizeof(float))) return false;
-    psi_map(s, D, is_e, c, w, [&](size_t r, size_t d) { v[r] = o[d]; });
+    std::copy(first, first + 4, D.jfirst);
     return true;
 }
 
-bool upload_group(cem_sim *s, unsigned g, bool from_host) {
+// The arrays of groups g as pieces of one stream, and where each is on the
+// host (the DFT slots: nullptr, first in the stream so that they stay aligned).
+struct Move {
+    MoveArgs a{};
+    double *host[kMovePieces];
+    unsigned long long words = 0;
+
+    void add(void *dev, double *h, size_t A, size_t B, size_t C, size_t sa, size_t sb, size_t sc,
+             const unsigned *map = nullptr) {
+        if (!A || !B || !C) return;
+        host[a.n] = h;
+        a.p[a.n++] = {static_cast<unsigned *>(dev), map, words, (unsigned)B, (unsigned)C, sa, sb, sc};
+        words += (unsigned long long)A * B * C;
+    }
+};
+
+Move state_move(cem_sim *s, unsigned g, const StateView &v) {
     Device &D = *s->dev;
+    Move m;
+    const size_t nx1 = s->n[0] + 1, ny1 = s->n[1] + 1, nz1 = s->n[2] + 1;
+    const size_t si = D.g.si, sj = D.g.sj;
+    if (g & kGroupDft) m.add(D.acc.p, nullptr, D.nslot, 1, 4 * (size_t)s->nf, 4 * (size_t)s->nf, 0, 1);
     for (int c = 0; c < 3; c++) {
-        if (g & (kGroupE0 << c)) {
-            if (from_host) { if (!upload_field(s, D.E[D.cur][c].p, s->E[c])) return false; }
-            else if (!zero_dev(s, D.E[D.cur][c].p, D.Np * sizeof(float))) return false;
-            D.vold_valid = false;
-        }
-        if (g & (kGroupH0 << c)) {
-            if (from_host) { if (!upload_field(s, D.H[D.cur][c].p, s->H[c])) return false; }
-            else if (!zero_dev(s, D.H[D.cur][c].p, D.Np * sizeof(float))) return false;
+        if ((g & (kGroupE0 << c)) && v.E[c]) m.add(D.E[D.cur][c].p, v.E[c], nx1, ny1, nz1, si, sj, 1);
+        if ((g & (kGroupH0 << c)) && v.H[c]) m.add(D.H[D.cur][c].p, v.H[c], nx1, ny1, nz1, si, sj, 1);
+    }
+    for (int q = 0; (g & kGroupPsi) && q < 12; q++) {
+        const int c = q / 4, w = q / 2 % 2, is_e = q % 2, ax = (c + w + 1) % 3;
+        double *h = is_e ? v.psiE[c][w] : v.psiH[c][w];
+        float *d = is_e ? D.psiE[c][w].p : D.psiH[D.cur][c][w].p;
+        const size_t planes = D.pml_planes[ax];
+        if (!h || !(is_e ? D.psi_dev_e[c][w] : D.psi_dev_h[c][w])) continue;
+        if (ax == 0) { m.add(d, h, planes, ny1, nz1, si, sj, 1); continue; }
+        if (ax == 1) { m.add(d, h, planes, nx1, nz1, sj, planes * sj, 1); continue; }
+        const size_t zw = is_e ? D.zw_e : D.zw_h;
+        int r[2][2];
+        pml_ranges(s, 2, is_e, r);
+        for (int sd = 0; sd < 2; sd++) {   // the planes of a slab follow one another in a window
+            if (r[sd][1] < r[sd][0]) continue;
+            const size_t np = r[sd][1] - r[sd][0] + 1;
+            m.add(d + D.zoff_host[is_e][r[sd][0]], h, np, nx1, ny1, 1, ny1 * zw, zw);
+            h += np * nx1 * ny1;
         }
     }
-    if (g & kGroupPsi)
-        for (int c = 0; c < 3; c++)
-            for (int w = 0; w < 2; w++) {
-                if (from_host) {
-                    if (!psi_upload(s, true, c, w, s->psiE[c][w], D.psiE[c][w].p) ||
-                        !psi_upload(s, false, c, w, s->psiH[c][w], D.psiH[D.cur][c][w].p))
-                        return false;
-                } else if (!zero_dev(s, D.psiE[c][w].p, D.psiE[c][w].n * 4) ||
-                           !zero_dev(s, D.psiH[D.cur][c][w].p, D.psiH[D.cur][c][w].n * 4)) {
-                    return false;
-                }
-            }
-    if (g & kGroupDebye)
-        for (int c = 0; c < 3; c++) {
-            if (!D.J[c].p) continue;
-            if (!from_host) { if (!zero_dev(s, D.J[c].p, D.J[c].n * 4)) return false; continue; }
-            const int *bx = D.jbox[c];
-            const size_t vol = (size_t)bx[3] * bx[4] * bx[5];
-            std::vector<float> box(D.J[c].n, 0.f);
-            for (int e = 0; e < s->ndisp; e++) {
-                if (s->d_comp[e] != c) continue;
-                const size_t q = s->d_idx[e];
-                const int i = (int)(q / s->si), j = (int)((q % s->si) / s->sj), k = (int)(q % s->sj);
-                const size_t o = ((size_t)(i - bx[0]) * bx[4] + (j - bx[1])) * bx[5] + (k - bx[2]);
-                for (int p = 0; p < s->npole; p++) box[jaddr(s->npole, vol, p, o)] = (float)s->d_J[(size_t)p * s->ndisp + e];
-            }
-            if (!h2d(s, D.J[c].p, box.data(), box.size() * 4)) return false;
+    for (int c = 0; c < 3 && (g & kGroupDebye) && v.d_J; c++) {
+        if (!D.J[c].p) continue;
+        const size_t vol = (size_t)D.jbox[c][3] * D.jbox[c][4] * D.jbox[c][5];
+        for (int p = 0; p < s->npole; p++) {
+            const size_t at = jaddr(vol, p, 0);
+            m.add(D.J[c].p + at, v.d_J + (size_t)p * s->ndisp + D.jfirst[c], 1, 1, D.jfirst[c + 1] - D.jfirst[c], 0, 0,
+                  1, D.jmap[c].p);
         }
-    if ((g & kGroupSibc) && s->nsb) {
-        if (!from_host) {
-            if (!zero_dev(s, D.sb_y.p, D.sb_y.n * 4)) return false;
+    }
+    if ((g & kGroupSibc) && s->nsb && v.sb_y)
+        m.add(D.sb_y.p, v.sb_y, 1, s->nsb, s->sibc_npole, 0, 1, s->nsb);
+    return m;
+}
+
+// Stream words [lo, lo + n) between the staging words st and the host arrays.
+template <bool Out>
+void move_host(cem_sim *s, const Move &m, const std::vector<double *> &slots, unsigned long long lo, size_t n,
+               unsigned *st) {
+    const unsigned long long hi = lo + n;
+    for (int q = 0; q < m.a.n; q++) {
+        const unsigned long long p0 = m.a.p[q].start, p1 = q + 1 < m.a.n ? m.a.p[q + 1].start : m.words;
+        const unsigned long long x = std::max(lo, p0), y = std::min(hi, p1);
+        if (x >= y) continue;
+        if (m.host[q]) {
+            float *f = reinterpret_cast<float *>(st) + (x - lo);
+            double *h = m.host[q] + (x - p0);
+            const size_t len = y - x;
+            for (size_t r = 0; r < len; r++) {
+                if (Out) h[r] = f[r];
+                else f[r] = (float)h[r];
+            }
         } else {
-            const int K = s->sibc_npole, ns = s->nsb;
-            std::vector<float> y((size_t)K * ns);
-            for (int e = 0; e < ns; e++)
-                for (int k = 0; k < K; k++) y[(size_t)k * ns + e] = (float)s->sb_y[(size_t)e * K + k];
-            if (!h2d(s, D.sb_y.p, y.data(), y.size() * 4)) return false;
+            const size_t len = 2 * (size_t)s->nf;
+            double *f = reinterpret_cast<double *>(st + (x - lo));
+            for (size_t r = (x - p0) / 2; r < (y - p0) / 2;) {
+                const size_t k = r % len, cnt = std::min(len - k, (size_t)(y - p0) / 2 - r);
+                double *h = slots[r / len] + k;
+                if (Out) std::memcpy(h, f, cnt * sizeof(double));
+                else std::memcpy(f, h, cnt * sizeof(double));
+                f += cnt;
+                r += cnt;
+            }
         }
     }
-    if (g & kGroupDft) {
-        const size_t len = 2 * (size_t)s->nf;
-        std::vector<double> acc((size_t)D.nslot * len, 0.0);
-        if (from_host) {
-            std::vector<double *> slots = dft_slots(s);
-            for (size_t q = 0; q < slots.size(); q++) std::memcpy(&acc[q * len], slots[q], len * sizeof(double));
+}
+
+// Runs a move in chunks of at most kStageWords. Pageable host memory: page-locking
+// even 64 KB takes 1-8 ms, more than 4 MB take to copy without it (0.4 ms).
+// Upwards nothing waits for the last chunk.
+constexpr size_t kStageWords = 1 << 20;
+
+template <bool Out>
+bool run_move(cem_sim *s, Move &m) {
+    Device &D = *s->dev;
+    if (!m.words) return true;
+    const size_t chunk = (size_t)std::min<unsigned long long>((m.words + 1) / 2 * 2, kStageWords);
+    if (!D.stage_ev) CB2_CHECK(s, cudaEventCreateWithFlags(&D.stage_ev, cudaEventDisableTiming));
+    CB2_CHECK(s, cudaEventSynchronize(D.stage_ev));   // an earlier upload may still read the host words
+    if (D.stage.n < chunk) {
+        if (D.stage.p) CB2_CHECK(s, cudaFree(D.stage.p));
+        D.stage.p = nullptr;
+        D.stage.n = 0;
+        CB2_CHECK(s, cudaMalloc(&D.stage.p, chunk * sizeof(unsigned)));
+        D.stage.n = chunk;
+    }
+    if (D.stage_host.size() < chunk) D.stage_host.resize(chunk);
+    unsigned *st = D.stage_host.data();
+    const std::vector<double *> slots = dft_slots(s);
+    m.a.stage = D.stage.p;
+    for (m.a.lo = 0; m.a.lo < m.words; m.a.lo += chunk) {
+        m.a.count = (unsigned)std::min<unsigned long long>(chunk, m.words - m.a.lo);
+        const size_t bytes = m.a.count * sizeof(unsigned);
+        if (!Out) {
+            if (m.a.lo) CB2_CHECK(s, cudaEventSynchronize(D.stage_ev));
+            move_host<Out>(s, m, slots, m.a.lo, m.a.count, st);
+            CB2_CHECK(s, cudaMemcpyAsync(D.stage.p, st, bytes, cudaMemcpyHostToDevice, D.stream));
+            CB2_CHECK(s, cudaEventRecord(D.stage_ev, D.stream));
         }
-        if (!h2d(s, D.acc.p, acc.data(), acc.size() * sizeof(double))) return false;
+        k_move<Out><<<std::min(8 * 148u, (m.a.count + 255) / 256), 256, 0, D.stream>>>(m.a);
+        CB2_CHECK(s, cudaGetLastError());
+        if (Out) {
+            if (!d2h(s, st, D.stage.p, bytes)) return false;
+            move_host<Out>(s, m, slots, m.a.lo, m.a.count, st);
+        }
+    }
+    return true;
+}
+
+// the host copies of groups g
+StateView host_view(cem_sim *s, unsigned g) {
+    host_state_alloc(s, g);
+    auto at = [](std::vector<double> &v) { return v.empty() ? nullptr : v.data(); };
+    StateView v;
+    for (int c = 0; c < 3; c++) {
+        v.E[c] = at(s->E[c]);
+        v.H[c] = at(s->H[c]);
+        for (int w = 0; w < 2; w++) {
+            v.psiE[c][w] = at(s->psiE[c][w]);
+            v.psiH[c][w] = at(s->psiH[c][w]);
+        }
+    }
+    v.d_J = at(s->d_J);
+    v.sb_y = at(s->sb_y);
+    return v;
+}
+
+// Groups g to the device: those of from_host from the host copies, the others zero.
+bool upload_groups(cem_sim *s, unsigned g, unsigned from_host) {
+    Device &D = *s->dev;
+    ClearArgs z{};
+    int nz = 0;
+    auto clear = [&](void *p, size_t words) {
+        if (!p || !words) return;
+        z.p[nz] = static_cast<unsigned *>(p);
+        z.n[nz++] = words;
+    };
+    for (int c = 0; c < 3; c++) {
+        if (g & (kGroupE0 << c)) clear(D.E[D.cur][c].p, D.Np);
+        if (g & (kGroupH0 << c)) clear(D.H[D.cur][c].p, D.Np);
+        for (int w = 0; w < 2 && (g & kGroupPsi); w++) {
+            clear(D.psiE[c][w].p, D.psiE[c][w].n);
+            clear(D.psiH[D.cur][c][w].p, D.psiH[D.cur][c][w].n);
+        }
+    }
+    for (int c = 0; c < 3 && (g & kGroupDebye); c++) clear(D.J[c].p, D.J[c].n);
+    if ((g & kGroupSibc) && s->nsb) clear(D.sb_y.p, D.sb_y.n);
+    if (g & kGroupDft) clear(D.acc.p, 2 * D.acc.n);
+    if (nz) {
+        k_clear<<<dim3(148, nz), 256, 0, D.stream>>>(z);
+        CB2_CHECK(s, cudaGetLastError());
+    }
+    if (g & (kGroupE0 | kGroupE1 | kGroupE2)) D.vold_valid = false;
+    if ((g & from_host & kGroupDebye) && !make_jmap(s)) return false;
+    Move m = state_move(s, g & from_host, host_view(s, g & from_host));
+    if (!run_move<false>(s, m)) return false;
+    if (g & kGroupDft) {
         D.ring_first = s->step;
         D.ring_count = 0;
     }
     return true;
 }
 
-bool download_group(cem_sim *s, unsigned g) {
+// Groups g from the device: the spectra to the host copies, the others to `to`.
+bool download_groups(cem_sim *s, unsigned g, const StateView &to) {
     Device &D = *s->dev;
     if ((g & kGroupDft) && !flush_dft(s)) return false;
-    for (int c = 0; c < 3; c++) {   // (each copy follows the work of the stream and is waited for)
-        if ((g & (kGroupE0 << c)) && !download_field(s, s->E[c], D.E[D.cur][c].p)) return false;
-        if ((g & (kGroupH0 << c)) && !download_field(s, s->H[c], D.H[D.cur][c].p)) return false;
-    }
-    if (g & kGroupPsi)
-        for (int c = 0; c < 3; c++)
-            for (int w = 0; w < 2; w++)
-                if (!psi_download(s, true, c, w, s->psiE[c][w], D.psiE[c][w].p) ||
-                    !psi_download(s, false, c, w, s->psiH[c][w], D.psiH[D.cur][c][w].p))
-                    return false;
-    if (g & kGroupDebye) {
-        s->d_J.assign((size_t)s->npole * s->ndisp, 0.0);
-        if (s->d_Eold.size() != (size_t)s->ndisp) s->d_Eold.assign(s->ndisp, 0.0);
-        for (int c = 0; c < 3; c++) {
-            if (!D.J[c].p) continue;
-            std::vector<float> box(D.J[c].n);
-            if (!d2h(s, box.data(), D.J[c].p, box.size() * 4)) return false;
-            const int *bx = D.jbox[c];
-            const size_t vol = (size_t)bx[3] * bx[4] * bx[5];
-            for (int e = 0; e < s->ndisp; e++) {
-                if (s->d_comp[e] != c) continue;
-                const size_t q = s->d_idx[e];
-                const int i = (int)(q / s->si), j = (int)((q % s->si) / s->sj), k = (int)(q % s->sj);
-                const size_t o = ((size_t)(i - bx[0]) * bx[4] + (j - bx[1])) * bx[5] + (k - bx[2]);
-                for (int p = 0; p < s->npole; p++) s->d_J[(size_t)p * s->ndisp + e] = box[jaddr(s->npole, vol, p, o)];
-            }
-        }
-    }
-    if ((g & kGroupSibc) && s->nsb) {
-        const int K = s->sibc_npole, ns = s->nsb;
-        std::vector<float> y((size_t)K * ns);
-        if (!d2h(s, y.data(), D.sb_y.p, y.size() * 4)) return false;
-        s->sb_y.resize((size_t)K * ns);
-        for (int e = 0; e < ns; e++)
-            for (int k = 0; k < K; k++) s->sb_y[(size_t)e * K + k] = y[(size_t)k * ns + e];
-    }
-    if (g & kGroupDft) {
-        const size_t len = 2 * (size_t)s->nf;
-        std::vector<double> acc((size_t)D.nslot * len);
-        if (!d2h(s, acc.data(), D.acc.p, acc.size() * sizeof(double))) return false;
-        std::vector<double *> slots = dft_slots(s);
-        for (size_t q = 0; q < slots.size(); q++) std::memcpy(slots[q], &acc[q * len], len * sizeof(double));
-    }
+    if ((g & kGroupDebye) && !make_jmap(s)) return false;
+    Move m = state_move(s, g, to);
+    if (!run_move<true>(s, m)) return false;
     return true;
 }
 
@@ -3185,11 +3257,7 @@ bool begin_device_op(cem_sim *s, bool steps = true) {
     if (D.failed) { set_error(D.error_msg.c_str()); return false; }
     CB2_CHECK(s, cudaSetDevice(D.device));
     const unsigned need = (~s->dev_valid | (s->exposed & ~kGroupDft)) & kGroupAll;
-    if (need) CB2_CHECK(s, cudaStreamSynchronize(D.stream));
-    for (unsigned g = 1; g & kGroupAll; g <<= 1) {
-        if (!(need & g)) continue;
-        if (!upload_group(s, g, (s->host_valid & g) != 0)) return false;
-    }
+    if (need && !upload_groups(s, need, s->host_valid)) return false;
     s->dev_valid = kGroupAll;
     if (!steps) return true;
     if (D.ring_count == 0) D.ring_first = s->step;
@@ -3222,7 +3290,7 @@ bool end_device_op(cem_sim *s) {
     }
     const unsigned stale = s->exposed & ~s->host_valid;
     if (stale) {
-        if (!download_group(s, stale)) return false;
+        if (!download_groups(s, stale, host_view(s, stale))) return false;
         s->host_valid |= stale;
     }
     return true;
@@ -3448,7 +3516,7 @@ int engine_pull(const cem_sim *cs, unsigned groups) {
     if (!missing) return 0;
     host_state_alloc(s, missing);
     const unsigned from_dev = s->dev && !s->dev->failed ? missing & s->dev_valid : 0u;
-    if (from_dev && !download_group(s, from_dev)) return -1;
+    if (from_dev && !download_groups(s, from_dev, host_view(s, from_dev))) return -1;
     // groups valid nowhere are all zero: the freshly allocated host copies
     if (missing & ~from_dev) {
         for (int c = 0; c < 3; c++) {
@@ -3458,6 +3526,14 @@ int engine_pull(const cem_sim *cs, unsigned groups) {
     }
     s->host_valid |= missing;
     return 0;
+}
+
+unsigned engine_device_only(const cem_sim *s, unsigned groups) {
+    return s->dev && !s->dev->failed ? groups & s->dev_valid & ~s->host_valid : 0u;
+}
+
+int engine_read(cem_sim *s, unsigned groups, const StateView &to) {
+    return !groups || download_groups(s, groups, to) ? 0 : -1;
 }
 
 void engine_expose(const cem_sim *cs, unsigned groups) { const_cast<cem_sim *>(cs)->exposed |= groups; }

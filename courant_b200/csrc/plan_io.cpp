@@ -34,38 +34,43 @@ void phasors_at(const cem_sim *s, long step, std::vector<double> &phE, std::vect
 }
 
 // Walk the checkpoint blocks in the reference order (export.c:187-213);
-// visit(ptr, n) gets each block's host array (or nullptr when absent).
+// visit(group, view, ptr, n, offset) gets each block's state group, its place
+// in v (nullptr: none) and its host array (nullptr when absent).
 template <class F>
-size_t checkpoint_blocks(cem_sim *s, F visit) {
+size_t checkpoint_blocks(cem_sim *s, StateView &v, F visit) {
     size_t o = 0;
-    auto block = [&](double *p, size_t n) { visit(p, n, o); o += n; };
-    for (int c = 0; c < 3; c++) block(s->E[c].empty() ? nullptr : s->E[c].data(), s->N);
-    for (int c = 0; c < 3; c++) block(s->H[c].empty() ? nullptr : s->H[c].data(), s->N);
+    auto block = [&](unsigned g, double **view, std::vector<double> &p, size_t n) {
+        visit(g, view, p.empty() ? nullptr : p.data(), n, o);
+        o += n;
+    };
+    for (int c = 0; c < 3; c++) block(kGroupE0 << c, &v.E[c], s->E[c], s->N);
+    for (int c = 0; c < 3; c++) block(kGroupH0 << c, &v.H[c], s->H[c], s->N);
     if (s->has_pml)
         for (int c = 0; c < 3; c++)
             for (int w = 0; w < 2; w++) {
-                block(s->psiE[c][w].empty() ? nullptr : s->psiE[c][w].data(), psi_len(s, 1, c, w));
-                block(s->psiH[c][w].empty() ? nullptr : s->psiH[c][w].data(), psi_len(s, 0, c, w));
+                block(kGroupPsi, &v.psiE[c][w], s->psiE[c][w], psi_len(s, 1, c, w));
+                block(kGroupPsi, &v.psiH[c][w], s->psiH[c][w], psi_len(s, 0, c, w));
             }
     if (s->ndisp) {
-        block(s->d_J.empty() ? nullptr : s->d_J.data(), (size_t)s->npole * s->ndisp);
-        block(s->d_Eold.empty() ? nullptr : s->d_Eold.data(), s->ndisp);
+        block(kGroupDebye, &v.d_J, s->d_J, (size_t)s->npole * s->ndisp);
+        block(0, nullptr, s->d_Eold, s->ndisp);
     }
-    if (s->nsb) block(s->sb_y.empty() ? nullptr : s->sb_y.data(), (size_t)s->nsb * s->sibc_npole);
+    if (s->nsb) block(kGroupSibc, &v.sb_y, s->sb_y, (size_t)s->nsb * s->sibc_npole);
     for (LumpedPort &p : s->port) {
-        block(p.V.data(), 2 * s->nf);
-        block(p.I.data(), 2 * s->nf);
+        block(kGroupDft, nullptr, p.V, 2 * s->nf);
+        block(kGroupDft, nullptr, p.I, 2 * s->nf);
     }
-    for (VoltageProbe &p : s->vp) block(p.acc.data(), 2 * s->nf);
-    for (CurrentProbe &p : s->ip) block(p.acc.data(), 2 * s->nf);
-    block(s->src_acc.data(), 2 * s->nf);
-    block(s->phE.empty() ? nullptr : s->phE.data(), 2 * s->nf);
-    block(s->phH.empty() ? nullptr : s->phH.data(), 2 * s->nf);
+    for (VoltageProbe &p : s->vp) block(kGroupDft, nullptr, p.acc, 2 * s->nf);
+    for (CurrentProbe &p : s->ip) block(kGroupDft, nullptr, p.acc, 2 * s->nf);
+    block(kGroupDft, nullptr, s->src_acc, 2 * s->nf);
+    block(kGroupDft, nullptr, s->phE, 2 * s->nf);
+    block(kGroupDft, nullptr, s->phH, 2 * s->nf);
     return o;
 }
 
 size_t checkpoint_body(const cem_sim *s) {
-    return checkpoint_blocks(const_cast<cem_sim *>(s), [](double *, size_t, size_t) {});
+    StateView v;
+    return checkpoint_blocks(const_cast<cem_sim *>(s), v, [](unsigned, double **, double *, size_t, size_t) {});
 }
 
 void report(const char *what) {
@@ -222,20 +227,29 @@ size_t cem_checkpoint_size(const cem_sim *s) {
 int cem_checkpoint_save(const cem_sim *cs, double *buf) {
     cem_sim *s = const_cast<cem_sim *>(cs);
     if (!s->finalized) { set_error("not finalized"); return -1; }
-    if (engine_pull(s, kGroupAll)) return -1;
+    // what only the device holds goes straight to its place in buf (the spectra are few)
+    const unsigned direct = engine_device_only(s, kGroupAll & ~kGroupDft);
+    if (engine_pull(s, kGroupAll & ~direct)) return -1;
+    StateView v;
+    const size_t body = checkpoint_blocks(s, v, [&](unsigned g, double **view, double *, size_t, size_t o) {
+        if (g & direct) *view = buf + 8 + o;
+    });
+    if (engine_read(s, direct, v)) return -1;
     phasors_at(s, s->step, s->phE, s->phH);
     // the ADE stores E before the last E update; the device folds that value
     // into the same pass, so the current E at the dispersive edges stands in
     if (s->ndisp) {
         s->d_Eold.resize(s->ndisp);
-        for (int e = 0; e < s->ndisp; e++) s->d_Eold[e] = s->E[s->d_comp[e]][s->d_idx[e]];
+        const double *E[3];
+        for (int c = 0; c < 3; c++) E[c] = v.E[c] ? v.E[c] : s->E[c].data();
+        for (int e = 0; e < s->ndisp; e++) s->d_Eold[e] = E[s->d_comp[e]][s->d_idx[e]];
     }
-    const size_t body = checkpoint_body(s);
     const double hdr[8] = {kCheckpointMagic, 1, (double)s->N, (double)s->nf, (double)s->step, (double)body,
                            (double)(s->port.size() + 100 * s->vp.size() + 10000 * s->ip.size()),
                            (double)(s->ndisp + s->nsb)};
     std::memcpy(buf, hdr, sizeof hdr);
-    checkpoint_blocks(s, [buf](double *p, size_t n, size_t o) {
+    checkpoint_blocks(s, v, [&](unsigned g, double **, double *p, size_t n, size_t o) {
+        if (g & direct) return;
         if (p) std::memcpy(buf + 8 + o, p, n * sizeof(double));
         else std::memset(buf + 8 + o, 0, n * sizeof(double));
     });
@@ -254,7 +268,8 @@ int cem_checkpoint_load(cem_sim *s, const double *buf) {
     host_state_alloc(s, kGroupAll);
     s->phE.assign(2 * s->nf, 0.0);
     s->phH.assign(2 * s->nf, 0.0);
-    checkpoint_blocks(s, [buf](double *p, size_t n, size_t o) {
+    StateView v;
+    checkpoint_blocks(s, v, [buf](unsigned, double **, double *p, size_t n, size_t o) {
         if (p) std::memcpy(p, buf + 8 + o, n * sizeof(double));
     });
     s->step = (long)buf[4];

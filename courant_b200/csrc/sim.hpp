@@ -199,11 +199,18 @@ enum StateGroup : unsigned {
     kGroupFields = 0x3f, kGroupAll = 0x3ff,
 };
 
+// where the arrays of the state are read to, in the reference's layout (nullptr: not)
+struct StateView {
+    double *E[3] = {}, *H[3] = {}, *psiE[3][2] = {}, *psiH[3][2] = {}, *d_J = nullptr, *sb_y = nullptr;
+};
+
 // engine entry points (engine.cu); all return 0 or -1 with the error set
 int engine_step(cem_sim *s, long n);
 int engine_phase(cem_sim *s, int phase, int i0, int i1);   // cem_mt_* on the device
 int engine_energy(const cem_sim *s, double *out);
 int engine_pull(const cem_sim *s, unsigned groups);   // device -> host copies (host becomes valid)
+unsigned engine_device_only(const cem_sim *s, unsigned groups);   // those of groups that only the device holds
+int engine_read(cem_sim *s, unsigned groups, const StateView &to);   // such groups (not the spectra) to the caller's arrays
 void engine_expose(const cem_sim *s, unsigned groups);  // caller holds pointers into these host copies
 void engine_host_modified(cem_sim *s, unsigned groups); // host copies were changed by the library
 bool engine_has_device(const cem_sim *s);
