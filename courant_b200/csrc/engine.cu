@@ -595,12 +595,98 @@ __device__ __forceinline__ Where h_where(const StepArgs &a, int i, int j, int k4
     return w;
 }
 
+__device__ __forceinline__ float4 all4(float v) { return make_float4(v, v, v, v); }
+
+__device__ __forceinline__ float4 sub4(const float4 &a, const float4 &b) {
+    return make_float4(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z), __fsub_rn(a.w, b.w));
+}
+__device__ __forceinline__ float4 add4(const float4 &a, const float4 &b) {
+    return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+}
+__device__ __forceinline__ float4 mul4(const float4 &a, const float4 &b) {
+    return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
+}
+__device__ __forceinline__ float4 fma4(const float4 &a, const float4 &b, const float4 &c) {
+    return make_float4(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y), __fmaf_rn(a.z, b.z, c.z),
+                       __fmaf_rn(a.w, b.w, c.w));
+}
+
+// the points of `in` from v, the others as they are
+__device__ __forceinline__ void pick4(float4 &to, const float4 &v, unsigned in) {
+    if (in & 1u) to.x = v.x;
+    if (in & 2u) to.y = v.y;
+    if (in & 4u) to.z = v.z;
+    if (in & 8u) to.w = v.w;
+}
+
+// One difference term of an update, d * c, and where auxiliaries lie (in: the
+// points that have one, psi their values) the CPML recursion psi_next and the
+// auxiliary's share: + dth * psi' for H, + psi' for E.
+template <bool E>
+__device__ __forceinline__ float4 term(const float4 &d, const float4 &c, float dth, float4 &psi, const float4 &b,
+                                       const float4 &cd, unsigned in) {
+    float4 t = mul4(d, c);
+    if (!in) return t;
+    const float4 n = fma4(b, psi, fma4(cd, d, psi));
+    const float4 u = E ? add4(t, n) : fma4(all4(dth), n, t);
+    if (in == 15u) {
+        psi = n;
+        return u;
+    }
+    pick4(psi, n, in);
+    pick4(t, u, in);
+    return t;
+}
+
 // H component C at points k4 .. k4+3 of row (i, j) from the E values there
 // (e2 = E_{C+2}, e1 = E_{C+1}) and one step along the derivative axes (e2n
 // along C+1, e1n along C+2), h the old H, w from h_where; the new H goes to
 // hq.
 template <int C>
 __device__ __forceinline__ void h_points(const StepArgs &a, int i, int j, int k4, float *hq, const Where &w,
+                                         const float4 &e2, const float4 &e2n, const float4 &e1, const float4 &e1n,
+                                         float4 h) {
+    constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
+    constexpr bool kz = A1 == 2 || A2 == 2;
+    const int nx = a.g.n[0], ny = a.g.n[1], nz = a.g.n[2];
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float ci = __ldg(a.hc[0] + min(i, nx - 1)), cj = __ldg(a.hc[1] + min(j, ny - 1));
+    const float4 ck = ldg4(a.hc[2] + k4);
+    const float4 c1 = A1 == 0 ? all4(ci) : (A1 == 1 ? all4(cj) : ck), c2 = A2 == 0 ? all4(ci) : (A2 == 1 ? all4(cj) : ck);
+    const int last = kz ? nz : nz + 1;
+    const unsigned own = k4 + 4 > last ? (1u << max(last - k4, 0)) - 1u : 15u;
+    const unsigned inz = (w.pk.x >= 0 ? 1u : 0u) | (w.pk.y >= 0 ? 2u : 0u) | (w.pk.z >= 0 ? 4u : 0u) | (w.pk.w >= 0 ? 8u : 0u);
+    const int pa[3] = {w.pi, w.pj, inz ? 0 : -1};
+    const unsigned in1 = (A1 == 2 ? inz : (pa[A1] >= 0 ? 15u : 0u)) & own, in2 = (A2 == 2 ? inz : (pa[A2] >= 0 ? 15u : 0u)) & own;
+    // auxiliaries: all loads before the arithmetic
+    float4 s1 = z4, s2 = z4, b1 = z4, b2 = z4, d1 = z4, d2 = z4;
+    int x1 = 0, x2 = 0;
+    if (in1) {
+        x1 = psi_at<A1, false>(a, pa[A1], i, j, k4);
+        s1 = ld4(a.psiH[C][0] + x1);
+        b1 = A1 == 2 ? ldg4(a.pml[2].bm1_h + k4) : all4(__ldg(a.pml[A1].bm1_h + (A1 == 0 ? i : j)));
+        d1 = A1 == 2 ? ldg4(a.pml[2].cid_h + k4) : all4(__ldg(a.pml[A1].cid_h + (A1 == 0 ? i : j)));
+    }
+    if (in2) {
+        x2 = psi_at<A2, false>(a, pa[A2], i, j, k4);
+        s2 = ld4(a.psiH[C][1] + x2);
+        b2 = A2 == 2 ? ldg4(a.pml[2].bm1_h + k4) : all4(__ldg(a.pml[A2].bm1_h + (A2 == 0 ? i : j)));
+        d2 = A2 == 2 ? ldg4(a.pml[2].cid_h + k4) : all4(__ldg(a.pml[A2].cid_h + (A2 == 0 ? i : j)));
+    }
+    const float4 t1 = term<false>(sub4(e2n, e2), c1, a.dth, s1, b1, d1, in1);
+    const float4 t2 = term<false>(sub4(e1n, e1), c2, a.dth, s2, b2, d2, in2);
+    if (in1) st4(a.psiH[C][0] + x1, s1);
+    if (in2) st4(a.psiH[C][1] + x2, s2);
+    const float4 v = sub4(h, sub4(t1, t2));
+    if (own == 15u) h = v;
+    else pick4(h, v, own);
+    st4(hq, h);
+}
+
+// The same point by point: auxiliaries and coefficients are fetched as they are
+// used, which takes fewer registers.
+template <int C>
+__device__ __forceinline__ void h_points_each(const StepArgs &a, int i, int j, int k4, float *hq, const Where &w,
                                          const float4 &e2, const float4 &e2n, const float4 &e1, const float4 &e1n,
                                          float4 h) {
     constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
@@ -652,8 +738,13 @@ __device__ __forceinline__ void h_points(const StepArgs &a, int i, int j, int k4
     if (any2) st4(a.psiH[C][1] + x2, s2);
 }
 
-// H component C on points k4 .. k4+3 of row (i, j) (segment [ks, ke))
-template <int C>
+// H component C on points k4 .. k4+3 of row (i, j) (segment [ks, ke)). Each:
+// h_points_each, for launches that are bound by HBM, where blocks in flight count
+// for more than a shorter chain (z tails and general blocks of large grids with
+// h_points: 10.9 M-cell board 331 -> 335 us per step). The launches of small grids
+// are bound by their threads' chains: h_points_each there 6.8 instead of 6.2 us per
+// step on the lossy scene, 10.5 instead of 9.9 on the 121 x 62 x 40 line.
+template <int C, bool Each = false>
 __device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r) {
     const int j = r.j, k4 = r.k4;
     const int m = j * a.g.sj + k4;
@@ -682,50 +773,8 @@ __device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r)
     if (A1 == 2) e2n = next_k(e2, E2 + q, row && k4 + 4 <= nz, edge);
     if (A2 == 2) e1n = next_k(e1, E1 + q, row && k4 + 4 <= nz, edge);
     if (!row) return;
-    h_points<C>(a, i, j, k4, H + q, w, e2, e2n, e1, e1n, h);
-}
-
-__device__ __forceinline__ float4 all4(float v) { return make_float4(v, v, v, v); }
-
-__device__ __forceinline__ float4 sub4(const float4 &a, const float4 &b) {
-    return make_float4(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z), __fsub_rn(a.w, b.w));
-}
-__device__ __forceinline__ float4 add4(const float4 &a, const float4 &b) {
-    return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
-}
-__device__ __forceinline__ float4 mul4(const float4 &a, const float4 &b) {
-    return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
-}
-__device__ __forceinline__ float4 fma4(const float4 &a, const float4 &b, const float4 &c) {
-    return make_float4(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y), __fmaf_rn(a.z, b.z, c.z),
-                       __fmaf_rn(a.w, b.w, c.w));
-}
-
-// the points of `in` from v, the others as they are
-__device__ __forceinline__ void pick4(float4 &to, const float4 &v, unsigned in) {
-    if (in & 1u) to.x = v.x;
-    if (in & 2u) to.y = v.y;
-    if (in & 4u) to.z = v.z;
-    if (in & 8u) to.w = v.w;
-}
-
-// One difference term of an update, d * c, and where auxiliaries lie (in: the
-// points that have one, psi their values) the CPML recursion psi_next and the
-// auxiliary's share: + dth * psi' for H, + psi' for E.
-template <bool E>
-__device__ __forceinline__ float4 term(const float4 &d, const float4 &c, float dth, float4 &psi, const float4 &b,
-                                       const float4 &cd, unsigned in) {
-    float4 t = mul4(d, c);
-    if (!in) return t;
-    const float4 n = fma4(b, psi, fma4(cd, d, psi));
-    const float4 u = E ? add4(t, n) : fma4(all4(dth), n, t);
-    if (in == 15u) {
-        psi = n;
-        return u;
-    }
-    pick4(psi, n, in);
-    pick4(t, u, in);
-    return t;
+    if (Each) h_points_each<C>(a, i, j, k4, H + q, w, e2, e2n, e1, e1n, h);
+    else h_points<C>(a, i, j, k4, H + q, w, e2, e2n, e1, e1n, h);
 }
 
 // E component C of four points from the curl: t per point (ca-1, cb, cs,
@@ -971,7 +1020,7 @@ __device__ __forceinline__ void h_lean(const StepArgs &a, int i, const RowPos &p
     if (A2 == 2) e1n = next_k(e1, E1 + q, row && k4 + 4 <= nz, !p.cont);
     if (!row) return;
     if (kz && p.tail) {
-        h_points<C>(a, i, j, k4, H + q, ztail_where(a.pml[2].plane_h, k4), e2, e2n, e1, e1n, h);
+        h_points_each<C>(a, i, j, k4, H + q, ztail_where(a.pml[2].plane_h, k4), e2, e2n, e1, e1n, h);
         return;
     }
     const float ci = __ldg(a.hc[0] + i), cj = __ldg(a.hc[1] + j);
@@ -1229,9 +1278,9 @@ __global__ void __launch_bounds__(kBlock, CB2_H_MINBLOCKS) k_update_h(const Step
     const int comp = w.y % 3;
     const RowPos p = general_pos<0>(a, w.x, w.y / 3);
     chain_wait();
-    if (comp == 0) h_vec<0>(a, w.x, p);
-    else if (comp == 1) h_vec<1>(a, w.x, p);
-    else h_vec<2>(a, w.x, p);
+    if (comp == 0) h_vec<0, true>(a, w.x, p);
+    else if (comp == 1) h_vec<1, true>(a, w.x, p);
+    else h_vec<2, true>(a, w.x, p);
 }
 
 // E over the general blocks (no Debye poles)
@@ -1294,11 +1343,12 @@ __device__ __forceinline__ int whole_place(const StepArgs &a, const Whole &l, in
     return deb ? 1 : 0;
 }
 
-// resident blocks per SM: 48 registers for H; for E 72, or 64 on large grids of up
+// resident blocks per SM: 56 registers for H (48 and 64: 250 k-cell board 13.3 and 12.8
+// us per step against 12.4); for E 72, or 64 on large grids of up
 // to four poles (they spill a little on the CPML paths there, but a bandwidth-bound
 // launch gains more from the eighth block: 334 against 341 us per step on the
 // 10.9 M-cell board; 13.1 against 15.1 the other way on the 250 k-cell one)
-constexpr int kWholeH = 10, kWholeE = 7, kWholeELarge = 8;
+constexpr int kWholeH = 9, kWholeE = 7, kWholeELarge = 8;
 __global__ void __launch_bounds__(kBlock, kWholeH) k_whole_h(const StepArgs a, const Whole l, const RunArgs r) {
     chain_next();
     if ((int)blockIdx.x < r.first) {
