@@ -744,8 +744,8 @@ __device__ __forceinline__ void h_points_each(const StepArgs &a, int i, int j, i
 // h_points: 10.9 M-cell board 331 -> 335 us per step). The launches of small grids
 // are bound by their threads' chains: h_points_each there 6.8 instead of 6.2 us per
 // step on the lossy scene, 10.5 instead of 9.9 on the 121 x 62 x 40 line.
-template <int C, bool Each = false>
-__device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r) {
+template <int C, bool Each = false, class Wait>
+__device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r, Wait wait) {
     const int j = r.j, k4 = r.k4;
     const int m = j * a.g.sj + k4;
     constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
@@ -760,6 +760,7 @@ __device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r)
     float *H = a.H[C];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 e2 = z4, e1 = z4, h = z4, e2n = z4, e1n = z4;
+    wait();
     if (row) {
         e2 = ld4(E2 + q);
         e1 = ld4(E1 + q);
@@ -950,8 +951,8 @@ __device__ __forceinline__ void e_points(const StepArgs &a, int i, int j, int k4
 }
 
 // E component C on points k4 .. k4+3 of row (i, j) (segment [ks, ke))
-template <int C, int P>
-__device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r, const float2 sv, unsigned skip) {
+template <int C, int P, class Wait>
+__device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r, unsigned skip, Wait wait) {
     const int j = r.j, k4 = r.k4;
     const int m = j * a.g.sj + k4;
     constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
@@ -967,11 +968,13 @@ __device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r,
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 h2 = z4, h1 = z4, ev = z4, h2m = z4, h1m = z4;
     uint2 mv = make_uint2(0, 0);
+    if (row) mv = __ldg(reinterpret_cast<const uint2 *>(a.mat[C] + q));
+    wait();
+    const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
     if (row) {
         h2 = ld4(H2 + q);
         h1 = ld4(H1 + q);
         ev = ld4(E + q);
-        mv = __ldg(reinterpret_cast<const uint2 *>(a.mat[C] + q));
         if (A1 != 2) h2m = ld4(H2 + q - stride_of<A1>(a));
         if (A2 != 2) h1m = ld4(H1 + q - stride_of<A2>(a));
     }
@@ -994,10 +997,10 @@ __device__ __forceinline__ Where ztail_where(const int *plane_z, int k4) {
 
 // H component C at points k4 .. k4+3 of row (i, j) of a fast piece: the
 // short path of h_points (no auxiliaries), every rounding the same; groups of
-// a z tail take h_points itself. All lanes of the warp call it (the k+1
+// a z tail take h_points_each. All lanes of the warp call it (the k+1
 // neighbours move by shuffle).
-template <int C>
-__device__ __forceinline__ void h_lean(const StepArgs &a, int i, const RowPos &p) {
+template <int C, class Wait>
+__device__ __forceinline__ void h_lean(const StepArgs &a, int i, const RowPos &p, Wait wait) {
     constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
     constexpr bool kz = A1 == 2 || A2 == 2;
     const int nx = a.g.n[0], ny = a.g.n[1], nz = a.g.n[2];
@@ -1009,6 +1012,7 @@ __device__ __forceinline__ void h_lean(const StepArgs &a, int i, const RowPos &p
     float *H = a.H[C];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 e2 = z4, e1 = z4, h = z4, e2n = z4, e1n = z4;
+    wait();
     if (row) {
         e2 = ld4(E2 + q);
         e1 = ld4(E1 + q);
@@ -1041,8 +1045,8 @@ __device__ __forceinline__ void h_lean(const StepArgs &a, int i, const RowPos &p
 // E component C at points k4 .. k4+3 of row (i, j) of a fast piece: the
 // short path of e_points (material table, sources; no auxiliaries, no Debye
 // currents), every rounding the same; groups of a z tail take e_points itself
-template <int C>
-__device__ __forceinline__ void e_lean(const StepArgs &a, int i, const RowPos &p, const float2 sv, unsigned skip) {
+template <int C, class Wait>
+__device__ __forceinline__ void e_lean(const StepArgs &a, int i, const RowPos &p, unsigned skip, Wait wait) {
     constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
     constexpr bool kz = A1 == 2 || A2 == 2;
     const int ny = a.g.n[1], nz = a.g.n[2];
@@ -1055,11 +1059,13 @@ __device__ __forceinline__ void e_lean(const StepArgs &a, int i, const RowPos &p
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 h2 = z4, h1 = z4, ev = z4, h2m = z4, h1m = z4;
     uint2 mv = make_uint2(0, 0);
+    if (row) mv = __ldg(reinterpret_cast<const uint2 *>(a.mat[C] + q));
+    wait();
+    const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
     if (row) {
         h2 = ld4(H2 + q);
         h1 = ld4(H1 + q);
         ev = ld4(E + q);
-        mv = __ldg(reinterpret_cast<const uint2 *>(a.mat[C] + q));
         if (A1 != 2) h2m = ld4(H2 + q - stride_of<A1>(a));
         if (A2 != 2) h1m = ld4(H1 + q - stride_of<A2>(a));
     }
@@ -1086,8 +1092,8 @@ __device__ __forceinline__ void e_lean(const StepArgs &a, int i, const RowPos &p
 // The P pole currents of the four points are read once as float4 and kept in
 // registers for both sum_p hk_p J_p and their own update, then written once;
 // beta_p/dt comes packed per table entry. Every rounding is that of e_points.
-template <int C, int P>
-__device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &p, const float2 sv, unsigned skip) {
+template <int C, int P, class Wait>
+__device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &p, unsigned skip, Wait wait) {
     constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
     constexpr bool kz = A1 == 2 || A2 == 2;
     const int ny = a.g.n[1], nz = a.g.n[2];
@@ -1106,11 +1112,13 @@ __device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &
     const int jo4 = row && k4 >= bx[2] && k4 < bx[2] + bx[5] ? jbox_at<C>(a, i, j, k4) : -1;
     const int jvol = jbox_volume<C>(a);
     float4 J[P > 0 ? P : 1];
+    if (row) mv = __ldg(reinterpret_cast<const uint2 *>(a.mat[C] + q));
+    wait();
+    const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
     if (row) {
         h2 = ld4(H2 + q);
         h1 = ld4(H1 + q);
         ev = ld4(E + q);
-        mv = __ldg(reinterpret_cast<const uint2 *>(a.mat[C] + q));
         if (A1 != 2) h2m = ld4(H2 + q - stride_of<A1>(a));
         if (A2 != 2) h1m = ld4(H1 + q - stride_of<A2>(a));
     }
@@ -1134,7 +1142,8 @@ __device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &
 
 // E = sum_k c_k (J - y_k) with y_k += (1 - e_k)(J - y_k), J from the faces' H.
 // (reference sibc.c:256-269)
-__device__ __forceinline__ void sibc_edge(const SibcArgs &a, int e) {
+template <class Wait>
+__device__ __forceinline__ void sibc_edge(const SibcArgs &a, int e, Wait wait) {
     // every load first: face tables (16-byte vectors), the convolution
     // states, then the H values of the faces
     const float4 w4 = __ldg(a.hw + e);
@@ -1142,6 +1151,7 @@ __device__ __forceinline__ void sibc_edge(const SibcArgs &a, int e) {
     const uchar4 c4 = __ldg(a.hcomp + e);
     const unsigned char ec = __ldg(a.ecomp + e);
     const unsigned ei = __ldg(a.eidx + e);
+    wait();
     float y[kSibcTerms];
 #pragma unroll
     for (int k = 0; k < kSibcTerms; k++)
@@ -1171,19 +1181,27 @@ __device__ __forceinline__ void sibc_edge(const SibcArgs &a, int e) {
     a.E[ec][ei] = E;
 }
 
-// samples of family u (0 E, 1 H) into the row of step t, by one block
-__device__ __forceinline__ void sample_family(const StepArgs &a, const RunArgs &r, int u, int t) {
+// samples of family u (0 E, 1 H) into their step's row, by one block: H in the step
+// in progress, E in the next one's H launch (of the first, none). Returns the step read.
+template <class Wait>
+__device__ __forceinline__ int sample_family(const StepArgs &a, const RunArgs &r, int u, Wait wait) {
     const uint4 *s = r.samples + (u ? r.nsample[0] : 0);
+    uint4 v;
+    if ((int)threadIdx.x < r.nsample[u]) v = __ldg(s + threadIdx.x);
+    wait();
+    const int at = r.at[u ? 0 : 1], t = u ? at : at - 1;
+    if (t < 0) return at;
     for (int e = threadIdx.x; e < r.nsample[u]; e += blockDim.x) {
-        const uint4 v = __ldg(s + e);
+        if (e != (int)threadIdx.x) v = __ldg(s + e);
         r.raw[(size_t)t * r.nent + v.z] = (u ? a.H[v.x - 3] : a.E[v.x])[v.y];
     }
+    return at;
 }
 
 // H launch of a run: E of the step before, and the new step's source values
-__device__ __forceinline__ void begin_step(const StepArgs &a, const RunArgs &r) {
-    const int t = r.at[1];
-    if (t > 0) sample_family(a, r, 0, t - 1);
+template <class Wait>
+__device__ __forceinline__ void begin_step(const StepArgs &a, const RunArgs &r, Wait wait) {
+    const int t = sample_family(a, r, 0, wait);
     __syncthreads();
     if (threadIdx.x == 0) {
         *r.srcv = r.src[t];
@@ -1214,11 +1232,16 @@ __device__ __forceinline__ void begin_step(const StepArgs &a, const RunArgs &r) 
 #endif
 
 // Chained launches (RunArgs::on): a launch that follows another on one stream
-// alone may start while that one ends; it works out its place meanwhile and
-// waits for the end before it touches what that one writes. (Fields are read by
+// alone may start while that one ends; meanwhile it works out its place and
+// fetches from the tables that no launch writes (CPML planes, material indices,
+// probe and surface-impedance entries), then waits for the end before it touches
+// what launches write (`wait` in the functions below, which others call with
+// nothing to wait for). (Fields are read by
 // plain loads for that: they change within the launch's life. The wait makes the
 // other's writes visible; the read-only path promises nothing there.) Parity
-// scene 6.8 to 5.9 us per step, lossy scene 8.2 to 6.9, cavity 5.8 to 5.4.
+// scene 6.8 to 5.9 us per step, lossy scene 8.2 to 6.9, cavity 5.8 to 5.4; with the
+// tables before the wait, 5.35 to 4.85, 6.25 to 5.3 and 5.0 to 4.65, 121 x 62 x 40
+// line 9.9 to 8.8, 250 k-cell board 12.5 to 11.7.
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -1227,35 +1250,30 @@ __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait
 __global__ void __launch_bounds__(kBlock, CB2_HF_MINBLOCKS) k_update_h_fast(const StepArgs a, int i0, const RunArgs r) {
     chain_next();
     if (r.first && blockIdx.x == gridDim.x - 1) {   // one column more: the run's own work
-        chain_wait();
-        if (blockIdx.y == 0) begin_step(a, r);
+        if (blockIdx.y == 0) begin_step(a, r, chain_wait);
         return;
     }
     const int comp = blockIdx.x % 3;
     const RowPos p = space_pos(a.item[0][kFast], blockIdx.x / 3);
-    chain_wait();
     const int i = i0 + blockIdx.y;
-    if (comp == 0) h_lean<0>(a, i, p);
-    else if (comp == 1) h_lean<1>(a, i, p);
-    else h_lean<2>(a, i, p);
+    if (comp == 0) h_lean<0>(a, i, p, chain_wait);
+    else if (comp == 1) h_lean<1>(a, i, p, chain_wait);
+    else h_lean<2>(a, i, p, chain_wait);
 }
 
 // E on the fast rectangles of node planes [i0, i0 + gridDim.y), from the last to the first
 __global__ void __launch_bounds__(kBlock, CB2_EF_MINBLOCKS) k_update_e_fast(const StepArgs a, int i0, const RunArgs r) {
     chain_next();
     if (r.first && blockIdx.x == gridDim.x - 1) {
-        chain_wait();
-        if (blockIdx.y == 0) sample_family(a, r, 1, r.at[0]);
+        if (blockIdx.y == 0) sample_family(a, r, 1, chain_wait);
         return;
     }
     const int comp = blockIdx.x % 3;
     const RowPos p = space_pos(a.item[1][kFast], blockIdx.x / 3);
-    chain_wait();
     const int i = i0 + (int)(gridDim.y - 1 - blockIdx.y);   // E begins where H ended, on what L2 still holds
-    const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
-    if (comp == 0) e_lean<0>(a, i, p, sv, r.skip);
-    else if (comp == 1) e_lean<1>(a, i, p, sv, r.skip);
-    else e_lean<2>(a, i, p, sv, r.skip);
+    if (comp == 0) e_lean<0>(a, i, p, r.skip, chain_wait);
+    else if (comp == 1) e_lean<1>(a, i, p, r.skip, chain_wait);
+    else e_lean<2>(a, i, p, r.skip, chain_wait);
 }
 
 // Position in the general space of update U: the general rectangles on an
@@ -1270,17 +1288,15 @@ __device__ __forceinline__ RowPos general_pos(const StepArgs &a, int i, int b) {
 __global__ void __launch_bounds__(kBlock, CB2_H_MINBLOCKS) k_update_h(const StepArgs a, const int2 *work, const RunArgs r) {
     chain_next();
     if ((int)blockIdx.x < r.first) {
-        chain_wait();
-        begin_step(a, r);
+        begin_step(a, r, chain_wait);
         return;
     }
     const int2 w = work[blockIdx.x - r.first];
     const int comp = w.y % 3;
     const RowPos p = general_pos<0>(a, w.x, w.y / 3);
-    chain_wait();
-    if (comp == 0) h_vec<0, true>(a, w.x, p);
-    else if (comp == 1) h_vec<1, true>(a, w.x, p);
-    else h_vec<2, true>(a, w.x, p);
+    if (comp == 0) h_vec<0, true>(a, w.x, p, chain_wait);
+    else if (comp == 1) h_vec<1, true>(a, w.x, p, chain_wait);
+    else h_vec<2, true>(a, w.x, p, chain_wait);
 }
 
 // E over the general blocks (no Debye poles)
@@ -1289,19 +1305,16 @@ __global__ void __launch_bounds__(kBlock, CB2_E_MINBLOCKS)
     chain_next();
     if ((int)blockIdx.x < r.first) {   // H samples, then the surface-impedance edges (their E is left alone below)
         const int e = ((int)blockIdx.x - 1) * kBlock + threadIdx.x;
-        chain_wait();
-        if (blockIdx.x == 0) sample_family(a, r, 1, r.at[0]);
-        else if (e < s.ns) sibc_edge(s, e);
+        if (blockIdx.x == 0) sample_family(a, r, 1, chain_wait);
+        else if (e < s.ns) sibc_edge(s, e, chain_wait);
         return;
     }
     const int2 w = work[gridDim.x - 1 - blockIdx.x];
     const int comp = w.y % 3;
     const RowPos p = general_pos<1>(a, w.x, w.y / 3);
-    chain_wait();
-    const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
-    if (comp == 0) e_vec<0, 0>(a, w.x, p, sv, r.skip);
-    else if (comp == 1) e_vec<1, 0>(a, w.x, p, sv, r.skip);
-    else e_vec<2, 0>(a, w.x, p, sv, r.skip);
+    if (comp == 0) e_vec<0, 0>(a, w.x, p, r.skip, chain_wait);
+    else if (comp == 1) e_vec<1, 0>(a, w.x, p, r.skip, chain_wait);
+    else e_vec<2, 0>(a, w.x, p, r.skip, chain_wait);
 }
 
 // All blocks of an update in one launch: the run's own work first, then the
@@ -1352,22 +1365,20 @@ constexpr int kWholeH = 9, kWholeE = 7, kWholeELarge = 8;
 __global__ void __launch_bounds__(kBlock, kWholeH) k_whole_h(const StepArgs a, const Whole l, const RunArgs r) {
     chain_next();
     if ((int)blockIdx.x < r.first) {
-        chain_wait();
-        begin_step(a, r);
+        begin_step(a, r, chain_wait);
         return;
     }
     int i, comp;
     RowPos p;
     const int kind = whole_place<false>(a, l, (int)blockIdx.x - r.first, i, comp, p);
-    chain_wait();
     if (kind == 2) {
-        if (comp == 0) h_vec<0>(a, i, p);
-        else if (comp == 1) h_vec<1>(a, i, p);
-        else h_vec<2>(a, i, p);
+        if (comp == 0) h_vec<0>(a, i, p, chain_wait);
+        else if (comp == 1) h_vec<1>(a, i, p, chain_wait);
+        else h_vec<2>(a, i, p, chain_wait);
     } else {
-        if (comp == 0) h_lean<0>(a, i, p);
-        else if (comp == 1) h_lean<1>(a, i, p);
-        else h_lean<2>(a, i, p);
+        if (comp == 0) h_lean<0>(a, i, p, chain_wait);
+        else if (comp == 1) h_lean<1>(a, i, p, chain_wait);
+        else h_lean<2>(a, i, p, chain_wait);
     }
 }
 
@@ -1377,28 +1388,25 @@ __global__ void __launch_bounds__(kBlock, P > 8 ? 4 : B)
     chain_next();
     if ((int)blockIdx.x < r.first) {   // H samples, then the surface-impedance edges (their E is left alone below)
         const int e = ((int)blockIdx.x - 1) * kBlock + threadIdx.x;
-        chain_wait();
-        if (blockIdx.x == 0) sample_family(a, r, 1, r.at[0]);
-        else if (e < s.ns) sibc_edge(s, e);
+        if (blockIdx.x == 0) sample_family(a, r, 1, chain_wait);
+        else if (e < s.ns) sibc_edge(s, e, chain_wait);
         return;
     }
     int i, comp;
     RowPos p;
     const int kind = whole_place<true>(a, l, (int)blockIdx.x - r.first, i, comp, p);
-    chain_wait();
-    const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
     if (kind == 2) {
-        if (comp == 0) e_vec<0, P>(a, i, p, sv, r.skip);
-        else if (comp == 1) e_vec<1, P>(a, i, p, sv, r.skip);
-        else e_vec<2, P>(a, i, p, sv, r.skip);
+        if (comp == 0) e_vec<0, P>(a, i, p, r.skip, chain_wait);
+        else if (comp == 1) e_vec<1, P>(a, i, p, r.skip, chain_wait);
+        else e_vec<2, P>(a, i, p, r.skip, chain_wait);
     } else if (P > 0 && kind == 1) {
-        if (comp == 0) e_debye<0, P>(a, i, p, sv, r.skip);
-        else if (comp == 1) e_debye<1, P>(a, i, p, sv, r.skip);
-        else e_debye<2, P>(a, i, p, sv, r.skip);
+        if (comp == 0) e_debye<0, P>(a, i, p, r.skip, chain_wait);
+        else if (comp == 1) e_debye<1, P>(a, i, p, r.skip, chain_wait);
+        else e_debye<2, P>(a, i, p, r.skip, chain_wait);
     } else {
-        if (comp == 0) e_lean<0>(a, i, p, sv, r.skip);
-        else if (comp == 1) e_lean<1>(a, i, p, sv, r.skip);
-        else e_lean<2>(a, i, p, sv, r.skip);
+        if (comp == 0) e_lean<0>(a, i, p, r.skip, chain_wait);
+        else if (comp == 1) e_lean<1>(a, i, p, r.skip, chain_wait);
+        else e_lean<2>(a, i, p, r.skip, chain_wait);
     }
 }
 
@@ -1625,7 +1633,7 @@ const WKernel kEWLarge[] = {k_whole_e<0, kWholeELarge>, k_whole_e<1, kWholeELarg
 
 __global__ void __launch_bounds__(kBlock) k_sibc(const SibcArgs a) {
     const int e = blockIdx.x * kBlock + threadIdx.x;
-    if (e < a.ns) sibc_edge(a, e);
+    if (e < a.ns) sibc_edge(a, e, [] {});
 }
 
 // ------------------------------------------------- probes, ports, DFT ring
@@ -1702,8 +1710,8 @@ __device__ __forceinline__ void post_block(const PostArgs &a) {
 __global__ void __launch_bounds__(kPostThreads) k_post(const PostArgs a) { post_block(a); }
 
 // the same as a launch of its own, where no update launch carries it
-__global__ void __launch_bounds__(kBlock) k_begin_step(const StepArgs a, const RunArgs r) { begin_step(a, r); }
-__global__ void __launch_bounds__(kBlock) k_sample_h(const StepArgs a, const RunArgs r) { sample_family(a, r, 1, r.at[0]); }
+__global__ void __launch_bounds__(kBlock) k_begin_step(const StepArgs a, const RunArgs r) { begin_step(a, r, [] {}); }
+__global__ void __launch_bounds__(kBlock) k_sample_h(const StepArgs a, const RunArgs r) { sample_family(a, r, 1, [] {}); }
 
 // before a run: its step count to zero, the source values of its steps
 __global__ void k_run_begin(const RunArgs r, const PostArgs p, float *src, int steps, long long step0) {
