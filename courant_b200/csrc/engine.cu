@@ -638,53 +638,71 @@ __device__ __forceinline__ float4 term(const float4 &d, const float4 &c, float d
     return t;
 }
 
-// H component C at points k4 .. k4+3 of row (i, j) from the E values there
-// (e2 = E_{C+2}, e1 = E_{C+1}) and one step along the derivative axes (e2n
-// along C+1, e1n along C+2), h the old H, w from h_where; the new H goes to
-// hq.
+// What the H update of four points takes from tables that no launch writes:
+// coefficients of the derivative axes, the points the component has (own), those
+// with an auxiliary on each axis (in1, in2), where these lie (x1, x2) and their
+// recursions' coefficients.
+struct HTables {
+    float4 c1, c2, b1, b2, d1, d2;
+    int x1, x2;
+    unsigned own, in1, in2;
+};
+
 template <int C>
-__device__ __forceinline__ void h_points(const StepArgs &a, int i, int j, int k4, float *hq, const Where &w,
-                                         const float4 &e2, const float4 &e2n, const float4 &e1, const float4 &e1n,
-                                         float4 h) {
+__device__ __forceinline__ HTables h_tables(const StepArgs &a, int i, int j, int k4, const Where &w) {
     constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
-    constexpr bool kz = A1 == 2 || A2 == 2;
-    const int nx = a.g.n[0], ny = a.g.n[1], nz = a.g.n[2];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float ci = __ldg(a.hc[0] + min(i, nx - 1)), cj = __ldg(a.hc[1] + min(j, ny - 1));
-    const float4 ck = ldg4(a.hc[2] + k4);
-    const float4 c1 = A1 == 0 ? all4(ci) : (A1 == 1 ? all4(cj) : ck), c2 = A2 == 0 ? all4(ci) : (A2 == 1 ? all4(cj) : ck);
-    const int last = kz ? nz : nz + 1;
-    const unsigned own = k4 + 4 > last ? (1u << max(last - k4, 0)) - 1u : 15u;
+    float ci = 0.f, cj = 0.f;
+    float4 ck = z4;
+    if (A1 == 0 || A2 == 0) ci = __ldg(a.hc[0] + i);
+    if (A1 == 1 || A2 == 1) cj = __ldg(a.hc[1] + j);
+    if (A1 == 2 || A2 == 2) ck = ldg4(a.hc[2] + k4);
+    HTables t{};
+    t.c1 = A1 == 0 ? all4(ci) : (A1 == 1 ? all4(cj) : ck);
+    t.c2 = A2 == 0 ? all4(ci) : (A2 == 1 ? all4(cj) : ck);
+    const int last = A1 == 2 || A2 == 2 ? a.g.n[2] : a.g.n[2] + 1;
+    t.own = k4 + 4 > last ? (1u << max(last - k4, 0)) - 1u : 15u;
     const unsigned inz = (w.pk.x >= 0 ? 1u : 0u) | (w.pk.y >= 0 ? 2u : 0u) | (w.pk.z >= 0 ? 4u : 0u) | (w.pk.w >= 0 ? 8u : 0u);
     const int pa[3] = {w.pi, w.pj, inz ? 0 : -1};
-    const unsigned in1 = (A1 == 2 ? inz : (pa[A1] >= 0 ? 15u : 0u)) & own, in2 = (A2 == 2 ? inz : (pa[A2] >= 0 ? 15u : 0u)) & own;
-    // auxiliaries: all loads before the arithmetic
-    float4 s1 = z4, s2 = z4, b1 = z4, b2 = z4, d1 = z4, d2 = z4;
-    int x1 = 0, x2 = 0;
-    if (in1) {
-        x1 = psi_at<A1, false>(a, pa[A1], i, j, k4);
-        s1 = ld4(a.psiH[C][0] + x1);
-        b1 = A1 == 2 ? ldg4(a.pml[2].bm1_h + k4) : all4(__ldg(a.pml[A1].bm1_h + (A1 == 0 ? i : j)));
-        d1 = A1 == 2 ? ldg4(a.pml[2].cid_h + k4) : all4(__ldg(a.pml[A1].cid_h + (A1 == 0 ? i : j)));
+    t.in1 = (A1 == 2 ? inz : (pa[A1] >= 0 ? 15u : 0u)) & t.own;
+    t.in2 = (A2 == 2 ? inz : (pa[A2] >= 0 ? 15u : 0u)) & t.own;
+    t.b1 = t.b2 = t.d1 = t.d2 = z4;
+    if (t.in1) {
+        t.x1 = psi_at<A1, false>(a, pa[A1], i, j, k4);
+        t.b1 = A1 == 2 ? ldg4(a.pml[2].bm1_h + k4) : all4(__ldg(a.pml[A1].bm1_h + (A1 == 0 ? i : j)));
+        t.d1 = A1 == 2 ? ldg4(a.pml[2].cid_h + k4) : all4(__ldg(a.pml[A1].cid_h + (A1 == 0 ? i : j)));
     }
-    if (in2) {
-        x2 = psi_at<A2, false>(a, pa[A2], i, j, k4);
-        s2 = ld4(a.psiH[C][1] + x2);
-        b2 = A2 == 2 ? ldg4(a.pml[2].bm1_h + k4) : all4(__ldg(a.pml[A2].bm1_h + (A2 == 0 ? i : j)));
-        d2 = A2 == 2 ? ldg4(a.pml[2].cid_h + k4) : all4(__ldg(a.pml[A2].cid_h + (A2 == 0 ? i : j)));
+    if (t.in2) {
+        t.x2 = psi_at<A2, false>(a, pa[A2], i, j, k4);
+        t.b2 = A2 == 2 ? ldg4(a.pml[2].bm1_h + k4) : all4(__ldg(a.pml[A2].bm1_h + (A2 == 0 ? i : j)));
+        t.d2 = A2 == 2 ? ldg4(a.pml[2].cid_h + k4) : all4(__ldg(a.pml[A2].cid_h + (A2 == 0 ? i : j)));
     }
-    const float4 t1 = term<false>(sub4(e2n, e2), c1, a.dth, s1, b1, d1, in1);
-    const float4 t2 = term<false>(sub4(e1n, e1), c2, a.dth, s2, b2, d2, in2);
-    if (in1) st4(a.psiH[C][0] + x1, s1);
-    if (in2) st4(a.psiH[C][1] + x2, s2);
+    return t;
+}
+
+// H component C at points k4 .. k4+3 of row (i, j) from the E values there
+// (e2 = E_{C+2}, e1 = E_{C+1}) and one step along the derivative axes (e2n
+// along C+1, e1n along C+2), h the old H, t from h_tables; the new H goes to
+// hq. Every rounding is that of h_value.
+template <int C>
+__device__ __forceinline__ void h_points(const StepArgs &a, float *hq, const HTables &t, const float4 &e2, const float4 &e2n,
+                                         const float4 &e1, const float4 &e1n, float4 h) {
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 s1 = z4, s2 = z4;
+    if (t.in1) s1 = ld4(a.psiH[C][0] + t.x1);
+    if (t.in2) s2 = ld4(a.psiH[C][1] + t.x2);
+    const float4 t1 = term<false>(sub4(e2n, e2), t.c1, a.dth, s1, t.b1, t.d1, t.in1);
+    const float4 t2 = term<false>(sub4(e1n, e1), t.c2, a.dth, s2, t.b2, t.d2, t.in2);
+    if (t.in1) st4(a.psiH[C][0] + t.x1, s1);
+    if (t.in2) st4(a.psiH[C][1] + t.x2, s2);
     const float4 v = sub4(h, sub4(t1, t2));
-    if (own == 15u) h = v;
-    else pick4(h, v, own);
+    if (t.own == 15u) h = v;
+    else pick4(h, v, t.own);
     st4(hq, h);
 }
 
-// The same point by point: auxiliaries and coefficients are fetched as they are
-// used, which takes fewer registers.
+// The same point by point, w from h_where: auxiliaries and coefficients are
+// fetched as they are used, which takes fewer registers.
 template <int C>
 __device__ __forceinline__ void h_points_each(const StepArgs &a, int i, int j, int k4, float *hq, const Where &w,
                                          const float4 &e2, const float4 &e2n, const float4 &e1, const float4 &e1n,
@@ -743,7 +761,8 @@ __device__ __forceinline__ void h_points_each(const StepArgs &a, int i, int j, i
 // for more than a shorter chain (z tails and general blocks of large grids with
 // h_points: 10.9 M-cell board 331 -> 335 us per step). The launches of small grids
 // are bound by their threads' chains: h_points_each there 6.8 instead of 6.2 us per
-// step on the lossy scene, 10.5 instead of 9.9 on the 121 x 62 x 40 line.
+// step on the lossy scene, 10.5 instead of 9.9 on the 121 x 62 x 40 line; h_tables
+// after the wait 5.2 instead of 4.8 and 8.8 instead of 8.65.
 template <int C, bool Each = false, class Wait>
 __device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r, Wait wait) {
     const int j = r.j, k4 = r.k4;
@@ -760,6 +779,8 @@ __device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r,
     float *H = a.H[C];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 e2 = z4, e1 = z4, h = z4, e2n = z4, e1n = z4;
+    HTables t{};
+    if (!Each && row) t = h_tables<C>(a, i, j, k4, w);
     wait();
     if (row) {
         e2 = ld4(E2 + q);
@@ -775,7 +796,7 @@ __device__ __forceinline__ void h_vec(const StepArgs &a, int i, const RowPos &r,
     if (A2 == 2) e1n = next_k(e1, E1 + q, row && k4 + 4 <= nz, edge);
     if (!row) return;
     if (Each) h_points_each<C>(a, i, j, k4, H + q, w, e2, e2n, e1, e1n, h);
-    else h_points<C>(a, i, j, k4, H + q, w, e2, e2n, e1, e1n, h);
+    else h_points<C>(a, H + q, t, e2, e2n, e1, e1n, h);
 }
 
 // E component C of four points from the curl: t per point (ca-1, cb, cs,
