@@ -925,54 +925,78 @@ __device__ __forceinline__ Where e_where(const StepArgs &a, int i, int j, int k4
     return w;
 }
 
+// As HTables for E, w from e_where.
+struct ETables {
+    float4 c1, c2, b1, b2, d1, d2;
+    int x1, x2;
+    unsigned own, in1, in2;
+};
+
+template <int C>
+__device__ __forceinline__ ETables e_tables(const StepArgs &a, int i, int j, int k4, const Where &w) {
+    constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int nz = a.g.n[2];
+    float ci = 0.f, cj = 0.f;
+    float4 ck = z4;
+    if (A1 == 0 || A2 == 0) ci = __ldg(a.ec[0] + i);
+    if (A1 == 1 || A2 == 1) cj = __ldg(a.ec[1] + j);
+    if (A1 == 2 || A2 == 2) ck = ldg4(a.ec[2] + k4);
+    ETables t{};
+    t.c1 = A1 == 0 ? all4(ci) : (A1 == 1 ? all4(cj) : ck);
+    t.c2 = A2 == 0 ? all4(ci) : (A2 == 1 ? all4(cj) : ck);
+    t.own = k4 + 4 > nz ? (1u << max(nz - k4, 0)) - 1u : 15u;
+    if (C != 2 && k4 == 0) t.own &= ~1u;
+    const unsigned inz = (w.pk.x >= 0 ? 1u : 0u) | (w.pk.y >= 0 ? 2u : 0u) | (w.pk.z >= 0 ? 4u : 0u) | (w.pk.w >= 0 ? 8u : 0u);
+    const int pa[3] = {w.pi, w.pj, inz ? 0 : -1};
+    t.in1 = (A1 == 2 ? inz : (pa[A1] >= 0 ? 15u : 0u)) & t.own;
+    t.in2 = (A2 == 2 ? inz : (pa[A2] >= 0 ? 15u : 0u)) & t.own;
+    t.b1 = t.b2 = t.d1 = t.d2 = z4;
+    if (t.in1) {
+        t.x1 = psi_at<A1, true>(a, pa[A1], i, j, k4);
+        t.b1 = A1 == 2 ? ldg4(a.pml[2].bm1_e + k4) : all4(__ldg(a.pml[A1].bm1_e + (A1 == 0 ? i : j)));
+        t.d1 = A1 == 2 ? ldg4(a.pml[2].cid_e + k4) : all4(__ldg(a.pml[A1].cid_e + (A1 == 0 ? i : j)));
+    }
+    if (t.in2) {
+        t.x2 = psi_at<A2, true>(a, pa[A2], i, j, k4);
+        t.b2 = A2 == 2 ? ldg4(a.pml[2].bm1_e + k4) : all4(__ldg(a.pml[A2].bm1_e + (A2 == 0 ? i : j)));
+        t.d2 = A2 == 2 ? ldg4(a.pml[2].cid_e + k4) : all4(__ldg(a.pml[A2].cid_e + (A2 == 0 ? i : j)));
+    }
+    return t;
+}
+
 // E component C at points k4 .. k4+3 of row (i, j) from the H values there
 // (h2 = H_{C+2}, h1 = H_{C+1}) and one step back along the derivative axes
 // (h2m along C+1, h1m along C+2), the old E ev and the material indices mv,
-// w from e_where; the new E goes to E[C] + q. Points with no CPML on a derivative
-// axis take no auxiliaries, those outside the Debye box no currents.
+// t from e_tables, jo4 from e_where; the new E goes to E[C] + q. Points with no
+// CPML on a derivative axis take no auxiliaries, those outside the Debye box no
+// currents.
 template <int C, int P>
-__device__ __forceinline__ void e_points(const StepArgs &a, int i, int j, int k4, int q, const Where &w,
+__device__ __forceinline__ void e_points(const StepArgs &a, int j, int k4, int q, const ETables &t, int jo4,
                                          const float4 &h2, const float4 &h2m, const float4 &h1, const float4 &h1m,
                                          const float4 &ev, const uint2 mv, const float2 sv, unsigned skip) {
-    constexpr int A1 = (C + 1) % 3, A2 = (C + 2) % 3;
-    const int nz = a.g.n[2];
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float ci = __ldg(a.ec[0] + i), cj = __ldg(a.ec[1] + j);
-    const float4 ck = ldg4(a.ec[2] + k4);
-    const float4 c1 = A1 == 0 ? all4(ci) : (A1 == 1 ? all4(cj) : ck), c2 = A2 == 0 ? all4(ci) : (A2 == 1 ? all4(cj) : ck);
-    unsigned own = k4 + 4 > nz ? (1u << max(nz - k4, 0)) - 1u : 15u;
-    if (C != 2 && k4 == 0) own &= ~1u;
-    const unsigned inz = (w.pk.x >= 0 ? 1u : 0u) | (w.pk.y >= 0 ? 2u : 0u) | (w.pk.z >= 0 ? 4u : 0u) | (w.pk.w >= 0 ? 8u : 0u);
-    const int pa[3] = {w.pi, w.pj, inz ? 0 : -1};
-    const unsigned in1 = (A1 == 2 ? inz : (pa[A1] >= 0 ? 15u : 0u)) & own, in2 = (A2 == 2 ? inz : (pa[A2] >= 0 ? 15u : 0u)) & own;
     // auxiliaries and currents: all loads before the arithmetic
-    float4 s1 = z4, s2 = z4, b1 = z4, b2 = z4, d1 = z4, d2 = z4;
-    int x1 = 0, x2 = 0;
-    if (in1) {
-        x1 = psi_at<A1, true>(a, pa[A1], i, j, k4);
-        s1 = ld4(a.psiE[C][0] + x1);
-        b1 = A1 == 2 ? ldg4(a.pml[2].bm1_e + k4) : all4(__ldg(a.pml[A1].bm1_e + (A1 == 0 ? i : j)));
-        d1 = A1 == 2 ? ldg4(a.pml[2].cid_e + k4) : all4(__ldg(a.pml[A1].cid_e + (A1 == 0 ? i : j)));
-    }
-    if (in2) {
-        x2 = psi_at<A2, true>(a, pa[A2], i, j, k4);
-        s2 = ld4(a.psiE[C][1] + x2);
-        b2 = A2 == 2 ? ldg4(a.pml[2].bm1_e + k4) : all4(__ldg(a.pml[A2].bm1_e + (A2 == 0 ? i : j)));
-        d2 = A2 == 2 ? ldg4(a.pml[2].cid_e + k4) : all4(__ldg(a.pml[A2].cid_e + (A2 == 0 ? i : j)));
-    }
+    float4 s1 = z4, s2 = z4;
+    if (t.in1) s1 = ld4(a.psiE[C][0] + t.x1);
+    if (t.in2) s2 = ld4(a.psiE[C][1] + t.x2);
     float4 J[P > 0 ? P : 1];
     const int jvol = P > 0 ? jbox_volume<C>(a) : 0;
 #pragma unroll
-    for (int p = 0; p < P; p++) J[p] = w.jo4 >= 0 ? ld4(a.J[C] + jaddr(jvol, p, w.jo4)) : z4;
-    const float4 t1 = term<true>(sub4(h2, h2m), c1, 0.f, s1, b1, d1, in1);
-    const float4 t2 = term<true>(sub4(h1, h1m), c2, 0.f, s2, b2, d2, in2);
-    if (in1) st4(a.psiE[C][0] + x1, s1);
-    if (in2) st4(a.psiE[C][1] + x2, s2);
-    e_four<C, P>(a, j, k4, q, ev, sub4(t1, t2), mv, own, w.jo4, J, sv, skip);
+    for (int p = 0; p < P; p++) J[p] = jo4 >= 0 ? ld4(a.J[C] + jaddr(jvol, p, jo4)) : z4;
+    const float4 t1 = term<true>(sub4(h2, h2m), t.c1, 0.f, s1, t.b1, t.d1, t.in1);
+    const float4 t2 = term<true>(sub4(h1, h1m), t.c2, 0.f, s2, t.b2, t.d2, t.in2);
+    if (t.in1) st4(a.psiE[C][0] + t.x1, s1);
+    if (t.in2) st4(a.psiE[C][1] + t.x2, s2);
+    e_four<C, P>(a, j, k4, q, ev, sub4(t1, t2), mv, t.own, jo4, J, sv, skip);
 }
 
-// E component C on points k4 .. k4+3 of row (i, j) (segment [ks, ke))
-template <int C, int P, class Wait>
+// E component C on points k4 .. k4+3 of row (i, j) (segment [ks, ke)). Early: the
+// tables before the wait, for the launches of small grids (parity scene 4.4 to 3.8
+// us per step, lossy scene 4.8 to 4.5, 121 x 62 x 40 line 8.8 to 8.7); not the
+// coefficients of the material table, whose registers cost the lean blocks of the
+// same launch more (line 9.4, 250 k-cell board 12.1 against 11.7).
+template <int C, int P, bool Early, class Wait>
 __device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r, unsigned skip, Wait wait) {
     const int j = r.j, k4 = r.k4;
     const int m = j * a.g.sj + k4;
@@ -990,6 +1014,8 @@ __device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r,
     float4 h2 = z4, h1 = z4, ev = z4, h2m = z4, h1m = z4;
     uint2 mv = make_uint2(0, 0);
     if (row) mv = __ldg(reinterpret_cast<const uint2 *>(a.mat[C] + q));
+    ETables t{};
+    if (Early && row) t = e_tables<C>(a, i, j, k4, w);
     wait();
     const float2 sv = *reinterpret_cast<const float2 *>(a.srcv);
     if (row) {
@@ -1005,7 +1031,8 @@ __device__ __forceinline__ void e_vec(const StepArgs &a, int i, const RowPos &r,
     if (A1 == 2) h2m = prev_k(h2, H2 + q, row && k4 > 0, edge);
     if (A2 == 2) h1m = prev_k(h1, H1 + q, row && k4 > 0, edge);
     if (!row) return;
-    e_points<C, P>(a, i, j, k4, q, w, h2, h2m, h1, h1m, ev, mv, sv, skip);
+    if (!Early) t = e_tables<C>(a, i, j, k4, w);
+    e_points<C, P>(a, j, k4, q, t, w.jo4, h2, h2m, h1, h1m, ev, mv, sv, skip);
 }
 
 // Where of a z-tail group: lean rows lie on interior planes outside the y
@@ -1095,7 +1122,7 @@ __device__ __forceinline__ void e_lean(const StepArgs &a, int i, const RowPos &p
     if (A2 == 2) h1m = prev_k(h1, H1 + q, row && k4 > 0, p.first);
     if (!row) return;
     if (kz && p.tail) {
-        e_points<C, 0>(a, i, j, k4, q, ztail_where(a.pml[2].plane_e, k4), h2, h2m, h1, h1m, ev, mv, sv, skip);
+        e_points<C, 0>(a, j, k4, q, e_tables<C>(a, i, j, k4, ztail_where(a.pml[2].plane_e, k4)), -1, h2, h2m, h1, h1m, ev, mv, sv, skip);
         return;
     }
     const float ci = __ldg(a.ec[0] + i), cj = __ldg(a.ec[1] + j);
@@ -1150,7 +1177,7 @@ __device__ __forceinline__ void e_debye(const StepArgs &a, int i, const RowPos &
     if (!row) return;
     // a z tail above the box (tails exist only where no box reaches a z slab)
     if (kz && p.tail) {
-        e_points<C, 0>(a, i, j, k4, q, ztail_where(a.pml[2].plane_e, k4), h2, h2m, h1, h1m, ev, mv, sv, skip);
+        e_points<C, 0>(a, j, k4, q, e_tables<C>(a, i, j, k4, ztail_where(a.pml[2].plane_e, k4)), -1, h2, h2m, h1, h1m, ev, mv, sv, skip);
         return;
     }
     const float ci = __ldg(a.ec[0] + i), cj = __ldg(a.ec[1] + j);
@@ -1235,9 +1262,10 @@ __device__ __forceinline__ void begin_step(const StepArgs &a, const RunArgs &r, 
 // Resident blocks (of kBlock threads) per SM the update kernels are
 // compiled for: register caps of 51 and 64 per thread for the general H and
 // E kernels at the default 10 and 8 (the rarer CPML and Debye paths spill a
-// little), 40 and 64 for the lean ones at 12 and 8 (the z-tail path of the
+// little), 40 and 56 for the lean ones at 12 and 9 (the z-tail path of the
 // lean kernels fits without spilling; at 16 and 10 it spills, and on the
-// large board the step is 5% slower)
+// large board the step is 5% slower; E at 8 with 64: 5.7 M-cell line 124.6
+// us per step against 120)
 #ifndef CB2_H_MINBLOCKS
 #define CB2_H_MINBLOCKS 10
 #endif
@@ -1249,7 +1277,7 @@ __device__ __forceinline__ void begin_step(const StepArgs &a, const RunArgs &r, 
 #define CB2_HF_MINBLOCKS 12
 #endif
 #ifndef CB2_EF_MINBLOCKS
-#define CB2_EF_MINBLOCKS 8
+#define CB2_EF_MINBLOCKS 9
 #endif
 
 // Chained launches (RunArgs::on): a launch that follows another on one stream
@@ -1261,40 +1289,46 @@ __device__ __forceinline__ void begin_step(const StepArgs &a, const RunArgs &r, 
 // plain loads for that: they change within the launch's life. The wait makes the
 // other's writes visible; the read-only path promises nothing there.) Parity
 // scene 6.8 to 5.9 us per step, lossy scene 8.2 to 6.9, cavity 5.8 to 5.4; with the
-// tables before the wait, 5.35 to 4.85, 6.25 to 5.3 and 5.0 to 4.65, 121 x 62 x 40
-// line 9.9 to 8.8, 250 k-cell board 12.5 to 11.7.
+// tables before the wait, 5.35 to 3.8, 6.25 to 4.5 and 5.0 to 4.6, 121 x 62 x 40
+// line 9.9 to 8.7, 250 k-cell board 12.5 to 11.6.
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+struct Chained {
+    __device__ __forceinline__ void operator()() const { chain_wait(); }
+};
+struct AtOnce {
+    __device__ __forceinline__ void operator()() const {}
+};
 
 // H on the fast rectangles of node planes [i0, i0 + gridDim.y); block x:
 // block x / 3 of the space, component x % 3
 __global__ void __launch_bounds__(kBlock, CB2_HF_MINBLOCKS) k_update_h_fast(const StepArgs a, int i0, const RunArgs r) {
     chain_next();
     if (r.first && blockIdx.x == gridDim.x - 1) {   // one column more: the run's own work
-        if (blockIdx.y == 0) begin_step(a, r, chain_wait);
+        if (blockIdx.y == 0) begin_step(a, r, Chained{});
         return;
     }
     const int comp = blockIdx.x % 3;
     const RowPos p = space_pos(a.item[0][kFast], blockIdx.x / 3);
     const int i = i0 + blockIdx.y;
-    if (comp == 0) h_lean<0>(a, i, p, chain_wait);
-    else if (comp == 1) h_lean<1>(a, i, p, chain_wait);
-    else h_lean<2>(a, i, p, chain_wait);
+    if (comp == 0) h_lean<0>(a, i, p, Chained{});
+    else if (comp == 1) h_lean<1>(a, i, p, Chained{});
+    else h_lean<2>(a, i, p, Chained{});
 }
 
 // E on the fast rectangles of node planes [i0, i0 + gridDim.y), from the last to the first
 __global__ void __launch_bounds__(kBlock, CB2_EF_MINBLOCKS) k_update_e_fast(const StepArgs a, int i0, const RunArgs r) {
     chain_next();
     if (r.first && blockIdx.x == gridDim.x - 1) {
-        if (blockIdx.y == 0) sample_family(a, r, 1, chain_wait);
+        if (blockIdx.y == 0) sample_family(a, r, 1, Chained{});
         return;
     }
     const int comp = blockIdx.x % 3;
     const RowPos p = space_pos(a.item[1][kFast], blockIdx.x / 3);
     const int i = i0 + (int)(gridDim.y - 1 - blockIdx.y);   // E begins where H ended, on what L2 still holds
-    if (comp == 0) e_lean<0>(a, i, p, r.skip, chain_wait);
-    else if (comp == 1) e_lean<1>(a, i, p, r.skip, chain_wait);
-    else e_lean<2>(a, i, p, r.skip, chain_wait);
+    if (comp == 0) e_lean<0>(a, i, p, r.skip, Chained{});
+    else if (comp == 1) e_lean<1>(a, i, p, r.skip, Chained{});
+    else e_lean<2>(a, i, p, r.skip, Chained{});
 }
 
 // Position in the general space of update U: the general rectangles on an
@@ -1309,15 +1343,15 @@ __device__ __forceinline__ RowPos general_pos(const StepArgs &a, int i, int b) {
 __global__ void __launch_bounds__(kBlock, CB2_H_MINBLOCKS) k_update_h(const StepArgs a, const int2 *work, const RunArgs r) {
     chain_next();
     if ((int)blockIdx.x < r.first) {
-        begin_step(a, r, chain_wait);
+        begin_step(a, r, Chained{});
         return;
     }
     const int2 w = work[blockIdx.x - r.first];
     const int comp = w.y % 3;
     const RowPos p = general_pos<0>(a, w.x, w.y / 3);
-    if (comp == 0) h_vec<0, true>(a, w.x, p, chain_wait);
-    else if (comp == 1) h_vec<1, true>(a, w.x, p, chain_wait);
-    else h_vec<2, true>(a, w.x, p, chain_wait);
+    if (comp == 0) h_vec<0, true>(a, w.x, p, Chained{});
+    else if (comp == 1) h_vec<1, true>(a, w.x, p, Chained{});
+    else h_vec<2, true>(a, w.x, p, Chained{});
 }
 
 // E over the general blocks (no Debye poles)
@@ -1326,16 +1360,16 @@ __global__ void __launch_bounds__(kBlock, CB2_E_MINBLOCKS)
     chain_next();
     if ((int)blockIdx.x < r.first) {   // H samples, then the surface-impedance edges (their E is left alone below)
         const int e = ((int)blockIdx.x - 1) * kBlock + threadIdx.x;
-        if (blockIdx.x == 0) sample_family(a, r, 1, chain_wait);
-        else if (e < s.ns) sibc_edge(s, e, chain_wait);
+        if (blockIdx.x == 0) sample_family(a, r, 1, Chained{});
+        else if (e < s.ns) sibc_edge(s, e, Chained{});
         return;
     }
     const int2 w = work[gridDim.x - 1 - blockIdx.x];
     const int comp = w.y % 3;
     const RowPos p = general_pos<1>(a, w.x, w.y / 3);
-    if (comp == 0) e_vec<0, 0>(a, w.x, p, r.skip, chain_wait);
-    else if (comp == 1) e_vec<1, 0>(a, w.x, p, r.skip, chain_wait);
-    else e_vec<2, 0>(a, w.x, p, r.skip, chain_wait);
+    if (comp == 0) e_vec<0, 0, false>(a, w.x, p, r.skip, Chained{});
+    else if (comp == 1) e_vec<1, 0, false>(a, w.x, p, r.skip, Chained{});
+    else e_vec<2, 0, false>(a, w.x, p, r.skip, Chained{});
 }
 
 // All blocks of an update in one launch: the run's own work first, then the
@@ -1379,27 +1413,28 @@ __device__ __forceinline__ int whole_place(const StepArgs &a, const Whole &l, in
 
 // resident blocks per SM: 56 registers for H (48 and 64: 250 k-cell board 13.3 and 12.8
 // us per step against 12.4); for E 72, or 64 on large grids of up
-// to four poles (they spill a little on the CPML paths there, but a bandwidth-bound
-// launch gains more from the eighth block: 334 against 341 us per step on the
-// 10.9 M-cell board; 13.1 against 15.1 the other way on the 250 k-cell one)
-constexpr int kWholeH = 9, kWholeE = 7, kWholeELarge = 8;
+// to six poles (they spill on the CPML paths there, but a bandwidth-bound launch
+// gains more from the eighth block: 334 against 341 us per step on the 10.9 M-cell
+// board of four poles, 98.4 against 100 on the 3.6 M-cell line of six; 13.1 against
+// 15.1 the other way on the 250 k-cell board)
+constexpr int kWholeH = 9, kWholeE = 7, kWholeELarge = 8, kLargePoles = 6;
 __global__ void __launch_bounds__(kBlock, kWholeH) k_whole_h(const StepArgs a, const Whole l, const RunArgs r) {
     chain_next();
     if ((int)blockIdx.x < r.first) {
-        begin_step(a, r, chain_wait);
+        begin_step(a, r, Chained{});
         return;
     }
     int i, comp;
     RowPos p;
     const int kind = whole_place<false>(a, l, (int)blockIdx.x - r.first, i, comp, p);
     if (kind == 2) {
-        if (comp == 0) h_vec<0>(a, i, p, chain_wait);
-        else if (comp == 1) h_vec<1>(a, i, p, chain_wait);
-        else h_vec<2>(a, i, p, chain_wait);
+        if (comp == 0) h_vec<0>(a, i, p, Chained{});
+        else if (comp == 1) h_vec<1>(a, i, p, Chained{});
+        else h_vec<2>(a, i, p, Chained{});
     } else {
-        if (comp == 0) h_lean<0>(a, i, p, chain_wait);
-        else if (comp == 1) h_lean<1>(a, i, p, chain_wait);
-        else h_lean<2>(a, i, p, chain_wait);
+        if (comp == 0) h_lean<0>(a, i, p, Chained{});
+        else if (comp == 1) h_lean<1>(a, i, p, Chained{});
+        else h_lean<2>(a, i, p, Chained{});
     }
 }
 
@@ -1409,25 +1444,25 @@ __global__ void __launch_bounds__(kBlock, P > 8 ? 4 : B)
     chain_next();
     if ((int)blockIdx.x < r.first) {   // H samples, then the surface-impedance edges (their E is left alone below)
         const int e = ((int)blockIdx.x - 1) * kBlock + threadIdx.x;
-        if (blockIdx.x == 0) sample_family(a, r, 1, chain_wait);
-        else if (e < s.ns) sibc_edge(s, e, chain_wait);
+        if (blockIdx.x == 0) sample_family(a, r, 1, Chained{});
+        else if (e < s.ns) sibc_edge(s, e, Chained{});
         return;
     }
     int i, comp;
     RowPos p;
     const int kind = whole_place<true>(a, l, (int)blockIdx.x - r.first, i, comp, p);
     if (kind == 2) {
-        if (comp == 0) e_vec<0, P>(a, i, p, r.skip, chain_wait);
-        else if (comp == 1) e_vec<1, P>(a, i, p, r.skip, chain_wait);
-        else e_vec<2, P>(a, i, p, r.skip, chain_wait);
+        if (comp == 0) e_vec<0, P, B == kWholeE>(a, i, p, r.skip, Chained{});
+        else if (comp == 1) e_vec<1, P, B == kWholeE>(a, i, p, r.skip, Chained{});
+        else e_vec<2, P, B == kWholeE>(a, i, p, r.skip, Chained{});
     } else if (P > 0 && kind == 1) {
-        if (comp == 0) e_debye<0, P>(a, i, p, r.skip, chain_wait);
-        else if (comp == 1) e_debye<1, P>(a, i, p, r.skip, chain_wait);
-        else e_debye<2, P>(a, i, p, r.skip, chain_wait);
+        if (comp == 0) e_debye<0, P>(a, i, p, r.skip, Chained{});
+        else if (comp == 1) e_debye<1, P>(a, i, p, r.skip, Chained{});
+        else e_debye<2, P>(a, i, p, r.skip, Chained{});
     } else {
-        if (comp == 0) e_lean<0>(a, i, p, r.skip, chain_wait);
-        else if (comp == 1) e_lean<1>(a, i, p, r.skip, chain_wait);
-        else e_lean<2>(a, i, p, r.skip, chain_wait);
+        if (comp == 0) e_lean<0>(a, i, p, r.skip, Chained{});
+        else if (comp == 1) e_lean<1>(a, i, p, r.skip, Chained{});
+        else e_lean<2>(a, i, p, r.skip, Chained{});
     }
 }
 
@@ -1645,7 +1680,8 @@ using WKernel = void (*)(StepArgs, Whole, RunArgs, SibcArgs);
 const FKernel kFKernels[] = {CB2_POLES(CB2_FK)};
 const WKernel kEWKernels[] = {CB2_POLES(CB2_WK)};
 const WKernel kEWLarge[] = {k_whole_e<0, kWholeELarge>, k_whole_e<1, kWholeELarge>, k_whole_e<2, kWholeELarge>,
-                            k_whole_e<3, kWholeELarge>, k_whole_e<4, kWholeELarge>};
+                            k_whole_e<3, kWholeELarge>, k_whole_e<4, kWholeELarge>, k_whole_e<5, kWholeELarge>,
+                            k_whole_e<kLargePoles, kWholeELarge>};
 #undef CB2_FK
 #undef CB2_WK
 #undef CB2_POLES
@@ -1654,7 +1690,7 @@ const WKernel kEWLarge[] = {k_whole_e<0, kWholeELarge>, k_whole_e<1, kWholeELarg
 
 __global__ void __launch_bounds__(kBlock) k_sibc(const SibcArgs a) {
     const int e = blockIdx.x * kBlock + threadIdx.x;
-    if (e < a.ns) sibc_edge(a, e, [] {});
+    if (e < a.ns) sibc_edge(a, e, AtOnce{});
 }
 
 // ------------------------------------------------- probes, ports, DFT ring
@@ -1731,8 +1767,8 @@ __device__ __forceinline__ void post_block(const PostArgs &a) {
 __global__ void __launch_bounds__(kPostThreads) k_post(const PostArgs a) { post_block(a); }
 
 // the same as a launch of its own, where no update launch carries it
-__global__ void __launch_bounds__(kBlock) k_begin_step(const StepArgs a, const RunArgs r) { begin_step(a, r, [] {}); }
-__global__ void __launch_bounds__(kBlock) k_sample_h(const StepArgs a, const RunArgs r) { sample_family(a, r, 1, [] {}); }
+__global__ void __launch_bounds__(kBlock) k_begin_step(const StepArgs a, const RunArgs r) { begin_step(a, r, AtOnce{}); }
+__global__ void __launch_bounds__(kBlock) k_sample_h(const StepArgs a, const RunArgs r) { sample_family(a, r, 1, AtOnce{}); }
 
 // before a run: its step count to zero, the source values of its steps
 __global__ void k_run_begin(const RunArgs r, const PostArgs p, float *src, int steps, long long step0) {
@@ -3526,7 +3562,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
             carry.first = !run ? 0 : own ? 1 + (sb.ns + kBlock - 1) / kBlock : 1;
             if (D.whole_e) {
                 const Whole l = whole(1, a, b, w, n);
-                const bool large = !D.whole_h && s->npole <= 4;
+                const bool large = !D.whole_h && s->npole <= kLargePoles;
                 launch(large ? kEWLarge[s->npole] : kEWKernels[s->npole],
                        dim3(carry.first + n + (unsigned)l.planes * (l.nd + l.nf)), D.sa[D.cur], l, carry, sb);
             } else {   // no poles: no Debye rectangles
