@@ -31,6 +31,16 @@ NVFLAGS = ["-O3", "--split-compile=0", "-std=c++17", "-lineinfo", *ARCH, "-Xcomp
            "-Xptxas", "-v", f'-DCEM_VERSION="{VERSION}"', f"-I{INCLUDE}"]
 
 
+# The compiler's choices follow the addresses of its own data: of two builds of one source, one ran the 5.7 M-cell line
+# at 119 and the other at 125 us per step. With fixed addresses (where the system allows it) every build is the same.
+FIXED = ["setarch", "-R"]
+try:
+    if subprocess.run([*FIXED, "true"], capture_output=True).returncode:
+        FIXED = []
+except OSError:
+    FIXED = []
+
+
 def _run(cmd: list[str], log) -> None:
     log.write(" ".join(cmd) + "\n")
     r = subprocess.run(cmd, capture_output=True, text=True)
@@ -71,7 +81,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         for src in sources():
             out = obj / (src.stem + (".cu.o" if src.suffix == ".cu" else ".o"))
             if src.suffix == ".cu":
-                _run([NVCC, *NVFLAGS, "-c", str(src), "-o", str(out)], log)
+                _run([*FIXED, NVCC, *NVFLAGS, "-c", str(src), "-o", str(out)], log)
             else:
                 # the mode solver's band loops are plain vector loops: -O3 vectorises them
                 # (element-wise, no contraction: the same bits as -O2)
