@@ -539,8 +539,8 @@ def s_params(v1, i1, v2, i2, R):
 
 
 class Batch:
-    """Several finalized simulations advanced together on one device: batched
-    launches over a work-list across the members, graph-captured chunks.
+    """Several finalized simulations advanced together on one device, each on
+    its own stream with its own replayed graphs.
     Results stay readable through each Sim between runs."""
 
     def __init__(self, c: Courant, h):

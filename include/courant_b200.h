@@ -102,9 +102,8 @@ CEM_API int cemx_tune_state(const cem_sim *s, double *out, int n);
 CEM_API int cemx_energy_noalloc(cem_sim *s, double *energy);
 
 /* Batches (no counterpart in the reference core). A batch advances several
- * finalized simulations on one device together: every batched launch walks a
- * work-list of blocks across all members (H, E, surface impedance, probes),
- * and runs of 16 steps replay one CUDA graph captured per composition. Each member
+ * finalized simulations on one device together: each steps on its own stream
+ * with its own replayed graphs, and the GPU runs them side by side. Each member
  * computes the same bits as when stepped alone with cem_step. Members keep
  * their own device state, so results are read with the usual courant.h calls
  * between runs. A simulation belongs to at most one batch and must not be
@@ -131,13 +130,12 @@ CEM_API long cemx_batch_left(const cemx_batch *b, const cem_sim *s);
  * Returns the number of members still short of their budget, or -1. */
 CEM_API int cemx_batch_run(cemx_batch *b, long max_steps);
 
-/* on = 1: the next run picks the work-list order (member-major or plane by
- * plane across members) by timing real steps, once per batch composition per
- * process. Returns the previous setting. */
+/* Kept for callers that set it: a batch has no choice left to time. Returns
+ * the previous setting. */
 CEM_API int cemx_batch_tune(cemx_batch *b, int on);
 
 /* Statistics of the last run, n entries of: device ms, steps, launches
- * (graph launches count once), graph length, work-list order, members.
+ * (graph launches count once), graph length, 0, members.
  * Returns 0 or -1. */
 CEM_API int cemx_batch_stats(const cemx_batch *b, double *out, int n);
 
