@@ -2117,12 +2117,22 @@ struct Device {
     bool tune = false, tuned = false, tuned_from_cache = false;
     double tuned_ms = 0;
     cudaEvent_t tev[2] = {nullptr, nullptr};   // tuner timing
-    cudaGraphExec_t graph = nullptr, tail = nullptr;   // graph_steps steps; the rest of the last run
-    int tail_steps = 0;
+    // per field buffer (a graph holds the arguments of the one that was current at its
+    // capture): graph_steps steps; the rest of the last run
+    cudaGraphExec_t graph[2] = {nullptr, nullptr}, tail[2] = {nullptr, nullptr};
+    int tail_steps[2] = {0, 0};
+
+    void drop_graphs() {   // of launches that have ended
+        for (int b = 0; b < 2; b++) {
+            if (graph[b]) cudaGraphExecDestroy(graph[b]);
+            if (tail[b]) cudaGraphExecDestroy(tail[b]);
+            graph[b] = tail[b] = nullptr;
+            tail_steps[b] = 0;
+        }
+    }
 
     ~Device() {
-        if (graph) cudaGraphExecDestroy(graph);
-        if (tail) cudaGraphExecDestroy(tail);
+        drop_graphs();
         for (cudaEvent_t e : tev)
             if (e) cudaEventDestroy(e);
         if (stage_ev) { cudaEventSynchronize(stage_ev); cudaEventDestroy(stage_ev); }
@@ -3688,10 +3698,13 @@ bool capture_steps(cem_sim *s, int n, cudaGraphExec_t &exec) {
 // n whole steps, n at most Device::run_steps and the room in the sample ring:
 // source values, the steps (with graphs on, groups of graph_steps replay one
 // captured graph; the graph holds the kernels' arguments, which stay fixed for
-// the life of the device state), then the sample rows.
+// the life of the device state and of its current field buffer), then the
+// sample rows.
 bool run_chunk(cem_sim *s, long n) {
     Device &D = *s->dev;
     const PostArgs &pa = D.pa[D.cur];
+    cudaGraphExec_t &tail = D.tail[D.cur];
+    int &tail_steps = D.tail_steps[D.cur];
     const long step0 = s->step;
     D.chained = false;
     k_run_begin<<<(unsigned)((n + 127) / 128), 128, 0, D.stream>>>(D.run, pa, reinterpret_cast<float *>(D.run_src.p), (int)n,
@@ -3706,18 +3719,18 @@ bool run_chunk(cem_sim *s, long n) {
     };
     long rest = n;
     for (const int gs = D.graph_steps; D.use_graphs && rest >= gs; rest -= gs)
-        if (!replay(D.graph, gs)) return false;
+        if (!replay(D.graph[D.cur], gs)) return false;
     // what is left over: one graph too when the run before left as much (a ten-step
     // call spends 55 us of the host's time on its launches, 8 on the graph's)
-    if (rest && rest != D.tail_steps) {
-        if (D.tail) {
+    if (rest && rest != tail_steps) {
+        if (tail) {
             CB2_CHECK(s, cudaStreamSynchronize(D.stream));
-            cudaGraphExecDestroy(D.tail);
+            cudaGraphExecDestroy(tail);
         }
-        D.tail = nullptr;
-        D.tail_steps = (int)rest;
+        tail = nullptr;
+        tail_steps = (int)rest;
     } else if (rest > 2 && D.use_graphs) {
-        if (!replay(D.tail, (int)rest)) return false;
+        if (!replay(tail, (int)rest)) return false;
         rest = 0;
     }
     for (; rest > 0; rest--)
@@ -3807,10 +3820,7 @@ bool apply_shape(cem_sim *s, Device &D, int thin, bool side, int graph, bool zta
         fill_args(s, D);
     }
     if (respace || graph != D.graph_steps) {
-        if (D.graph) cudaGraphExecDestroy(D.graph);
-        if (D.tail) cudaGraphExecDestroy(D.tail);
-        D.graph = D.tail = nullptr;
-        D.tail_steps = 0;
+        D.drop_graphs();
         D.graph_steps = graph;
     }
     D.side_on = side;

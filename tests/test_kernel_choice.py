@@ -1,0 +1,27 @@
+"""The kernel choice (cemx_use_fused) in mid-run. A fused step writes the other
+one of two field buffers; what is stepped with the separate kernels afterwards,
+replayed graphs included, must go on from there."""
+import numpy as np
+import pytest
+
+from courant_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 10, 32, 75])
+def test_separate_kernels_go_on_from_a_fused_step(lib, n):
+    a, b = scenes.lossy_scene(lib)[0], scenes.lossy_scene(lib)[0]
+    a.step(n)
+    a.step(n)            # a run of this length has its graph now
+    for _ in range(2):   # to the second buffer, and back to the first
+        a.useFused(True)
+        a.step(1)
+        a.useFused(False)
+        a.step(n)
+        a.step(n)
+    for _ in range(6 * n + 2):
+        b.step(1)
+    assert a.steps == b.steps
+    assert np.array_equal(a.checkpoint(), b.checkpoint())
+    assert np.array_equal(a.portV(0), b.portV(0)) and a.energy() == b.energy()
