@@ -2191,6 +2191,20 @@ bool fail(cem_sim *s, const char *what, cudaError_t e) {
         if (e_ != cudaSuccess) return fail((s), #call, e_); \
     } while (0)
 
+// A simulation's device as the thread's current one for a scope, then the
+// caller's again: a launch on a stream needs the stream's device current, and
+// state is read by threads that are at work on another device.
+struct OnDevice {
+    int prev = -1;
+    cudaError_t err;
+    explicit OnDevice(int device) {
+        err = cudaGetDevice(&prev);
+        if (err == cudaSuccess && prev != device) err = cudaSetDevice(device);
+        else prev = -1;
+    }
+    ~OnDevice() { if (prev >= 0) cudaSetDevice(prev); }
+};
+
 // All copies and fills are ordered on the engine stream (a non-blocking
 // stream does not synchronise with the legacy default stream).
 bool h2d(cem_sim *s, void *dst, const void *src, size_t bytes) {
@@ -3362,6 +3376,8 @@ bool upload_groups(cem_sim *s, unsigned g, unsigned from_host) {
 // Groups g from the device: the spectra to the host copies, the others to `to`.
 bool download_groups(cem_sim *s, unsigned g, const StateView &to) {
     Device &D = *s->dev;
+    const OnDevice here(D.device);
+    CB2_CHECK(s, here.err);
     if ((g & kGroupDft) && !flush_dft(s)) return false;
     if ((g & kGroupDebye) && !make_jmap(s)) return false;
     Move m = state_move(s, g, to);

@@ -1,0 +1,55 @@
+"""What the engine asks of the CUDA runtime, with a runtime of two devices in
+host memory in its place (fake_cudart.cpp; kernels do not run)."""
+import ctypes
+import subprocess
+
+import numpy as np
+import pytest
+
+from courant_b200 import build, scenes
+from courant_b200.api import Courant
+
+
+class Fake:
+    def __init__(self, path):
+        self.lib = Courant(path)
+        self.so = ctypes.CDLL(str(path))
+        self.so.fake_count.restype = ctypes.c_long
+        self.so.fake_fail_copy.argtypes = [ctypes.c_long]
+
+    def count(self, what):
+        return self.so.fake_count(what.encode())
+
+    current = property(lambda self: self.so.fake_current(), lambda self, d: self.so.fake_set_current(d))
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    if build.needs_build():
+        build.build()
+    objs = [build.PKG / "_build" / (p.stem + (".cu.o" if p.suffix == ".cu" else ".o")) for p in build.sources()]
+    if not all(o.exists() for o in objs):
+        pytest.skip("the library's objects are not here")
+    out = tmp_path_factory.mktemp("fake") / "libcourant_fake.so"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wall", "-Wextra", f"-I{build.CUDA_LIB.parent / 'include'}",
+                    str(build.PKG.parent / "tests" / "fake_cudart.cpp"), *map(str, objs), "-o", str(out), "-Wl,-Bsymbolic",
+                    "-lpthread"], check=True)
+    return Fake(out)
+
+
+READS = {"field": lambda s: s.field(4), "spectrum": lambda s: s.portV(0), "checkpoint": lambda s: s.checkpoint(),
+         "release": lambda s: s.releaseDevice(), "state": lambda s: s.c.ex.cem_state_array(s.h, 2, 0, 0)}
+
+
+@pytest.mark.parametrize("read", READS)
+def test_state_is_read_from_a_thread_on_another_device(fake, read):
+    fake.current = 0
+    s = scenes.lossy_scene(fake.lib)[0]
+    s.prepareDevice(1)
+    s.step(10)
+    fake.current = 0
+    before = fake.count("k_move")
+    READS[read](s)
+    assert fake.count("k_move") > before and fake.current == 0
+    s.step(1)   # still in order
+    s.destroy()
