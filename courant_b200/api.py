@@ -389,12 +389,13 @@ class Sim:
 
     # ---- fields and state
     def field(self, comp: int) -> np.ndarray:
-        p = self.c.ex.cem_field(self.h, comp)
-        return np.ctypeslib.as_array(p, shape=(self.N,)).copy()
+        return self.fieldView(comp).copy()
 
     def fieldView(self, comp: int) -> np.ndarray:
         """Writable view of the library's host copy of a field (cem_field)."""
         p = self.c.ex.cem_field(self.h, comp)
+        if not p and 0 <= comp <= 5:
+            raise CourantError(f"field: {self.c.last_error()}")
         return np.ctypeslib.as_array(p, shape=(self.N,))
 
     def setField(self, comp: int, data):

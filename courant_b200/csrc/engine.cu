@@ -3656,7 +3656,8 @@ int engine_pull(const cem_sim *cs, unsigned groups) {
     const unsigned missing = groups & ~s->host_valid & kGroupAll;
     if (!missing) return 0;
     host_state_alloc(s, missing);
-    const unsigned from_dev = s->dev && !s->dev->failed ? missing & s->dev_valid : 0u;
+    const unsigned from_dev = s->dev ? missing & s->dev_valid : 0u;
+    if (from_dev && s->dev->failed) { set_error(s->dev->error_msg.c_str()); return -1; }
     if (from_dev && !download_groups(s, from_dev, host_view(s, from_dev))) return -1;
     // groups valid nowhere are all zero: the freshly allocated host copies
     if (missing & ~from_dev) {

@@ -279,6 +279,7 @@ int cem_mode_port_waves(cem_sim *s, int port, double *a, double *b, double *z0, 
     ModePort &p = s->mport[port];
     if (!p.solved && solve_all_ports(s)) return -1;
     const double *V0 = cem_vprobe(s, p.vp0), *V1 = cem_vprobe(s, p.vp1), *Ix = cem_iprobe(s, p.ip);
+    if (!V0 || !V1 || !Ix) return -1;
     const cem_mode_port_def &d = p.def;
     const double dx = s->d[0][d.i_mon];
     const double xmon = 0.5 * (s->node[0][d.i_mon] + s->node[0][d.i_mon + 1]);

@@ -187,7 +187,7 @@ int cem_plan_sibc(const cem_sim *s, double *idx, double *hidx, double *hw, doubl
 // Samples recorded by an external engine, folded into the DFTs exactly as the
 // reference does it (export.c:121-149), on the host in FP64.
 void cem_push_samples(cem_sim *s, int n, const double *ip, const double *vold, const double *vnew, const double *vp) {
-    if (engine_pull(s, kGroupDft)) return;
+    if (engine_pull(s, kGroupDft)) { report("cem_push_samples"); return; }
     const int nf = s->nf;
     std::vector<double> phE, phH;
     auto acc = [nf](double *a, const std::vector<double> &ph, double v) {
@@ -318,7 +318,7 @@ size_t cem_state_len(const cem_sim *s, int which, int comp, int w) {
 
 void cem_set_step(cem_sim *s, long step) {
     // the DFT ring is indexed by step: fold pending rows before renumbering
-    if (engine_has_device(s)) engine_pull(s, kGroupDft);
+    if (engine_has_device(s) && engine_pull(s, kGroupDft)) report("cem_set_step");
     s->step = step;
 }
 

@@ -747,38 +747,41 @@ int cem_finalize(cem_sim *s, double cfl) {
 
 // ---- results ------------------------------------------------------------
 
+// Pointers into groups g may go to the caller: false, with the error set, when
+// the device that holds them cannot be read.
+static bool hand_out(const cem_sim *s, unsigned g) {
+    if (engine_pull(s, g)) return false;
+    engine_expose(s, g);
+    return true;
+}
+
 const double *cem_port_v(const cem_sim *s, int p) {
     if (p < 0 || p >= (int)s->port.size() || s->port[p].V.empty()) return nullptr;
-    engine_pull(s, kGroupDft);
-    engine_expose(s, kGroupDft);
+    if (!hand_out(s, kGroupDft)) return nullptr;
     return s->port[p].V.data();
 }
 
 const double *cem_port_i(const cem_sim *s, int p) {
     if (p < 0 || p >= (int)s->port.size() || s->port[p].I.empty()) return nullptr;
-    engine_pull(s, kGroupDft);
-    engine_expose(s, kGroupDft);
+    if (!hand_out(s, kGroupDft)) return nullptr;
     return s->port[p].I.data();
 }
 
 const double *cem_source_spectrum(const cem_sim *s) {
     if (s->src_acc.empty()) return nullptr;
-    engine_pull(s, kGroupDft);
-    engine_expose(s, kGroupDft);
+    if (!hand_out(s, kGroupDft)) return nullptr;
     return s->src_acc.data();
 }
 
 const double *cem_vprobe(const cem_sim *s, int p) {
     if (p < 0 || p >= (int)s->vp.size() || s->vp[p].acc.empty()) return nullptr;
-    engine_pull(s, kGroupDft);
-    engine_expose(s, kGroupDft);
+    if (!hand_out(s, kGroupDft)) return nullptr;
     return s->vp[p].acc.data();
 }
 
 const double *cem_iprobe(const cem_sim *s, int p) {
     if (p < 0 || p >= (int)s->ip.size() || s->ip[p].acc.empty()) return nullptr;
-    engine_pull(s, kGroupDft);
-    engine_expose(s, kGroupDft);
+    if (!hand_out(s, kGroupDft)) return nullptr;
     return s->ip[p].acc.data();
 }
 
@@ -789,8 +792,7 @@ double *cem_field(cem_sim *s, int comp) {
     if (comp < 0 || comp > 5) return nullptr;
     const unsigned g = 1u << comp;
     host_state_alloc(s, g);
-    engine_pull(s, g);
-    engine_expose(s, g);
+    if (!hand_out(s, g)) return nullptr;
     return comp < 3 ? s->E[comp].data() : s->H[comp - 3].data();
 }
 

@@ -71,7 +71,10 @@ __attribute__((visibility("default"))) long fake_count(const char *what) {
             n += c.second;
     return n;
 }
-__attribute__((visibility("default"))) void fake_fail_copy(long after) { copies_left = after; }
+__attribute__((visibility("default"))) void fake_fail_copy(long after) {
+    copies_left = after;
+    last = cudaSuccess;
+}
 __attribute__((visibility("default"))) int fake_current() { return current; }
 __attribute__((visibility("default"))) void fake_set_current(int d) { current = d; }
 

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from courant_b200 import build, scenes
-from courant_b200.api import Courant
+from courant_b200.api import Courant, CourantError
 
 
 class Fake:
@@ -52,4 +52,36 @@ def test_state_is_read_from_a_thread_on_another_device(fake, read):
     READS[read](s)
     assert fake.count("k_move") > before and fake.current == 0
     s.step(1)   # still in order
+    s.destroy()
+
+
+@pytest.mark.parametrize("read", ["field", "spectrum", "checkpoint", "release"])
+def test_a_read_that_fails_is_an_error(fake, read):
+    """A copy from the device that fails, and any read of the failed device after it: no zeros in place of the state."""
+    fake.current = 0
+    s = scenes.lossy_scene(fake.lib)[0]
+    s.step(10)
+    fake.so.fake_fail_copy(0)
+    try:
+        for _ in range(2):
+            with pytest.raises(CourantError):
+                READS[read](s)
+    finally:
+        fake.so.fake_fail_copy(-1)
+    for later in (s.checkpoint, lambda: s.field(1), lambda: s.sourceSpectrum()):
+        with pytest.raises(CourantError):
+            later()
+    s.destroy()
+
+
+def test_mode_port_waves_of_a_failed_read_are_an_error(fake):
+    fake.current = 0
+    s, meta = scenes.modeport_scene(fake.lib)
+    s.step(10)
+    fake.so.fake_fail_copy(0)
+    try:
+        with pytest.raises(CourantError):
+            s.modePortWaves(meta["modeports"][0])
+    finally:
+        fake.so.fake_fail_copy(-1)
     s.destroy()
