@@ -2110,9 +2110,10 @@ struct Device {
     DevBuf<float> raw;
     DevBuf<float2> run_src;
     DevBuf<int> run_at;
-    // words that state moves pass through, on the device and on the host (kStageWords at most)
+    // words that state moves pass through, on the device and on the host (the whole state, or
+    // kStageWords of it); made with the device state, so that reading results allocates nothing there
     DevBuf<unsigned> stage;
-    std::vector<unsigned> stage_host;
+    std::unique_ptr<unsigned[]> stage_host;
     cudaEvent_t stage_ev = nullptr;
     bool tune = false, tuned = false, tuned_from_cache = false;
     double tuned_ms = 0;
@@ -3021,6 +3022,7 @@ void fill_args(cem_sim *s, Device &D) {
 }
 
 bool create_device_impl(cem_sim *s);
+bool make_stage(cem_sim *s);
 
 // a device that failed to build is dropped, so the next call starts over
 bool create_device(cem_sim *s) {
@@ -3136,6 +3138,7 @@ bool create_device_impl(cem_sim *s) {
     CB2_CHECK(s, cudaFuncSetAttribute(kFKernels[s->npole], cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedSmem));
     const long long nblk = (long long)((g.plane + kEnergyBlock - 1) / kEnergyBlock) * (s->n[0] + 1);
     if (!dev_alloc(s, D.partial, (size_t)nblk) || !dev_alloc(s, D.scalar, 1)) return false;
+    if (!make_stage(s)) return false;
     fill_args(s, D);
     return true;
 }
@@ -3282,22 +3285,24 @@ void move_host(cem_sim *s, const Move &m, const std::vector<double *> &slots, un
 // Upwards nothing waits for the last chunk.
 constexpr size_t kStageWords = 1 << 20;
 
+bool make_stage(cem_sim *s) {
+    Device &D = *s->dev;
+    size_t words = 4 * (size_t)s->nf * D.nslot + 6 * s->N + (size_t)s->npole * s->ndisp + (size_t)s->nsb * s->sibc_npole;
+    for (int c = 0; c < 3; c++)
+        for (int w = 0; w < 2; w++) words += D.psi_len_h[c][w] + D.psi_len_e[c][w];
+    CB2_CHECK(s, cudaEventCreateWithFlags(&D.stage_ev, cudaEventDisableTiming));
+    if (!dev_alloc(s, D.stage, std::min((words + 1) / 2 * 2, kStageWords))) return false;
+    D.stage_host.reset(new unsigned[D.stage.n]);
+    return true;
+}
+
 template <bool Out>
 bool run_move(cem_sim *s, Move &m) {
     Device &D = *s->dev;
     if (!m.words) return true;
-    const size_t chunk = (size_t)std::min<unsigned long long>((m.words + 1) / 2 * 2, kStageWords);
-    if (!D.stage_ev) CB2_CHECK(s, cudaEventCreateWithFlags(&D.stage_ev, cudaEventDisableTiming));
+    const size_t chunk = D.stage.n;
     CB2_CHECK(s, cudaEventSynchronize(D.stage_ev));   // an earlier upload may still read the host words
-    if (D.stage.n < chunk) {
-        if (D.stage.p) CB2_CHECK(s, cudaFree(D.stage.p));
-        D.stage.p = nullptr;
-        D.stage.n = 0;
-        CB2_CHECK(s, cudaMalloc(&D.stage.p, chunk * sizeof(unsigned)));
-        D.stage.n = chunk;
-    }
-    if (D.stage_host.size() < chunk) D.stage_host.resize(chunk);
-    unsigned *st = D.stage_host.data();
+    unsigned *st = D.stage_host.get();
     const std::vector<double *> slots = dft_slots(s);
     m.a.stage = D.stage.p;
     for (m.a.lo = 0; m.a.lo < m.words; m.a.lo += chunk) {

@@ -85,3 +85,20 @@ def test_mode_port_waves_of_a_failed_read_are_an_error(fake):
     finally:
         fake.so.fake_fail_copy(-1)
     s.destroy()
+
+
+@pytest.mark.parametrize("read", ["field", "spectrum", "checkpoint", "release"])
+@pytest.mark.parametrize("scene", [scenes.parity_scene], ids=["plain"])
+def test_moving_state_allocates_nothing_on_the_device(fake, scene, read):
+    """Callers may have given all device memory away by the time they read results or go back to a saved state."""
+    fake.current = 0
+    s = scene(fake.lib)[0]
+    s.step(10)
+    made = fake.count("malloc")
+    saved = READS[read](s)
+    assert fake.count("malloc") == made
+    if read == "checkpoint":
+        s.restore(saved)
+        s.step(1)
+        assert fake.count("malloc") == made
+    s.destroy()
