@@ -2028,8 +2028,14 @@ struct Device {
     int ntab[3] = {0, 0, 0};
     DevBuf<float> J[3];
     int jbox[3][6] = {};
-    DevBuf<unsigned> jmap[3];   // offset in the box of each dispersive edge (made for the first move)
-    size_t jfirst[4] = {};      // first dispersive edge of each component
+    // dispersive edges [e, e + n) of a component, at offsets [o, o + n) of its box (made for the first move)
+    struct JRun {
+        size_t e;
+        unsigned o, n;
+    };
+    std::vector<JRun> jruns[3];
+    size_t jfirst[4] = {};        // first dispersive edge of each component
+    bool jmap_made = false;
     // Update kernels [H, E]: thread spaces [kFast, kGeneral, kAll], the
     // interior node planes [p0, p1), and the work-list of the general blocks
     // (entries: node plane, block of the plane's general space incl.
@@ -2111,8 +2117,10 @@ struct Device {
     DevBuf<float2> run_src;
     DevBuf<int> run_at;
     // words that state moves pass through, on the device and on the host (the whole state, or
-    // kStageWords of it); made with the device state, so that reading results allocates nothing there
+    // kStageWords of it); made with the device state, so that reading results allocates nothing there.
+    // Behind the stage_words, where the dispersive edges are few: each one's offset in its box.
     DevBuf<unsigned> stage;
+    size_t stage_words = 0;
     std::unique_ptr<unsigned[]> stage_host;
     cudaEvent_t stage_ev = nullptr;
     bool tune = false, tuned = false, tuned_from_cache = false;
@@ -3169,24 +3177,39 @@ bool flush_dft(cem_sim *s) {
     return true;
 }
 
-// The dispersive edges follow one another by component.
+// Where the dispersive edges, which follow one another by component and in
+// index order, lie in the Debye boxes. Up to kMapEdges of them move packed, by a
+// map of four bytes an edge on the device; of more, the boxes move whole and the
+// host takes the edges from them (a map of the 97 M-cell board's edges held 743 MB).
+// On a 6e3-cell scene of three poles, saving, restoring and 200 steps are 1230 us with
+// the map and 1258 with whole boxes.
+constexpr size_t kMapEdges = 1 << 20;
+
 bool make_jmap(cem_sim *s) {
     Device &D = *s->dev;
-    if (D.jfirst[3]) return true;
-    size_t first[4] = {};
+    if (D.jmap_made) return true;
+    size_t e = 0;
     for (int c = 0; c < 3; c++) {
         const int *bx = D.jbox[c];
-        std::vector<unsigned> map;
-        size_t e = first[c];
-        for (; e < (size_t)s->ndisp && s->d_comp[e] == c; e++) {
+        while (e < (size_t)s->ndisp && s->d_comp[e] == c) {
             const size_t q = s->d_idx[e];
             const int i = (int)(q / s->si), j = (int)((q % s->si) / s->sj), k = (int)(q % s->sj);
-            map.push_back((unsigned)(((size_t)(i - bx[0]) * bx[4] + (j - bx[1])) * bx[5] + (k - bx[2])));
+            unsigned n = 1;
+            while (e + n < (size_t)s->ndisp && s->d_comp[e + n] == c && s->d_idx[e + n] == q + n && k + (int)n <= s->n[2]) n++;
+            D.jruns[c].push_back({e, (unsigned)(((size_t)(i - bx[0]) * bx[4] + (j - bx[1])) * bx[5] + (k - bx[2])), n});
+            e += n;
         }
-        first[c + 1] = e;
-        if (!dev_renew(s, D.jmap[c], map)) return false;
+        D.jfirst[c + 1] = e;
     }
-    std::copy(first, first + 4, D.jfirst);
+    if ((size_t)s->ndisp <= kMapEdges) {
+        std::vector<unsigned> map;
+        map.reserve(s->ndisp);
+        for (const auto &runs : D.jruns)
+            for (const Device::JRun &r : runs)
+                for (unsigned t = 0; t < r.n; t++) map.push_back(r.o + t);
+        if (!h2d(s, D.stage.p + D.stage_words, map.data(), map.size() * sizeof(unsigned))) return false;
+    }
+    D.jmap_made = true;
     return true;
 }
 
@@ -3195,12 +3218,14 @@ bool make_jmap(cem_sim *s) {
 struct Move {
     MoveArgs a{};
     double *host[kMovePieces];
+    const std::vector<Device::JRun> *runs[kMovePieces];   // of a Debye pole's whole box
     unsigned long long words = 0;
 
     void add(void *dev, double *h, size_t A, size_t B, size_t C, size_t sa, size_t sb, size_t sc,
-             const unsigned *map = nullptr) {
+             const unsigned *map = nullptr, const std::vector<Device::JRun> *r = nullptr) {
         if (!A || !B || !C) return;
         host[a.n] = h;
+        runs[a.n] = r;
         a.p[a.n++] = {static_cast<unsigned *>(dev), map, words, (unsigned)B, (unsigned)C, sa, sb, sc};
         words += (unsigned long long)A * B * C;
     }
@@ -3238,9 +3263,13 @@ Move state_move(cem_sim *s, unsigned g, const StateView &v) {
         if (!D.J[c].p) continue;
         const size_t vol = (size_t)D.jbox[c][3] * D.jbox[c][4] * D.jbox[c][5];
         for (int p = 0; p < s->npole; p++) {
-            const size_t at = jaddr(vol, p, 0);
-            m.add(D.J[c].p + at, v.d_J + (size_t)p * s->ndisp + D.jfirst[c], 1, 1, D.jfirst[c + 1] - D.jfirst[c], 0, 0,
-                  1, D.jmap[c].p);
+            float *d = D.J[c].p + jaddr(vol, p, 0);
+            double *h = v.d_J + (size_t)p * s->ndisp;
+            const size_t e = D.jfirst[c];
+            if ((size_t)s->ndisp <= kMapEdges)
+                m.add(d, h + e, 1, 1, D.jfirst[c + 1] - e, 0, 0, 1, D.stage.p + D.stage_words + e);
+            else
+                m.add(d, h, 1, 1, vol, 0, 0, 1, nullptr, &D.jruns[c]);
         }
     }
     if ((g & kGroupSibc) && s->nsb && v.sb_y)
@@ -3257,7 +3286,23 @@ void move_host(cem_sim *s, const Move &m, const std::vector<double *> &slots, un
         const unsigned long long p0 = m.a.p[q].start, p1 = q + 1 < m.a.n ? m.a.p[q + 1].start : m.words;
         const unsigned long long x = std::max(lo, p0), y = std::min(hi, p1);
         if (x >= y) continue;
-        if (m.host[q]) {
+        if (m.host[q] && m.runs[q]) {
+            float *f = reinterpret_cast<float *>(st) + (x - lo);
+            const unsigned long long b0 = x - p0, b1 = y - p0;   // offsets in the box
+            if (!Out) std::memset(f, 0, (b1 - b0) * sizeof(float));
+            auto r = std::partition_point(m.runs[q]->begin(), m.runs[q]->end(),
+                                          [b0](const Device::JRun &t) { return t.o + (unsigned long long)t.n <= b0; });
+            for (; r != m.runs[q]->end() && r->o < b1; ++r) {
+                const unsigned long long from = std::max<unsigned long long>(r->o, b0);
+                const unsigned long long to = std::min<unsigned long long>(r->o + (unsigned long long)r->n, b1);
+                double *h = m.host[q] + r->e + (from - r->o);
+                float *w = f + (from - b0);
+                for (size_t t = 0; t < to - from; t++) {
+                    if (Out) h[t] = w[t];
+                    else w[t] = (float)h[t];
+                }
+            }
+        } else if (m.host[q]) {
             float *f = reinterpret_cast<float *>(st) + (x - lo);
             double *h = m.host[q] + (x - p0);
             const size_t len = y - x;
@@ -3287,12 +3332,17 @@ constexpr size_t kStageWords = 1 << 20;
 
 bool make_stage(cem_sim *s) {
     Device &D = *s->dev;
-    size_t words = 4 * (size_t)s->nf * D.nslot + 6 * s->N + (size_t)s->npole * s->ndisp + (size_t)s->nsb * s->sibc_npole;
-    for (int c = 0; c < 3; c++)
+    const bool packed = (size_t)s->ndisp <= kMapEdges;
+    size_t words = 4 * (size_t)s->nf * D.nslot + 6 * s->N + (size_t)s->nsb * s->sibc_npole;
+    if (packed) words += (size_t)s->npole * s->ndisp;
+    for (int c = 0; c < 3; c++) {
+        if (!packed) words += D.J[c].n;
         for (int w = 0; w < 2; w++) words += D.psi_len_h[c][w] + D.psi_len_e[c][w];
+    }
     CB2_CHECK(s, cudaEventCreateWithFlags(&D.stage_ev, cudaEventDisableTiming));
-    if (!dev_alloc(s, D.stage, std::min((words + 1) / 2 * 2, kStageWords))) return false;
-    D.stage_host.reset(new unsigned[D.stage.n]);
+    D.stage_words = std::min((words + 1) / 2 * 2, kStageWords);
+    if (!dev_alloc(s, D.stage, D.stage_words + (packed ? s->ndisp : 0))) return false;
+    D.stage_host.reset(new unsigned[D.stage_words]);
     return true;
 }
 
@@ -3300,7 +3350,7 @@ template <bool Out>
 bool run_move(cem_sim *s, Move &m) {
     Device &D = *s->dev;
     if (!m.words) return true;
-    const size_t chunk = D.stage.n;
+    const size_t chunk = D.stage_words;
     CB2_CHECK(s, cudaEventSynchronize(D.stage_ev));   // an earlier upload may still read the host words
     unsigned *st = D.stage_host.get();
     const std::vector<double *> slots = dft_slots(s);

@@ -88,7 +88,7 @@ def test_mode_port_waves_of_a_failed_read_are_an_error(fake):
 
 
 @pytest.mark.parametrize("read", ["field", "spectrum", "checkpoint", "release"])
-@pytest.mark.parametrize("scene", [scenes.parity_scene], ids=["plain"])
+@pytest.mark.parametrize("scene", [scenes.parity_scene, scenes.lossy_scene], ids=["plain", "lossy"])
 def test_moving_state_allocates_nothing_on_the_device(fake, scene, read):
     """Callers may have given all device memory away by the time they read results or go back to a saved state."""
     fake.current = 0
