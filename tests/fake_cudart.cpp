@@ -56,7 +56,7 @@ CUresult encode(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cu
 
 extern "C" {
 
-// what the tests ask: "malloc", "free", "live" (bytes), "launch", "graph" (replays), "capture", or a kernel's name
+// what the tests ask: "malloc", "free", "live" (bytes), "up" (copies to the device), "launch", "graph" (replays), "capture", or a kernel's name
 __attribute__((visibility("default"))) long fake_count(const char *what) {
     std::lock_guard<std::mutex> l(mu);
     if (!std::strcmp(what, "live")) {
@@ -120,7 +120,11 @@ cudaError_t cudaFree(void *p) {
     counts["free"]++;
     return cudaSuccess;
 }
-cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, cudaMemcpyKind, cudaStream_t) {
+cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, cudaMemcpyKind kind, cudaStream_t) {
+    if (kind == cudaMemcpyHostToDevice) {
+        std::lock_guard<std::mutex> l(mu);
+        counts["up"]++;
+    }
     if (copies_left >= 0 && copies_left-- == 0) return ret(cudaErrorUnknown);
     std::memcpy(to, from, n);
     return cudaSuccess;

@@ -102,3 +102,14 @@ def test_moving_state_allocates_nothing_on_the_device(fake, scene, read):
         s.step(1)
         assert fake.count("malloc") == made
     s.destroy()
+
+
+@pytest.mark.parametrize("scene", [scenes.parity_scene, scenes.lossy_scene], ids=["plain", "lossy"])
+def test_small_tables_go_up_together(fake, scene):
+    """Dozens of tables of a few kilobytes: one copy, and one more for each array too large to share it."""
+    fake.current = 0
+    s = scene(fake.lib)[0]
+    before = fake.count("up")
+    s.prepareDevice()
+    assert fake.count("up") - before <= 8
+    s.destroy()
