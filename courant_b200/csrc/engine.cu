@@ -2003,6 +2003,8 @@ struct Device {
     bool failed = false;
     std::string error_msg;
 
+    size_t held = 0;   // bytes allocated on the device
+
     // The small tables of a new device state go up together: pool_host collects them, pool_at
     // says whose place is where, flush_pool allocates and copies once. (An allocation, a copy
     // and a wait for each of 56 tables: 1.95 instead of 1.35 ms for the device state of a 6e3-cell scene.)
@@ -2251,6 +2253,7 @@ bool dev_alloc(cem_sim *s, DevBuf<T> &b, size_t n) {
     b.own = true;
     if (!n) return true;
     CB2_CHECK(s, cudaMalloc(&b.p, n * sizeof(T)));
+    s->dev->held += n * sizeof(T);
     return true;
 }
 
@@ -2276,7 +2279,10 @@ bool dev_upload(cem_sim *s, DevBuf<T> &b, const std::vector<T> &v) {
 // the same into a buffer that may hold an older table (of launches that have ended)
 template <class T>
 bool dev_renew(cem_sim *s, DevBuf<T> &b, const std::vector<T> &v) {
-    if (b.p && b.own) CB2_CHECK(s, cudaFree(b.p));
+    if (b.p && b.own) {
+        CB2_CHECK(s, cudaFree(b.p));
+        s->dev->held -= b.n * sizeof(T);
+    }
     b.p = nullptr;
     return dev_upload(s, b, v);
 }
@@ -2669,6 +2675,9 @@ bool build_pml(cem_sim *s, Device &D) {
     return true;
 }
 
+// most steps of a run whose rows hold n samples: up to 16 MB of them
+int sample_rows(long long n) { return (int)std::max(1ll, std::min((long long)kRing, (4ll << 20) / std::max(n, 1ll))); }
+
 bool build_probes(cem_sim *s, Device &D) {
     D.nip = (int)s->ip.size();
     D.nport = (int)s->port.size();
@@ -2716,7 +2725,7 @@ bool build_probes(cem_sim *s, Device &D) {
         D.run.nsample[u] = (int)samp.size() - (u ? D.run.nsample[0] : 0);
     }
     D.run.nent = (int)idx.size();
-    D.run_steps = (int)std::max(1ll, std::min((long long)kRing, (4ll << 20) / std::max(D.run.nent, 1)));
+    D.run_steps = sample_rows(D.run.nent);
     if (!dev_upload(s, D.samples, samp) || !dev_alloc(s, D.raw, (size_t)D.run_steps * D.run.nent) ||
         !dev_alloc(s, D.run_src, kRing) || !dev_alloc(s, D.run_at, 2))
         return false;
@@ -3364,6 +3373,24 @@ void move_host(cem_sim *s, const Move &m, const std::vector<double *> &slots, un
 // even 64 KB takes 1-8 ms, more than 4 MB take to copy without it (0.4 ms).
 // Upwards nothing waits for the last chunk.
 constexpr size_t kStageWords = 1 << 20;
+
+// Device bytes of a simulation beside its fields, materials, auxiliaries and
+// currents, known before the device state exists: samples, spectra, staging
+// words, place tables, work-lists, partial sums, and room for the small tables.
+long long side_bytes(const cem_sim *s) {
+    long long n = 0, b = 1 << 18;
+    for (const CurrentProbe &p : s->ip) n += (long long)p.idx.size();
+    for (const LumpedPort &p : s->port) n += (long long)p.edge.size();
+    for (const VoltageProbe &p : s->vp) n += (long long)p.edge.size();
+    const long long nslot = (long long)(s->ip.size() + 2 * s->port.size() + 1 + s->vp.size());
+    b += n * (sizeof(uint4) + sizeof(unsigned char) + sizeof(unsigned) + sizeof(double)) + sample_rows(n) * n * 4;
+    b += nslot * 8 * (kRing + 2ll * s->nf) + kRing * 8;
+    b += kStageWords * 4 + (s->ndisp <= (long long)kMapEdges ? s->ndisp * 4ll : 0);
+    const long long groups = (s->n[1] + 1ll) * ((s->n[2] + 4) / 4), blocks = (groups + kBlock - 1) / kBlock + kMaxRects;
+    b += 4 * (groups + kBlock) * 8 + 2 * 3 * (s->n[0] + 1ll) * blocks * 8;
+    b += (s->n[0] + 1ll) * (groups * 8 / kEnergyBlock + 1) * 8;
+    return b;
+}
 
 bool make_stage(cem_sim *s) {
     Device &D = *s->dev;
@@ -4206,7 +4233,7 @@ int cemx_profile_steps(cem_sim *s, long n, double *kernel_ms, long *launches) {
 
 int cemx_sizes(const cem_sim *s, long long *out, int n) {
     if (!s->finalized) { set_error("not finalized"); return -1; }
-    long long v[19] = {0};
+    long long v[20] = {0};
     v[0] = (long long)s->n[0] * s->n[1] * s->n[2];
     v[1] = (long long)s->N;
     for (int c = 0; c < 3; c++)
@@ -4220,16 +4247,7 @@ int cemx_sizes(const cem_sim *s, long long *out, int n) {
     v[7] = s->sibc_npole;
     if (s->dev) {
         for (int c = 0; c < 3; c++) v[8 + c] = s->dev->ntab[c];
-        long long bytes = 0;
-        const Device &D = *s->dev;
-        for (int c = 0; c < 3; c++) {
-            bytes += (long long)(2 * D.E[0][c].n + 2 * D.H[0][c].n + D.hc[c].n + D.ec[c].n) * 4 +
-                     (long long)D.mat[c].n * 2 + (long long)D.tab[c].n * 4 + (long long)D.J[c].n * 4;
-            for (int w = 0; w < 2; w++) bytes += (long long)(D.psiE[c][w].n + 2 * D.psiH[0][c][w].n) * 4;
-        }
-        bytes += (long long)D.sb_y.n * 4 + (long long)(D.sb_hw.n + D.sb_hidx.n) * 16 + (long long)D.sb_eidx.n * 4 +
-                 (long long)(D.ring.n + D.acc.n) * 8;
-        v[11] = bytes;
+        v[11] = (long long)s->dev->held;
     }
     // kernels per step: H and E, each over its fast and general blocks (or one fused kernel)
     int upd = 4;
@@ -4261,7 +4279,8 @@ int cemx_sizes(const cem_sim *s, long long *out, int n) {
         }
         for (int c = 0; c < 3; c++) v[18] += (long long)D.jbox[c][3] * D.jbox[c][4] * D.jbox[c][5];
     }
-    for (int q = 0; q < n && q < 19; q++) out[q] = v[q];
+    v[19] = side_bytes(s);
+    for (int q = 0; q < n && q < 20; q++) out[q] = v[q];
     return 0;
 }
 

@@ -32,18 +32,19 @@ from .api import Courant, Sim
 
 def footprint(sim: Sim) -> int:
     """Device bytes a simulation will hold, from its sizes before its device
-    state exists: padded FP32 fields (6), u16 material indices (3), CPML
-    auxiliaries (padded layout, about 1.5x the compact count), Debye currents,
-    surface-impedance states, and a 10% margin for tables and probes."""
+    state exists: padded FP32 fields (6, in two buffers), u16 material indices
+    (3), CPML auxiliaries (padded layout, about 1.5x the compact count), Debye
+    currents, surface-impedance states, a 10% margin, and what the library
+    holds beside these (samples, spectra, staging words, launch tables)."""
     z = sim.sizes()
     nx, ny, nz = sim.nx, sim.ny, sim.nz
     sj = (nz + 1 + 7) // 8 * 8
     npts = (nx + 1) * (ny + 1) * sj
-    b = npts * (6 * 4 + 3 * 2)
+    b = npts * (2 * 6 * 4 + 3 * 2)
     b += int(1.5 * 4 * (z["psiE"] + 2 * z["psiH"]))
     b += int(1.3 * 4 * z["npole"] * z["ndisp"])
     b += 4 * z["sibc_terms"] * z["nsibc"] + 48 * z["nsibc"]
-    return int(b * 1.1)
+    return int(b * 1.1) + z.get("side_bytes", 0)
 
 
 def results(sim: Sim, meta: dict) -> dict:

@@ -35,7 +35,9 @@ CEM_API int cemx_profile_steps(cem_sim *s, long n, double *kernel_ms, long *laun
  *   11 device bytes held (0 before the first step), 12 kernel launches per step,
  *   13-17 point-components the update classes cover per step (H fast, H
  *   general, E fast, E general, E Debye; 0 before the first step),
- *   18 points of the Debye boxes (all three components).
+ *   18 points of the Debye boxes (all three components),
+ *   19 device bytes beside fields, materials, auxiliaries and currents: samples,
+ *   spectra, staging words, launch tables (an upper estimate, at any time).
  * Returns 0 or -1. */
 CEM_API int cemx_sizes(const cem_sim *s, long long *out, int n);
 

@@ -6,7 +6,7 @@ import subprocess
 import numpy as np
 import pytest
 
-from courant_b200 import build, scenes
+from courant_b200 import boards, build, scenes, serve
 from courant_b200.api import Courant, CourantError
 
 
@@ -113,3 +113,33 @@ def test_small_tables_go_up_together(fake, scene):
     s.prepareDevice()
     assert fake.count("up") - before <= 8
     s.destroy()
+
+
+def probed_box(c):
+    """A small closed box full of probes: the samples outweigh the fields."""
+    s = c.createSim(1e-4 * np.arange(31), 1e-4 * np.arange(29), 1e-4 * np.arange(25))
+    s.setFrequencies(np.linspace(1e9, 20e9, 50))
+    for q in range(60):
+        s.addIProbe(0, 2 + q % 26, 2, 26, 2, 22)
+    s.finalize(0.9)
+    return s, {}
+
+
+@pytest.mark.parametrize("make", [scenes.parity_scene, scenes.lossy_scene, scenes.modeport_scene, probed_box,
+                                  lambda c: boards.seeded_board(c, seed=4, cells=8e4, ports="lumped", nf=8),
+                                  lambda c: boards.seeded_board(c, seed=6, cells=3e5, ports="mode", nf=8)],
+                         ids=["plain", "lossy", "mode ports", "probes", "board", "larger board"])
+def test_device_bytes_are_all_counted(fake, make):
+    """sizes() tells what is allocated, before and after results were read, and a server's estimate covers it."""
+    fake.current = 0
+    s = make(fake.lib)[0]
+    estimate, before = serve.footprint(s), fake.count("live")
+    s.prepareDevice()
+    assert s.sizes()["device_bytes"] == fake.count("live") - before
+    s.step(40)
+    s.checkpoint(), s.sourceSpectrum(), s.energy()
+    held = fake.count("live") - before
+    assert s.sizes()["device_bytes"] == held
+    assert held <= estimate <= 1.3 * held + (6 << 20)
+    s.destroy()
+    assert fake.count("live") == before
