@@ -215,7 +215,13 @@ struct RunArgs {
     float2 *srcv;            // the current step's, which the E update reads
     int *at;                 // [0] step of the run in progress, [1] the next one
     int on;                  // whether the launch belongs to a run
-    int first;               // blocks of the launch before the update's own: sampling, surface impedance
+    // blocks of the launch before the update's own: sampling, then surface impedance (of the
+    // per-class fast launches: one column more, whose first rows sample)
+    int first;
+    // sampling blocks, one entry per thread. us per step of the 61 x 47 x 35 cavity with 378
+    // to 6048 entries: 4.6, with 15120: 4.8 (by one block: 4.6 with 378, 13, 23 and 51 with
+    // 3024, 6048 and 15120)
+    int blocks;
     unsigned skip;           // table flags whose points the E update leaves to those blocks
 };
 
@@ -1229,33 +1235,41 @@ __device__ __forceinline__ void sibc_edge(const SibcArgs &a, int e, Wait wait) {
     a.E[ec][ei] = E;
 }
 
-// samples of family u (0 E, 1 H) into their step's row, by one block: H in the step
-// in progress, E in the next one's H launch (of the first, none). Returns the step read.
+// samples of family u (0 E, 1 H) into their step's row, by block b of n (one entry per
+// thread, see RunArgs::blocks): H in the step in progress, E in the next one's H launch (of
+// the first, none). Returns the step sampled. The H launch reads at[1] and writes at[0], the
+// E launch the other way round: no block reads what another of its launch writes.
 template <class Wait>
-__device__ __forceinline__ int sample_family(const StepArgs &a, const RunArgs &r, int u, Wait wait) {
+__device__ __forceinline__ int sample_family(const StepArgs &a, const RunArgs &r, int u, int b, int n, Wait wait) {
     const uint4 *s = r.samples + (u ? r.nsample[0] : 0);
+    const int first = b * kBlock + (int)threadIdx.x;
     uint4 v;
-    if ((int)threadIdx.x < r.nsample[u]) v = __ldg(s + threadIdx.x);
+    if (first < r.nsample[u]) v = __ldg(s + first);
     wait();
-    const int at = r.at[u ? 0 : 1], t = u ? at : at - 1;
-    if (t < 0) return at;
-    for (int e = threadIdx.x; e < r.nsample[u]; e += blockDim.x) {
-        if (e != (int)threadIdx.x) v = __ldg(s + e);
+    const int t = u ? r.at[0] : r.at[1] - 1;
+    if (t < 0) return t;
+    for (int e = first; e < r.nsample[u]; e += n * kBlock) {
+        if (e != first) v = __ldg(s + e);
         r.raw[(size_t)t * r.nent + v.z] = (u ? a.H[v.x - 3] : a.E[v.x])[v.y];
     }
-    return at;
+    return t;
 }
 
 // H launch of a run: E of the step before, and the new step's source values
 template <class Wait>
-__device__ __forceinline__ void begin_step(const StepArgs &a, const RunArgs &r, Wait wait) {
-    const int t = sample_family(a, r, 0, wait);
-    __syncthreads();
-    if (threadIdx.x == 0) {
+__device__ __forceinline__ void begin_step(const StepArgs &a, const RunArgs &r, int b, int n, Wait wait) {
+    const int t = sample_family(a, r, 0, b, n, wait) + 1;
+    if (b == 0 && threadIdx.x == 0) {
         *r.srcv = r.src[t];
         r.at[0] = t;
-        r.at[1] = t + 1;
     }
+}
+
+// E launch: H of the step
+template <class Wait>
+__device__ __forceinline__ void sample_h(const StepArgs &a, const RunArgs &r, int b, int n, Wait wait) {
+    const int t = sample_family(a, r, 1, b, n, wait);
+    if (b == 0 && threadIdx.x == 0) r.at[1] = t + 1;
 }
 
 // H over node planes [i0, i0 + gridDim.y) (cem_mt_H and the unfused step)
@@ -1305,7 +1319,8 @@ struct AtOnce {
 __global__ void __launch_bounds__(kBlock, CB2_HF_MINBLOCKS) k_update_h_fast(const StepArgs a, int i0, const RunArgs r) {
     chain_next();
     if (r.first && blockIdx.x == gridDim.x - 1) {   // one column more: the run's own work
-        if (blockIdx.y == 0) begin_step(a, r, Chained{});
+        const int n = min(r.blocks, (int)gridDim.y);
+        if ((int)blockIdx.y < n) begin_step(a, r, (int)blockIdx.y, n, Chained{});
         return;
     }
     const int comp = blockIdx.x % 3;
@@ -1320,7 +1335,8 @@ __global__ void __launch_bounds__(kBlock, CB2_HF_MINBLOCKS) k_update_h_fast(cons
 __global__ void __launch_bounds__(kBlock, CB2_EF_MINBLOCKS) k_update_e_fast(const StepArgs a, int i0, const RunArgs r) {
     chain_next();
     if (r.first && blockIdx.x == gridDim.x - 1) {
-        if (blockIdx.y == 0) sample_family(a, r, 1, Chained{});
+        const int n = min(r.blocks, (int)gridDim.y);
+        if ((int)blockIdx.y < n) sample_h(a, r, (int)blockIdx.y, n, Chained{});
         return;
     }
     const int comp = blockIdx.x % 3;
@@ -1343,7 +1359,7 @@ __device__ __forceinline__ RowPos general_pos(const StepArgs &a, int i, int b) {
 __global__ void __launch_bounds__(kBlock, CB2_H_MINBLOCKS) k_update_h(const StepArgs a, const int2 *work, const RunArgs r) {
     chain_next();
     if ((int)blockIdx.x < r.first) {
-        begin_step(a, r, Chained{});
+        begin_step(a, r, (int)blockIdx.x, r.blocks, Chained{});
         return;
     }
     const int2 w = work[blockIdx.x - r.first];
@@ -1359,8 +1375,8 @@ __global__ void __launch_bounds__(kBlock, CB2_E_MINBLOCKS)
     k_update_e(const StepArgs a, const int2 *work, const RunArgs r, const SibcArgs s) {
     chain_next();
     if ((int)blockIdx.x < r.first) {   // H samples, then the surface-impedance edges (their E is left alone below)
-        const int e = ((int)blockIdx.x - 1) * kBlock + threadIdx.x;
-        if (blockIdx.x == 0) sample_family(a, r, 1, Chained{});
+        const int e = ((int)blockIdx.x - r.blocks) * kBlock + (int)threadIdx.x;
+        if (e < 0) sample_h(a, r, (int)blockIdx.x, r.blocks, Chained{});
         else if (e < s.ns) sibc_edge(s, e, Chained{});
         return;
     }
@@ -1421,7 +1437,7 @@ constexpr int kWholeH = 9, kWholeE = 7, kWholeELarge = 8, kLargePoles = 6;
 __global__ void __launch_bounds__(kBlock, kWholeH) k_whole_h(const StepArgs a, const Whole l, const RunArgs r) {
     chain_next();
     if ((int)blockIdx.x < r.first) {
-        begin_step(a, r, Chained{});
+        begin_step(a, r, (int)blockIdx.x, r.blocks, Chained{});
         return;
     }
     int i, comp;
@@ -1443,8 +1459,8 @@ __global__ void __launch_bounds__(kBlock, P > 8 ? 4 : B)
     k_whole_e(const StepArgs a, const Whole l, const RunArgs r, const SibcArgs s) {
     chain_next();
     if ((int)blockIdx.x < r.first) {   // H samples, then the surface-impedance edges (their E is left alone below)
-        const int e = ((int)blockIdx.x - 1) * kBlock + threadIdx.x;
-        if (blockIdx.x == 0) sample_family(a, r, 1, Chained{});
+        const int e = ((int)blockIdx.x - r.blocks) * kBlock + (int)threadIdx.x;
+        if (e < 0) sample_h(a, r, (int)blockIdx.x, r.blocks, Chained{});
         else if (e < s.ns) sibc_edge(s, e, Chained{});
         return;
     }
@@ -1767,10 +1783,10 @@ __device__ __forceinline__ void post_block(const PostArgs &a) {
 __global__ void __launch_bounds__(kPostThreads) k_post(const PostArgs a) { post_block(a); }
 
 // the same as a launch of its own, where no update launch carries it
-__global__ void __launch_bounds__(kBlock) k_begin_step(const StepArgs a, const RunArgs r) { begin_step(a, r, AtOnce{}); }
-__global__ void __launch_bounds__(kBlock) k_sample_h(const StepArgs a, const RunArgs r) { sample_family(a, r, 1, AtOnce{}); }
+__global__ void __launch_bounds__(kBlock) k_begin_step(const StepArgs a, const RunArgs r) { begin_step(a, r, 0, 1, AtOnce{}); }
+__global__ void __launch_bounds__(kBlock) k_sample_h(const StepArgs a, const RunArgs r) { sample_h(a, r, 0, 1, AtOnce{}); }
 
-// before a run: its step count to zero, the source values of its steps
+// before a run: its next step is the first, the source values of its steps
 __global__ void k_run_begin(const RunArgs r, const PostArgs p, float *src, int steps, long long step0) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
     if (t == 0) r.at[1] = 0;
@@ -3608,8 +3624,9 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
     SibcArgs sb = D.sb[D.cur];
     if (!run || !D.sibc_flagged) sb.ns = 0;
     RunArgs none = D.run, carry = D.run;   // a launch with nothing of the run's, and the phase's one with it
-    none.first = carry.first = 0;
+    none.first = carry.first = none.blocks = carry.blocks = 0;
     none.skip = carry.skip = sb.ns ? kFlagSibc : 0u;
+    auto sample_blocks = [&](int u) { return std::max(1, (D.run.nsample[u] + kBlock - 1) / kBlock); };
     // general work-list entries of update u for node planes [a, b)
     auto span = [&](int u, int a, int b, const int2 *&p) {
         const std::vector<int> &st = D.wl_start[u];
@@ -3640,12 +3657,13 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
         cudaLaunchKernelEx(&c, kernel, args...);
         D.chained = run;
     };
-    // fast (or Debye) rectangles of update u on node planes [a, b), with one block column more for r.first
-    auto fast = [&](int u, int a, int b, auto kernel, const RunArgs &r, int cls = kFast) {
-        const int nb = space_blocks(D.sp[u][cls]);
+    // fast rectangles of update u on node planes [a, b), with one block column more for r.first
+    auto fast = [&](int u, int a, int b, auto kernel, const RunArgs &r) {
+        const int nb = space_blocks(D.sp[u][kFast]);
         const int c0 = std::max(a, D.p0[u]), c1 = std::min(b, D.p1[u]);
         if (nb == 0) return;
         RunArgs q = r;
+        q.first = r.first > 0;
         for (int c = c0; c < c1; c += kMaxGridY, q.first = 0)
             launch(kernel, dim3(3 * nb + q.first, std::min(kMaxGridY, c1 - c)), D.sa[D.cur], c, q);
     };
@@ -3667,7 +3685,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
             const int2 *w;
             const unsigned n = span(0, a, b, w);
             const bool side = n && D.side_on && space_blocks(D.sp[0][kFast]);   // beside the fast launch
-            carry.first = run ? 1 : 0;
+            carry.blocks = carry.first = run ? sample_blocks(0) : 0;
             if (D.whole_h) {
                 const Whole l = whole(0, a, b, w, n);
                 launch(k_whole_h, dim3(carry.first + n + (unsigned)l.planes * (l.nd + l.nf)), D.sa[D.cur], l, carry);
@@ -3702,7 +3720,8 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
             const unsigned n = span(1, a, b, w);
             const bool own = n || sb.ns;   // the general launch carries the run's
             const bool side = own && D.side_on && space_blocks(D.sp[1][kFast]);
-            carry.first = !run ? 0 : own ? 1 + (sb.ns + kBlock - 1) / kBlock : 1;
+            carry.blocks = run ? sample_blocks(1) : 0;
+            carry.first = carry.blocks + (run ? (sb.ns + kBlock - 1) / kBlock : 0);
             if (D.whole_e) {
                 const Whole l = whole(1, a, b, w, n);
                 const bool large = !D.whole_h && s->npole <= kLargePoles;
