@@ -1432,7 +1432,11 @@ __device__ __forceinline__ int whole_place(const StepArgs &a, const Whole &l, in
 // to six poles (they spill on the CPML paths there, but a bandwidth-bound launch
 // gains more from the eighth block: 334 against 341 us per step on the 10.9 M-cell
 // board of four poles, 98.4 against 100 on the 3.6 M-cell line of six; 13.1 against
-// 15.1 the other way on the 250 k-cell board)
+// 15.1 the other way on the 250 k-cell board; with seven and eight poles 93.4 and 97.7
+// against 92.8 and 96.1 on the 3.4 M-cell line). More poles keep the small grids' form
+// on large ones: their tables fetched before the wait cost 0-1% there (3.4 M cells, the
+// lean blocks apart: 89.7, 92.8, 99.0, 104.3 us with 7, 8, 12 and 16 poles, 89.8, 91.9, 98.2,
+// 104.0 with the tables after it).
 constexpr int kWholeH = 9, kWholeE = 7, kWholeELarge = 8, kLargePoles = 6;
 __global__ void __launch_bounds__(kBlock, kWholeH) k_whole_h(const StepArgs a, const Whole l, const RunArgs r) {
     chain_next();
@@ -2137,6 +2141,7 @@ struct Device {
     int run_steps = 0;                // most steps of a run (sample rows)
     bool sibc_flagged = false;        // the tables mark the surface-impedance edges
     bool whole_h = true, whole_e = true;   // an update's blocks in one launch (Whole), or a kernel per class
+    bool split_e = false;   // of whole_e: the lean rectangles in a launch of their own
     bool chained = false;   // the last launch on the main stream is one of a run, nothing else since
     RunArgs run{};
     DevBuf<uint4> samples;
@@ -3146,6 +3151,15 @@ bool create_device_impl(cem_sim *s) {
     // one launch an update below 2 M cells; above, for E with poles (Whole has both sides measured)
     D.whole_h = (long long)s->n[0] * s->n[1] * s->n[2] < 2000000;
     D.whole_e = D.whole_h || s->npole > 0;
+    // With many poles the registers of their general and Debye blocks (from nine poles on 128, four
+    // blocks per SM) cost the lean blocks of the same launch more than sharing a row's ends saves. us
+    // per step, all in one launch / the lean blocks apart, of lossy lines: 1.0 M cells, 9, 12 and 16
+    // poles 31.2 / 30.5, 31.7 / 31.5, 33.6 / 34.4; 1.7 M cells 53.1 / 48.7, 55.3 / 50.9, 58.6 / 54.5, with 7
+    // and 8 poles 46.3 / 47.6, 49.7 / 50.6; 3.4 M cells, 7, 8, 9, 12 and 16 poles 92.6 / 89.7, 95.8 / 92.8,
+    // 118.5 / 94.7, 121.2 / 99.0, 124.6 / 104.3; with 4 and 6 poles (eight blocks per SM) 82.7 / 84.1,
+    // 89.2 / 90.2.
+    const long long cells = (long long)s->n[0] * s->n[1] * s->n[2];
+    D.split_e = s->npole > kLargePoles + 2 ? cells >= 1000000 : s->npole > kLargePoles && cells >= 2000000;
     if (const char *e = std::getenv("CEM_B200_ZTAIL")) {
         D.ztail = e[0] != '0';
         D.ztail_split = e[0] != '1';
@@ -3725,8 +3739,24 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
             if (D.whole_e) {
                 const Whole l = whole(1, a, b, w, n);
                 const bool large = !D.whole_h && s->npole <= kLargePoles;
-                launch(large ? kEWLarge[s->npole] : kEWKernels[s->npole],
-                       dim3(carry.first + n + (unsigned)l.planes * (l.nd + l.nf)), D.sa[D.cur], l, carry, sb);
+                const WKernel kernel = large ? kEWLarge[s->npole] : kEWKernels[s->npole];
+                const unsigned others = carry.first + n + (unsigned)l.planes * l.nd;   // than the lean blocks
+                if (!D.split_e || !l.planes || !l.nf) {
+                    launch(kernel, dim3(others + (unsigned)l.planes * l.nf), D.sa[D.cur], l, carry, sb);
+                } else {
+                    Whole g = l;
+                    g.nf = 0;
+                    const bool beside = others && D.side_on;
+                    if (beside) {
+                        fork();
+                        kernel<<<others, blk, 0, D.side>>>(D.sa[D.cur], g, carry, sb);
+                        cudaEventRecord(D.join, D.side);
+                    } else if (others) {
+                        launch(kernel, dim3(others), D.sa[D.cur], g, carry, sb);
+                    }
+                    fast(1, a, b, k_update_e_fast, none);
+                    if (beside) join();
+                }
             } else {   // no poles: no Debye rectangles
                 if (side) {
                     fork();
@@ -4273,7 +4303,7 @@ int cemx_sizes(const cem_sim *s, long long *out, int n) {
     if (s->dev) {
         const Device &D = *s->dev;
         for (int u = 0; u < 2; u++) {
-            if (u ? D.whole_e : D.whole_h) { upd--; continue; }
+            if (u ? D.whole_e && !D.split_e : D.whole_h) { upd--; continue; }
             upd -= space_blocks(D.sp[u][kFast]) == 0 || D.p1[u] <= D.p0[u];
             upd -= D.wl_start[u].empty() || D.wl_start[u].back() == 0;
         }

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from courant_b200 import boards, build, scenes, serve
-from courant_b200.api import Courant, CourantError
+from courant_b200.api import Courant, CourantError, DebyeModel
 
 
 class Fake:
@@ -143,3 +143,30 @@ def test_device_bytes_are_all_counted(fake, make):
     assert held <= estimate <= 1.3 * held + (6 << 20)
     s.destroy()
     assert fake.count("live") == before
+
+
+def debye_box(c, n, poles):
+    """CPML round a box whose lower half is Debye material."""
+    s = c.createSim(*(1e-4 * np.arange(q + 1) for q in n))
+    for f in (0, 1, 2, 3, 5):
+        s.setBoundary(f, 1, 6)
+    fp = np.geomspace(1e9, 40e9, poles)
+    s.setDebyePoles(fp)
+    s.materialBoxDebye(-1, 1, -1, 1, 0, 1e-4 * (n[2] // 2), DebyeModel(3.5, fp, np.full(poles, 0.05), 0.0))
+    p = s.addLumpedPort(2, n[0] // 2, n[1] // 2, 0, 4, 1, 50.0)
+    s.setGaussian(p, 1.0, 8e-12, 3e-12)
+    s.setFrequencies([5e9])
+    s.finalize(0.9)
+    return s
+
+
+@pytest.mark.parametrize("n,poles,apart", [((120, 104, 84), 12, True), ((80, 72, 60), 12, False), ((140, 132, 112), 7, True),
+                                           ((140, 132, 112), 6, False), ((120, 104, 84), 8, False)])
+def test_lean_blocks_of_grids_with_many_poles_run_by_themselves(fake, n, poles, apart):
+    fake.current = 0
+    s = debye_box(fake.lib, n, poles)
+    before = {k: fake.count(k) for k in ("k_whole_e", "k_update_e_fast")}
+    s.step(3)
+    assert fake.count("k_whole_e") - before["k_whole_e"] == 3
+    assert fake.count("k_update_e_fast") - before["k_update_e_fast"] == (3 if apart else 0)
+    s.destroy()

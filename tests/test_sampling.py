@@ -4,6 +4,8 @@ carries them, give the bits of the phases; and many entries cost a step little."
 import numpy as np
 import pytest
 
+from courant_b200.api import DebyeModel
+
 pytestmark = pytest.mark.gpu
 
 BIG = (172, 130, 96)   # above 2 M cells: a kernel per class of blocks
@@ -27,6 +29,26 @@ def box(c, n, edges, loops, cpml=False, copper=False):
         edges -= m
     for q in range(loops):
         s.addIProbe(0, 9 + q % (n[0] - 18), 8, n[1] - 8, 8, n[2] - 8)
+    s.finalize(0.9)
+    return s
+
+
+def debye_box(c, n, poles, copper):
+    """CPML round a box whose lower half is Debye material, with or without a block of copper in it."""
+    s = c.createSim(*(1e-4 * np.arange(q + 1) for q in n))
+    for f in (0, 1, 2, 3, 5):
+        s.setBoundary(f, 1, 6)
+    fp = np.geomspace(1e9, 40e9, poles)
+    s.setDebyePoles(fp)
+    s.materialBoxDebye(-1, 1, -1, 1, 0, 1e-4 * (n[2] // 2), DebyeModel(3.5, fp, np.full(poles, 0.05), 0.0))
+    if copper:
+        s.setConductorLoss(5.8e7, 1e9, 40e9)
+        s.pecBox(2e-3, 2.4e-3, 2e-3, 2.5e-3, 0.9e-3, 1.2e-3)
+    p = s.addLumpedPort(2, n[0] // 2, n[1] // 2, 0, 4, 1, 50.0)
+    s.setGaussian(p, 1.0, 8e-12, 3e-12)
+    s.setFrequencies([5e9])
+    s.addVProbe(2, n[0] // 2 + 3, n[1] // 2, 0, 6, 1)
+    s.addIProbe(2, 5, n[0] // 2 - 3, n[0] // 2 + 3, n[1] // 2 - 3, n[1] // 2 + 3)
     s.finalize(0.9)
     return s
 
@@ -55,6 +77,18 @@ def test_runs_sample_what_the_phases_do(lib, kw, steps):
     phases(b, steps)
     assert np.array_equal(a.checkpoint(), b.checkpoint())   # fields and all spectra
     assert np.abs(a.portV(0)).max() > 0
+    a.destroy()
+    b.destroy()
+
+
+@pytest.mark.parametrize("n,poles,copper", [((120, 104, 84), 9, True), ((140, 132, 112), 7, False), ((140, 132, 112), 16, True)])
+def test_lean_blocks_apart_give_the_bits_of_the_phases(lib, n, poles, copper):
+    """Many poles on large grids: the lean rectangles of E in a launch beside the others."""
+    a, b = debye_box(lib, n, poles, copper), debye_box(lib, n, poles, copper)
+    for k in (33, 1, 6):
+        a.step(k)
+    phases(b, 40)
+    assert np.array_equal(a.checkpoint(), b.checkpoint())
     a.destroy()
     b.destroy()
 
