@@ -2140,6 +2140,7 @@ struct Device {
     // runs of whole steps (RunArgs)
     int run_steps = 0;                // most steps of a run (sample rows)
     bool sibc_flagged = false;        // the tables mark the surface-impedance edges
+    bool large = false;   // from 2 M cells
     bool whole_h = true, whole_e = true;   // an update's blocks in one launch (Whole), or a kernel per class
     bool split_e = false;   // of whole_e: the lean rectangles in a launch of their own
     bool chained = false;   // the last launch on the main stream is one of a run, nothing else since
@@ -2968,6 +2969,28 @@ bool build_spaces(cem_sim *s, Device &D, int u) {
     return dev_renew(s, D.wl[u], wl);
 }
 
+// The spaces of both updates, and which of them run as one launch: below 2 M
+// cells, and E with poles (Whole has both sides measured). Where all blocks are
+// lean (no CPML, no poles, no surface impedance) an update is one launch either
+// way, and the lean kernels have more blocks per SM: closed boxes of 1.0e5, 6.5e5,
+// 1.05e6 and 1.8e6 cells 4.6, 12.7, 18.5 and 29.4 us per step as k_whole_*, 4.3, 11.9,
+// 16.9 and 27.2 as the lean kernels. Beside blocks of another kind they gain from 1 M
+// cells (closed boxes with copper of 1.0e5, 1.05e6 and 1.8e6 cells: 5.0, 21.6 and 36.0 as
+// k_whole_*, 5.4, 20.7 and 34.3 as a kernel per class). They have a column of blocks
+// more that samples, so planes of fewer than four blocks stay with k_whole_* (2000
+// x 20 x 20 cells: 16.7 and 18.8).
+bool build_launches(cem_sim *s, Device &D) {
+    if (!build_spaces(s, D, 0) || !build_spaces(s, D, 1)) return false;
+    auto lean = [&](int u) {
+        return !D.wl_start[u].back() && !space_blocks(D.sp[u][kDebye]) && space_blocks(D.sp[u][kFast]) >= 4;
+    };
+    const bool all_lean = lean(0) && lean(1) && !s->nsb && !s->npole;
+    const bool apart = all_lean || (long long)s->n[0] * s->n[1] * s->n[2] >= 1000000;
+    D.whole_h = !D.large && !(apart && lean(0));
+    D.whole_e = s->npole > 0 || (!D.large && !(apart && lean(1)));
+    return true;
+}
+
 bool build_sources(cem_sim *s, Device &D) {
     const size_t plane = (size_t)(s->n[1] + 1) * (s->n[2] + 1);
     if (s->msrc >= 0) {
@@ -3147,10 +3170,8 @@ bool create_device_impl(cem_sim *s) {
     CB2_CHECK(s, cudaGetDevice(&D.device));
     if (const char *e = std::getenv("CEM_B200_FUSED")) D.use_fused = e[0] == '1';
     if (const char *e = std::getenv("CEM_B200_GRAPHS")) D.use_graphs = e[0] != '0';
-    D.ztail = (long long)s->n[0] * s->n[1] * s->n[2] >= 2000000;
-    // one launch an update below 2 M cells; above, for E with poles (Whole has both sides measured)
-    D.whole_h = (long long)s->n[0] * s->n[1] * s->n[2] < 2000000;
-    D.whole_e = D.whole_h || s->npole > 0;
+    const long long cells = (long long)s->n[0] * s->n[1] * s->n[2];
+    D.ztail = D.large = cells >= 2000000;
     // With many poles the registers of their general and Debye blocks (from nine poles on 128, four
     // blocks per SM) cost the lean blocks of the same launch more than sharing a row's ends saves. us
     // per step, all in one launch / the lean blocks apart, of lossy lines: 1.0 M cells, 9, 12 and 16
@@ -3158,7 +3179,6 @@ bool create_device_impl(cem_sim *s) {
     // and 8 poles 46.3 / 47.6, 49.7 / 50.6; 3.4 M cells, 7, 8, 9, 12 and 16 poles 92.6 / 89.7, 95.8 / 92.8,
     // 118.5 / 94.7, 121.2 / 99.0, 124.6 / 104.3; with 4 and 6 poles (eight blocks per SM) 82.7 / 84.1,
     // 89.2 / 90.2.
-    const long long cells = (long long)s->n[0] * s->n[1] * s->n[2];
     D.split_e = s->npole > kLargePoles + 2 ? cells >= 1000000 : s->npole > kLargePoles && cells >= 2000000;
     if (const char *e = std::getenv("CEM_B200_ZTAIL")) {
         D.ztail = e[0] != '0';
@@ -3210,7 +3230,7 @@ bool create_device_impl(cem_sim *s) {
     };
     if (!phase("fields", true) || !phase("pml", build_pml(s, D)) || !phase("tables", build_tables(s, D)) ||
         !phase("probes", build_probes(s, D)) || !phase("sibc", build_sibc(s, D)) ||
-        !phase("sources", build_sources(s, D)) || !phase("spaces", build_spaces(s, D, 0) && build_spaces(s, D, 1)))
+        !phase("sources", build_sources(s, D)) || !phase("spaces", build_launches(s, D)))
         return false;
     for (int b = 0; b < 2; b++)
         for (int c = 0; c < 3; c++)
@@ -3738,7 +3758,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
             carry.first = carry.blocks + (run ? (sb.ns + kBlock - 1) / kBlock : 0);
             if (D.whole_e) {
                 const Whole l = whole(1, a, b, w, n);
-                const bool large = !D.whole_h && s->npole <= kLargePoles;
+                const bool large = D.large && s->npole <= kLargePoles;
                 const WKernel kernel = large ? kEWLarge[s->npole] : kEWKernels[s->npole];
                 const unsigned others = carry.first + n + (unsigned)l.planes * l.nd;   // than the lean blocks
                 if (!D.split_e || !l.planes || !l.nf) {
@@ -3999,7 +4019,7 @@ bool apply_shape(cem_sim *s, Device &D, int thin, bool side, int graph, bool zta
     if (respace) {
         D.thin = thin;
         D.ztail = ztail;
-        if (!build_spaces(s, D, 0) || !build_spaces(s, D, 1)) return false;
+        if (!build_launches(s, D)) return false;
         fill_args(s, D);
     }
     if (respace || graph != D.graph_steps) {

@@ -170,3 +170,28 @@ def test_lean_blocks_of_grids_with_many_poles_run_by_themselves(fake, n, poles, 
     assert fake.count("k_whole_e") - before["k_whole_e"] == 3
     assert fake.count("k_update_e_fast") - before["k_update_e_fast"] == (3 if apart else 0)
     s.destroy()
+
+
+def closed_box(c, n, copper=False):
+    s = c.createSim(*(1e-4 * np.arange(q + 1) for q in n))
+    if copper:
+        s.setConductorLoss(5.8e7, 1e9, 40e9)
+        s.pecBox(1e-3, 1.4e-3, 1e-3, 1.5e-3, 0.9e-3, 1.2e-3)
+    p = s.addLumpedPort(2, n[0] // 2, n[1] // 2, 0, n[2] // 4, 1, 50.0)
+    s.setGaussian(p, 1.0, 8e-12, 3e-12)
+    s.setFrequencies([5e9])
+    s.finalize(0.9)
+    return s
+
+
+@pytest.mark.parametrize("n,copper,lean", [((60, 50, 40), False, True), ((120, 120, 90), False, True), ((60, 50, 40), True, False),
+                                           ((110, 110, 90), True, True), ((300, 8, 8), False, False)])
+def test_grids_of_lean_blocks_run_in_the_lean_kernels(fake, n, copper, lean):
+    fake.current = 0
+    s = closed_box(fake.lib, n, copper)
+    before = {k: fake.count(k) for k in ("k_whole_h", "k_whole_e", "k_update_h_fast", "k_update_e_fast")}
+    s.step(3)
+    made = {k: fake.count(k) - v for k, v in before.items()}
+    whole, fast = (0, 3) if lean else (3, 0)
+    assert made == {"k_whole_h": whole, "k_whole_e": whole, "k_update_h_fast": fast, "k_update_e_fast": fast}
+    s.destroy()
