@@ -2991,6 +2991,13 @@ bool build_launches(cem_sim *s, Device &D) {
     return true;
 }
 
+// whether an update has blocks on the second stream when that is on
+bool uses_side(const cem_sim *s, const Device &D) {
+    auto fast = [&](int u) { return space_blocks(D.sp[u][kFast]) > 0 && D.p1[u] > D.p0[u]; };
+    return (!D.whole_h && D.wl_start[0].back() && fast(0)) ||
+           (D.whole_e ? D.split_e && fast(1) : (D.wl_start[1].back() || s->nsb) && fast(1));
+}
+
 bool build_sources(cem_sim *s, Device &D) {
     const size_t plane = (size_t)(s->n[1] + 1) * (s->n[2] + 1);
     if (s->msrc >= 0) {
@@ -4022,7 +4029,7 @@ bool apply_shape(cem_sim *s, Device &D, int thin, bool side, int graph, bool zta
         if (!build_launches(s, D)) return false;
         fill_args(s, D);
     }
-    if (respace || graph != D.graph_steps) {
+    if (respace || graph != D.graph_steps || side != D.side_on) {
         D.drop_graphs();
         D.graph_steps = graph;
     }
@@ -4050,7 +4057,7 @@ bool shape_ms(cem_sim *s, long warm, long n, double *ms, long *used) {
 }
 
 // choose the launch shape of s (cache, else coordinate descent over the
-// choices, 672 steps); `used` returns the steps it ran
+// choices, up to 672 steps); `used` returns the steps it ran
 bool tune_shape(cem_sim *s, long *used) {
     Device &D = *s->dev;
     const std::string key = shape_key(s);
@@ -4076,7 +4083,7 @@ bool tune_shape(cem_sim *s, long *used) {
     };
     if (!trial(thin, side, graph, !zt)) return false;
     for (int t : {8, 32}) if (!trial(t, side, graph, zt)) return false;
-    if (!trial(thin, !side, graph, zt)) return false;
+    if (uses_side(s, D) && !trial(thin, !side, graph, zt)) return false;
     for (int g : {16, 64}) if (!trial(thin, side, g, zt)) return false;
     D.tuned_ms = best;
     store_shape(key, {(double)thin, side ? 1.0 : 0.0, (double)graph, best, zt ? 1.0 : 0.0});

@@ -68,7 +68,7 @@ CEM_API int cemx_use_fused(cem_sim *s, int on);
  * kernels' thread spaces (8, 16 or 32 points), the z CPML slabs inside the
  * lean kernels' rows or as general blocks, general CPML blocks on a second
  * stream or after the others, 16, 32 or 64 steps per replayed CUDA graph - by
- * timing about 672 of those steps under each choice in turn (every choice
+ * timing up to 672 of those steps under each choice in turn (every choice
  * computes the same bits, so they are ordinary steps), and records the result
  * per grid shape (cells, poles, surface impedance, CPML faces) in a cache file,
  * $CEM_B200_TUNE_CACHE or ~/.cache/courant-b200/launch-shapes.txt, which later

@@ -29,6 +29,7 @@ std::map<const void *, std::string> kernels;
 std::map<std::string, long> counts;
 long copies_left = -1;   // copies until one fails (-1: none does)
 double static_scratch[1 << 17];
+float elapsed = 1.f, elapsed_factor = 1.f;   // what the next pair of events measures, and how it changes
 
 Stream *S(cudaStream_t s) { return reinterpret_cast<Stream *>(s); }
 cudaError_t ret(cudaError_t e) { return e == cudaSuccess ? e : last = e; }
@@ -75,6 +76,7 @@ __attribute__((visibility("default"))) void fake_fail_copy(long after) {
     copies_left = after;
     last = cudaSuccess;
 }
+__attribute__((visibility("default"))) void fake_elapsed(float ms, float factor) { elapsed = ms; elapsed_factor = factor; }
 __attribute__((visibility("default"))) int fake_current() { return current; }
 __attribute__((visibility("default"))) void fake_set_current(int d) { current = d; }
 
@@ -157,7 +159,11 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
     return ret(reinterpret_cast<Event *>(e)->device == S(s)->device ? cudaSuccess : cudaErrorInvalidResourceHandle);
 }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { *ms = 1.f; return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) {
+    *ms = elapsed;
+    elapsed *= elapsed_factor;
+    return cudaSuccess;
+}
 
 cudaError_t cudaStreamBeginCapture(cudaStream_t s, cudaStreamCaptureMode) {
     S(s)->capturing = true;

@@ -16,6 +16,7 @@ class Fake:
         self.so = ctypes.CDLL(str(path))
         self.so.fake_count.restype = ctypes.c_long
         self.so.fake_fail_copy.argtypes = [ctypes.c_long]
+        self.so.fake_elapsed.argtypes = [ctypes.c_float, ctypes.c_float]
 
     def count(self, what):
         return self.so.fake_count(what.encode())
@@ -194,4 +195,36 @@ def test_grids_of_lean_blocks_run_in_the_lean_kernels(fake, n, copper, lean):
     made = {k: fake.count(k) - v for k, v in before.items()}
     whole, fast = (0, 3) if lean else (3, 0)
     assert made == {"k_whole_h": whole, "k_whole_e": whole, "k_update_h_fast": fast, "k_update_e_fast": fast}
+    s.destroy()
+
+
+def open_box(c, n):
+    s = c.createSim(*(1e-4 * np.arange(q + 1) for q in n))
+    for f in (0, 1, 2, 3, 5):
+        s.setBoundary(f, 1, 6)
+    s.setFrequencies([5e9])
+    s.finalize(0.9)
+    return s
+
+
+@pytest.mark.parametrize("n,streams", [((140, 132, 112), 2), ((40, 36, 30), 1)], ids=["two streams", "one stream"])
+def test_the_tuner_times_each_choice_on_its_own_graph(fake, tmp_path, monkeypatch, n, streams):
+    """Every choice times faster than the one before, so each is kept: a graph of its own must have been captured for
+    it (as it is, z tails, two thin-segment thresholds, streams, two graph lengths), none for a stream that is not used.
+    Of the steps left, with 7 choices 1376, the first run ends with the sample ring after 352: 5 graphs of 64 and one of
+    the 32 steps that were left over before as well; with 6 choices 1472, after 448, 7 graphs of 64."""
+    monkeypatch.setenv("CEM_B200_TUNE_CACHE", str(tmp_path / "shapes.txt"))
+    fake.current = 0
+    s = open_box(fake.lib, n)
+    s.prepareDevice()
+    s.tune(True)
+    fake.so.fake_elapsed(1.0, 0.5)
+    before = fake.count("capture")
+    try:
+        s.step(2048)
+    finally:
+        fake.so.fake_elapsed(1.0, 1.0)
+    st = s.tuneState()
+    assert st["tuned"] and fake.count("capture") - before == (8 if streams == 2 else 6)
+    assert st["side_stream"] == (streams == 1)
     s.destroy()
