@@ -2298,10 +2298,11 @@ bool dev_upload(cem_sim *s, DevBuf<T> &b, const std::vector<T> &v) {
     return h2d(s, b.p, v.data(), v.size() * sizeof(T));
 }
 
-// the same into a buffer that may hold an older table (of launches that have ended)
+// the same into a buffer that may hold an older table, which launches in flight may use
 template <class T>
 bool dev_renew(cem_sim *s, DevBuf<T> &b, const std::vector<T> &v) {
     if (b.p && b.own) {
+        CB2_CHECK(s, cudaStreamSynchronize(s->dev->stream));
         CB2_CHECK(s, cudaFree(b.p));
         s->dev->held -= b.n * sizeof(T);
     }

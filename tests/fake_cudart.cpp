@@ -20,11 +20,12 @@ thread_local int current = 0;
 thread_local cudaError_t last = cudaSuccess;
 thread_local struct { dim3 grid, block; size_t smem; cudaStream_t stream; } pushed;
 
-struct Stream { int device; long captured; bool capturing; };
-struct Event { int device; };
+struct Stream { int device; long captured; bool capturing, busy; };
+struct Event { int device; Stream *stream; };
 struct Graph { long launches; };
 
 std::map<void *, std::pair<int, size_t>> memory;
+std::map<Stream *, int> streams;
 std::map<const void *, std::string> kernels;
 std::map<std::string, long> counts;
 long copies_left = -1;   // copies until one fails (-1: none does)
@@ -42,6 +43,7 @@ cudaError_t launch(const void *f, dim3 grid, cudaStream_t stream) {
         S(stream)->captured++;
         return cudaSuccess;
     }
+    S(stream)->busy = true;
     counts["launch"]++;
     counts[kernels[f]]++;
     return cudaSuccess;
@@ -57,7 +59,7 @@ CUresult encode(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cu
 
 extern "C" {
 
-// what the tests ask: "malloc", "free", "live" (bytes), "up" (copies to the device), "launch", "graph" (replays), "capture", or a kernel's name
+// what the tests ask: "malloc", "free", "free in flight" (with launches that nothing has waited for), "live" (bytes), "up" (copies to the device), "launch", "graph" (replays), "capture", or a kernel's name
 __attribute__((visibility("default"))) long fake_count(const char *what) {
     std::lock_guard<std::mutex> l(mu);
     if (!std::strcmp(what, "live")) {
@@ -120,6 +122,8 @@ cudaError_t cudaFree(void *p) {
     if (!memory.erase(p)) return ret(cudaErrorInvalidValue);
     std::free(p);
     counts["free"]++;
+    for (auto &s : streams)
+        if (s.first->busy) { counts["free in flight"]++; break; }
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, cudaMemcpyKind kind, cudaStream_t) {
@@ -143,22 +147,35 @@ cudaError_t cudaGetDriverEntryPoint(const char *, void **f, unsigned long long, 
 }
 
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
-    *s = reinterpret_cast<cudaStream_t>(new Stream{current, 0, false});
+    std::lock_guard<std::mutex> l(mu);
+    Stream *n = new Stream{current, 0, false, false};
+    streams[n] = 1;
+    *s = reinterpret_cast<cudaStream_t>(n);
     return cudaSuccess;
 }
-cudaError_t cudaStreamDestroy(cudaStream_t s) { delete S(s); return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t s) {
+    std::lock_guard<std::mutex> l(mu);
+    streams.erase(S(s));
+    delete S(s);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { S(s)->busy = false; return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
-    *e = reinterpret_cast<cudaEvent_t>(new Event{current});
+    *e = reinterpret_cast<cudaEvent_t>(new Event{current, nullptr});
     return cudaSuccess;
 }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { return cudaEventCreateWithFlags(e, 0); }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { delete reinterpret_cast<Event *>(e); return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    reinterpret_cast<Event *>(e)->stream = S(s);
     return ret(reinterpret_cast<Event *>(e)->device == S(s)->device ? cudaSuccess : cudaErrorInvalidResourceHandle);
 }
-cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {   // (of all that its stream has: enough for a wait at the end)
+    Stream *s = reinterpret_cast<Event *>(e)->stream;
+    if (s && streams.count(s)) s->busy = false;
+    return cudaSuccess;
+}
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) {
     *ms = elapsed;
     elapsed *= elapsed_factor;
@@ -186,6 +203,7 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t x) { delete reinterpret_cast<Gr
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t s) {
     std::lock_guard<std::mutex> l(mu);
     if (S(s)->device != current) return ret(cudaErrorInvalidResourceHandle);
+    S(s)->busy = true;
     counts["graph"]++;
     return cudaSuccess;
 }

@@ -228,3 +228,25 @@ def test_the_tuner_times_each_choice_on_its_own_graph(fake, tmp_path, monkeypatc
     assert st["tuned"] and fake.count("capture") - before == (8 if streams == 2 else 6)
     assert st["side_stream"] == (streams == 1)
     s.destroy()
+
+
+def test_tables_of_launches_in_flight_are_not_freed(fake, tmp_path, monkeypatch):
+    """A tuned shape from the cache file replaces the place tables of a simulation that has steps in flight."""
+    cache = tmp_path / "shapes.txt"
+    monkeypatch.setenv("CEM_B200_TUNE_CACHE", str(cache))
+    fake.current = 0
+    a, b = open_box(fake.lib, (60, 200, 180)), open_box(fake.lib, (60, 200, 180))
+    a.tune(True)
+    fake.so.fake_elapsed(1.0, 0.5)
+    a.step(2048)
+    fake.so.fake_elapsed(1.0, 1.0)
+    assert len(cache.read_text().splitlines()) == 1 and a.tuneState()["z_tails"] != b.tuneState()["z_tails"]
+    a.synchronize()
+    b.step(40)
+    b.tune(True)
+    before = fake.count("free"), fake.count("free in flight")
+    b.step(2048)
+    assert b.tuneState()["from_cache"] and fake.count("free") > before[0]
+    assert fake.count("free in flight") == before[1]
+    a.destroy()
+    b.destroy()
