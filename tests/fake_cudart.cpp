@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <set>
 #include <mutex>
 #include <string>
 
@@ -20,7 +21,12 @@ thread_local int current = 0;
 thread_local cudaError_t last = cudaSuccess;
 thread_local struct { dim3 grid, block; size_t smem; cudaStream_t stream; } pushed;
 
-struct Stream { int device; long captured; bool capturing, busy; };
+struct Stream {
+    int device;
+    long captured;
+    bool capturing, busy;
+    std::set<Stream *> after;   // streams whose work it has waited for
+};
 struct Event { int device; Stream *stream; };
 struct Graph { long launches; };
 
@@ -34,6 +40,14 @@ float elapsed = 1.f, elapsed_factor = 1.f;   // what the next pair of events mea
 
 Stream *S(cudaStream_t s) { return reinterpret_cast<Stream *>(s); }
 cudaError_t ret(cudaError_t e) { return e == cudaSuccess ? e : last = e; }
+
+void settle(Stream *s) {   // what s has, and what it has waited for, is done
+    std::lock_guard<std::mutex> l(mu);
+    if (!streams.count(s)) return;
+    s->busy = false;
+    for (Stream *t : s->after)
+        if (streams.count(t)) t->busy = false;
+}
 
 cudaError_t launch(const void *f, dim3 grid, cudaStream_t stream) {
     std::lock_guard<std::mutex> l(mu);
@@ -148,7 +162,7 @@ cudaError_t cudaGetDriverEntryPoint(const char *, void **f, unsigned long long, 
 
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
     std::lock_guard<std::mutex> l(mu);
-    Stream *n = new Stream{current, 0, false, false};
+    Stream *n = new Stream{current, 0, false, false, {}};
     streams[n] = 1;
     *s = reinterpret_cast<cudaStream_t>(n);
     return cudaSuccess;
@@ -159,8 +173,11 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) {
     delete S(s);
     return cudaSuccess;
 }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { S(s)->busy = false; return cudaSuccess; }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { settle(S(s)); return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
+    if (reinterpret_cast<Event *>(e)->stream) S(s)->after.insert(reinterpret_cast<Event *>(e)->stream);
+    return cudaSuccess;
+}
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
     *e = reinterpret_cast<cudaEvent_t>(new Event{current, nullptr});
     return cudaSuccess;
@@ -173,7 +190,7 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
 }
 cudaError_t cudaEventSynchronize(cudaEvent_t e) {   // (of all that its stream has: enough for a wait at the end)
     Stream *s = reinterpret_cast<Event *>(e)->stream;
-    if (s && streams.count(s)) s->busy = false;
+    if (s) settle(s);
     return cudaSuccess;
 }
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) {
