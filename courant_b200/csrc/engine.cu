@@ -3989,10 +3989,13 @@ std::string shape_cache_path() {
     return base + "/courant-b200/launch-shapes.txt";
 }
 
+// which launches a shape was measured with: counted up when the update kernels change what it is for
+constexpr int kLaunchLayout = 2;   // 1: a kernel per class of blocks on every grid (no mark in the key)
+
 std::string shape_key(const cem_sim *s) {
     char k[160];
-    std::snprintf(k, sizeof k, "%dx%dx%d/p%d/sibc%d/pml%d.%d.%d.%d.%d.%d", s->n[0], s->n[1], s->n[2], s->npole,
-                  s->nsb > 0, s->npml[0], s->npml[1], s->npml[2], s->npml[3], s->npml[4], s->npml[5]);
+    std::snprintf(k, sizeof k, "%dx%dx%d/p%d/sibc%d/pml%d.%d.%d.%d.%d.%d/l%d", s->n[0], s->n[1], s->n[2], s->npole,
+                  s->nsb > 0, s->npml[0], s->npml[1], s->npml[2], s->npml[3], s->npml[4], s->npml[5], kLaunchLayout);
     return k;
 }
 

@@ -1,6 +1,7 @@
 """What the engine asks of the CUDA runtime, with a runtime of two devices in
 host memory in its place (fake_cudart.cpp; kernels do not run)."""
 import ctypes
+import shutil
 import subprocess
 
 import numpy as np
@@ -25,7 +26,7 @@ class Fake:
 
 
 @pytest.fixture(scope="module")
-def fake(tmp_path_factory):
+def fake_path(tmp_path_factory):
     if build.needs_build():
         build.build()
     objs = [build.PKG / "_build" / (p.stem + (".cu.o" if p.suffix == ".cu" else ".o")) for p in build.sources()]
@@ -35,7 +36,12 @@ def fake(tmp_path_factory):
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wall", "-Wextra", f"-I{build.CUDA_LIB.parent / 'include'}",
                     str(build.PKG.parent / "tests" / "fake_cudart.cpp"), *map(str, objs), "-o", str(out), "-Wl,-Bsymbolic",
                     "-lpthread"], check=True)
-    return Fake(out)
+    return out
+
+
+@pytest.fixture(scope="module")
+def fake(fake_path):
+    return Fake(fake_path)
 
 
 READS = {"field": lambda s: s.field(4), "spectrum": lambda s: s.portV(0), "checkpoint": lambda s: s.checkpoint(),
@@ -250,3 +256,23 @@ def test_tables_of_launches_in_flight_are_not_freed(fake, tmp_path, monkeypatch)
     assert fake.count("free in flight") == before[1]
     a.destroy()
     b.destroy()
+
+
+def test_shapes_tuned_for_earlier_kernels_are_measured_again(fake_path, tmp_path, monkeypatch):
+    """A cache file from before the merged launches: its lines are of the same grid, but of other kernels."""
+    cache = tmp_path / "shapes.txt"
+    monkeypatch.setenv("CEM_B200_TUNE_CACHE", str(cache))
+    old = "40x36x30/p0/sibc0/pml6.6.6.6.0.6 8 0 64 0.05 1\n"
+    cache.write_text(old)
+    for name, from_cache in (("first", False), ("second", True)):   # copies of their own: the file is read once a process
+        own = tmp_path / f"lib{name}.so"
+        shutil.copy(fake_path, own)
+        f = Fake(own)
+        s = open_box(f.lib, (40, 36, 30))
+        s.tune(True)
+        s.step(2048)
+        st = s.tuneState()
+        assert st["tuned"] and st["from_cache"] == from_cache
+        s.destroy()
+    lines = cache.read_text().splitlines()
+    assert lines[0] + "\n" == old and len(lines) == 2
