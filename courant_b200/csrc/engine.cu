@@ -2023,7 +2023,8 @@ struct Device {
     bool failed = false;
     std::string error_msg;
 
-    size_t held = 0;   // bytes allocated on the device
+    size_t held = 0;     // bytes allocated on the device
+    long launches = 0;   // kernels and graphs launched (not those of a capture)
 
     // The small tables of a new device state go up together: pool_host collects them, pool_at
     // says whose place is where, flush_pool allocates and copies once. (An allocation, a copy
@@ -3272,6 +3273,7 @@ bool flush_dft(cem_sim *s) {
     t_begin(4);
     k_dft<<<grid, 128, 0, D.stream>>>(D.ring.p, D.nslot, D.nip + 2 * D.nport + 1, D.ring_first, D.ring_count, s->dt,
                                       D.omega.p, s->nf, D.acc.p);
+    D.launches++;
     t_end();
     CB2_CHECK(s, cudaGetLastError());
     D.ring_first += D.ring_count;
@@ -3485,6 +3487,7 @@ bool run_move(cem_sim *s, Move &m) {
             CB2_CHECK(s, cudaEventRecord(D.stage_ev, D.stream));
         }
         k_move<Out><<<std::min(8 * 148u, (m.a.count + 255) / 256), 256, 0, D.stream>>>(m.a);
+        D.launches++;
         CB2_CHECK(s, cudaGetLastError());
         if (Out) {
             if (!d2h(s, st, D.stage.p, bytes)) return false;
@@ -3535,6 +3538,7 @@ bool upload_groups(cem_sim *s, unsigned g, unsigned from_host) {
     if (g & kGroupDft) clear(D.acc.p, 2 * D.acc.n);
     if (nz) {
         k_clear<<<dim3(148, nz), 256, 0, D.stream>>>(z);
+        D.launches++;
         CB2_CHECK(s, cudaGetLastError());
     }
     if (g & (kGroupE0 | kGroupE1 | kGroupE2)) D.vold_valid = false;
@@ -3578,11 +3582,13 @@ bool begin_device_op(cem_sim *s, bool steps = true) {
     if (!steps) return true;
     if (D.ring_count == 0) D.ring_first = s->step;
     k_set_step<<<1, 1, 0, D.stream>>>(D.pa[D.cur], s->step);
+    D.launches++;
     CB2_CHECK(s, cudaGetLastError());
     if (!D.vold_valid && D.nport) {
         PostArgs pa = D.pa[D.cur];
         pa.advance = 0;
         k_post<<<1, kPostThreads, 0, D.stream>>>(pa);
+        D.launches++;
         CB2_CHECK(s, cudaGetLastError());
         D.vold_valid = true;
     }
@@ -3626,14 +3632,17 @@ void launch_sibc_post(cem_sim *s, Device &D) {
         cudaEventRecord(D.fork, D.stream);
         cudaStreamWaitEvent(D.side, D.fork, 0);
         k_sibc<<<nb, kBlock, 0, D.side>>>(D.sb[D.cur]);
+        D.launches++;
         cudaEventRecord(D.join, D.side);
     } else if (s->nsb) {
         t_begin(2);
         k_sibc<<<nb, kBlock, 0, D.stream>>>(D.sb[D.cur]);
+        D.launches++;
         t_end();
     }
     t_begin(3);
     k_post<<<1, kPostThreads, 0, D.stream>>>(pa);
+    D.launches++;
     t_end();
     if (beside) cudaStreamWaitEvent(D.stream, D.join, 0);
 }
@@ -3645,6 +3654,7 @@ bool launch_fused_step(cem_sim *s) {
     const dim3 grid((s->n[2] + 1 + kFK - 1) / kFK, (s->n[1] + 1 + kFJ - 1) / kFJ, (s->n[0] + 1 + kFX - 1) / kFX);
     t_begin(1);
     kFKernels[s->npole]<<<grid, dim3(kFK, kFJ), kFusedSmem, D.stream>>>(D.sa[D.cur], D.fa[D.cur], D.maps[D.cur]);
+    D.launches++;
     t_end();
     D.cur ^= 1;
     launch_sibc_post(s, D);
@@ -3697,6 +3707,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
         c.attrs = &at;
         c.numAttrs = run && D.chained ? 1 : 0;
         cudaLaunchKernelEx(&c, kernel, args...);
+        D.launches++;
         D.chained = run;
     };
     // fast rectangles of update u on node planes [a, b), with one block column more for r.first
@@ -3735,6 +3746,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
                 if (side) {
                     fork();
                     k_update_h<<<n + carry.first, blk, 0, D.side>>>(D.sa[D.cur], w, carry);
+                    D.launches++;
                     cudaEventRecord(D.join, D.side);
                 }
                 const bool here = !n && space_blocks(D.sp[0][kFast]);   // no general blocks: the fast launch carries the run's
@@ -3742,6 +3754,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
                 if (n && !side) launch(k_update_h, dim3(n + carry.first), D.sa[D.cur], w, carry);
                 if (run && !n && !here) {
                     k_begin_step<<<1, blk, 0, D.stream>>>(D.sa[D.cur], carry);
+                    D.launches++;
                     D.chained = false;
                 }
                 if (side) join();
@@ -3752,7 +3765,10 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
     if (phase_mask & 2) {   // port voltages before the E update
         PostArgs pa = D.pa[D.cur];
         pa.advance = 0;
-        if (D.nport) k_post<<<1, kPostThreads, 0, D.stream>>>(pa);
+        if (D.nport) {
+            k_post<<<1, kPostThreads, 0, D.stream>>>(pa);
+            D.launches++;
+        }
     }
     if (phase_mask & 4) {   // E over node planes [i0, i1) within [0, nx)
         const int a = std::max(0, i0), b = std::min(nx, i1);
@@ -3778,6 +3794,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
                     if (beside) {
                         fork();
                         kernel<<<others, blk, 0, D.side>>>(D.sa[D.cur], g, carry, sb);
+                        D.launches++;
                         cudaEventRecord(D.join, D.side);
                     } else if (others) {
                         launch(kernel, dim3(others), D.sa[D.cur], g, carry, sb);
@@ -3789,6 +3806,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
                 if (side) {
                     fork();
                     k_update_e<<<n + carry.first, blk, 0, D.side>>>(D.sa[D.cur], w, carry, sb);
+                    D.launches++;
                     cudaEventRecord(D.join, D.side);
                 }
                 const bool here = !own && space_blocks(D.sp[1][kFast]);
@@ -3796,6 +3814,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
                 if (own && !side) launch(k_update_e, dim3(n + carry.first), D.sa[D.cur], w, carry, sb);
                 if (run && !own && !here) {
                     k_sample_h<<<1, blk, 0, D.stream>>>(D.sa[D.cur], carry);
+                    D.launches++;
                     D.chained = false;
                 }
                 if (side) join();
@@ -3808,6 +3827,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
             if (s->nsb && !D.sibc_flagged) {
                 D.chained = false;
                 k_sibc<<<(unsigned)((s->nsb + kBlock - 1) / kBlock), kBlock, 0, D.stream>>>(D.sb[D.cur]);
+                D.launches++;
             }
         } else {
             if (D.ring_count == kRing && !flush_dft(s)) return false;
@@ -3885,7 +3905,7 @@ namespace {
 bool capture_steps(cem_sim *s, int n, cudaGraphExec_t &exec) {
     Device &D = *s->dev;
     const int rc = D.ring_count;
-    const long st = s->step;
+    const long st = s->step, made = D.launches;
     CB2_CHECK(s, cudaStreamBeginCapture(D.stream, cudaStreamCaptureModeThreadLocal));
     D.chained = false;
     bool ok = true;
@@ -3894,6 +3914,7 @@ bool capture_steps(cem_sim *s, int n, cudaGraphExec_t &exec) {
     const cudaError_t ec = cudaStreamEndCapture(D.stream, &g);
     D.ring_count = rc;
     s->step = st;
+    D.launches = made;
     if (!ok) {
         if (g) cudaGraphDestroy(g);
         return false;
@@ -3920,9 +3941,11 @@ bool run_chunk(cem_sim *s, long n) {
     D.chained = false;
     k_run_begin<<<(unsigned)((n + 127) / 128), 128, 0, D.stream>>>(D.run, pa, reinterpret_cast<float *>(D.run_src.p), (int)n,
                                                                   step0);
+    D.launches++;
     auto replay = [&](cudaGraphExec_t &graph, int k) {
         if (!graph && !capture_steps(s, k, graph)) return false;
         CB2_CHECK(s, cudaGraphLaunch(graph, D.stream));
+        D.launches++;
         D.chained = false;
         D.ring_count += k;
         s->step += k;
@@ -3947,20 +3970,20 @@ bool run_chunk(cem_sim *s, long n) {
     for (; rest > 0; rest--)
         if (!launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1, true)) return false;
     k_rows<<<(unsigned)n, kRowThreads, 0, D.stream>>>(D.run, pa, (int)n, step0);
+    D.launches++;
     CB2_CHECK(s, cudaGetLastError());
     return true;
 }
 
 // n whole steps: in runs with the separate kernels, one by one with the fused
 // kernel and while kernels are timed one by one
-bool run_steps(cem_sim *s, long n, long *launches = nullptr) {
+bool run_steps(cem_sim *s, long n) {
     Device &D = *s->dev;
     const bool runs = !D.use_fused && !g_timer;
     while (n > 0) {
         if (D.ring_count == kRing && !flush_dft(s)) return false;
         const long k = runs ? std::min<long>(n, std::min(D.run_steps, kRing - D.ring_count)) : 1;
         if (runs ? !run_chunk(s, k) : !launch_step(s, 1 | 4 | 8, 0, s->n[0] + 1)) return false;
-        if (launches) *launches += runs ? k / D.graph_steps + k % D.graph_steps + 2 : 1;   // a graph counts once, as does a step
         n -= k;
     }
     CB2_CHECK(s, cudaGetLastError());
@@ -4281,6 +4304,7 @@ struct cemx_batch {
     cudaEvent_t join = nullptr;
     double last_ms = 0;
     long last_steps = 0, last_launches = 0;
+    int last_graph = 32;
 };
 
 namespace {
@@ -4508,10 +4532,13 @@ int cemx_batch_run(cemx_batch *b, long max_steps) {
     if (!b) { set_error("batch: null argument"); return -1; }
     if (cudaSetDevice(b->device) != cudaSuccess) { set_error("batch: cannot select its device"); return -1; }
     std::vector<cem_sim *> touched;
+    long before = 0;
     for (auto &m : b->members)
         if (m.left > 0) {
+            const long made = m.s->dev ? m.s->dev->launches : 0;
             if (!begin_device_op(m.s)) return -1;
             touched.push_back(m.s);
+            before += made;
         }
     b->last_ms = 0;
     b->last_steps = 0;
@@ -4525,7 +4552,7 @@ int cemx_batch_run(cemx_batch *b, long max_steps) {
         for (auto &m : b->members) {
             if (m.left <= 0) continue;
             const long n = std::min({m.left, kTurn, max_steps - done});
-            if (!run_steps(m.s, n, &b->last_launches)) return -1;
+            if (!run_steps(m.s, n)) return -1;
             m.left -= n;
             more += m.left > 0;
             b->last_steps = std::max(b->last_steps, done + n);
@@ -4544,6 +4571,12 @@ int cemx_batch_run(cemx_batch *b, long max_steps) {
     b->last_ms = ms;
     for (cem_sim *s : touched)
         if (!end_device_op(s)) return -1;
+    b->last_launches = -before;
+    b->last_graph = 0;
+    for (cem_sim *s : touched) {
+        b->last_launches += s->dev->launches;
+        b->last_graph = std::max(b->last_graph, s->dev->graph_steps);
+    }
     int left = 0;
     for (auto &m : b->members) left += m.left > 0;
     return left;
@@ -4551,7 +4584,7 @@ int cemx_batch_run(cemx_batch *b, long max_steps) {
 
 int cemx_batch_stats(const cemx_batch *b, double *out, int n) {
     if (!b) return -1;
-    const double v[6] = {b->last_ms, (double)b->last_steps, (double)b->last_launches, 32.0, 0.0,
+    const double v[6] = {b->last_ms, (double)b->last_steps, (double)b->last_launches, (double)b->last_graph, 0.0,
                          (double)b->members.size()};
     for (int q = 0; q < n && q < 6; q++) out[q] = v[q];
     return 0;

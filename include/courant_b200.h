@@ -137,7 +137,8 @@ CEM_API int cemx_batch_run(cemx_batch *b, long max_steps);
 CEM_API int cemx_batch_tune(cemx_batch *b, int on);
 
 /* Statistics of the last run, n entries of: device ms, steps, launches
- * (graph launches count once), graph length, 0, members.
+ * (kernels and graphs, of all members), steps of the members' longest
+ * replayed graph, 0, members.
  * Returns 0 or -1. */
 CEM_API int cemx_batch_stats(const cemx_batch *b, double *out, int n);
 

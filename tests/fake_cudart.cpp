@@ -24,10 +24,11 @@ thread_local struct { dim3 grid, block; size_t smem; cudaStream_t stream; } push
 struct Stream {
     int device;
     long captured;
-    bool capturing, busy;
+    Stream *capture;            // the stream whose capture takes what is launched here
+    bool busy;
     std::set<Stream *> after;   // streams whose work it has waited for
 };
-struct Event { int device; Stream *stream; };
+struct Event { int device; Stream *stream, *capture; };
 struct Graph { long launches; };
 
 std::map<void *, std::pair<int, size_t>> memory;
@@ -53,8 +54,8 @@ cudaError_t launch(const void *f, dim3 grid, cudaStream_t stream) {
     std::lock_guard<std::mutex> l(mu);
     if (!grid.x || !grid.y || !grid.z) return ret(cudaErrorInvalidConfiguration);
     if (S(stream)->device != current) return ret(cudaErrorInvalidResourceHandle);
-    if (S(stream)->capturing) {
-        S(stream)->captured++;
+    if (S(stream)->capture) {
+        S(stream)->capture->captured++;
         return cudaSuccess;
     }
     S(stream)->busy = true;
@@ -162,7 +163,7 @@ cudaError_t cudaGetDriverEntryPoint(const char *, void **f, unsigned long long, 
 
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
     std::lock_guard<std::mutex> l(mu);
-    Stream *n = new Stream{current, 0, false, false, {}};
+    Stream *n = new Stream{current, 0, nullptr, false, {}};
     streams[n] = 1;
     *s = reinterpret_cast<cudaStream_t>(n);
     return cudaSuccess;
@@ -175,17 +176,20 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) {
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { settle(S(s)); return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
-    if (reinterpret_cast<Event *>(e)->stream) S(s)->after.insert(reinterpret_cast<Event *>(e)->stream);
+    const Event *ev = reinterpret_cast<Event *>(e);
+    if (ev->stream) S(s)->after.insert(ev->stream);
+    if (ev->capture && ev->capture->capture) S(s)->capture = ev->capture;
     return cudaSuccess;
 }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
-    *e = reinterpret_cast<cudaEvent_t>(new Event{current, nullptr});
+    *e = reinterpret_cast<cudaEvent_t>(new Event{current, nullptr, nullptr});
     return cudaSuccess;
 }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { return cudaEventCreateWithFlags(e, 0); }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { delete reinterpret_cast<Event *>(e); return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
     reinterpret_cast<Event *>(e)->stream = S(s);
+    reinterpret_cast<Event *>(e)->capture = S(s)->capture;
     return ret(reinterpret_cast<Event *>(e)->device == S(s)->device ? cudaSuccess : cudaErrorInvalidResourceHandle);
 }
 cudaError_t cudaEventSynchronize(cudaEvent_t e) {   // (of all that its stream has: enough for a wait at the end)
@@ -200,14 +204,18 @@ cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) {
 }
 
 cudaError_t cudaStreamBeginCapture(cudaStream_t s, cudaStreamCaptureMode) {
-    S(s)->capturing = true;
+    S(s)->capture = S(s);
     S(s)->captured = 0;
     std::lock_guard<std::mutex> l(mu);
     counts["capture"]++;
     return cudaSuccess;
 }
 cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t *g) {
-    S(s)->capturing = false;
+    {
+        std::lock_guard<std::mutex> l(mu);
+        for (auto &t : streams)
+            if (t.first->capture == S(s)) t.first->capture = nullptr;
+    }
     *g = reinterpret_cast<cudaGraph_t>(new Graph{S(s)->captured});
     return cudaSuccess;
 }

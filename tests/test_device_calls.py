@@ -276,3 +276,30 @@ def test_shapes_tuned_for_earlier_kernels_are_measured_again(fake_path, tmp_path
         s.destroy()
     lines = cache.read_text().splitlines()
     assert lines[0] + "\n" == old and len(lines) == 2
+
+
+def test_batch_statistics_are_what_was_launched(fake, tmp_path, monkeypatch):
+    """Runs without a graph, with graphs of 32 steps, and with one of the steps left over as well."""
+    monkeypatch.setenv("CEM_B200_TUNE_CACHE", str(tmp_path / "shapes.txt"))
+    fake.current = 0
+    sims = [scenes.parity_scene(fake.lib)[0], scenes.lossy_scene(fake.lib)[0], open_box(fake.lib, (140, 132, 112))]
+    b = fake.lib.createBatch()
+    for s in sims:
+        b.add(s, 5000)
+    for n in (7, 1, 42, 42, 300, 1100, 64):
+        before = fake.count("launch") + fake.count("graph")
+        b.run(n)
+        made = fake.count("launch") + fake.count("graph") - before
+        st = b.stats()
+        assert (st["launches"], st["chunk"], st["steps"]) == (made, 32, n)
+    b.remove(sims[2])
+    sims[2].tune(True)
+    fake.so.fake_elapsed(1.0, 0.5)
+    sims[2].step(2048)
+    fake.so.fake_elapsed(1.0, 1.0)
+    b.add(sims[2], 10)
+    b.run(10)
+    assert b.stats()["chunk"] == sims[2].tuneState()["graph_steps"] == 64
+    b.destroy()
+    for s in sims:
+        s.destroy()
