@@ -4545,6 +4545,10 @@ int cemx_batch_run(cemx_batch *b, long max_steps) {
     b->last_launches = 0;
     // members take turns of kTurn steps at most, so that the host feeds all their streams
     constexpr long kTurn = 256;
+    for (cem_sim *s : touched) {   // what members had in flight is not of this run's time
+        CB2_BCHECK(cudaEventRecord(b->join, s->dev->stream));
+        CB2_BCHECK(cudaStreamWaitEvent(b->stream, b->join, 0));
+    }
     CB2_BCHECK(cudaEventRecord(b->ev0, b->stream));
     for (cem_sim *s : touched) CB2_BCHECK(cudaStreamWaitEvent(s->dev->stream, b->ev0, 0));
     for (long done = 0, more = 1; done < max_steps && more; done += kTurn) {
