@@ -128,25 +128,14 @@ struct StepArgs {
     PmlAxis pml[3];
     float *psiH[3][2], *psiE[3][2];
     const unsigned short *mat[3];
-    const float *tab[3];          // field-major: ca-1, cb, cs, beta_p/dt (p = 0..P-1)
     const float4 *tab4[3];        // packed per entry: ca-1, cb, cs, flags (bit pattern)
     const float4 *beta4[3];       // per entry: beta_p/dt of the P poles, nb4 float4 (zero beyond P)
     int nb4;
-    int ntab[3];
-    int npole;
     float omk[kMaxPoles], hk[kMaxPoles];
     float *J[3];
     int jbox[3][6];          // i0, j0, k0, ni, nj, nk of each component's Debye box
-    double dt;
-    double src_amp, src_t0, src_tau;   // lumped Gaussian (amp 0 when none)
-    int msrc_on, i_src;
-    double m_t0, m_tau;
     const float *wsrc[2];    // mode-source weights of Ey and Ez on plane i_src
-    const long long *dstep;
     const float *srcv;       // lumped Vs and modal Vm at this step's H time, FP32 (source_values)
-    // [H, E]: k ranges [zt[u][0], zt[u][1]) and [zt[u][2], zt[u][3]) (four-point groups) where the
-    // lean kernels' rows reach into a z CPML slab and take its auxiliaries (empty: they never do)
-    int zt[2][4];
     const uint2 *item[2][4];   // [H, E][kFast, kGeneral, kAll, kDebye]: the spaces' threads (RowPos)
     int p0[2], p1[2];        // interior node planes of H and E
 };
@@ -535,7 +524,7 @@ __device__ __forceinline__ float4 prev_k(const float4 &v, const float *p, bool n
 // its four, whether it has work (`act`; a thread past the end takes the last
 // thread's position), whether the next lane holds the next four points of the
 // same row (`cont`), whether the previous lane does not hold the previous four
-// (`first`) and whether the four lie in a z tail (StepArgs::zt). One word pair
+// (`first`) and whether the four lie in a z tail (Device::zt). One word pair
 // per thread of the space from a table, the same for every plane: finding the
 // rectangle and dividing by its width took 60-80 of a thread's 300 instructions
 // and a chain of indexed constant loads.
@@ -1691,7 +1680,6 @@ __global__ void __launch_bounds__(kFT, 3) k_step_fused(const StepArgs a, const F
 }
 
 // launchers of the pole-count instantiations
-using HKernel = void (*)(StepArgs, int, RunArgs);
 using FKernel = void (*)(StepArgs, FusedArgs, TmaMaps);
 using WKernel = void (*)(StepArgs, Whole, RunArgs, SibcArgs);
 #define CB2_POLES(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
@@ -1699,7 +1687,7 @@ using WKernel = void (*)(StepArgs, Whole, RunArgs, SibcArgs);
 #define CB2_WK(p) k_whole_e<p, kWholeE>,
 const FKernel kFKernels[] = {CB2_POLES(CB2_FK)};
 const WKernel kEWKernels[] = {CB2_POLES(CB2_WK)};
-const WKernel kEWLarge[] = {k_whole_e<0, kWholeELarge>, k_whole_e<1, kWholeELarge>, k_whole_e<2, kWholeELarge>,
+const WKernel kEWLarge[] = {nullptr /* large grids without poles: a kernel per class */, k_whole_e<1, kWholeELarge>, k_whole_e<2, kWholeELarge>,
                             k_whole_e<3, kWholeELarge>, k_whole_e<4, kWholeELarge>, k_whole_e<5, kWholeELarge>,
                             k_whole_e<kLargePoles, kWholeELarge>};
 #undef CB2_FK
@@ -1785,10 +1773,6 @@ __device__ __forceinline__ void post_block(const PostArgs &a) {
 }
 
 __global__ void __launch_bounds__(kPostThreads) k_post(const PostArgs a) { post_block(a); }
-
-// the same as a launch of its own, where no update launch carries it
-__global__ void __launch_bounds__(kBlock) k_begin_step(const StepArgs a, const RunArgs r) { begin_step(a, r, 0, 1, AtOnce{}); }
-__global__ void __launch_bounds__(kBlock) k_sample_h(const StepArgs a, const RunArgs r) { sample_h(a, r, 0, 1, AtOnce{}); }
 
 // before a run: its next step is the first, the source values of its steps
 __global__ void k_run_begin(const RunArgs r, const PostArgs p, float *src, int steps, long long step0) {
@@ -2053,7 +2037,6 @@ struct Device {
     int zw_h = 0, zw_e = 0;
     std::vector<int> zoff_host[2];   // H, E
     DevBuf<unsigned short> mat[3];
-    DevBuf<float> tab[3];
     DevBuf<float4> tab4[3];
     DevBuf<float4> beta4[3];   // beta_p/dt per table entry, (P + 3) / 4 float4 each
     DevBuf<double> cb64[3];
@@ -2075,7 +2058,9 @@ struct Device {
     Space sp[2][kSpaces]{};
     DevBuf<uint2> item[2][kSpaces];
     int p0[2] = {0, 0}, p1[2] = {0, 0};
-    int zt[2][4] = {};       // z CPML groups the lean kernels' rows reach (StepArgs::zt)
+    // k ranges [zt[u][0], zt[u][1]) and [zt[u][2], zt[u][3]) (four-point groups) where the lean kernels'
+    // rows reach into a z CPML slab and take its auxiliaries (empty: they never do)
+    int zt[2][4] = {};
     DevBuf<int2> wl[2];
     std::vector<int> wl_start[2];
     DevBuf<float> wsrc[2];
@@ -2362,13 +2347,6 @@ struct TableBuilder {
         cb64.push_back(cb);
         return id;
     }
-    std::vector<float> field_major() const {
-        const size_t n = flags.size();
-        std::vector<float> o(n * nf);
-        for (size_t e = 0; e < n; e++)
-            for (int f = 0; f < nf; f++) o[f * n + e] = rows[e * nf + f];
-        return o;
-    }
 };
 
 // Material tables of the three E components. Entries are
@@ -2577,7 +2555,6 @@ bool build_tables(cem_sim *s, Device &D) {
         const int *box_lo = b.box_lo, *box_hi = b.box_hi;
         D.ntab[c] = (int)tb.flags.size();
         if (!dev_upload(s, D.mat[c], b.mat)) return false;
-        if (!dev_upload(s, D.tab[c], tb.field_major())) return false;
         {
             const size_t ne = tb.flags.size();
             std::vector<float4> packed(ne);
@@ -3023,7 +3000,6 @@ void fill_args_for(cem_sim *s, Device &D, int cur) {
         for (int c = 0; c < kSpaces; c++) a.item[u][c] = D.item[u][c].p;
         a.p0[u] = D.p0[u];
         a.p1[u] = D.p1[u];
-        for (int q = 0; q < 4; q++) a.zt[u][q] = D.zt[u][q];
     }
     for (int c = 0; c < 3; c++) {
         a.E[c] = D.E[cur][c].p;
@@ -3037,16 +3013,13 @@ void fill_args_for(cem_sim *s, Device &D, int cur) {
             a.psiE[c][w] = D.psiE[c][w].p;
         }
         a.mat[c] = D.mat[c].p;
-        a.tab[c] = D.tab[c].p;
         a.tab4[c] = D.tab4[c].p;
         a.beta4[c] = D.beta4[c].p;
-        a.ntab[c] = D.ntab[c];
         a.J[c] = D.J[c].p;
         for (int q = 0; q < 6; q++) a.jbox[c][q] = D.jbox[c][q];
     }
     a.dth = (float)(s->dt / CEM_MU0);
     a.has_pml = s->has_pml;
-    a.npole = s->npole;
     a.nb4 = (s->npole + 3) / 4;
     for (int p = 0; p < s->npole; p++) {
         const double tau = 1.0 / (2 * M_PI * s->pole_f[p]);
@@ -3054,19 +3027,10 @@ void fill_args_for(cem_sim *s, Device &D, int cur) {
         a.omk[p] = (float)(2 * r / (1 + r));   // 1 - k_p
         a.hk[p] = (float)(0.5 * (1 + s->d_k[p]));
     }
-    a.dt = s->dt;
-    a.src_amp = s->src_port >= 0 ? s->src_amp : 0.0;
-    a.src_t0 = s->src_t0;
-    a.src_tau = s->src_tau;
-    a.msrc_on = s->msrc >= 0;
-    if (a.msrc_on) {
-        a.i_src = s->mport[s->msrc].def.i_src;
-        a.m_t0 = s->msrc_t0;
-        a.m_tau = s->msrc_tau;
+    if (s->msrc >= 0) {
         a.wsrc[0] = D.wsrc[0].p;
         a.wsrc[1] = D.wsrc[1].p;
     }
-    a.dstep = D.dstep.p;
     a.srcv = D.srcv.p;
 
     FusedArgs &f = D.fa[cur];
@@ -3749,14 +3713,8 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
                     D.launches++;
                     cudaEventRecord(D.join, D.side);
                 }
-                const bool here = !n && space_blocks(D.sp[0][kFast]);   // no general blocks: the fast launch carries the run's
-                fast(0, a, b, k_update_h_fast, here ? carry : none);
+                fast(0, a, b, k_update_h_fast, n ? none : carry);   // without general blocks it carries the run's
                 if (n && !side) launch(k_update_h, dim3(n + carry.first), D.sa[D.cur], w, carry);
-                if (run && !n && !here) {
-                    k_begin_step<<<1, blk, 0, D.stream>>>(D.sa[D.cur], carry);
-                    D.launches++;
-                    D.chained = false;
-                }
                 if (side) join();
             }
             t_end();
@@ -3809,14 +3767,8 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
                     D.launches++;
                     cudaEventRecord(D.join, D.side);
                 }
-                const bool here = !own && space_blocks(D.sp[1][kFast]);
-                fast(1, a, b, k_update_e_fast, here ? carry : none);
+                fast(1, a, b, k_update_e_fast, own ? none : carry);
                 if (own && !side) launch(k_update_e, dim3(n + carry.first), D.sa[D.cur], w, carry, sb);
-                if (run && !own && !here) {
-                    k_sample_h<<<1, blk, 0, D.stream>>>(D.sa[D.cur], carry);
-                    D.launches++;
-                    D.chained = false;
-                }
                 if (side) join();
             }
             t_end();
