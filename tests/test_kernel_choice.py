@@ -25,3 +25,19 @@ def test_separate_kernels_go_on_from_a_fused_step(lib, n):
     assert a.steps == b.steps
     assert np.array_equal(a.checkpoint(), b.checkpoint())
     assert np.array_equal(a.portV(0), b.portV(0)) and a.energy() == b.energy()
+
+
+def test_replayed_graphs_give_the_bits_of_launches(lib, monkeypatch):
+    """Graphs of 32 steps and of the 12 left over, a graph of 7 steps replayed, and no graph at all
+    (CEM_B200_GRAPHS=0), past a flush of the sample ring (1024 steps)."""
+    monkeypatch.setenv("CEM_B200_GRAPHS", "0")
+    plain = scenes.lossy_scene(lib)[0]
+    plain.prepareDevice()
+    monkeypatch.delenv("CEM_B200_GRAPHS")
+    a, b = scenes.lossy_scene(lib)[0], scenes.lossy_scene(lib)[0]
+    plain.step(1100)
+    a.step(1100)
+    for n in [7] * 157 + [1]:
+        b.step(n)
+    want = plain.checkpoint()
+    assert np.array_equal(a.checkpoint(), want) and np.array_equal(b.checkpoint(), want)

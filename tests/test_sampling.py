@@ -81,9 +81,10 @@ def test_runs_sample_what_the_phases_do(lib, kw, steps):
     b.destroy()
 
 
-@pytest.mark.parametrize("n,poles,copper", [((120, 104, 84), 9, True), ((140, 132, 112), 7, False), ((140, 132, 112), 16, True)])
-def test_lean_blocks_apart_give_the_bits_of_the_phases(lib, n, poles, copper):
-    """Many poles on large grids: the lean rectangles of E in a launch beside the others."""
+@pytest.mark.parametrize("n,poles,copper", [((120, 104, 84), 9, True), ((140, 132, 112), 7, False), ((140, 132, 112), 16, True),
+                                            ((140, 132, 112), 4, True), ((140, 132, 112), 1, False)])
+def test_e_of_large_grids_with_poles_gives_the_bits_of_the_phases(lib, n, poles, copper):
+    """All blocks of E in one launch, and with many poles the lean rectangles in a launch beside the others."""
     a, b = debye_box(lib, n, poles, copper), debye_box(lib, n, poles, copper)
     for k in (33, 1, 6):
         a.step(k)
