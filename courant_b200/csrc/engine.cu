@@ -3537,8 +3537,7 @@ bool download_groups(cem_sim *s, unsigned g, const StateView &to) {
 // Make the device state current before a device operation. What callers may
 // have written through a pointer they hold goes up again (the spectra are handed
 // out as const: they stay); steps: the operation advances the simulation, so
-// the step count, source values and port voltages are set and the host copies
-// cease to be current. Nothing waits for the device unless something goes up.
+// the port voltages are set and the host copies cease to be current. Nothing waits for the device unless something goes up.
 // (Five waits and two small copies an operation were half of a ten-step call
 // on a small grid.)
 bool begin_device_op(cem_sim *s, bool steps = true) {
@@ -3551,9 +3550,6 @@ bool begin_device_op(cem_sim *s, bool steps = true) {
     s->dev_valid = kGroupAll;
     if (!steps) return true;
     if (D.ring_count == 0) D.ring_first = s->step;
-    k_set_step<<<1, 1, 0, D.stream>>>(D.pa[D.cur], s->step);
-    D.launches++;
-    CB2_CHECK(s, cudaGetLastError());
     if (!D.vold_valid && D.nport) {
         PostArgs pa = D.pa[D.cur];
         pa.advance = 0;
@@ -3563,6 +3559,16 @@ bool begin_device_op(cem_sim *s, bool steps = true) {
         D.vold_valid = true;
     }
     s->host_valid = 0;
+    return true;
+}
+
+// Before steps that are launched one by one: the step count and its source
+// values. (A run brings its own, k_run_begin.)
+bool set_device_step(cem_sim *s) {
+    Device &D = *s->dev;
+    k_set_step<<<1, 1, 0, D.stream>>>(D.pa[D.cur], s->step);
+    D.launches++;
+    CB2_CHECK(s, cudaGetLastError());
     return true;
 }
 
@@ -3938,6 +3944,7 @@ bool run_chunk(cem_sim *s, long n) {
 bool run_steps(cem_sim *s, long n) {
     Device &D = *s->dev;
     const bool runs = !D.use_fused && !g_timer;
+    if (!runs && !set_device_step(s)) return false;
     while (n > 0) {
         if (D.ring_count == kRing && !flush_dft(s)) return false;
         const long k = runs ? std::min<long>(n, std::min(D.run_steps, kRing - D.ring_count)) : 1;
@@ -4092,7 +4099,7 @@ int engine_step(cem_sim *s, long n) {
 }
 
 int engine_phase(cem_sim *s, int phase, int i0, int i1) {
-    if (!begin_device_op(s)) return -1;
+    if (!begin_device_op(s) || !set_device_step(s)) return -1;
     static const int masks[5] = {0, 1, 2, 4, 8};
     if (phase < 0 || phase > 4) return 0;
     if (phase == 2) s->dev->vold_valid = true;
@@ -4217,7 +4224,7 @@ bool timed_steps(cem_sim *s, long n, double *ms) {
 }
 
 bool profiled_steps(cem_sim *s, long n, double *kernel_ms, long *launches) {
-    if (!begin_device_op(s)) return false;
+    if (!begin_device_op(s) || !set_device_step(s)) return false;
     Device &D = *s->dev;
     KernelTimer timer;
     timer.stream = D.stream;
@@ -4489,11 +4496,15 @@ int cemx_batch_tune(cemx_batch *b, int on) {
 int cemx_batch_run(cemx_batch *b, long max_steps) {
     if (!b) { set_error("batch: null argument"); return -1; }
     if (cudaSetDevice(b->device) != cudaSuccess) { set_error("batch: cannot select its device"); return -1; }
-    std::vector<cem_sim *> touched;
+    std::vector<cem_sim *> touched, busy;   // busy: with earlier work in flight
     long before = 0;
     for (auto &m : b->members)
         if (m.left > 0) {
             const long made = m.s->dev ? m.s->dev->launches : 0;
+            if (m.s->dev && cudaStreamQuery(m.s->dev->stream) == cudaErrorNotReady) {
+                cudaGetLastError();   // no error of a launch
+                busy.push_back(m.s);
+            }
             if (!begin_device_op(m.s)) return -1;
             touched.push_back(m.s);
             before += made;
@@ -4503,7 +4514,7 @@ int cemx_batch_run(cemx_batch *b, long max_steps) {
     b->last_launches = 0;
     // members take turns of kTurn steps at most, so that the host feeds all their streams
     constexpr long kTurn = 256;
-    for (cem_sim *s : touched) {   // what members had in flight is not of this run's time
+    for (cem_sim *s : busy) {   // that work is not of this run's time
         CB2_BCHECK(cudaEventRecord(b->join, s->dev->stream));
         CB2_BCHECK(cudaStreamWaitEvent(b->stream, b->join, 0));
     }

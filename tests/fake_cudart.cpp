@@ -175,6 +175,7 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) {
     return cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { settle(S(s)); return cudaSuccess; }
+cudaError_t cudaStreamQuery(cudaStream_t s) { return ret(S(s)->busy ? cudaErrorNotReady : cudaSuccess); }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
     const Event *ev = reinterpret_cast<Event *>(e);
     if (ev->stream) S(s)->after.insert(ev->stream);

@@ -298,8 +298,20 @@ def test_batch_statistics_are_what_was_launched(fake, tmp_path, monkeypatch):
     sims[2].step(2048)
     fake.so.fake_elapsed(1.0, 1.0)
     b.add(sims[2], 10)
+    sims[2].step(3)   # in flight when the run begins
     b.run(10)
     assert b.stats()["chunk"] == sims[2].tuneState()["graph_steps"] == 64
     b.destroy()
     for s in sims:
         s.destroy()
+
+
+def test_a_short_call_launches_no_more_than_its_run(fake):
+    """One step: the run's begin, H, E and its sample rows; the step count and source values are the run's own."""
+    fake.current = 0
+    s = scenes.parity_scene(fake.lib)[0]
+    s.step(5)
+    before = fake.count("launch")
+    s.step(1)
+    assert fake.count("launch") - before == 4
+    s.destroy()
