@@ -2155,6 +2155,7 @@ struct Device {
     // capture): graph_steps steps; the rest of the last run
     cudaGraphExec_t graph[2] = {nullptr, nullptr}, tail[2] = {nullptr, nullptr};
     int tail_steps[2] = {0, 0};
+    bool graph_wanted[2] = {false, false};   // a run of graph_steps has been launched without one
 
     void drop_graphs() {   // of launches that have ended
         for (int b = 0; b < 2; b++) {
@@ -2162,6 +2163,7 @@ struct Device {
             if (tail[b]) cudaGraphExecDestroy(tail[b]);
             graph[b] = tail[b] = nullptr;
             tail_steps[b] = 0;
+            graph_wanted[b] = false;
         }
     }
 
@@ -3916,11 +3918,20 @@ bool run_chunk(cem_sim *s, long n) {
         return true;
     };
     long rest = n;
-    for (const int gs = D.graph_steps; D.use_graphs && rest >= gs; rest -= gs)
+    const int gs = D.graph_steps;
+    bool &wanted = D.graph_wanted[D.cur];
+    // a graph is captured for four replays at once, or when the run before could have used it: a
+    // capture takes 450 us of the host's time, the launches of 32 steps 140 (first run of 32
+    // steps of a batch of 24 small members: 12 ms with a capture each, 6 without)
+    const bool graphs = D.use_graphs && (wanted || rest >= 4 * gs);
+    wanted = wanted || rest >= gs;
+    for (; graphs && rest >= gs; rest -= gs)
         if (!replay(D.graph[D.cur], gs)) return false;
     // what is left over: one graph too when the run before left as much (a ten-step
     // call spends 55 us of the host's time on its launches, 8 on the graph's)
-    if (rest && rest != tail_steps) {
+    if (rest >= gs) {
+        // launched one by one below
+    } else if (rest && rest != tail_steps) {
         if (tail) {
             CB2_CHECK(s, cudaStreamSynchronize(D.stream));
             cudaGraphExecDestroy(tail);
@@ -4036,6 +4047,7 @@ bool shape_ms(cem_sim *s, long warm, long n, double *ms, long *used) {
         CB2_CHECK(s, cudaEventCreate(&D.tev[0]));
         CB2_CHECK(s, cudaEventCreate(&D.tev[1]));
     }
+    D.graph_wanted[D.cur] = true;   // captured before the timed steps
     if (!run_steps(s, warm)) return false;
     CB2_CHECK(s, cudaEventRecord(D.tev[0], D.stream));
     if (!run_steps(s, n)) return false;
