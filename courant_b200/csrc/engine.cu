@@ -533,7 +533,9 @@ __device__ __forceinline__ float4 prev_k(const float4 &v, const float *p, bool n
 // (`first`) and whether the four lie in a z tail (Device::zt). One word pair
 // per thread of the space from a table, the same for every plane: finding the
 // rectangle and dividing by its width took 60-80 of a thread's 300 instructions
-// and a chain of indexed constant loads.
+// and a chain of indexed constant loads. (Where a plane holds a few groups only, one
+// load more before the fields is the longer way: 20000 x 3 x 3 cells 126 us per step,
+// with the division 76; 4000 x 8 x 8 27 and 23.)
 struct RowPos {
     int j, k4;
     bool act, cont, first, tail;
@@ -1395,7 +1397,10 @@ __global__ void __launch_bounds__(kBlock, CB2_E_MINBLOCKS)
 // 13.1, 1.1 M-cell board 41.2 / 40.2 / 38.3, lossy line (6 poles, 3.6 M cells)
 // 102 / 99.4 / 101, 10.9 M-cell board 364 / 334 / 352, 5.7 M-cell line (no
 // poles) 123 / 125 / 128. (General blocks spread evenly over the launch
-// instead: 1.1 M-cell board 43.7, 10.9 M-cell 373.)
+// instead: 1.1 M-cell board 43.7, 10.9 M-cell 373.) About the border of 2 M cells, H per
+// class / in one launch: boards of 1.30, 1.73, 2.15, 2.61 and 3.05 M cells 47.1 / 44.3,
+// 64.8 / 62.6, 75.2 / 75.7, 90.3 / 91.2, 102.4 / 103.4; both updates, lines without poles of
+// 1.43, 1.81, 2.19 and 2.55 M cells 28.2 / 28.0, 35.6 / 35.9, 44.0 / 45.5, 53.1 / 55.3.
 struct Whole {
     const int2 *work;    // general entries (node plane, block)
     int n;
@@ -4263,11 +4268,13 @@ bool profiled_steps(cem_sim *s, long n, double *kernel_ms, long *launches) {
 
 // Simulations advanced together on one device (cemx_batch_*). Each member keeps
 // its own device state and steps on its own stream with its own replayed
-// graphs; the GPU runs the members' launches side by side, so small members
-// fill what one of them leaves idle, a change of members costs nothing, and a
-// member at the end of its budget holds none of the others up. (Work-lists of
-// all members' blocks in common launches, in lockstep: 189 us per step for
-// eight boards of 5e4-8e5 cells, 2.6 M in all.)
+// graphs, so a change of members costs nothing and a member at the end of its
+// budget holds none of the others up. us per step of boards of 6e4-8.5e5 cells, one
+// after another / as a batch: two members (1.0 M cells) 37.9 / 33.6, eight (2.7 M) 112 /
+// 120, 24 (8.0 M) 332 / 354: running side by side gains where members leave the GPU
+// idle and costs where each launch fills it. (Without chained launches 43.6 / 37.0, 133 /
+// 126, 394 / 370. Work-lists of all members' blocks in common launches, in lockstep: 189
+// for the eight.)
 struct cemx_batch {
     struct Member {
         cem_sim *s;
