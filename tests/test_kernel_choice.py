@@ -41,3 +41,19 @@ def test_replayed_graphs_give_the_bits_of_launches(lib, monkeypatch):
         b.step(n)
     want = plain.checkpoint()
     assert np.array_equal(a.checkpoint(), want) and np.array_equal(b.checkpoint(), want)
+
+
+def test_state_is_read_from_a_thread_without_a_device(lib):
+    """A thread that has made no CUDA call reads fields, spectra and a checkpoint of another thread's simulation."""
+    import threading
+
+    s = scenes.lossy_scene(lib)[0]
+    s.step(50)
+    got = []
+    t = threading.Thread(target=lambda: got.extend([s.portV(0), s.field(2), s.checkpoint()]))
+    t.start()
+    t.join()
+    want = scenes.lossy_scene(lib)[0]
+    want.step(50)
+    assert len(got) == 3
+    assert np.array_equal(got[0], want.portV(0)) and np.array_equal(got[1], want.field(2)) and np.array_equal(got[2], want.checkpoint())
