@@ -2098,6 +2098,7 @@ struct Device {
     long long ring_first = 0;
     int ring_count = 0;
     bool vold_valid = false;
+    bool vold_taken = false;   // by cem_mt_mid, for the cem_mt_post to come
 
     TmaMaps maps[2]{};
     DevBuf<int> error;
@@ -3544,10 +3545,11 @@ bool download_groups(cem_sim *s, unsigned g, const StateView &to) {
 // Make the device state current before a device operation. What callers may
 // have written through a pointer they hold goes up again (the spectra are handed
 // out as const: they stay); steps: the operation advances the simulation, so
-// the port voltages are set and the host copies cease to be current. Nothing waits for the device unless something goes up.
+// the port voltages are set and the host copies cease to be current; phase: of
+// engine_phase. Nothing waits for the device unless something goes up.
 // (Five waits and two small copies an operation were half of a ten-step call
 // on a small grid.)
-bool begin_device_op(cem_sim *s, bool steps = true) {
+bool begin_device_op(cem_sim *s, bool steps = true, int phase = 0) {
     if (!create_device(s)) return false;
     Device &D = *s->dev;
     if (D.failed) { set_error(D.error_msg.c_str()); return false; }
@@ -3557,7 +3559,9 @@ bool begin_device_op(cem_sim *s, bool steps = true) {
     s->dev_valid = kGroupAll;
     if (!steps) return true;
     if (D.ring_count == 0) D.ring_first = s->step;
-    if (!D.vold_valid && D.nport) {
+    // what cem_mt_mid has taken stands until cem_mt_post, however often E goes up and down between them
+    if (phase < 3) D.vold_taken = false;
+    if (!D.vold_valid && !D.vold_taken && D.nport) {
         PostArgs pa = D.pa[D.cur];
         pa.advance = 0;
         k_post<<<1, kPostThreads, 0, D.stream>>>(pa);
@@ -4116,11 +4120,12 @@ int engine_step(cem_sim *s, long n) {
 }
 
 int engine_phase(cem_sim *s, int phase, int i0, int i1) {
-    if (!begin_device_op(s) || !set_device_step(s)) return -1;
+    if (!begin_device_op(s, true, phase) || !set_device_step(s)) return -1;
     static const int masks[5] = {0, 1, 2, 4, 8};
     if (phase < 0 || phase > 4) return 0;
-    if (phase == 2) s->dev->vold_valid = true;
+    if (phase == 2) s->dev->vold_valid = s->dev->vold_taken = true;
     if (!launch_step(s, masks[phase], i0, i1)) return -1;
+    if (phase == 4) s->dev->vold_taken = false;
     if (!end_device_op(s)) return -1;
     return 0;
 }
