@@ -3929,10 +3929,12 @@ bool run_chunk(cem_sim *s, long n) {
     long rest = n;
     const int gs = D.graph_steps;
     bool &wanted = D.graph_wanted[D.cur];
-    // a graph is captured for four replays at once, or when the run before could have used it: a
+    // a graph is captured for two replays at once, or when the run before could have used it: a
     // capture takes 450 us of the host's time, the launches of 32 steps 140 (first run of 32
-    // steps of a batch of 24 small members: 12 ms with a capture each, 6 without)
-    const bool graphs = D.use_graphs && (wanted || rest >= 4 * gs);
+    // steps of a batch of 24 small members: 12 ms with a capture each, 6 without). Not for more
+    // at once: a program that starts with some hundred steps has its graph then, not in the
+    // first run that it waits for.
+    const bool graphs = D.use_graphs && (wanted || rest >= 2 * gs);
     wanted = wanted || rest >= gs;
     for (; graphs && rest >= gs; rest -= gs)
         if (!replay(D.graph[D.cur], gs)) return false;

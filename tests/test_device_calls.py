@@ -318,14 +318,14 @@ def test_a_short_call_launches_no_more_than_its_run(fake):
 
 
 def test_a_graph_is_captured_when_it_will_be_replayed(fake):
-    """Not for the first 32 steps (a capture costs the host more than their launches); for the next, or for 128 at once."""
+    """Not for the first 32 steps (a capture costs the host more than their launches); for the next, or for 64 at once."""
     fake.current = 0
     a, b = scenes.parity_scene(fake.lib)[0], scenes.parity_scene(fake.lib)[0]
     made = fake.count("capture")
     a.step(32)
     assert fake.count("capture") == made
     a.step(32)
-    b.step(128)
+    b.step(64)
     assert fake.count("capture") == made + 2
     a.destroy()
     b.destroy()
