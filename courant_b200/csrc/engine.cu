@@ -4351,7 +4351,8 @@ int cemx_sizes(const cem_sim *s, long long *out, int n) {
         for (int u = 0; u < 2; u++) {
             if (u ? D.whole_e && !D.split_e : D.whole_h) { upd--; continue; }
             upd -= space_blocks(D.sp[u][kFast]) == 0 || D.p1[u] <= D.p0[u];
-            upd -= D.wl_start[u].empty() || D.wl_start[u].back() == 0;
+            const bool edges = u && s->nsb && D.sibc_flagged;   // the general launch carries them
+            upd -= (D.wl_start[u].empty() || D.wl_start[u].back() == 0) && !edges;
         }
     }
     // with the fused kernel also the surface impedance and the probes

@@ -329,3 +329,20 @@ def test_a_graph_is_captured_when_it_will_be_replayed(fake):
     assert fake.count("capture") == made + 2
     a.destroy()
     b.destroy()
+
+
+LAUNCHES = {"plain": lambda c: scenes.parity_scene(c)[0], "lossy": lambda c: scenes.lossy_scene(c)[0],
+            "closed": lambda c: closed_box(c, (60, 50, 40)), "closed copper": lambda c: closed_box(c, (60, 50, 40), True),
+            "larger closed copper": lambda c: closed_box(c, (110, 110, 90), True), "large": lambda c: open_box(c, (140, 132, 112)),
+            "many poles": lambda c: debye_box(c, (120, 104, 84), 12), "large, poles": lambda c: debye_box(c, (140, 132, 112), 4)}
+
+
+@pytest.mark.parametrize("name", LAUNCHES)
+def test_launches_per_step_are_what_is_launched(fake, name):
+    fake.current = 0
+    s = LAUNCHES[name](fake.lib)
+    s.step(1)
+    before = fake.count("launch")
+    s.step(5)   # and the run's begin and its sample rows
+    assert fake.count("launch") - before == 5 * s.sizes()["launches_per_step"] + 2
+    s.destroy()
