@@ -570,6 +570,7 @@ class Batch:
         return self._check(self.c.ex.cemx_batch_run(self.h, int(max_steps)), "batch_run")
 
     def tune(self, on: bool = True) -> bool:
+        """Kept for callers that set it: a batch has nothing to choose. Returns the previous setting."""
         return bool(self.c.ex.cemx_batch_tune(self.h, int(on)))
 
     def stats(self) -> dict:

@@ -43,6 +43,7 @@
 #include <array>
 #include <chrono>
 #include <mutex>
+#include <new>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -3272,6 +3273,7 @@ bool make_jmap(cem_sim *s) {
     if (D.jmap_made) return true;
     size_t e = 0;
     for (int c = 0; c < 3; c++) {
+        D.jruns[c].clear();
         const int *bx = D.jbox[c];
         while (e < (size_t)s->ndisp && s->d_comp[e] == c) {
             const size_t q = s->d_idx[e];
@@ -3442,7 +3444,8 @@ bool make_stage(cem_sim *s) {
     CB2_CHECK(s, cudaEventCreateWithFlags(&D.stage_ev, cudaEventDisableTiming));
     D.stage_words = std::min((words + 1) / 2 * 2, kStageWords);
     if (!dev_alloc(s, D.stage, D.stage_words + (packed ? s->ndisp : 0))) return false;
-    D.stage_host.reset(new unsigned[D.stage_words]);
+    D.stage_host.reset(new (std::nothrow) unsigned[D.stage_words]);
+    if (!D.stage_host) { set_error("out of memory"); return false; }
     return true;
 }
 

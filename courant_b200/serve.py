@@ -82,7 +82,7 @@ class Server:
         self.lib = lib
         self.budget = int(budget_bytes)
         self.chunk = chunk
-        self.tune = tune
+        self.tune = tune   # handed on for callers that set it: a batch has nothing to choose
         self.batch = lib.createBatch(device)
         self.batch.tune(tune)
         self.incoming: queue.Queue = queue.Queue()
