@@ -210,7 +210,7 @@ struct RunArgs {
     const float2 *src;       // per step of the run: lumped and modal source values
     float2 *srcv;            // the current step's, which the E update reads
     int *at;                 // [0] step of the run in progress, [1] the next one
-    int on;                  // whether the launch belongs to a run
+    int chain;               // whether the launch lets the next one begin early (chain_next)
     // blocks of the launch before the update's own: sampling, then surface impedance (of the
     // per-class fast launches: one column more, whose first rows sample)
     int first;
@@ -534,9 +534,7 @@ __device__ __forceinline__ float4 prev_k(const float4 &v, const float *p, bool n
 // (`first`) and whether the four lie in a z tail (Device::zt). One word pair
 // per thread of the space from a table, the same for every plane: finding the
 // rectangle and dividing by its width took 60-80 of a thread's 300 instructions
-// and a chain of indexed constant loads. (Where a plane holds a few groups only, one
-// load more before the fields is the longer way: 20000 x 3 x 3 cells 126 us per step,
-// with the division 76; 4000 x 8 x 8 27 and 23.)
+// and a chain of indexed constant loads.
 struct RowPos {
     int j, k4;
     bool act, cont, first, tail;
@@ -1292,7 +1290,7 @@ __device__ __forceinline__ void sample_h(const StepArgs &a, const RunArgs &r, in
 #define CB2_EF_MINBLOCKS 9
 #endif
 
-// Chained launches (RunArgs::on): a launch that follows another on one stream
+// Chained launches: a launch that follows another on one stream
 // alone may start while that one ends; meanwhile it works out its place and
 // fetches from the tables that no launch writes (CPML planes, material indices,
 // probe and surface-impedance entries), then waits for the end before it touches
@@ -1302,7 +1300,9 @@ __device__ __forceinline__ void sample_h(const StepArgs &a, const RunArgs &r, in
 // other's writes visible; the read-only path promises nothing there.) Parity
 // scene 6.8 to 5.9 us per step, lossy scene 8.2 to 6.9, cavity 5.8 to 5.4; with the
 // tables before the wait, 5.35 to 3.8, 6.25 to 4.5 and 5.0 to 4.6, 121 x 62 x 40
-// line 9.9 to 8.7, 250 k-cell board 12.5 to 11.6.
+// line 9.9 to 8.7, 250 k-cell board 12.5 to 11.6. Letting the next one begin costs the
+// launch something per block, 950 blocks a us at most: for thousands of planes of one
+// block of a few threads that is the launch's time, and it is left out (Device::thin).
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 struct Chained {
@@ -1315,7 +1315,7 @@ struct AtOnce {
 // H on the fast rectangles of node planes [i0, i0 + gridDim.y); block x:
 // block x / 3 of the space, component x % 3
 __global__ void __launch_bounds__(kBlock, CB2_HF_MINBLOCKS) k_update_h_fast(const StepArgs a, int i0, const RunArgs r) {
-    chain_next();
+    if (r.chain) chain_next();
     if (r.first && blockIdx.x == gridDim.x - 1) {   // one column more: the run's own work
         const int n = min(r.blocks, (int)gridDim.y);
         if ((int)blockIdx.y < n) begin_step(a, r, (int)blockIdx.y, n, Chained{});
@@ -1331,7 +1331,7 @@ __global__ void __launch_bounds__(kBlock, CB2_HF_MINBLOCKS) k_update_h_fast(cons
 
 // E on the fast rectangles of node planes [i0, i0 + gridDim.y), from the last to the first
 __global__ void __launch_bounds__(kBlock, CB2_EF_MINBLOCKS) k_update_e_fast(const StepArgs a, int i0, const RunArgs r) {
-    chain_next();
+    if (r.chain) chain_next();
     if (r.first && blockIdx.x == gridDim.x - 1) {
         const int n = min(r.blocks, (int)gridDim.y);
         if ((int)blockIdx.y < n) sample_h(a, r, (int)blockIdx.y, n, Chained{});
@@ -1355,7 +1355,7 @@ __device__ __forceinline__ RowPos general_pos(const StepArgs &a, int i, int b) {
 // Work entry of the general blocks: x node plane, y block of the plane's
 // general space (component y % 3, block y / 3).
 __global__ void __launch_bounds__(kBlock, CB2_H_MINBLOCKS) k_update_h(const StepArgs a, const int2 *work, const RunArgs r) {
-    chain_next();
+    if (r.chain) chain_next();
     if ((int)blockIdx.x < r.first) {
         begin_step(a, r, (int)blockIdx.x, r.blocks, Chained{});
         return;
@@ -1371,7 +1371,7 @@ __global__ void __launch_bounds__(kBlock, CB2_H_MINBLOCKS) k_update_h(const Step
 // E over the general blocks (no Debye poles)
 __global__ void __launch_bounds__(kBlock, CB2_E_MINBLOCKS)
     k_update_e(const StepArgs a, const int2 *work, const RunArgs r, const SibcArgs s) {
-    chain_next();
+    if (r.chain) chain_next();
     if ((int)blockIdx.x < r.first) {   // H samples, then the surface-impedance edges (their E is left alone below)
         const int e = ((int)blockIdx.x - r.blocks) * kBlock + (int)threadIdx.x;
         if (e < 0) sample_h(a, r, (int)blockIdx.x, r.blocks, Chained{});
@@ -1440,7 +1440,7 @@ __device__ __forceinline__ int whole_place(const StepArgs &a, const Whole &l, in
 // 104.0 with the tables after it).
 constexpr int kWholeH = 9, kWholeE = 7, kWholeELarge = 8, kLargePoles = 6;
 __global__ void __launch_bounds__(kBlock, kWholeH) k_whole_h(const StepArgs a, const Whole l, const RunArgs r) {
-    chain_next();
+    if (r.chain) chain_next();
     if ((int)blockIdx.x < r.first) {
         begin_step(a, r, (int)blockIdx.x, r.blocks, Chained{});
         return;
@@ -1462,7 +1462,7 @@ __global__ void __launch_bounds__(kBlock, kWholeH) k_whole_h(const StepArgs a, c
 template <int P, int B>
 __global__ void __launch_bounds__(kBlock, P > 8 ? 4 : B)
     k_whole_e(const StepArgs a, const Whole l, const RunArgs r, const SibcArgs s) {
-    chain_next();
+    if (r.chain) chain_next();
     if ((int)blockIdx.x < r.first) {   // H samples, then the surface-impedance edges (their E is left alone below)
         const int e = ((int)blockIdx.x - r.blocks) * kBlock + (int)threadIdx.x;
         if (e < 0) sample_h(a, r, (int)blockIdx.x, r.blocks, Chained{});
@@ -2116,10 +2116,10 @@ struct Device {
     // runs of kGraphSteps whole steps replay one captured graph (CEM_B200_GRAPHS=0: never)
     bool use_graphs = true;
     // launch shape, chosen by the tuner per grid shape (defaults otherwise):
-    // k segments thinner than `thin` points join a neighbour; general blocks on
+    // k segments thinner than `thin_k` points join a neighbour; general blocks on
     // the second stream beside the others (`side_on`) or after them on the main
     // one; `graph_steps` steps per replayed graph
-    int thin = 16;
+    int thin_k = 16;
     bool side_on = true;
     int graph_steps = 32;
     // the z CPML slabs run inside the lean kernels' rows (z tails) or as general blocks;
@@ -2140,6 +2140,7 @@ struct Device {
     int run_steps = 0;                // most steps of a run (sample rows)
     bool sibc_flagged = false;        // the tables mark the surface-impedance edges
     bool large = false;   // from 2 M cells
+    bool thin = false;    // thousands of node planes, each within a block per component
     bool whole_h = true, whole_e = true;   // an update's blocks in one launch (Whole), or a kernel per class
     bool split_e = false;   // of whole_e: the lean rectangles in a launch of their own
     bool chained = false;   // the last launch on the main stream is one of a run, nothing else since
@@ -2878,7 +2879,7 @@ bool build_spaces(cem_sim *s, Device &D, int u) {
         for (const int *bx : boxes) deb = deb || (ke > bx[2] && ks < bx[2] + bx[5]);
         if (zs && !tails) return 2;
         return deb ? 1 : 0;
-    }, D.thin);
+    }, D.thin_k);
     if (tails && D.ztail_split) {   // the slabs' groups as segments of their own, after the thin merges
         for (int q = 0; q < 4; q += 2)
             if (D.zt[u][q + 1] > D.zt[u][q]) { kcut(D.zt[u][q]); kcut(D.zt[u][q + 1]); }
@@ -2972,16 +2973,20 @@ bool build_spaces(cem_sim *s, Device &D, int u) {
 // cells (closed boxes with copper of 1.0e5, 1.05e6 and 1.8e6 cells: 5.0, 21.6 and 36.0 as
 // k_whole_*, 5.4, 20.7 and 34.3 as a kernel per class). They have a column of blocks
 // more that samples, so planes of fewer than four blocks stay with k_whole_* (2000
-// x 20 x 20 cells: 16.7 and 18.8).
+// x 20 x 20 cells: 16.7 and 18.8), but for thousands of planes, where short blocks
+// count and launches don't chain: 20000 x 3 x 3, 8000 x 5 x 40 and 4000 x 8 x 8 cells 126, 52.7
+// and 27.0 us as chained k_whole_*, 90.7, 47.5 and 23.2 not chained, 86.0, 41.5 and 20.6 as a
+// kernel per class (with CPML at the x ends 69.7, 36.2 and 18.5).
 bool build_launches(cem_sim *s, Device &D) {
     if (!build_spaces(s, D, 0) || !build_spaces(s, D, 1)) return false;
+    D.thin = s->n[0] >= 3000 && space_blocks(D.sp[0][kAll]) == 1 && space_blocks(D.sp[1][kAll]) == 1;
     auto lean = [&](int u) {
         return !D.wl_start[u].back() && !space_blocks(D.sp[u][kDebye]) && space_blocks(D.sp[u][kFast]) >= 4;
     };
     const bool all_lean = lean(0) && lean(1) && !s->nsb && !s->npole;
     const bool apart = all_lean || (long long)s->n[0] * s->n[1] * s->n[2] >= 1000000;
-    D.whole_h = !D.large && !(apart && lean(0));
-    D.whole_e = s->npole > 0 || (!D.large && !(apart && lean(1)));
+    D.whole_h = !D.large && !D.thin && !(apart && lean(0));
+    D.whole_e = s->npole > 0 || (!D.large && !D.thin && !(apart && lean(1)));
     return true;
 }
 
@@ -3667,6 +3672,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
     if (!run || !D.sibc_flagged) sb.ns = 0;
     RunArgs none = D.run, carry = D.run;   // a launch with nothing of the run's, and the phase's one with it
     none.first = carry.first = none.blocks = carry.blocks = 0;
+    none.chain = carry.chain = run && !D.thin;
     none.skip = carry.skip = sb.ns ? kFlagSibc : 0u;
     auto sample_blocks = [&](int u) { return std::max(1, (D.run.nsample[u] + kBlock - 1) / kBlock); };
     // general work-list entries of update u for node planes [a, b)
@@ -3695,7 +3701,7 @@ bool launch_step(cem_sim *s, int phase_mask, int i0, int i1, bool run = false) {
         at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at.val.programmaticStreamSerializationAllowed = 1;
         c.attrs = &at;
-        c.numAttrs = run && D.chained ? 1 : 0;
+        c.numAttrs = none.chain && D.chained ? 1 : 0;
         cudaLaunchKernelEx(&c, kernel, args...);
         D.launches++;
         D.chained = run;
@@ -4039,9 +4045,9 @@ void store_shape(const std::string &key, const std::array<double, 5> &v) {   // 
 }
 
 bool apply_shape(cem_sim *s, Device &D, int thin, bool side, int graph, bool ztail) {
-    const bool respace = thin != D.thin || ztail != D.ztail;
+    const bool respace = thin != D.thin_k || ztail != D.ztail;
     if (respace) {
-        D.thin = thin;
+        D.thin_k = thin;
         D.ztail = ztail;
         if (!build_launches(s, D)) return false;
         fill_args(s, D);
@@ -4089,7 +4095,7 @@ bool tune_shape(cem_sim *s, long *used) {
         const bool zt = it->second[4] < 0 ? D.ztail : it->second[4] != 0;
         return apply_shape(s, D, (int)it->second[0], it->second[1] != 0, (int)it->second[2], zt);
     }
-    int thin = D.thin, graph = D.graph_steps;
+    int thin = D.thin_k, graph = D.graph_steps;
     bool side = D.side_on, zt = D.ztail;
     double best;
     if (!shape_ms(s, 32, 64, &best, used)) return false;
@@ -4432,7 +4438,7 @@ int cemx_tune_state(const cem_sim *s, double *out, int n) {
         const Device &D = *s->dev;
         v[0] = D.tuned;
         v[1] = D.tuned_from_cache;
-        v[2] = D.thin;
+        v[2] = D.thin_k;
         v[3] = D.side_on;
         v[4] = D.graph_steps;
         v[5] = D.tuned_ms;

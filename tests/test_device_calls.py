@@ -346,3 +346,15 @@ def test_launches_per_step_are_what_is_launched(fake, name):
     s.step(5)   # and the run's begin and its sample rows
     assert fake.count("launch") - before == 5 * s.sizes()["launches_per_step"] + 2
     s.destroy()
+
+
+@pytest.mark.parametrize("n,lean", [((3000, 6, 6), True), ((2999, 6, 6), False), ((3000, 60, 40), True), ((3000, 24, 20), False)])
+def test_thousands_of_short_planes_run_in_the_lean_kernels(fake, n, lean):
+    """One block of a few threads per plane and component, thousands of times (and not with planes of more than one block,
+    unless they are four)."""
+    fake.current = 0
+    s = closed_box(fake.lib, n)
+    before = fake.count("k_whole_h"), fake.count("k_update_h_fast")
+    s.step(3)
+    assert (fake.count("k_whole_h") - before[0], fake.count("k_update_h_fast") - before[1]) == ((0, 3) if lean else (3, 0))
+    s.destroy()

@@ -103,3 +103,26 @@ def test_many_probes_cost_a_step_little(lib):
         t.append(min(s.stepTimed(320) for _ in range(5)))
         s.destroy()
     assert t[1] < 2 * t[0]
+
+
+@pytest.mark.parametrize("faces", [(), (0, 1), (0, 1, 5)], ids=["closed", "x", "x and z"])
+def test_thousands_of_short_planes_give_the_bits_of_the_phases(lib, faces):
+    def make():
+        s = lib.createSim(*(1e-4 * np.arange(q + 1) for q in (3001, 7, 9)))
+        for f in faces:
+            s.setBoundary(f, 1, 4 if f < 2 else 2)
+        p = s.addLumpedPort(2, 1500, 3, 0, 4, 1, 50.0)
+        s.setGaussian(p, 1.0, 8e-12, 3e-12)
+        s.setFrequencies([5e9])
+        for q in range(60):
+            s.addVProbe(0, 3, 4, 1400 + q, 1480 + q, 1)
+        s.addIProbe(0, 1520, 1, 5, 1, 6)
+        s.finalize(0.9)
+        return s
+
+    a, b = make(), make()
+    for n in (64, 1, 7):
+        a.step(n)
+    phases(b, 72)
+    assert np.array_equal(a.checkpoint(), b.checkpoint())
+    assert np.abs(a.portV(0)).max() > 0
